@@ -272,6 +272,7 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
     }
     if (s->bp.enabled) b.max_bil_radius = std::max(b.max_bil_radius, s->btab.radius);
     b.max_rb_tiles = std::max(b.max_rb_tiles, std::max(1, s->rb_tx * s->rb_ty));
+    if (s->vol.grid) b.max_grid = std::max(b.max_grid, s->vol.grid_cap);
     b.kahan_mask |= s->icp_params().kahan ? 2 : 1;
     b.fp16_mask |= s->vol.fp16 ? 2 : 1;
   }
@@ -588,12 +589,16 @@ size_t session_bytes(const dyn_tsdf_params& t, const dyn_sensor& s, int precisio
   b += sizeof(Entry) * (size_t)t.num_buckets * t.bucket_size;
   b += sizeof(unsigned long long) * (size_t)t.num_blocks;
   if (precision != DYN_PRECISION_FP32)
-    b += (4 + (colour ? 4 : 0)) * (size_t)t.num_blocks * kBlockVox;
+    b += (4 + (colour ? 4 : 0)) * ((size_t)t.num_blocks + 1) * kBlockVox;
   else
-    b += sizeof(dyn_voxel) * (size_t)t.num_blocks * kBlockVox;
+    b += sizeof(dyn_voxel) * ((size_t)t.num_blocks + 1) * kBlockVox;
   b += sizeof(int2) * (size_t)t.num_blocks;  // visible list
   if (precision == DYN_PRECISION_MIXED)
     b += (sizeof(int) + 1) * (size_t)t.num_blocks;  // free-space summaries
+  {
+    const DSensor ds = dsensor(s);
+    b += sizeof(unsigned) * (size_t)grid_entries(ds, dtsdf(t, precision));  // raycast block grid
+  }
   b += n * (2 + 3 + 4 + 4 + 4 + 3);  // inputs, raw, filtered, ray depth, target rgb
   {  // ray depth bounds and the free-space tile map
     const int tx = ((int)s.cols + 7) / 8, ty = ((int)s.rows + 7) / 8;
@@ -697,7 +702,8 @@ dyn_status alloc_device_buffers(dyn_session* s) {
   s->vol.free_ok = (double)s->vol.sat_lo >= (double)tsdf->voxel_size ? 1 : 0;
   DYN_TRY(s->dalloc(&s->vol.entries, sizeof(Entry) * (size_t)tsdf->num_buckets * tsdf->bucket_size));
   DYN_TRY(s->dalloc(&s->vol.block_keys, sizeof(unsigned long long) * (size_t)tsdf->num_blocks));
-  const size_t nvox = (size_t)tsdf->num_blocks * kBlockVox;
+  // one block more than the heap, never written: what a missing block reads as
+  const size_t nvox = ((size_t)tsdf->num_blocks + 1) * kBlockVox;
   s->vol.voxels = nullptr;
   s->vol.vox16 = nullptr;
   s->vol.colors = nullptr;
@@ -715,6 +721,10 @@ dyn_status alloc_device_buffers(dyn_session* s) {
     DYN_TRY(s->dalloc(&s->vol.freecell, (size_t)tsdf->num_blocks));
   }
   DYN_TRY(s->dalloc(&s->vol.cnt, sizeof(Counters)));
+  s->vol.grid = nullptr;
+  s->vol.grid_cap = (int)grid_entries(s->ls[0], s->vol.t);
+  DYN_TRY(s->dalloc(&s->vol.gbox, sizeof(GridBox)));
+  if (s->vol.grid_cap > 0) DYN_TRY(s->dalloc(&s->vol.grid, sizeof(unsigned) * (size_t)s->vol.grid_cap));
   DYN_TRY(s->dalloc(&s->d_gvis, sizeof(int2) * (size_t)tsdf->num_blocks));
   s->rb_tx = ((int)s->sensor.cols + 7) / 8;
   s->rb_ty = ((int)s->sensor.rows + 7) / 8;
@@ -745,6 +755,12 @@ size_t session_device_bytes(const dyn_tsdf_params* tsdf, const dyn_gn_params* gn
   const size_t b = s->measured;
   delete s;
   return b;
+}
+
+// Whether the session's block grid covers the rays of sensor 'virt'.
+static bool raycast_grid_fits(const dyn_session* s, const dyn_sensor& virt) {
+  const long long n = grid_entries(dsensor(virt), s->vol.t);
+  return s->vol.grid && n > 0 && n <= s->vol.grid_cap;
 }
 
 dyn_status ensure_staging(dyn_session* s) {
@@ -1059,7 +1075,7 @@ dyn_status dyn_raycast(dyn_session* s, const float pose[16], const dyn_sensor* v
   DYN_CUDA(cudaMemcpyAsync(s->d_pose_override, pose, 64, cudaMemcpyHostToDevice, s->stream));
   size_t n = (size_t)vs.rows * vs.cols;
   launch_raycast(s->vol, dsensor(vs), s->d_pose, s->d_pose_override, s->d_ray,
-                 rgb_host ? s->d_trgb : nullptr, s->stream);
+                 rgb_host ? s->d_trgb : nullptr, raycast_grid_fits(s, vs), s->stream);
   DYN_CUDA(cudaGetLastError());
   DYN_CUDA(cudaMemcpyAsync(depth_host, s->d_ray, n * 4, cudaMemcpyDeviceToHost, s->stream));
   if (rgb_host)
@@ -1080,7 +1096,7 @@ dyn_status dyn_raycast_maps(dyn_session* s, const float pose[16], const dyn_sens
   DYN_CUDA(cudaMemcpyAsync(s->d_pose_override, pose, 64, cudaMemcpyHostToDevice, st));
   const size_t n = (size_t)vs.rows * vs.cols;
   launch_raycast(s->vol, dsensor(vs), s->d_pose, s->d_pose_override, s->d_ray,
-                 rgb_host ? s->d_trgb : nullptr, st);
+                 rgb_host ? s->d_trgb : nullptr, raycast_grid_fits(s, vs), st);
   // misses (at max_sensor_depth or beyond) become invalid depth, then the
   // maps of that depth in the raycast camera's frame
   launch_target_prepare(s->d_ray, s->d_filt, s->tp.max_sensor_depth, nullptr, nullptr, (int)n,

@@ -18,12 +18,82 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "sessdev.cuh"
 
 namespace dyn {
 
 namespace {
 
+// ------------------------------------------------------------ the block grid
+// The raycast looks blocks up by their coordinates far more often than
+// anything else (every sample, up to eight blocks), so each frame's blocks are
+// also laid out in a dense grid over the box the frame's rays can reach
+// (GridBox; z fastest): entry = first voxel of the block (512 x heap index),
+// or of the empty block after the heap.  A lookup is one multiply-add chain
+// and one load without branches, where the hash takes a bucket scan in a
+// divergent branch for every lane that changes block: with the exact march
+// below and hash lookups a 640x480 FP32 target took 257 M warp instructions at
+// 20 of 32 lanes (485 us, as before it); with the grid 138 M at 28 lanes
+// (260 us; 320x240 225 -> 98 us).  The mixed march, whose arithmetic did not
+// change: 640x480 136 -> 61 us, 1280x720 band 200 -> 100 us, and a 32-session
+// band batch 667 -> 351 us.
+__device__ inline GridBox grid_box(const float* __restrict__ T, const DSensor& s, const DTsdf& t,
+                                   int cap) {
+  GridBox b;
+  float lo[3], hi[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) lo[a] = hi[a] = T[4 * a + 3];
+  const float u0 = (0.0f - s.cx) / s.fx, u1 = ((float)(s.cols - 1) - s.cx) / s.fx;
+  const float v0 = (0.0f - s.cy) / s.fy, v1 = ((float)(s.rows - 1) - s.cy) / s.fy;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float e = (T[4 * a] * ((k & 1) ? u1 : u0) + T[4 * a + 1] * ((k & 2) ? v1 : v0) +
+                       T[4 * a + 2]) * t.dmax + T[4 * a + 3];
+      lo[a] = fminf(lo[a], e);
+      hi[a] = fmaxf(hi[a], e);
+    }
+  int n[3], o[3];
+  bool ok = cap > 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    // a block of margin below, two above (a cell's high corners); 2^20 blocks
+    // is the key's range
+    const float l = floorf(lo[a] / t.bsm) - 1.0f, h = floorf(hi[a] / t.bsm) + 2.0f;
+    ok = ok && l > -1048576.0f && h < 1048576.0f;
+    o[a] = ok ? (int)l : 0;
+    n[a] = ok ? (int)h - (int)l + 1 : 0;
+  }
+  ok = ok && (double)n[0] * (double)n[1] * (double)n[2] <= (double)cap;
+  b.x0 = o[0];
+  b.y0 = o[1];
+  b.z0 = o[2];
+  b.nx = n[0];
+  b.ny = n[1];
+  b.nz = n[2];
+  b.ok = ok ? 1 : 0;
+  return b;
+}
+// The grid emptied at pose T by 'threads' threads, this one number 'thread'.
+__device__ inline void grid_clear(const VolumeDev& v, const float* __restrict__ T,
+                                  const DSensor& s, int thread, int threads) {
+  const GridBox b = grid_box(T, s, v.t, v.grid_cap);
+  if (thread == 0) *v.gbox = b;
+  if (!b.ok) return;
+  const int n4 = (b.nx * b.ny * b.nz + 3) / 4;  // (the buffer holds whole vectors)
+  const unsigned e = (unsigned)v.t.num_blocks * (unsigned)kBlockVox;
+  for (int i = thread; i < n4; i += threads)
+    reinterpret_cast<uint4*>(v.grid)[i] = make_uint4(e, e, e, e);
+}
+__device__ inline void grid_put(const VolumeDev& v, const GridBox& b, unsigned long long key,
+                                int ptr, unsigned flag) {
+  const int x = key_x(key) - b.x0, y = key_y(key) - b.y0, z = key_z(key) - b.z0;
+  if ((unsigned)x < (unsigned)b.nx && (unsigned)y < (unsigned)b.ny && (unsigned)z < (unsigned)b.nz)
+    v.grid[(x * b.ny + y) * b.nz + z] = ((unsigned)ptr * (unsigned)kBlockVox) | flag;
+}
 // ------------------------------------------------------------ allocation
 constexpr int kAllocT = 16;          // 16x16 pixel tile per CTA
 constexpr int kSetSlots = 2048;      // CTA-local dedup set (16 KB)
@@ -200,10 +270,20 @@ __device__ inline void allocate_tile(const float* __restrict__ depth, const DSen
 
 // (8 CTAs per SM -- at most 32 registers, 24.7 KB of shared memory each --
 // so that a 640x480 frame's 1,200 tiles run in one wave instead of 1.35)
+// The tiles' rows of CTAs are followed by rows that empty the raycast's grid at
+// the frame's pose (memory-bound work beside the rays' latency-bound one).
 __global__ void __launch_bounds__(kAllocT* kAllocT, 8)
-    fused_allocate_kernel(const SessDev* __restrict__ tab) {
+    fused_allocate_kernel(const SessDev* __restrict__ tab, int tile_rows) {
   const SessDev& S = tab[blockIdx.z];
   const DSensor& s = S.ls[0];
+  if ((int)blockIdx.y >= tile_rows) {
+    if (S.vol.grid && S.mode == 1)
+      grid_clear(S.vol, S.pose->posef, s,
+                 (((int)blockIdx.y - tile_rows) * (int)gridDim.x + (int)blockIdx.x) * kAllocT * kAllocT +
+                     (int)threadIdx.y * kAllocT + (int)threadIdx.x,
+                 ((int)gridDim.y - tile_rows) * (int)gridDim.x * kAllocT * kAllocT);
+    return;
+  }
   if ((int)blockIdx.x * kAllocT >= s.cols || (int)blockIdx.y * kAllocT >= s.rows) return;
   allocate_tile(S.raw, s, S.vol, S.pose, blockIdx.x, blockIdx.y);
 }
@@ -402,6 +482,20 @@ __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, 
   return dm * (1.0f + 1e-5f) + 1e-5f < __uint_as_float(mn);
 }
 
+// one volume's grid at a caller's pose: emptied, then its blocks entered
+__global__ void grid_clear_kernel(const __grid_constant__ VolumeDev v,
+                                  const __grid_constant__ DSensor s,
+                                  const float* __restrict__ pose16) {
+  grid_clear(v, pose16, s, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+__global__ void grid_fill_kernel(const __grid_constant__ VolumeDev v) {
+  const GridBox b = *v.gbox;
+  if (!b.ok) return;
+  const int n = min(v.cnt->nalloc, v.t.num_blocks);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    grid_put(v, b, v.block_keys[i], i, v.freecell && v.freecell[i] ? 1u : 0u);
+}
+
 // Every session's visible blocks appended to one batch-wide list of
 // (session, heap index), so integration balances across sessions; the
 // session index carries kVisFree for free-space blocks.
@@ -415,11 +509,14 @@ __global__ void fused_visible_kernel(const SessDev* __restrict__ tab, int2* __re
   int n = v.cnt->nalloc;
   if (n > v.t.num_blocks) n = v.t.num_blocks;
   const int lane = threadIdx.x & 31;
+  // (mixed carving sessions enter their blocks after the free-cell pass)
+  const bool put = v.grid && S.mode == 1 && !v.nonsat && v.gbox->ok;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     int i = base + threadIdx.x;
     bool vis = false;
     if (i < n) {
       const unsigned long long key = v.block_keys[i];
+      if (put) grid_put(v, *v.gbox, key, i, 0u);
       vis = block_visible(key, v.t, S.ls[0], invT);
       // every allocated block (visible or not) enters the ray-start bound
       if (S.rbound) bound_block(key, v.t, S.ls[0], invT, S.rbound, S.rb_tx, S.rb_ty, v.t.band, true);
@@ -448,18 +545,25 @@ __global__ void fused_visible_kernel(const SessDev* __restrict__ tab, int2* __re
 // march (free_ok) -- as the free-cell shortcut does; so the near bound of a
 // tile is the nearest depth of the boxes of the blocks that hold such
 // voxels (VolumeDev::nonsat > 0), widened as bound_block widens every box.
+// Every block also enters the raycast's grid here, with its free-cell flag.
 __global__ void fused_surface_bound_kernel(const SessDev* __restrict__ tab) {
   const SessDev& S = tab[blockIdx.z];
   const VolumeDev& v = S.vol;
-  if (!S.rbound || !v.nonsat || !v.free_ok || v.t.band) return;
+  if (!v.nonsat) return;
+  const bool bound = S.rbound && v.free_ok && !v.t.band;
+  const bool put = v.grid && S.mode == 1 && v.gbox->ok;
   __shared__ M4f invT;
   if (threadIdx.x < 16) invT.m[threadIdx.x] = S.pose->invf[threadIdx.x];
   __syncthreads();
   int n = v.cnt->nalloc;
   if (n > v.t.num_blocks) n = v.t.num_blocks;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (v.nonsat[i] > 0)
-      bound_block(v.block_keys[i], v.t, S.ls[0], invT, S.rbound, S.rb_tx, S.rb_ty, true, false);
+    {
+      const unsigned long long key = v.block_keys[i];
+      if (put) grid_put(v, *v.gbox, key, i, v.freecell[i] ? 1u : 0u);
+      if (bound && v.nonsat[i] > 0)
+        bound_block(key, v.t, S.ls[0], invT, S.rbound, S.rb_tx, S.rb_ty, true, false);
+    }
 }
 
 // ------------------------------------------------------------ integration
@@ -891,9 +995,6 @@ __device__ inline VoxelSample get_interpolated(const VolumeDev& v, F3 position, 
   return out;
 }
 
-constexpr int kRayTX = 16, kRayTY = 16;
-
-
 // tsdfVolume raycast (tsdf.cu:471-526) of pixel (x, y) from camera pose T:
 // march from 0 by the interpolated sdf (a truncation where unobserved) until
 // the sdf drops under a voxel or the depth passes max_sensor_depth; then the
@@ -901,7 +1002,7 @@ constexpr int kRayTX = 16, kRayTY = 16;
 // skip_to or after skip_far (the tile's ray depth bounds: no allocated block
 // there) step by the truncation without a lookup -- what the lookup would
 // have returned.  Returns true when the march hit the step cap.
-__device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
+__device__ __noinline__ bool raycast_exact_hash_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
                                         int y, float skip_to, float skip_far,
                                         float* __restrict__ depth_out,
                                         uint8_t* __restrict__ rgb_out) {
@@ -950,6 +1051,318 @@ __device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, co
   return over;
 }
 
+// ---- the exact march over the block grid
+// A sample of the reference's march needs the voxel its point lies in and the
+// low corner of its trilinear cell, each the truncation of an IEEE quotient
+// plus or minus a half (voxel_index), and the weights p * (1/vs) - floor.  All
+// of them follow from e = p / vs: the voxel is e rounded to nearest, the low
+// corner floor(e), the high corner floor(e) + 1.  The march takes both from
+// vp = fl(p * fl(1/vs)), which the weights need anyway, rounded by adding and
+// subtracting 1.5 * 2^23 (two additions and no conversion: the sum's low bits
+// are the integer).  With u = 2^-24 the roundings of vp (2u|e|) and of the
+// reference's corner, quotient and half additions (4u|e| + 3u at most, the
+// high corner's) move a value across a rounding boundary only within
+// 6u|e| + 3u of it, so where every axis is farther than 8u(max|vp| + 2) from
+// every multiple of one half the indices are the reference's; else
+// (exact_axis) they are computed with its own expressions.
+//
+// (x - cx) * z / fx by the hoisted reciprocal: yh = fl(1/b), yl the rest of
+// 1/b; q = fl(a * yh + fl(a * yl)) is within an ulp of a / b, and
+// fma(fma(-b, q, a), yh, q) is then the correctly rounded quotient (Markstein,
+// IBM J. Res. Dev. 34, 1990) unless a step under- or overflows, which the
+// ranges of march_setup exclude.  A zero dividend gives zero (of either sign:
+// the sign reaches only sums with the pose's translation, and a zero's sign
+// changes no index, weight or depth).
+constexpr float kRint = 12582912.0f;   // 1.5 * 2^23
+constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
+
+// v rounded to the nearest integer (|v| < 2^22): its integer biased by
+// kRintBits, the integer of floor(v) likewise, and v - round(v).
+struct Rounded {
+  int near, low;
+  float diff;
+};
+__device__ inline Rounded round_near(float v) {
+  Rounded r;
+  const float t = v + kRint;
+  r.near = __float_as_int(t);
+  r.diff = v - (t - kRint);
+  r.low = r.near - (r.diff < 0.0f ? 1 : 0);  // (not for -0)
+  return r;
+}
+__device__ inline float biased_float(int i) { return __int_as_float(i) - kRint; }
+
+// The block grid of the march (GridBox): entry of the block that holds voxel
+// (x, y, z), biased as round_near gives them.
+struct GridView {
+  const unsigned* __restrict__ e;
+  unsigned sx, sy, off;
+};
+__device__ inline GridView grid_view(const VolumeDev& v) {
+  const GridBox& b = *v.gbox;
+  GridView g;
+  g.e = v.grid;
+  g.sy = (unsigned)b.nz;
+  g.sx = (unsigned)b.ny * g.sy;
+  constexpr unsigned bias = (unsigned)kRintBits >> 3;
+  g.off = ((unsigned)b.x0 + bias) * g.sx + ((unsigned)b.y0 + bias) * g.sy + (unsigned)b.z0 + bias;
+  return g;
+}
+__device__ inline unsigned grid_index(const GridView& g, int x, int y, int z) {
+  return (unsigned)(x >> 3) * g.sx + (unsigned)(y >> 3) * g.sy + (unsigned)(z >> 3) - g.off;
+}
+
+// Voxel indices of the eight corners of the cell whose low corner is (x, y, z)
+// (biased), in the reference's order: g the grid index of the low corner's
+// block, e0 that block's first voxel; the other blocks are read only where the
+// cell crosses a block boundary.  FLAG: entries carry the free-cell flag in
+// bit 0.
+template <bool FLAG>
+__device__ inline void cell_corners(const GridView& G, unsigned g, unsigned e0, int x, int y,
+                                    int z, unsigned (&i)[8]) {
+  const bool kx = (x & 7) == 7, ky = (y & 7) == 7, kz = (z & 7) == 7;
+  unsigned b[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) b[k] = e0;
+  if (kx | ky | kz) {
+    const unsigned mx = kx ? G.sx : 0u, my = ky ? G.sy : 0u, mz = kz ? 1u : 0u;
+    const unsigned gx = g + mx, gy = g + my, gxy = gx + my;
+    b[1] = __ldg(G.e + gx);
+    b[2] = __ldg(G.e + gy);
+    b[3] = __ldg(G.e + (g + mz));
+    b[4] = __ldg(G.e + gxy);
+    b[5] = __ldg(G.e + (gy + mz));
+    b[6] = __ldg(G.e + (gx + mz));
+    b[7] = __ldg(G.e + (gxy + mz));
+  }
+  const unsigned xl = (unsigned)(x & 7) << 6, yl = (unsigned)(y & 7) << 3, zl = (unsigned)(z & 7);
+  const unsigned xh = kx ? 0u : xl + 64u, yh = ky ? 0u : yl + 8u, zh = kz ? 0u : zl + 1u;
+  if (FLAG) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) b[k] &= ~1u;
+  }
+  i[0] = b[0] + (xl + yl) + zl;
+  i[1] = b[1] + (xh + yl) + zl;
+  i[2] = b[2] + (xl + yh) + zl;
+  i[3] = b[3] + (xl + yl) + zh;
+  i[4] = b[4] + (xh + yh) + zl;
+  i[5] = b[5] + (xl + yh) + zh;
+  i[6] = b[6] + (xh + yl) + zh;
+  i[7] = b[7] + (xh + yh) + zh;
+}
+
+struct MarchRay {
+  float yhx, ylx, yhy, yly;  // reciprocals of fx and fy
+};
+
+__device__ inline bool recip_ok(float x) {
+  return fabsf(x) >= 9.5367431640625e-7f && fabsf(x) <= 1048576.0f;  // 2^-20 .. 2^20
+}
+
+// The largest |coordinate| in voxels of the samples of pixel offset (px, py)
+// (per unit depth) from pose T, up to dmax; NaN for a pose that is not finite.
+__device__ inline float march_extent(const DTsdf& t, const M4f& T, float px, float py,
+                                     float inv_vs) {
+  float far = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float e = (fabsf(T.m[4 * i]) * fabsf(px) + fabsf(T.m[4 * i + 1]) * fabsf(py) +
+                     fabsf(T.m[4 * i + 2])) * t.dmax + fabsf(T.m[4 * i + 3]);
+    far = e > far ? e : (e <= far ? far : e);  // NaN passes on
+  }
+  return far * inv_vs * 1.001f + 2.0f;
+}
+
+// Every step of a march is at least min(voxel, truncation): below 4096 of them
+// up to dmax the roundings of cur add up to less than a step, so the march
+// ends within the step cap (rc_cap, four steps more) and needs no count.
+__device__ inline bool march_bounded(const DTsdf& t) {
+  return t.dmax <= 4096.0f * fminf(t.vs, t.trunc);
+}
+
+// Whether the fast indices and divisions hold along the whole ray of pixel
+// offset (ax, ay) from pose T, with their constants.
+__device__ inline bool march_setup(const DTsdf& t, const DSensor& s, const M4f& T, float ax,
+                                   float ay, float inv_vs, MarchRay& m) {
+  const bool ok = recip_ok(s.fx) && recip_ok(s.fy) && (ax == 0.0f || recip_ok(ax)) &&
+                  (ay == 0.0f || recip_ok(ay)) && recip_ok(t.vs) && recip_ok(t.trunc) &&
+                  recip_ok(t.dmax) && march_bounded(t);
+  m.yhx = 1.0f / s.fx;
+  m.yhy = 1.0f / s.fy;
+  m.ylx = __fmaf_rn(-s.fx, m.yhx, 1.0f) * m.yhx;
+  m.yly = __fmaf_rn(-s.fy, m.yhy, 1.0f) * m.yhy;
+  const float far = march_extent(t, T, ax * m.yhx, ay * m.yhy, inv_vs);
+  return ok && far < 131072.0f;
+}
+
+// The depths of a march: samples below the near distance, then steps without a
+// lookup up to the tile's near bound (no allocated block there, so each sample
+// would step by the truncation), samples up to the far bound, and steps
+// without a lookup to the end.  Depths only grow, so one comparison per sample
+// tells whether its range is left.  The sum is taken step by step, as the
+// samples would take it.
+struct MarchRange {
+  float skip_to, last;  // last: the first depth past the far bound or the end
+  float lim;
+  bool near;
+  __device__ MarchRange(float znear, float skip_to_, float skip_far, float dmax)
+      : skip_to(fminf(skip_to_, dmax)), near(true) {
+    // the least float above skip_far (>= 0)
+    last = skip_far < dmax ? fminf(__int_as_float(__float_as_int(skip_far) + 1), dmax) : dmax;
+    lim = fminf(znear, dmax);
+  }
+  // whether a sample is taken at 'cur'; moves it past depths without one
+  __device__ bool sample(float& cur, float trunc, float dmax) {
+    if (cur < lim) return true;
+    if (near) {
+      near = false;
+      while (cur < skip_to) cur += trunc;
+      lim = last;
+      if (cur < lim) return true;
+    }
+    while (cur < dmax) cur += trunc;
+    return false;
+  }
+};
+
+__device__ inline float div_by(float a, float b, float yh, float yl) {
+  const float q = __fmaf_rn(a, yh, __fmul_rn(a, yl));
+  return __fmaf_rn(__fmaf_rn(-b, q, a), yh, q);
+}
+
+// One axis by the reference's expressions: (low corner, voxel - low corner),
+// or a second value of 2 where the high corner is not low + 1 or the voxel is
+// neither.  (Quotients too small for div_by's exactness are lost in the half.)
+__device__ __noinline__ int2 exact_axis(float p, float vs, float inv_vs) {
+  const float yl = __fmaf_rn(-vs, inv_vs, 1.0f) * inv_vs;
+  auto index = [&](float q) {
+    const float sg = (float)((q > 0.0f) - (q < 0.0f));
+    return (int)(div_by(q, vs, inv_vs, yl) + sg * 0.5f);
+  };
+  const float pd = p - vs / 2.0f;
+  const int g = index(p), g0 = index(pd + 0.0f), g1 = index(pd + vs);
+  return make_int2(g0, (g1 - g0 == 1 && (g == g0 || g == g1)) ? g - g0 : 2);
+}
+
+// get_interpolated without colour, out of line (rare in the march).
+__device__ __noinline__ float2 interpolated_generic(const VolumeDev& v, float x, float y, float z,
+                                                    float inv_vs) {
+  BlockCache bc;
+  bc.x = bc.y = bc.z = 0x7fffffff;
+  bc.ptr = -1;
+  const VoxelSample s = get_interpolated<false>(v, f3(x, y, z), inv_vs, bc);
+  return make_float2(s.sdf, s.w ? 1.0f : 0.0f);
+}
+
+// The march of raycast_exact_hash_px, its blocks looked up in the grid: every
+// sample reads the entry of its voxel's block, an observed one those of its
+// cell's blocks.  Rays outside march_setup's ranges, and volumes without a
+// grid, take raycast_exact_hash_px.
+__device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
+                                        int y, float skip_to, float skip_far,
+                                        float* __restrict__ depth_out,
+                                        uint8_t* __restrict__ rgb_out) {
+  const DTsdf& t = v.t;
+  const float inv_vs = 1.0f / t.vs;
+  // getPoint3d (utils.h:104-112) with the pixel's (u - cx), (v - cy) hoisted
+  const float ax = (float)x - s.cx, ay = (float)y - s.cy;
+  MarchRay R;
+  if (!v.grid || !v.gbox->ok || !march_setup(t, s, T, ax, ay, inv_vs, R))
+    return raycast_exact_hash_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  const GridView G = grid_view(v);
+  const uint2* __restrict__ vox = reinterpret_cast<const uint2*>(v.voxels);
+  const float fx = s.fx, fy = s.fy, dmax = t.dmax, trunc = t.trunc, vs = t.vs;
+  const unsigned empty = (unsigned)t.num_blocks * (unsigned)kBlockVox;
+  float cur = 0.0f;
+  MarchRange range(ray_near(t), skip_to, skip_far, dmax);
+  while (range.sample(cur, trunc, dmax)) {
+    const F3 p = xform(T, f3(div_by(ax * cur, fx, R.yhx, R.ylx), div_by(ay * cur, fy, R.yhy, R.yly),
+                             cur));
+    const F3 vp = p * inv_vs;
+    const Rounded rx = round_near(vp.x), ry = round_near(vp.y), rz = round_near(vp.z);
+    // the weights, from the floors of vp whatever the indices
+    const float wx = vp.x - biased_float(rx.low), wy = vp.y - biased_float(ry.low),
+                wz = vp.z - biased_float(rz.low);
+    int lx = rx.low, ly = ry.low, lz = rz.low, ix = rx.near, iy = ry.near, iz = rz.near;
+    int odd = 0;
+    // margin: 1/4 - 8u(max|vp| + 2)
+    const float thr = __fmaf_rn(fmaxf(fmaxf(fabsf(vp.x), fabsf(vp.y)), fabsf(vp.z)),
+                                -4.76837158203125e-7f, 0.25f - 9.5367431640625e-7f);
+    if (!(fmaxf(fmaxf(fabsf(fabsf(rx.diff) - 0.25f), fabsf(fabsf(ry.diff) - 0.25f)),
+                fabsf(fabsf(rz.diff) - 0.25f)) < thr)) {
+      auto check = [&](float diff, float pos, int& l, int& i) {
+        if (!(fabsf(fabsf(diff) - 0.25f) < thr)) {
+          const int2 e = exact_axis(pos, vs, inv_vs);
+          l = e.x + kRintBits;
+          i = l + e.y;
+          odd |= e.y & 2;
+        }
+      };
+      check(rx.diff, p.x, lx, ix);
+      check(ry.diff, p.y, ly, iy);
+      check(rz.diff, p.z, lz, iz);
+    }
+    if (odd) {
+      const float2 g = interpolated_generic(v, p.x, p.y, p.z, inv_vs);
+      cur += g.y == 0.0f ? trunc : g.x;
+      if (g.y != 0.0f && g.x < vs) break;
+      continue;
+    }
+    // (both entries at once: one load's latency instead of two)
+    const unsigned g = grid_index(G, lx, ly, lz);
+    const unsigned own = __ldg(G.e + grid_index(G, ix, iy, iz)), e0 = __ldg(G.e + g);
+    if (own == empty) {  // no block: weight 0
+      cur += trunc;
+      continue;
+    }
+    // the voxel and the cell's corners together
+    unsigned c[8];
+    cell_corners<false>(G, g, e0, lx, ly, lz, c);
+    const uint2 v0 = __ldg(vox + (own + (unsigned)(((ix & 7) << 6) | ((iy & 7) << 3) | (iz & 7))));
+    uint2 r[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r[k] = __ldg(vox + c[k]);
+    if (v0.x < 0x01000000u) {  // weight 0
+      cur += trunc;
+      continue;
+    }
+    const float x0 = 1.0f - wx, y0 = 1.0f - wy, z0 = 1.0f - wz;
+    const float a00 = x0 * y0, a10 = wx * y0, a01 = x0 * wy, a11 = wx * wy;
+    const float coef[8] = {a00 * z0, a10 * z0, a01 * z0, a00 * wz,
+                           a11 * z0, a01 * wz, a10 * wz, a11 * wz};
+    // an unobserved corner takes the voxel's value
+    const unsigned least = min(min(min(r[0].x, r[1].x), min(r[2].x, r[3].x)),
+                               min(min(r[4].x, r[5].x), min(r[6].x, r[7].x)));
+    if (least < 0x01000000u) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) r[k].y = r[k].x < 0x01000000u ? v0.y : r[k].y;
+    }
+    float sdf = coef[0] * vsdf(r[0]);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) sdf += coef[k] * vsdf(r[k]);
+    cur += sdf;
+    if (sdf < vs) break;
+  }
+  const int i = y * s.cols + x;
+  depth_out[i] = cur;
+  if (rgb_out) {
+    uint8_t r = 0, g = 0, b = 0;
+    if (cur < dmax) {
+      BlockCache bc;
+      bc.x = bc.y = bc.z = 0x7fffffff;
+      bc.ptr = -1;
+      F3 point = xform(T, point3d_uv(x, y, cur, s));
+      VoxelSample vx = get_interpolated<true>(v, point, inv_vs, bc);
+      r = (uint8_t)vx.r;
+      g = (uint8_t)vx.g;
+      b = (uint8_t)vx.b;
+    }
+    rgb_out[3 * (size_t)i] = r;
+    rgb_out[3 * (size_t)i + 1] = g;
+    rgb_out[3 * (size_t)i + 2] = b;
+  }
+  return false;
+}
 
 // ------------------------------------------------------------ mixed-precision raycast
 // The mixed forms' march: tsdfVolume::GenerateDepthKernel /
@@ -1049,6 +1462,24 @@ __device__ inline VoxelSample interp(const VolumeDev& v, F3 q, typename Vox<FP16
   return out;
 }
 
+// The interpolated colour at depth 'cur' of the ray q = o + cur * d (voxel
+// units); of an unobserved voxel its own.
+__device__ __noinline__ uchar4 mixed_colour(const VolumeDev& v, F3 o, F3 d, float cur) {
+  using V = Vox<true>;
+  const F3 q = f3(__fmaf_rn(cur, d.x, o.x), __fmaf_rn(cur, d.y, o.y), __fmaf_rn(cur, d.z, o.z));
+  const int gx = (int)floorf(q.x + 0.5f), gy = (int)floorf(q.y + 0.5f),
+            gz = (int)floorf(q.z + 0.5f);
+  BlockCache bc;
+  bc.x = bc.y = bc.z = 0x7fffffff;
+  bc.ptr = -1;
+  const int ptr = block_ptr(v, blk_of(gx), blk_of(gy), blk_of(gz), bc);
+  const int lin = lin_of(gx, gy, gz);
+  const typename V::raw_t raw = V::load(v, ptr, lin);
+  if (V::w(raw) == 0) return V::color(v, raw, ptr, lin);
+  const VoxelSample vx = interp<true, true>(v, q, raw, ptr, lin, bc);
+  return make_uchar4((uint8_t)vx.r, (uint8_t)vx.g, (uint8_t)vx.b, 0);
+}
+
 // The block of a cell's low corner through the ray's cache, with its
 // free-cell flag (0 where no flags are kept).
 __device__ inline int cell_block_free(const VolumeDev& v, int bx, int by, int bz, FreeCache& bc,
@@ -1070,9 +1501,10 @@ __device__ inline int cell_block_free(const VolumeDev& v, int bx, int by, int bz
 // free-cell flags (mixed form with carving); without them (band sessions)
 // the cell's and the centre voxel's blocks share one lookup cache.
 template <bool FP16, bool FREE>
-__device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
-                                  int y, float skip_to, float skip_far,
-                                  float* __restrict__ depth_out, uint8_t* __restrict__ rgb_out) {
+__device__ __noinline__ bool raycast_hash_px(const VolumeDev& v, const DSensor& s, const M4f& T,
+                                             int x, int y, float skip_to, float skip_far,
+                                             float* __restrict__ depth_out,
+                                             uint8_t* __restrict__ rgb_out) {
   using V = Vox<FP16>;
   const int i = y * s.cols + x;
   const DTsdf& t = v.t;
@@ -1129,88 +1561,147 @@ __device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4
   }
   depth_out[i] = cur;
   if (rgb_out) {
-    uint8_t r = 0, g = 0, b = 0;
-    if (cur < t.dmax) {
-      const F3 q =
-          f3(__fmaf_rn(cur, d.x, o.x), __fmaf_rn(cur, d.y, o.y), __fmaf_rn(cur, d.z, o.z));
-      const int gx = (int)floorf(q.x + 0.5f), gy = (int)floorf(q.y + 0.5f),
-                gz = (int)floorf(q.z + 0.5f);
-      const int ptr = block_ptr(v, blk_of(gx), blk_of(gy), blk_of(gz), bc0);
-      const int lin = lin_of(gx, gy, gz);
-      const typename V::raw_t raw = V::load(v, ptr, lin);
-      uchar4 c;
-      if (V::w(raw) != 0) {
-        const VoxelSample vx = interp<FP16, true>(v, q, raw, ptr, lin, bc);
-        c = make_uchar4((uint8_t)vx.r, (uint8_t)vx.g, (uint8_t)vx.b, 0);
-      } else {
-        c = V::color(v, raw, ptr, lin);  // GetInterpolatedVoxel returns the centre voxel
-      }
-      r = c.x;
-      g = c.y;
-      b = c.z;
-    }
-    rgb_out[3 * (size_t)i] = r;
-    rgb_out[3 * (size_t)i + 1] = g;
-    rgb_out[3 * (size_t)i + 2] = b;
+    uchar4 c = make_uchar4(0, 0, 0, 0);
+    if (cur < t.dmax) c = mixed_colour(v, o, d, cur);
+    rgb_out[3 * (size_t)i] = c.x;
+    rgb_out[3 * (size_t)i + 1] = c.y;
+    rgb_out[3 * (size_t)i + 2] = c.z;
   }
   return over;
 }
 
-// One 16x16 pixel tile (tile bx, by) from pose16 (a float 4x4); warps cover
-// 8x4 pixel sub-tiles for coherent rays.  Step-cap overruns are counted.
-// The tile is TX x TY pixels (multiples of 8 x 4; TX * TY >= 64).
-template <bool MIXED, int TX = kRayTX, int TY = kRayTY>
+// raycast_hash_px over the block grid: the same samples, each with the entries
+// of its cell's blocks read from the grid.  FREE: bit 0 of a block's entry is
+// its free-cell flag.
+template <bool FREE>
+__device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
+                                  int y, float skip_to, float skip_far,
+                                  float* __restrict__ depth_out, uint8_t* __restrict__ rgb_out) {
+  const DTsdf& t = v.t;
+  const float inv_vs = 1.0f / t.vs;
+  const float axf = ((float)x - s.cx) / s.fx, ayf = ((float)y - s.cy) / s.fy;
+  if (!v.grid || !v.gbox->ok || !march_bounded(t) ||
+      !(march_extent(t, T, axf, ayf, inv_vs) < 131072.0f))
+    return raycast_hash_px<true, FREE>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  const F3 o = f3(T.m[3] * inv_vs, T.m[7] * inv_vs, T.m[11] * inv_vs);
+  const F3 d = f3((T.m[0] * axf + T.m[1] * ayf + T.m[2]) * inv_vs,
+                  (T.m[4] * axf + T.m[5] * ayf + T.m[6]) * inv_vs,
+                  (T.m[8] * axf + T.m[9] * ayf + T.m[10]) * inv_vs);
+  const GridView G = grid_view(v);
+  const unsigned* __restrict__ vox = v.vox16;
+  const float dmax = t.dmax, trunc = t.trunc, vs = t.vs;
+  float cur = 0.0f;
+  MarchRange range(ray_near(t), skip_to, skip_far, dmax);
+  auto half_of = [](unsigned r) {
+    return __half2float(__ushort_as_half((unsigned short)(r & 0xffffu)));
+  };
+  while (range.sample(cur, trunc, dmax)) {
+    const F3 q = f3(__fmaf_rn(cur, d.x, o.x), __fmaf_rn(cur, d.y, o.y), __fmaf_rn(cur, d.z, o.z));
+    const int lx = round_near(q.x).low, ly = round_near(q.y).low, lz = round_near(q.z).low;
+    const float wx = q.x - biased_float(lx), wy = q.y - biased_float(ly),
+                wz = q.z - biased_float(lz);
+    const unsigned g = grid_index(G, lx, ly, lz);
+    const unsigned e0 = __ldg(G.e + g);
+    if (FREE && (e0 & 1u)) {  // the interpolated sdf is the truncation distance
+      cur += trunc;
+      continue;
+    }
+    const int ix = lx + (wx >= 0.5f), iy = ly + (wy >= 0.5f), iz = lz + (wz >= 0.5f);
+    // the voxel's block: mostly the cell's own
+    unsigned own = e0;
+    if ((unsigned)((ix ^ lx) | (iy ^ ly) | (iz ^ lz)) >= 8u)
+      own = __ldg(G.e + grid_index(G, ix, iy, iz));
+    const unsigned raw =
+        __ldg(vox + ((FREE ? own & ~1u : own) + (unsigned)(((ix & 7) << 6) | ((iy & 7) << 3) | (iz & 7))));
+    if (raw < 0x10000u) {  // weight 0
+      cur += trunc;
+      continue;
+    }
+    unsigned c[8], r[8];
+    cell_corners<FREE>(G, g, e0, lx, ly, lz, c);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r[k] = __ldg(vox + c[k]);
+    const float n0 = half_of(raw);
+    const float x0 = 1.0f - wx, y0 = 1.0f - wy, z0 = 1.0f - wz;
+    const float a00 = x0 * y0, a10 = wx * y0, a01 = x0 * wy, a11 = wx * wy;
+    const float coef[8] = {a00 * z0, a10 * z0, a01 * z0, a00 * wz,
+                           a11 * z0, a01 * wz, a10 * wz, a11 * wz};
+    float dist = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dist = __fmaf_rn(coef[k], r[k] < 0x10000u ? n0 : half_of(r[k]), dist);
+    const float sdf = dist * trunc;
+    cur += sdf;
+    if (sdf < vs) break;
+  }
+  const int i = y * s.cols + x;
+  depth_out[i] = cur;
+  if (rgb_out) {
+    uchar4 c = make_uchar4(0, 0, 0, 0);
+    if (cur < dmax) c = mixed_colour(v, o, d, cur);
+    rgb_out[3 * (size_t)i] = c.x;
+    rgb_out[3 * (size_t)i + 1] = c.y;
+    rgb_out[3 * (size_t)i + 2] = c.z;
+  }
+  return false;
+}
+
+// One pixel's ray of a TX x TY pixel tile (bx, by) from pose16 (a float 4x4);
+// warps cover 8x4 pixel sub-tiles for coherent rays.  Step-cap overruns are
+// counted.
+template <bool MIXED, int TX, int TY>
 __device__ inline void raycast_tile(const VolumeDev& v, const DSensor& s,
                                     const float* __restrict__ pose16, float* __restrict__ depth_out,
                                     uint8_t* __restrict__ rgb_out, int bx, int by,
                                     const unsigned* __restrict__ rbound, int tiles_x) {
-  static_assert(TX % 8 == 0 && TY % 4 == 0 && TX * TY >= 64, "tile of 8x4 warps");
-  __shared__ M4f Ts;
-  __shared__ int over;
-  const int tid = threadIdx.y * TX + threadIdx.x;
-  if (tid < 16) Ts.m[tid] = pose16[tid];
-  if (tid == 0) over = 0;
-  __syncthreads();
-  const M4f T = Ts;  // the pose in registers for the whole march
-  const int warp = tid >> 5, lane = tid & 31;
-  const int lx = (warp % (TX / 8)) * 8 + (lane & 7);
-  const int ly = (warp / (TX / 8)) * 4 + (lane >> 3);
-  const int x = bx * TX + lx, y = by * TY + ly;
-  if (x < s.cols && y < s.rows) {
-    float skip_to = 0.0f, skip_far = 3.402823466e+38f;
-    if (rbound) {
-      const int tx = x / kRbTile, ty = y / kRbTile;
-      const RayBounds B =
-          ray_bounds(const_cast<unsigned*>(rbound), tiles_x, (s.rows + kRbTile - 1) / kRbTile);
-      const int f = ty * tiles_x + tx, c = (ty / kRbCoarse) * B.cx + tx / kRbCoarse;
-      skip_to = fminf(__uint_as_float(B.near8[f]), __uint_as_float(B.near64[c]));
-      skip_far = fmaxf(__uint_as_float(B.far8[f]), __uint_as_float(B.far64[c]));
-    }
-    const bool o = MIXED ? (v.freecell ? raycast_px<true, true>(v, s, T, x, y, skip_to, skip_far,
-                                                                 depth_out, rgb_out)
-                                       : raycast_px<true, false>(v, s, T, x, y, skip_to,
-                                                                  skip_far, depth_out, rgb_out))
-                         : raycast_exact_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
-    if (o) atomicAdd(&over, 1);
+  static_assert(TX % 8 == 0 && TY % 4 == 0, "tile of 8x4 warps");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int x = bx * TX + (warp % (TX / 8)) * 8 + (lane & 7);
+  const int y = by * TY + (warp / (TX / 8)) * 4 + (lane >> 3);
+  if (x >= s.cols || y >= s.rows) return;
+  M4f T;  // the pose in registers for the whole march
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float4 r = __ldg(reinterpret_cast<const float4*>(pose16) + k);
+    T.m[4 * k] = r.x;
+    T.m[4 * k + 1] = r.y;
+    T.m[4 * k + 2] = r.z;
+    T.m[4 * k + 3] = r.w;
   }
-  __syncthreads();
-  if (tid == 0 && over) atomicAdd(&v.cnt->raycast_overruns, over);
+  float skip_to = 0.0f, skip_far = 3.402823466e+38f;
+  if (rbound) {
+    const int tx = x / kRbTile, ty = y / kRbTile;
+    const RayBounds B =
+        ray_bounds(const_cast<unsigned*>(rbound), tiles_x, (s.rows + kRbTile - 1) / kRbTile);
+    const int f = ty * tiles_x + tx, c = (ty / kRbCoarse) * B.cx + tx / kRbCoarse;
+    skip_to = fminf(__uint_as_float(B.near8[f]), __uint_as_float(B.near64[c]));
+    skip_far = fmaxf(__uint_as_float(B.far8[f]), __uint_as_float(B.far64[c]));
+  }
+  const bool over = MIXED ? (v.freecell ? raycast_px<true>(v, s, T, x, y, skip_to, skip_far,
+                                                           depth_out, rgb_out)
+                                        : raycast_px<false>(v, s, T, x, y, skip_to, skip_far,
+                                                            depth_out, rgb_out))
+                          : raycast_exact_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  if (over) atomicAdd(&v.cnt->raycast_overruns, 1);
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kRayTX* kRayTY)
-    raycast_kernel(VolumeDev v, DSensor s, const PoseState* __restrict__ ps,
-                   const float* __restrict__ pose_override, float* __restrict__ depth_out,
-                   uint8_t* __restrict__ rgb_out) {
-  raycast_tile<MIXED>(v, s, pose_override ? pose_override : ps->posef, depth_out, rgb_out,
-                      blockIdx.x, blockIdx.y, nullptr, 0);
+__global__ void __launch_bounds__(256)
+    raycast_kernel(const __grid_constant__ VolumeDev v, const __grid_constant__ DSensor s,
+                   const PoseState* __restrict__ ps, const float* __restrict__ pose_override,
+                   float* __restrict__ depth_out, uint8_t* __restrict__ rgb_out) {
+  raycast_tile<MIXED, 16, 16>(v, s, pose_override ? pose_override : ps->posef, depth_out, rgb_out,
+                              blockIdx.x, blockIdx.y, nullptr, 0);
 }
 
 // next frame's target of every mode-1 session (blockIdx.z) at its new pose;
 // one instantiation per voxel form (sessions of the other form return) and
 // per tile shape (every pixel's march is independent of the tiling)
-// (at least 1024 threads resident per SM: the march is latency-bound, and
-// 4 CTAs of 256 hide more of it than the 3 that 76 registers allow)
+// (at least 1024 threads resident per SM: the march waits on its own loads --
+// grid entry, voxel, corners -- and issues in 60 % of the cycles, and 4 CTAs of
+// 256 hide more of it than the 3 that 76 registers allow.  A persistent launch
+// whose warps fetch 8x4 tiles from an even sample of the image balanced the
+// SMs but spilled in the loop: 272 against 253 us.  All nine loads of a sample
+// issued together: 275 against 265 us, the weight test saves more.)
 template <bool MIXED, int TX, int TY>
 __global__ void __launch_bounds__(TX* TY, 1024 / (TX * TY))
     fused_raycast_kernel(const SessDev* __restrict__ tab) {
@@ -1226,8 +1717,8 @@ __global__ void __launch_bounds__(TX* TY, 1024 / (TX * TY))
 template <int TX, int TY>
 void launch_fused_raycast(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   dim3 grid((b.max_cols + TX - 1) / TX, (b.max_rows + TY - 1) / TY, b.n);
-  if (b.fp16_mask & 1) fused_raycast_kernel<false, TX, TY><<<grid, dim3(TX, TY), 0, st>>>(tab);
-  if (b.fp16_mask & 2) fused_raycast_kernel<true, TX, TY><<<grid, dim3(TX, TY), 0, st>>>(tab);
+  if (b.fp16_mask & 1) fused_raycast_kernel<false, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
+  if (b.fp16_mask & 2) fused_raycast_kernel<true, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
 }
 
 // per-frame counters of every session (all but nalloc, the heap top) and
@@ -1300,7 +1791,7 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 void launch_volume_clear(const VolumeDev& v, cudaStream_t st) {
   size_t ne = (size_t)v.t.num_buckets * v.t.bucket_size;
   clear_entries_kernel<<<nblk((long long)ne, 256), 256, 0, st>>>(v.entries, ne);
-  const size_t nv = (size_t)v.t.num_blocks * kBlockVox;
+  const size_t nv = ((size_t)v.t.num_blocks + 1) * kBlockVox;  // and the empty block
   if (v.voxels) cudaMemsetAsync(v.voxels, 0, sizeof(dyn_voxel) * nv, st);
   if (v.vox16) cudaMemsetAsync(v.vox16, 0, sizeof(unsigned) * nv, st);
   if (v.colors) cudaMemsetAsync(v.colors, 0, sizeof(uchar4) * nv, st);
@@ -1311,13 +1802,19 @@ void launch_volume_clear(const VolumeDev& v, cudaStream_t st) {
 
 void launch_raycast(const VolumeDev& v, const DSensor& s, const PoseState* ps,
                     const float* pose_override, float* depth_out, uint8_t* rgb_out,
-                    cudaStream_t st) {
-  dim3 grid(nblk(s.cols, kRayTX), nblk(s.rows, kRayTY));
+                    bool use_grid, cudaStream_t st) {
+  if (use_grid) {
+    grid_clear_kernel<<<148 * 4, 256, 0, st>>>(v, s, pose_override ? pose_override : ps->posef);
+    grid_fill_kernel<<<148 * 4, 256, 0, st>>>(v);
+  }
+  VolumeDev w = v;
+  if (!use_grid) w.grid = nullptr;
+  const dim3 grid(nblk(s.cols, 16), nblk(s.rows, 16));
   if (v.fp16)
-    raycast_kernel<true><<<grid, dim3(kRayTX, kRayTY), 0, st>>>(v, s, ps, pose_override,
+    raycast_kernel<true><<<grid, 256, 0, st>>>(w, s, ps, pose_override,
                                                                 depth_out, rgb_out);
   else
-    raycast_kernel<false><<<grid, dim3(kRayTX, kRayTY), 0, st>>>(v, s, ps, pose_override,
+    raycast_kernel<false><<<grid, 256, 0, st>>>(w, s, ps, pose_override,
                                                                  depth_out, rgb_out);
 }
 
@@ -1337,8 +1834,10 @@ void fused_reset_counters(const SessDev* tab, const BatchShape& b, cudaStream_t 
 }
 
 void fused_allocate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  dim3 grid(nblk(b.max_cols, kAllocT), nblk(b.max_rows, kAllocT), b.n);
-  fused_allocate_kernel<<<grid, dim3(kAllocT, kAllocT), 0, st>>>(tab);
+  const int tx = nblk(b.max_cols, kAllocT), ty = nblk(b.max_rows, kAllocT);
+  // about two CTAs per SM for the grids (enough for their writes)
+  const int extra = b.max_grid > 0 ? nblk(std::max(8, 148 * 2 / b.n), tx) : 0;
+  fused_allocate_kernel<<<dim3(tx, ty + extra, b.n), dim3(kAllocT, kAllocT), 0, st>>>(tab, ty);
 }
 
 void fused_visible(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
