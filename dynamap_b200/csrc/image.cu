@@ -10,6 +10,7 @@
 #include "image.cuh"
 
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "dyn_exp.h"
@@ -42,78 +43,166 @@ __global__ void ingest_kernel(const uint16_t* __restrict__ raw,
   ingest_px(raw, rgb, scaler, depth, inten, i);
 }
 
-constexpr int BTX = 32, BTY = 8;
-
-// pyramid::applyBilateralFilter, pyramid.cu:213-233, one thread per pixel,
-// window rows x-r..x+r-1, cols y-r..y+r-1, summed row-major.  The depth tile
-// plus halo is staged in shared memory; the spatial weights, a pure function
-// of the tap offset, come precomputed on the host in double and rounded to
-// float exactly as the reference rounds them per tap (read as warp-uniform
-// values).  The range weight uses dyn_expf, the same operation sequence the
-// oracle runs, so the filtered depth is bit-identical to the oracle's.  Taps
-// outside the image or with depth <= 0 are skipped; invalid centres stay 0.
+// pyramid::applyBilateralFilter, pyramid.cu:213-233, window rows x-r..x+r-1,
+// cols y-r..y+r-1, summed row-major.  The depth tile plus halo is staged in
+// shared memory (0 where outside the image or not > 0: such taps are skipped,
+// such centres stay 0); the spatial weights, a pure function of the tap
+// offset, come precomputed on the host in double and rounded to float exactly
+// as the reference rounds them per tap (read as warp-uniform values).  The
+// range weight uses dyn_expf, the same operation sequence the oracle runs, so
+// the filtered depth is bit-identical to the oracle's.
 // FAST (mixed-precision sessions): each tap's weight in one hardware
 // base-2 exponential, gs * exp(-dn^2 / (2 s^2)) = 2^(log2 gs - dn^2 c) with
 // c = log2(e) / (2 s^2), the spatial weights staged as their logarithms;
 // the range normalisation 1/(2 pi s^2), common to every weight, cancels in
 // acc / wp and is left out.
+//
+// Bound by the FP32 pipe: 15 operations per tap (dyn_expf's polynomial is 7 of
+// them), 256 taps per pixel at the reference's diameter.  So everything else
+// is kept off the tap:
+//  * SMALL: where the depths of the CTA's tile span so little that every tap's
+//    exponent rounds to k = 0 (sigma_i 10 m: always), dyn_expf's reduction is
+//    the identity and is left out -- the conversions it needs run at an eighth
+//    of the FP32 rate;
+//  * MASK false: where no staged pixel is invalid, no test per tap;
+//  * the taps of a window row unroll (DT the window size, 0: any), so that
+//    their weights overlap; only the two sums are serial.
+// A call at diameter 8, before -> now: 160x120 43.3 -> 12.4 us (the kernel 8),
+// 320x240 45 -> 14, 640x480 80 -> 33, 1280x720 146 -> 71.  Two pixels of a
+// column per thread, each staged depth read once for both, measured 16, 37 and
+// 72 us: the shared-memory reads are not what it waits for.
+constexpr int BTX = 32;
+
+__device__ __host__ inline int bil_pitch(int D) { return BTX + D - 1; }
+// Floats before the spatial weights (a multiple of four: they are read as
+// vectors).
+__device__ __host__ inline int bil_tile_floats(int D, int rows) {
+  return (bil_pitch(D) * (rows + D - 1) + 3) / 4 * 4;
+}
+
+// exp(x) of dyn_expf for |x log2(e)| <= 1/2, where its k is 0: p * 2^0.
+__device__ inline float expf_k0(float r) {
+  float p = 1.98412698412698413e-4f;   // the terms of dyn_expf
+  p = __fmaf_rn(p, r, 1.38888888888888889e-3f);
+  p = __fmaf_rn(p, r, 8.33333333333333333e-3f);
+  p = __fmaf_rn(p, r, 4.16666666666666667e-2f);
+  p = __fmaf_rn(p, r, 1.66666666666666667e-1f);
+  p = __fmaf_rn(p, r, 0.5f);
+  p = __fmaf_rn(p, r, 1.0f);
+  return __fmaf_rn(p, r, 1.0f);
+}
+
+template <bool FAST, bool SMALL, bool MASK, int DT>
+__device__ inline float bilateral_sum(const float* __restrict__ t, const float* __restrict__ gs,
+                                      int pitch, int D_, float inv2s2, float norm, float c) {
+  const int D = DT ? DT : D_;
+  const float c2 = inv2s2 * 1.4426950408889634f;  // FAST: log2(e) / (2 s^2)
+  float acc = 0.0f, wp = 0.0f;
+  auto tap = [&](float nv, float g) {
+    const float dn = nv - c;
+    float w;
+    if (FAST) {
+      asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmaf_rn(-(dn * dn), c2, g)));
+      if (MASK) w = nv > 0.0f ? w : 0.0f;
+      acc = __fmaf_rn(nv, w, acc);
+    } else {
+      w = (SMALL ? expf_k0(-(dn * dn) * inv2s2) * norm : range_weight(dn, inv2s2, norm)) * g;
+      if (MASK) w = nv > 0.0f ? w : 0.0f;
+      acc += nv * w;
+    }
+    wp += w;
+  };
+#pragma unroll 1
+  for (int i = 0; i < D; ++i) {
+    const float* tr = t + i * pitch;
+    const float* gr = gs + i * D;
+    if (DT) {
+#pragma unroll
+      for (int j = 0; j < DT; j += 4) {
+        const float4 g = *reinterpret_cast<const float4*>(gr + j);
+        tap(tr[j], g.x);
+        tap(tr[j + 1], g.y);
+        tap(tr[j + 2], g.z);
+        tap(tr[j + 3], g.w);
+      }
+    } else {
+#pragma unroll 2
+      for (int j = 0; j < D; ++j) tap(tr[j], gr[j]);
+    }
+  }
+  return acc / wp;
+}
+
+// One tile of 32 x blockDim.y pixels, tile column bx and row by.
 template <bool FAST>
 __device__ inline void bilateral_tile(const float* __restrict__ src, float* __restrict__ dst,
                                       int rows, int cols, const BilateralTable& tb, int bx,
                                       int by, float* tile) {
-  const int D = 2 * tb.radius, half = tb.radius;
-  const int TW = BTX + D - 1, TH = BTY + D - 1;
-  float* gs = tile + TW * TH;  // the spatial weights, staged once per CTA
-  const int tid = threadIdx.y * BTX + threadIdx.x;
-  const int row0 = by * BTY - half, col0 = bx * BTX - half;
-  for (int k = tid; k < TW * TH; k += BTX * BTY) {
-    int tr = k / TW, tc = k - (k / TW) * TW;
-    int gr = row0 + tr, gc = col0 + tc;
-    tile[k] = (gr >= 0 && gr < rows && gc >= 0 && gc < cols) ? src[gr * cols + gc] : 0.0f;
+  __shared__ unsigned lo_s, hi_s;
+  const int D = 2 * tb.radius, half = tb.radius, TY = blockDim.y;
+  const int TW = bil_pitch(D), TH = TY + D - 1;
+  float* gs = tile + bil_tile_floats(D, TY);  // the spatial weights, staged once per CTA
+  const int tid = threadIdx.y * BTX + threadIdx.x, threads = TY * BTX;
+  if (tid == 0) {
+    lo_s = 0xffffffffu;
+    hi_s = 0u;
   }
-  for (int k = tid; k < D * D; k += BTX * BTY) gs[k] = FAST ? __log2f(tb.gs[k]) : tb.gs[k];
   __syncthreads();
-  const int x = by * BTY + threadIdx.y;  // row (the reference's x)
-  const int y = bx * BTX + threadIdx.x;  // column
-  if (x >= rows || y >= cols) return;
-  const float c = tile[(threadIdx.y + half) * TW + threadIdx.x + half];
-  if (!(c > 0.0f)) {
-    dst[x * cols + y] = 0.0f;
-    return;
-  }
-  const float inv2s2 = tb.inv2s2, norm = tb.norm;
-  const float c2 = inv2s2 * 1.4426950408889634f;  // FAST: log2(e) / (2 s^2)
-  float acc = 0.0f, wp = 0.0f;
-  // the taps inside the image: row x - half + i in [0, rows), column
-  // y - half + j in [0, cols); summed in the reference's order
-  const int i0 = max(0, half - x), i1 = min(D, rows - x + half);
-  const int j0 = max(0, half - y), j1 = min(D, cols - y + half);
-  for (int i = i0; i < i1; ++i) {
-    const float* trow = tile + (threadIdx.y + i) * TW + threadIdx.x;
-    const float* grow = gs + i * D;
-    for (int j = j0; j < j1; ++j) {
-      float nv = trow[j];
-      if (!(nv > 0.0f)) continue;
-      const float dn = nv - c;
-      if (FAST) {
-        float w;
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmaf_rn(-(dn * dn), c2, grow[j])));
-        acc = __fmaf_rn(nv, w, acc);
-        wp += w;
+  const int row0 = by * TY - half, col0 = bx * BTX - half;
+  unsigned lo = 0xffffffffu, hi = 0u;  // valid depths as bits (positive floats order as theirs)
+  bool hole = false;
+  for (int tr = threadIdx.y; tr < TH; tr += TY) {
+    const int gr = row0 + tr;
+    const bool in = gr >= 0 && gr < rows;
+    for (int tc = threadIdx.x; tc < TW; tc += BTX) {
+      const int gc = col0 + tc;
+      float d = (in && gc >= 0 && gc < cols) ? src[gr * cols + gc] : 0.0f;
+      if (!(d > 0.0f)) {
+        d = 0.0f;
+        hole = true;
       } else {
-        float w = range_weight(dn, inv2s2, norm) * grow[j];
-        acc += nv * w;
-        wp += w;
+        lo = min(lo, __float_as_uint(d));
+        hi = max(hi, __float_as_uint(d));
       }
+      tile[tr * TW + tc] = d;
     }
   }
-  dst[x * cols + y] = acc / wp;
+  for (int k = tid; k < D * D; k += threads) gs[k] = FAST ? __log2f(tb.gs[k]) : tb.gs[k];
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (threadIdx.x == 0 && hi) {
+    atomicMin(&lo_s, lo);
+    atomicMax(&hi_s, hi);
+  }
+  const bool mask = __syncthreads_or(hole) != 0;
+  const int y = bx * BTX + threadIdx.x;  // column
+  const int x = by * TY + threadIdx.y;   // row (the reference's x)
+  if (x >= rows || y >= cols) return;
+  const float* t = tile + (int)threadIdx.y * TW + threadIdx.x;
+  const float c = t[half * TW + half];
+  float out = 0.0f;
+  if (c > 0.0f) {
+    // the largest |exponent| of the tile's taps, by the taps' own (monotone)
+    // operations
+    const float span = __uint_as_float(hi_s) - __uint_as_float(lo_s);
+    const float i2 = tb.inv2s2, nm = tb.norm;
+    if (!FAST && !(span * span * i2 * 1.44269504088896341f <= 0.5f))
+      out = bilateral_sum<FAST, false, true, 0>(t, gs, TW, D, i2, nm, c);
+    else if (D != 16)
+      out = bilateral_sum<FAST, true, true, 0>(t, gs, TW, D, i2, nm, c);
+    else if (mask)
+      out = bilateral_sum<FAST, true, true, 16>(t, gs, TW, D, i2, nm, c);
+    else
+      out = bilateral_sum<FAST, true, false, 16>(t, gs, TW, D, i2, nm, c);
+  }
+  dst[x * cols + y] = out;
 }
 
 __global__ void bilateral_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                  int rows, int cols, const __grid_constant__ BilateralTable tb) {
-  extern __shared__ float tile[];
-  bilateral_tile<false>(src, dst, rows, cols, tb, blockIdx.x, blockIdx.y, tile);
+  extern __shared__ float4 smem4[];
+  bilateral_tile<false>(src, dst, rows, cols, tb, blockIdx.x, blockIdx.y,
+                        reinterpret_cast<float*>(smem4));
 }
 
 // One 2x pyramid step: mean of the valid depths of each 2x2 cell (fix of
@@ -265,11 +354,12 @@ __global__ void fused_free_tiles_kernel(const SessDev* __restrict__ tab) {
 }
 
 __global__ void fused_bilateral_kernel(const SessDev* __restrict__ tab) {
-  extern __shared__ float tile[];
+  extern __shared__ float4 smem4[];
+  float* tile = reinterpret_cast<float*>(smem4);
   const SessDev& S = tab[blockIdx.z];
   if (!S.bil_enabled) return;
   const int rows = S.ls[0].rows, cols = S.ls[0].cols;
-  if ((int)blockIdx.x * BTX >= cols || (int)blockIdx.y * BTY >= rows) return;
+  if ((int)blockIdx.x * BTX >= cols || (int)(blockIdx.y * blockDim.y) >= rows) return;
   if (S.vol.fp16)  // mixed-precision session
     bilateral_tile<true>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
   else
@@ -338,16 +428,21 @@ static double gaussian_d(double x, double sigma) {
 
 BilateralTable make_bilateral_table(int radius, float sigma_i, float sigma_s) {
   BilateralTable tb;
-  std::memset(&tb, 0, sizeof(tb));
   tb.radius = radius;
   const int D = 2 * radius, half = radius;
-  for (int i = 0; i < D; ++i)
-    for (int j = 0; j < D; ++j) {
-      // vertexDistance (pyramid.cu:201-206) in float, gaussian in double
-      float dx = (float)(half - i), dy = (float)(half - j);
-      float dd = std::sqrt(dx * dx + dy * dy + 0.0f * 0.0f);
-      tb.gs[i * D + j] = (float)gaussian_d((double)dd, (double)sigma_s);
+  // vertexDistance (pyramid.cu:201-206) in float, gaussian in double; a
+  // weight depends on the offsets' magnitudes alone, in either order: 45
+  // exponentials instead of 256 at radius 8 (the table is made per call:
+  // 8.0 -> 2.0 us of host time there)
+  float w[17][17];
+  for (int i = 0; i <= half; ++i)
+    for (int j = 0; j <= i; ++j) {
+      const float dx = (float)i, dy = (float)j;
+      const float dd = std::sqrt(dx * dx + dy * dy + 0.0f * 0.0f);
+      w[i][j] = w[j][i] = (float)gaussian_d((double)dd, (double)sigma_s);
     }
+  for (int i = 0; i < D; ++i)
+    for (int j = 0; j < D; ++j) tb.gs[i * D + j] = w[std::abs(half - i)][std::abs(half - j)];
   double si = (double)sigma_i;
   tb.inv2s2 = (float)(1.0 / (2.0 * si * si));
   tb.norm = (float)(1.0 / (2.0 * 3.14159265358979323846 * si * si));
@@ -355,16 +450,21 @@ BilateralTable make_bilateral_table(int radius, float sigma_i, float sigma_s) {
 }
 
 // depth tile with its halo, then the D x D spatial weights
-static size_t bilateral_smem(int radius) {
-  int D = 2 * radius;
-  return sizeof(float) * ((size_t)(BTX + D - 1) * (BTY + D - 1) + (size_t)D * D);
+static size_t bilateral_smem(int radius, int rows) {
+  const int D = 2 * radius;
+  return sizeof(float) * ((size_t)bil_tile_floats(D, rows) + (size_t)D * D);
+}
+// Rows of a CTA's tile: 8 stage less halo per pixel, 4 balance small images
+// over the SMs (453x340: 20.2 us with 4, 23.4 with 8; 640x480: 35.1 and 32.6).
+static int bilateral_rows(long long cols, long long rows, int n) {
+  return (cols + BTX - 1) / BTX * ((rows + 7) / 8) * n >= 6 * 148 ? 8 : 4;
 }
 
 void launch_bilateral(const float* src, float* dst, int rows, int cols, const BilateralTable& tb,
                       cudaStream_t st) {
-  dim3 grid(nblk(cols, BTX), nblk(rows, BTY));
-  bilateral_kernel<<<grid, dim3(BTX, BTY), bilateral_smem(tb.radius), st>>>(src, dst, rows, cols,
-                                                                            tb);
+  const int ty = bilateral_rows(cols, rows, 1);
+  bilateral_kernel<<<dim3(nblk(cols, BTX), nblk(rows, ty)), dim3(BTX, ty),
+                     bilateral_smem(tb.radius, ty), st>>>(src, dst, rows, cols, tb);
 }
 
 void launch_downsample_depth(const float* src, int rows, int cols, float* dst, cudaStream_t st) {
@@ -395,9 +495,10 @@ void fused_ingest(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
 }
 
 void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  if (b.max_bil_radius > 0)
-    fused_bilateral_kernel<<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, BTY), b.n),
-                             dim3(BTX, BTY), bilateral_smem(b.max_bil_radius), st>>>(tab);
+  if (b.max_bil_radius <= 0) return;
+  const int ty = bilateral_rows(b.max_cols, b.max_rows, b.n);
+  fused_bilateral_kernel<<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, ty), b.n), dim3(BTX, ty),
+                           bilateral_smem(b.max_bil_radius, ty), st>>>(tab);
 }
 
 void fused_pyramid(const SessDev* tab, const BatchShape& b, int target, cudaStream_t st) {
