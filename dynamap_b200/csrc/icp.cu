@@ -27,6 +27,15 @@ namespace dyn {
 
 namespace {
 
+// A level as the per-frame kernels keep it in shared memory, with its tiles'
+// shape and the session's parameters (read again and again while a thread's
+// registers hold sums).
+struct FrameLevel : IcpLevel {
+  int n, group, slots, tile, ntiles;  // pixels; icp_group, icp_slots, icp_tile_slots, icp_tiles
+  int parts_log2;                     // a tile's parts, one per warp: 16 or 8
+  IcpParams P;
+};
+
 __device__ inline bool normal_ok(float4 n) {
   if (isnan(n.x) || isnan(n.y) || isnan(n.z)) return false;
   return !(n.x == 0.0f && n.y == 0.0f && n.z == 0.0f);
@@ -150,7 +159,7 @@ __device__ inline PixTgt load_tgt(const IcpLevel& L, const IcpParams& P, const P
 // multiply-adds: b_k = cn_k (pq . n), the reference's three-product sum in
 // exact arithmetic) added into FP32 per-thread sums.
 __device__ inline void accumulate_mixed(const IcpParams& P, const F3 p, const F3 n, const F3 pq,
-                                        const PixTgt& t, Acc& a) {
+                                        const PixTgt& t, float count, Acc& a) {
   const F3 c = cross3(p, n);
   const float cn[6] = {c.x, c.y, c.z, n.x, n.y, n.z};
   const float r = __fmaf_rn(pq.x, n.x, __fmaf_rn(pq.y, n.y, __fmul_rn(pq.z, n.z)));
@@ -184,7 +193,7 @@ __device__ inline void accumulate_mixed(const IcpParams& P, const F3 p, const F3
     for (int k = 0; k < 6; ++k) a.v[21 + k] = __fmaf_rn(-cn[k], r, a.v[21 + k]);
   }
   a.v[27] = __fmaf_rn(r, r, a.v[27]);
-  a.v[28] = __fadd_rn(a.v[28], 1.0f);
+  a.v[28] = __fadd_rn(a.v[28], count);
 }
 
 template <bool KAHAN>
@@ -200,7 +209,7 @@ __device__ inline void accumulate(const IcpLevel& L, const IcpParams& P, const P
   if (!(fabsf(cosT) > P.cos_thr)) return;
   F3 pq = p - qq;
   if (KAHAN) {
-    accumulate_mixed(P, p, n, pq, t, a);
+    accumulate_mixed(P, p, n, pq, t, 1.0f, a);
     return;
   }
   F3 c = cross3(p, n);
@@ -246,23 +255,49 @@ __device__ inline void pixel_terms(const IcpLevel& L, const IcpParams& P, const 
   accumulate<KAHAN>(L, P, q, load_tgt(L, P, q, idx), a);
 }
 
-// Two pixels with their loads issued together (source, then target), then
-// added in order: the same sums as pixel_terms on i0, then on i1.
-template <bool KAHAN>
-__device__ inline void pixel_pair(const IcpLevel& L, const IcpParams& P, const M4f& T, int i0,
-                                  int i1, int n, Acc& a) {
-  const bool v0 = i0 < n, v1 = i1 < n;
-  PixSrc a0, a1;
-  if (v0) a0 = load_src(L, i0);
-  if (v1) a1 = load_src(L, i1);
-  PixProj q0, q1;
-  const bool ok0 = v0 && project_src<KAHAN>(L, P, T, i0, a0, q0);
-  const bool ok1 = v1 && project_src<KAHAN>(L, P, T, i1, a1, q1);
-  PixTgt t0, t1;
-  if (ok0) t0 = load_tgt(L, P, q0, i0);
-  if (ok1) t1 = load_tgt(L, P, q1, i1);
-  if (ok0) accumulate<KAHAN>(L, P, q0, t0, a);
-  if (ok1) accumulate<KAHAN>(L, P, q1, t1, a);
+// N pixels i, i + stride, ... below n of the mixed form, added in order: the
+// terms of pixel_terms on one after the other, without branches, so that the
+// pixels' latencies overlap (at 16 warps per SM nothing else hides them).  A
+// pixel without a correspondence loads pixel 0, counts 0, and its vectors are
+// zero: its terms are zeros, which change no sum.
+template <int N>
+__device__ inline void pixel_group(const FrameLevel& L, const M4f& T, int i, int stride, int n,
+                                   Acc& a) {
+  const IcpParams& P = L.P;
+  PixSrc src[N];
+  PixProj q[N];
+  PixTgt t[N];
+  bool ok[N];
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    ok[m] = i + m * stride < n;
+    src[m] = load_src(L, ok[m] ? i + m * stride : 0);
+  }
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    const bool in = project_src<true>(L, P, T, i + m * stride, src[m], q[m]);
+    ok[m] = ok[m] && in;
+    q[m].index = ok[m] ? q[m].index : 0;
+    q[m].px = ok[m] ? q[m].px : 0;
+    q[m].py = ok[m] ? q[m].py : 0;
+  }
+#pragma unroll
+  for (int m = 0; m < N; ++m) t[m] = load_tgt(L, P, q[m], ok[m] ? i + m * stride : 0);
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    const F3 n = f3(t[m].tn.x, t[m].tn.y, t[m].tn.z);
+    const float cosT = dot3(n, f3(q[m].sn.x, q[m].sn.y, q[m].sn.z));
+    const bool in = ok[m] && !(t[m].td < P.dmin || t[m].td > P.dmax) && normal_ok(t[m].tn) &&
+                    fabsf(cosT) > P.cos_thr;
+    const F3 pq = q[m].p - point3d_fast(q[m].px, q[m].py, t[m].td, L.s);
+    auto sel = [in](F3 v) { return f3(in ? v.x : 0.0f, in ? v.y : 0.0f, in ? v.z : 0.0f); };
+    PixTgt u = t[m];
+    u.ic = in ? u.ic : 0.0f;
+    u.il = in ? u.il : 0.0f;
+    u.iu = in ? u.iu : 0.0f;
+    u.si = in ? u.si : 0.0f;
+    accumulate_mixed(P, sel(q[m].p), sel(n), sel(pq), u, in ? 1.0f : 0.0f, a);
+  }
 }
 
 // ---- block and tile sums
@@ -292,27 +327,35 @@ __device__ inline void unpack_pair(double d, float& s, float& c) {
   c = __uint_as_float((unsigned)(u >> 32));
 }
 
-// Block sum of the 29 accumulators in a fixed order; result in red[0..28]
-// (shared) after the call: FP64 values, or packed compensated pairs (KAHAN).
+// Warp sum of the 29 accumulators in a fixed order: lane l < 29 gets the total
+// of value l (FP64, or a compensated pair).
 // The warp sum is a halving exchange over 32 slots (values 29..31 zero):
 // at offset o every lane keeps the half of its remaining slots that its
 // bit o selects, sends the other half to lane ^ o and adds what that lane
 // sent; after offsets 16, 8, 4, 2, 1 lane l holds the warp's total of value
 // l.  31 exchanges per lane instead of 29 x 5 for a butterfly per value.
+struct LaneSum {
+  double d;    // plain
+  float s, c;  // compensated
+};
 template <bool KAHAN>
-__device__ inline void block_reduce(const Acc& a, double* red /*[8][29]*/) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ inline LaneSum warp_reduce(const Acc& a) {
+  const int lane = threadIdx.x & 31;
+  LaneSum out;
   if (KAHAN) {
-    float s[32], c[32];
+    float s[32], c[16];
 #pragma unroll
-    for (int k = 0; k < kIcpVals; ++k) {
-      s[k] = a.v[k];
-      c[k] = 0.0f;
+    for (int k = 0; k < kIcpVals; ++k) s[k] = a.v[k];
+#pragma unroll
+    for (int k = kIcpVals; k < 32; ++k) s[k] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {  // the first exchange: no corrections yet
+      const bool up = (lane & 16) != 0;
+      const float ks = up ? s[k + 16] : s[k], gs = up ? s[k] : s[k + 16];
+      two_sum(ks, __shfl_xor_sync(0xffffffffu, gs, 16), s[k], c[k]);
     }
 #pragma unroll
-    for (int k = kIcpVals; k < 32; ++k) s[k] = c[k] = 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 8; o > 0; o >>= 1) {
       const bool up = (lane & o) != 0;
 #pragma unroll
       for (int k = 0; k < o; ++k) {
@@ -325,7 +368,8 @@ __device__ inline void block_reduce(const Acc& a, double* red /*[8][29]*/) {
         pair_add(s[k], c[k], rs, rc);
       }
     }
-    if (lane < kIcpVals) red[warp * kIcpVals + lane] = pack_pair(s[0], c[0]);
+    out.s = s[0];
+    out.c = c[0];
   } else {
     double s[32];
 #pragma unroll
@@ -341,34 +385,50 @@ __device__ inline void block_reduce(const Acc& a, double* red /*[8][29]*/) {
         s[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
       }
     }
-    if (lane < kIcpVals) red[warp * kIcpVals + lane] = s[0];
+    out.d = s[0];
   }
-  __syncthreads();
-  if (threadIdx.x < kIcpVals) {
-    if (KAHAN) {
-      float sv = 0.0f, sc = 0.0f;
-      for (int w = 0; w < kIcpThreads / 32; ++w) {
+  return out;
+}
+
+// One value of the first nw of NW warps (red[0], red[29], ...: shared) added in
+// warp order.
+template <bool KAHAN, int NW>
+__device__ inline double add_warps(const double* red, int nw = NW) {
+  if (KAHAN) {
+    float sv = 0.0f, sc = 0.0f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w)
+      if (w < nw) {
         float s2, c2;
-        unpack_pair(red[w * kIcpVals + threadIdx.x], s2, c2);
+        unpack_pair(red[w * kIcpVals], s2, c2);
         pair_add(sv, sc, s2, c2);
       }
-      red[threadIdx.x] = pack_pair(sv, sc);  // row 0 reused: each thread its own column
-    } else {
-      double sum = 0.0;
-      for (int w = 0; w < kIcpThreads / 32; ++w) sum += red[w * kIcpVals + threadIdx.x];
-      red[threadIdx.x] = sum;
-    }
+    return pack_pair(sv, sc);
   }
+  double sum = 0.0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w)
+    if (w < nw) sum += red[w * kIcpVals];
+  return sum;
+}
+
+// Block sum in red[0..28] (shared, NW x 29) after the call.
+template <bool KAHAN, int NW>
+__device__ inline void block_reduce(const Acc& a, double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const LaneSum l = warp_reduce<KAHAN>(a);
+  if (lane < kIcpVals) red[warp * kIcpVals + lane] = KAHAN ? pack_pair(l.s, l.c) : l.d;
+  __syncthreads();
+  // (row 0 reused: each thread its own column)
+  if (threadIdx.x < kIcpVals) red[threadIdx.x] = add_warps<KAHAN, NW>(red + threadIdx.x);
   __syncthreads();
 }
 
-// Sum of the per-tile (or per-block) partials in a fixed order: thread
+// Sum of the stage kernel's per-block partials in a fixed order: thread
 // (g, k) of 8 x 29 sums value k of rows g, g + 8, g + 16, ... (all 29
 // values' loads in flight at once, coalesced along k), then thread k adds
 // the 8 group sums in group order.  'scratch' is 8 x 29 doubles of shared
-// memory; out[29] (shared) receives FP64 values (a compensated pair's
-// s + c in the KAHAN form).
-template <bool KAHAN>
+// memory; out[29] (shared).
 __device__ inline void final_reduce(const double* __restrict__ partials, int nblocks,
                                     double* out, double* scratch) {
   constexpr int kGroups = kIcpThreads / 32;  // 8: scratch is the block-reduce array
@@ -376,41 +436,62 @@ __device__ inline void final_reduce(const double* __restrict__ partials, int nbl
   const int t = threadIdx.x;
   if (t < kGroups * kIcpVals) {
     const int g = t / kIcpVals, k = t - g * kIcpVals;
-    if (KAHAN) {
-      float sv = 0.0f, sc = 0.0f;
+    double sum = 0.0;
 #pragma unroll 4
-      for (int b = g; b < nblocks; b += kGroups) {
-        float s2, c2;
-        unpack_pair(__ldcg(partials + (size_t)b * kIcpVals + k), s2, c2);
-        pair_add(sv, sc, s2, c2);
-      }
-      scratch[g * kIcpVals + k] = pack_pair(sv, sc);
-    } else {
-      double sum = 0.0;
-#pragma unroll 4
-      for (int b = g; b < nblocks; b += kGroups) sum += __ldcg(partials + (size_t)b * kIcpVals + k);
-      scratch[g * kIcpVals + k] = sum;
-    }
+    for (int b = g; b < nblocks; b += kGroups) sum += __ldcg(partials + (size_t)b * kIcpVals + k);
+    scratch[g * kIcpVals + k] = sum;
   }
   __syncthreads();
   if (t < kIcpVals) {
+    double sum = 0.0;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) sum += scratch[g * kIcpVals + t];
+    out[t] = sum;
+  }
+  __syncthreads();
+}
+
+// The level's total of its tiles' partials, in a fixed order: warp w sums rows
+// w, w + 16, ... (v[i] lane k's value k of row w + 16 i, zero past the last
+// tile), then lane k of warp 0 adds the 16 warps' sums.  'red' is 16 x 29
+// doubles of shared memory; out[29] (shared) is there for warp 0 after the
+// call: FP64 values (a compensated pair's s + c in the KAHAN form).
+constexpr int kFrameWarps = kIcpFrameThreads / 32;
+constexpr int kWarpRows = (kIcpMaxTiles + kFrameWarps - 1) / kFrameWarps;
+template <bool KAHAN>
+__device__ inline void level_total(const double (&v)[kWarpRows], double* out, double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane < kIcpVals) {
     if (KAHAN) {
       float sv = 0.0f, sc = 0.0f;
 #pragma unroll
-      for (int g = 0; g < kGroups; ++g) {
+      for (int i = 0; i < kWarpRows; ++i) {  // (rows that are not there add zero pairs)
         float s2, c2;
-        unpack_pair(scratch[g * kIcpVals + t], s2, c2);
+        unpack_pair(v[i], s2, c2);
         pair_add(sv, sc, s2, c2);
       }
-      out[t] = (double)sv + (double)sc;  // FP64 from here on: the 6x6 solve
+      red[w * kIcpVals + lane] = pack_pair(sv, sc);
     } else {
       double sum = 0.0;
 #pragma unroll
-      for (int g = 0; g < kGroups; ++g) sum += scratch[g * kIcpVals + t];
-      out[t] = sum;
+      for (int i = 0; i < kWarpRows; ++i) sum += v[i];
+      red[w * kIcpVals + lane] = sum;
     }
   }
   __syncthreads();
+  if (threadIdx.x < 32) {
+    if (lane < kIcpVals) {
+      const double t = add_warps<KAHAN, kFrameWarps>(red + lane);
+      if (KAHAN) {
+        float s2, c2;
+        unpack_pair(t, s2, c2);
+        out[lane] = (double)s2 + (double)c2;  // FP64 from here on: the 6x6 solve
+      } else {
+        out[lane] = t;
+      }
+    }
+    __syncwarp();
+  }
 }
 
 // ---- FP64 6x6 algebra (one thread) --------------------------------------
@@ -423,13 +504,12 @@ __device__ inline void final_reduce(const double* __restrict__ partials, int nbl
 __host__ __device__ constexpr int tri(int i, int j) { return i * (i + 1) / 2 + j; }
 
 // LDL^T of a symmetric positive definite 6x6 in place (stands in for
-// Eigen's A.ldlt().solve(b), gnSolver.cu:439-442): column j gives the pivot
-// D[j] = A[j][j] - sum_k L[j][k]^2 D[k] and L[i][j] = (A[i][j] - sum_k
-// L[i][k] L[j][k] D[k]) / D[j], each sum in increasing k; then forward
-// substitution, division by D, back substitution.  L overwrites the strict
-// lower triangle of a, D its diagonal.  Each pivot's reciprocal is taken
-// once and multiplies (one FP64 division per column instead of one per
-// entry: the one-thread solve sits between every two ICP iterations).
+// Eigen's A.ldlt().solve(b), gnSolver.cu:439-442), column by column: with
+// D[j] = A[j][j], L[i][j] = A[i][j] / D[j], then A[i][k] -= L[i][j] A[k][j]
+// for the columns behind -- so that only a reciprocal, a product and a fused
+// multiply-add lie between two pivots (this one thread sits between every two
+// ICP iterations); then forward substitution, division by D, back
+// substitution.  L overwrites the strict lower triangle of a, D its diagonal.
 // Returns false on a zero pivot.
 __device__ __forceinline__ bool ldlt6(double (&a)[21], const double (&b)[6], double (&x)[6]) {
   double rd[6];  // 1 / D[j]
@@ -437,22 +517,20 @@ __device__ __forceinline__ bool ldlt6(double (&a)[21], const double (&b)[6], dou
   // every loop has a constant trip count and unrolls completely
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    double s = a[tri(j, j)];
+    if (!(fabs(a[tri(j, j)]) > 0.0)) return false;
+    rd[j] = 1.0 / a[tri(j, j)];
+    double l[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-      if (k < j) s -= a[tri(j, k)] * a[tri(j, k)] * a[tri(k, k)];
-    a[tri(j, j)] = s;
-    if (!(fabs(s) > 0.0)) return false;
-    rd[j] = 1.0 / s;
+    for (int i = 0; i < 6; ++i)
+      if (i > j) l[i] = a[tri(i, j)] * rd[j];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      if (i <= j) continue;
-      double t = a[tri(i, j)];
+    for (int i = 0; i < 6; ++i)
 #pragma unroll
       for (int k = 0; k < 6; ++k)
-        if (k < j) t -= a[tri(i, k)] * a[tri(j, k)] * a[tri(k, k)];
-      a[tri(i, j)] = t * rd[j];
-    }
+        if (k > j && k <= i) a[tri(i, k)] = fma(-l[i], a[tri(k, j)], a[tri(i, k)]);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      if (i > j) a[tri(i, j)] = l[i];
   }
   double y[6];
 #pragma unroll
@@ -460,7 +538,7 @@ __device__ __forceinline__ bool ldlt6(double (&a)[21], const double (&b)[6], dou
     double t = b[i];
 #pragma unroll
     for (int k = 0; k < 6; ++k)
-      if (k < i) t -= a[tri(i, k)] * y[k];
+      if (k < i) t = fma(-a[tri(i, k)], y[k], t);
     y[i] = t;
   }
 #pragma unroll
@@ -469,8 +547,8 @@ __device__ __forceinline__ bool ldlt6(double (&a)[21], const double (&b)[6], dou
   for (int i = 5; i >= 0; --i) {
     double t = y[i];
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-      if (k > i) t -= a[tri(k, i)] * x[k];
+    for (int k = 5; k >= 0; --k)
+      if (k > i) t = fma(-a[tri(k, i)], x[k], t);
     x[i] = t;
   }
   return true;
@@ -479,17 +557,34 @@ __device__ __forceinline__ bool ldlt6(double (&a)[21], const double (&b)[6], dou
 // exp of the twist matrix v2t(xi) (gnSolver.cu:443-455): rotation by
 // Rodrigues' formula and translation through the SE(3) left Jacobian,
 // R = I + a W + b W^2, t = (I + b W + c W^2) v, with a = sin t / t,
-// b = (1 - cos t)/t^2, c = (t - sin t)/t^3 (Taylor below t = 1e-4).
+// b = (1 - cos t)/t^2, c = (t - sin t)/t^3.  Up to half a radian they are
+// their Taylor series in t^2 to the eighth term (the rest is below 1e-19 of
+// the value; the closed forms lose digits to cancellation there, and their
+// square root, sine, cosine and divisions are a serial chain between every two
+// ICP iterations).
 __device__ __forceinline__ void se3_exp(const double* xi, double* T) {
   double w0 = xi[0], w1 = xi[1], w2 = xi[2];
-  double th2 = w0 * w0 + w1 * w1 + w2 * w2, th = sqrt(th2);
+  double th2 = w0 * w0 + w1 * w1 + w2 * w2;
   double a, b, c;
-  if (th < 1e-4) {
-    a = 1.0 - th2 / 6.0;
-    b = 0.5 - th2 / 24.0;
-    c = 1.0 / 6.0 - th2 / 120.0;
+  if (th2 < 0.25) {
+    // 1 / n! for n = 1 .. 17
+    const double f[18] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040,
+                          1.0 / 40320, 1.0 / 362880, 1.0 / 3628800, 1.0 / 39916800,
+                          1.0 / 479001600, 1.0 / 6227020800.0, 1.0 / 87178291200.0,
+                          1.0 / 1307674368000.0, 1.0 / 20922789888000.0,
+                          1.0 / 355687428096000.0};
+    a = f[15];
+    b = f[16];
+    c = f[17];
+#pragma unroll
+    for (int k = 6; k >= 0; --k) {
+      a = fma(-a, th2, f[2 * k + 1]);
+      b = fma(-b, th2, f[2 * k + 2]);
+      c = fma(-c, th2, f[2 * k + 3]);
+    }
   } else {
     double sn, cs;
+    const double th = sqrt(th2);
     sincos(th, &sn, &cs);
     a = sn / th;
     b = (1.0 - cs) / th2;
@@ -607,7 +702,7 @@ __device__ bool gn_update(const double* acc, const IcpParams& P, int it, double*
   for (int k = 0; k < 6; ++k) b[k] *= scaling;
 #pragma unroll
   for (int k = 0; k < 21; ++k) a[k] *= scaling;
-  const double mx2 = max21(a);
+  const double mx2 = mx * scaling;  // the scaled entries' maximum (rounding is monotone)
   const double alpha = (double)P.reg * mx2;
 #pragma unroll
   for (int k = 0; k < 6; ++k) a[tri(k, k)] += alpha / (double)it;
@@ -632,65 +727,104 @@ __device__ bool gn_update(const double* acc, const IcpParams& P, int it, double*
   return conv;
 }
 
-// Blocks of a level's chained reduction: one per tile, at most
-// kIcpMaxBlocks (a block then takes several tiles).
-inline __host__ __device__ int icp_grid(int n) {
-  int g = icp_tiles(n);
+// Blocks of the stage entry points' reduction: about 256, 512 or 1024 pixels
+// each, at most kIcpMaxBlocks (a block then strides).
+inline __host__ __device__ int icp_stage_grid(int n) {
+  const int t = n <= 8192 ? 256 : (n <= 65536 ? 512 : 1024);
+  int g = (n + t - 1) / t;
   if (g > kIcpMaxBlocks) g = kIcpMaxBlocks;
   if (g < 1) g = 1;
   return g;
 }
 
-// The partial sums of tile 'tile' of level L into row[0..28]: each thread
-// accumulates its pixels (tile * tile_px + threadIdx.x + m * 256) in
-// FP32, the block adds them in FP64 in a fixed order.  Every thread of the
-// block calls it; 'red' is the block's shared scratch.
+// Part 'part' (of nw) of tile 'tile' of level L, slots part * 32 + lane + m * 512
+// of the tile, by one warp, added in a fixed order into red[0..28] (shared).  The
+// compensated form's warp totals move into compensated pairs, one value per
+// lane, after every slot's pixels.
 template <bool KAHAN>
-__device__ inline void tile_partial(const IcpLevel& L, const IcpParams& P, const M4f& T,
-                                    int tile, double* red, double* __restrict__ row) {
+__device__ inline void tile_warp_sum(const FrameLevel& L, const M4f& T, int tile, int part,
+                                     double* red) {
+  const int lane = threadIdx.x & 31;
+  const int end = min(L.slots, (tile + 1) * L.tile), first = tile * L.tile + part * 32 + lane;
   Acc a;
+  if (KAHAN) {
+    const int group = L.group;
+    LaneSum l;
+    l.s = l.c = 0.0f;
+    // (whole warps: slots come in runs of 256)
+    for (int g = first; g < end; g += kIcpFrameThreads) {
+      const int i = (g >> 8) * group * 256 + (g & 255);
 #pragma unroll
-  for (int k = 0; k < kIcpVals; ++k) {
-    a.v[k] = 0.0f;
-    a.d[k] = 0.0;
+      for (int k = 0; k < kIcpVals; ++k) a.v[k] = 0.0f;
+#pragma unroll 1
+      for (int m = 0; m < group; m += 2)  // (a group of one: its second pixel is out)
+        pixel_group<2>(L, T, i + m * 256, 256, group > 1 ? L.n : min(L.n, i + 1), a);
+      const LaneSum w = warp_reduce<KAHAN>(a);
+      pair_add(l.s, l.c, w.s, w.c);
+    }
+    if (lane < kIcpVals) red[lane] = pack_pair(l.s, l.c);
+  } else {  // FP64 sums hold most registers: one pixel at a time
+#pragma unroll
+    for (int k = 0; k < kIcpVals; ++k) a.d[k] = 0.0;
+    for (int i = first; i < end; i += kIcpFrameThreads) pixel_terms<KAHAN>(L, L.P, T, i, a);
+    __syncwarp();
+    const LaneSum w = warp_reduce<KAHAN>(a);
+    if (lane < kIcpVals) red[lane] = w.d;
   }
-  const int n = L.s.rows * L.s.cols;
-  const int tpx = icp_tile_px(n);
-  const int base = tile * tpx + (int)threadIdx.x;
-  if (tpx == kIcpThreads) {
-    if (base < n) pixel_terms<KAHAN>(L, P, T, base, a);
-  } else if (!KAHAN) {  // FP64 sums hold most registers: one pixel at a time
-    for (int m = 0; m < tpx / kIcpThreads; ++m)
-      if (base + m * kIcpThreads < n) pixel_terms<KAHAN>(L, P, T, base + m * kIcpThreads, a);
-  } else {
-    for (int m = 0; m < tpx / kIcpThreads; m += 2)
-      pixel_pair<KAHAN>(L, P, T, base + m * kIcpThreads, base + (m + 1) * kIcpThreads, n, a);
-  }
-  block_reduce<KAHAN>(a, red);
-  if (threadIdx.x < kIcpVals) row[threadIdx.x] = red[threadIdx.x];
-  __syncthreads();  // red is reused by the next tile
 }
 
-// The level's total (tiles in index order), the iteration's statistics, the
-// GN update and the next transform, for a solver state held at st_* (global
-// memory in the chained kernels, shared memory in the persistent one).
-// tot[] must be shared; the update runs on thread 0.
+// The partial sums of the block's tiles first, first + step, ... of level L,
+// each value handed to put(tile, k, value).  The warps go through up to
+// kTileBatch tiles on their own (their loads' latencies overlap: a block of
+// few warps and many tiles waits on nothing else) before the block adds their
+// parts, in warp order.  Every thread of the block calls it; red: kTileBatch x
+// 16 x 29.
+constexpr int kTileBatch = 8;
+template <bool KAHAN, class Put>
+__device__ inline void tile_partials(const FrameLevel& L, const M4f& T, int first, int step,
+                                     double* red, Put&& put) {
+  const int warp = threadIdx.x >> 5, lg = L.parts_log2, ntiles = L.ntiles;
+  for (int t0 = first; t0 < ntiles; t0 += kTileBatch * step) {
+    int m = 1;  // tiles of this batch
+    while (m < kTileBatch && t0 + m * step < ntiles) ++m;
+#pragma unroll 1
+    for (int p = warp; p < m << lg; p += kFrameWarps) {  // each tile's parts in order
+      const int u = p >> lg, part = p - (u << lg);
+      tile_warp_sum<KAHAN>(L, T, t0 + u * step, part, red + (u * kFrameWarps + part) * kIcpVals);
+    }
+    __syncthreads();
+    // (a value per thread, a tile per warp)
+    const int k = threadIdx.x & 31;
+    if (warp < m && k < kIcpVals)
+      put(t0 + warp * step, k,
+          add_warps<KAHAN, kFrameWarps>(red + warp * kFrameWarps * kIcpVals + k, 1 << lg));
+    if (t0 + kTileBatch * step < ntiles) __syncthreads();  // red is reused
+  }
+}
+
+// The iteration's GN update and the next transform from the rows' values v
+// (level_total), for a solver state held at st_* (global memory in the chained
+// kernels, shared memory in the persistent one), and its statistics.  tot[]
+// must be shared; the update runs on thread 0, then the statistics on another
+// warp.
 template <bool KAHAN>
-__device__ inline void level_update(const double* __restrict__ partials, int ntiles,
-                                    const IcpParams& P, int pl, int it, double* tot, double* red,
-                                    double* st_inc, double* st_prev, float* st_T,
-                                    int* st_converged, int* st_iters, int* st_inliers,
-                                    float* st_rms) {
-  final_reduce<KAHAN>(partials, ntiles, tot, red);
+__device__ inline void level_update(const double (&v)[kWarpRows], const IcpParams& P, int pl,
+                                    int it, double* tot, double* red, double* st_inc,
+                                    double* st_prev, float* st_T, int* st_converged,
+                                    int* st_iters, int* st_inliers, float* st_rms) {
+  level_total<KAHAN>(v, tot, red);
   if (threadIdx.x == 0) {
-    st_iters[pl] = it;
-    st_inliers[pl] = (int)tot[28];
-    st_rms[pl] = tot[28] > 0 ? (float)sqrt(tot[27] / tot[28]) : 0.0f;
     const bool conv = gn_update(tot, P, it, st_inc, st_prev);
     *st_converged = conv ? 1 : 0;
     double Td[16];
     se3_exp(st_inc, Td);
     for (int k = 0; k < 16; ++k) st_T[k] = (float)Td[k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 32) {
+    st_iters[pl] = it;
+    st_inliers[pl] = (int)tot[28];
+    st_rms[pl] = tot[28] > 0 ? (float)sqrt(tot[27] / tot[28]) : 0.0f;
   }
 }
 
@@ -698,10 +832,10 @@ __device__ inline void level_update(const double* __restrict__ partials, int nti
 // 'nb' blocks: the partial sums of the block's tiles, then -- in the last
 // block to finish -- the FP64 total and the GN update (gnSolver.cu:379-415).
 template <bool KAHAN>
-__device__ inline void icp_iteration_body(const IcpLevel& L, const IcpParams& P, int pl, int it,
-                                          IcpState* st, double* __restrict__ partials, int bid,
+__device__ inline void icp_iteration_body(const FrameLevel& L, int pl, int it, IcpState* st,
+                                          double* __restrict__ partials, int bid,
                                           int nb) {
-  __shared__ double red[(kIcpThreads / 32) * kIcpVals];
+  __shared__ double red[kTileBatch * kFrameWarps * kIcpVals];
   __shared__ M4f Ts;
   __shared__ int skip;
   if (threadIdx.x == 0) {
@@ -712,9 +846,9 @@ __device__ inline void icp_iteration_body(const IcpLevel& L, const IcpParams& P,
   __syncthreads();
   if (skip) return;
   // the transform stays in shared memory (registers go to the sums)
-  const int ntiles = icp_tiles(L.s.rows * L.s.cols);
-  for (int tile = bid; tile < ntiles; tile += nb)
-    tile_partial<KAHAN>(L, P, Ts, tile, red, partials + (size_t)tile * kIcpVals);
+  tile_partials<KAHAN>(L, Ts, bid, nb, red, [&](int tile, int k, double x) {
+    partials[(size_t)tile * kIcpVals + k] = x;
+  });
   __threadfence();
   __shared__ unsigned int ticket;
   if (threadIdx.x == 0) ticket = atomicAdd(&st->ticket, 1u);
@@ -722,8 +856,14 @@ __device__ inline void icp_iteration_body(const IcpLevel& L, const IcpParams& P,
   if (ticket != (unsigned)nb - 1) return;
   __threadfence();
   __shared__ double tot[kIcpVals];
-  level_update<KAHAN>(partials, ntiles, P, pl, it, tot, red, st->inc, st->prev, st->T,
-                      &st->converged, st->iters, st->inliers, st->rms);
+  double v[kWarpRows];
+#pragma unroll
+  for (int i = 0; i < kWarpRows; ++i) {  // every row's load in flight at once
+    const int b = (threadIdx.x >> 5) + i * kFrameWarps, k = threadIdx.x & 31;
+    v[i] = (b < L.ntiles && k < kIcpVals) ? __ldcg(partials + (size_t)b * kIcpVals + k) : 0.0;
+  }
+  level_update<KAHAN>(v, L.P, pl, it, tot, red, st->inc, st->prev, st->T, &st->converged, st->iters,
+                      st->inliers, st->rms);
   if (threadIdx.x == 0) st->ticket = 0;
 }
 
@@ -739,8 +879,8 @@ __device__ inline void release_successor() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-__device__ inline IcpLevel level_of(const SessDev& S, int l) {
-  IcpLevel L;
+__device__ inline FrameLevel level_of(const SessDev& S, int l) {
+  FrameLevel L;
   L.sd = S.sdep[l];
   L.sn = S.snrm[l];
   L.si = S.sint[l];
@@ -748,6 +888,14 @@ __device__ inline IcpLevel level_of(const SessDev& S, int l) {
   L.tn = S.tnrm[l];
   L.ti = S.tint[l];
   L.s = S.ls[l];
+  L.n = L.s.rows * L.s.cols;
+  const int kahan = S.icpp.kahan;
+  L.group = icp_group(L.n);
+  L.slots = icp_slots(L.n, kahan);
+  L.tile = icp_tile_slots(L.n, kahan);
+  L.ntiles = icp_tiles(L.n, kahan);
+  L.parts_log2 = L.tile >= kIcpFrameThreads ? 4 : 3;
+  L.P = S.icpp;
   return L;
 }
 
@@ -755,33 +903,50 @@ __device__ inline IcpLevel level_of(const SessDev& S, int l) {
 // only the blocks of its own grid.  One instantiation per summation kind;
 // sessions of the other kind return.
 template <bool KAHAN>
-__global__ void __launch_bounds__(kIcpThreads, 2)
+__global__ void __launch_bounds__(kIcpFrameThreads, 1)
     fused_icp_iteration_kernel(const SessDev* __restrict__ tab, int pl, int it) {
   const SessDev& S = tab[blockIdx.z];
   if ((S.icpp.kahan != 0) != KAHAN) return;
   if (it >= S.slot_iters[pl]) return;  // the reference runs iterations 1 .. N-1
   const int l = S.slot_level[pl];
-  const int nb = icp_grid(S.ls[l].rows * S.ls[l].cols);
+  const int nb = icp_tiles(S.ls[l].rows * S.ls[l].cols, KAHAN);
   if ((int)blockIdx.x >= nb) return;
-  __shared__ IcpLevel L;  // shared: registers go to the sums
+  __shared__ FrameLevel L;  // shared: registers go to the sums
   if (threadIdx.x == 0) L = level_of(S, l);
   wait_predecessor();  // the solver state and partials of the previous iteration
   release_successor();
-  icp_iteration_body<KAHAN>(L, S.icpp, pl, it, S.icp, S.partials, blockIdx.x, nb);
+  icp_iteration_body<KAHAN>(L, pl, it, S.icp, S.partials, blockIdx.x, nb);
 }
 
 // ---- the persistent form: one launch walks every level and iteration
 //
-// A cooperative launch (all blocks resident at once) over the table: each
-// session owns a run of blocks (icp_share: about its share of the tiles),
-// every block keeps its session's solver state in shared memory, and one
-// grid-wide barrier per iteration separates the tiles' partial sums from
-// their use: after it, every block of the session adds the partials (the
-// same sums, in the same order, so every block holds the same state) and
-// runs the GN update itself -- no second barrier.  Iterations alternate
-// between two rows of partials, so a block may start the next iteration's
-// tiles while another still reads this one's.  The results are those of the
-// chained kernels bit for bit (the same tiles, summed in the same order).
+// A cooperative launch (all blocks resident at once, one per SM) over the
+// table: each session owns a run of blocks (icp_share: its share of the
+// work), every block keeps its session's solver state in shared memory, sums
+// its tiles, and then waits for the rows of the level's other tiles, adds them
+// (the same sums, in the same order, so every block holds the same state) and
+// runs the GN update itself.
+//
+// There is no barrier: a row is 29 doubles as tagged words {32 data bits, tag},
+// written and read as single 64-bit accesses, and a reader polls the rows
+// themselves until they carry the iteration's tag -- one store's and one
+// load's way through L2 between two blocks, with no fence (whose acquire side
+// also empties L1, where the images stay from iteration to iteration).
+// Iterations alternate between two rows per tile: a block writes its row of an
+// iteration only after reading every row of the one before, so the rows it
+// overwrites have been read.  Blocks without a tile of a level wait for the
+// state that the session's first block leaves at the level's end; those
+// without a tile of a later level return.
+//
+// The coarse levels are a chain of latencies, about six iterations of a
+// frame's nine: the block's sums 2,500 (sky) to 6,000 cycles, the rows 2,000,
+// the 6x6 solve 3,000; a finest iteration of 640x480 is 22,000 and 8,000.
+// Live ICP stage, before (256-thread blocks, 300 rows that every block read, a
+// hub block's barrier over the whole table, a square root, sine and cosine per
+// update) -> now: 640x480 FP32 132 -> 85 us, mixed 112 -> 94, 1280x720 band
+// 123 -> 101, 320x240 FP32 97 -> 66, 32-session band batch in one group 460 ->
+// 408.  A barrier of one counter instead of the tagged rows measured 88, 91,
+// 96, 68 and 396; finishing the pose in this kernel 4 us more than in its own.
 
 // Current value of the GPU's nanosecond timer.
 __device__ inline unsigned long long global_ns() {
@@ -790,200 +955,306 @@ __device__ inline unsigned long long global_ns() {
   return t;
 }
 
-// Grid-wide barrier number k (1, 2, ...) of a launch of 'nb' blocks (the
-// grid) whose barrier words (kIcpBarWords, zero at launch) are 'bar'.
-// Arrivals and releases are spread over kIcpBarSpread counters and flags,
-// each on its own 128-byte line: block b adds one to counter
-// b % kIcpBarSpread; block 0 alone polls the counters (one thread each)
-// until each holds k times its blocks, then writes k to every release
-// flag; block b polls flag b % kIcpBarSpread.  So no line takes
-// more than a few dozen blocks' polls beside the arrivals it counts.  Every
-// wait is bounded: after kBarrierWaitNs (or once the abort word is raised)
-// the block gives up, raises the abort word and returns false.
-constexpr unsigned long long kBarrierWaitNs = 500000000ull;  // half a second
-__device__ inline unsigned* bar_counter(unsigned* bar, int i) { return bar + 32 * i; }
-__device__ inline unsigned* bar_flag(unsigned* bar, int i) {
-  return bar + 32 * (kIcpBarSpread + i);
-}
-__device__ inline int* bar_abort(unsigned* bar) {
-  return reinterpret_cast<int*>(bar + 32 * (2 * kIcpBarSpread));
-}
-__device__ inline bool grid_barrier(unsigned* bar, unsigned k, unsigned nb) {
-  __shared__ int ok;
-  const unsigned me = blockIdx.x;
-  int* abort = bar_abort(bar);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // this block's partial sums before its arrival
-    atomicAdd(bar_counter(bar, (int)(me % kIcpBarSpread)), 1u);
+// A wait's bound: expired() after kWaitNs, or once the abort word is raised
+// (looked at every 64th try); it raises the word.
+constexpr unsigned long long kWaitNs = 500000000ull;  // half a second
+struct BoundedWait {
+  unsigned n = 0;
+  unsigned long long t0 = 0;
+  __device__ bool expired(unsigned* abort_word) {
+    if ((++n & 63u) != 0) return false;
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    if (*(volatile unsigned*)abort_word == 0 && t - t0 <= kWaitNs) return false;
+    atomicExch(abort_word, 1u);
+    return true;
   }
-  if (me == 0) {  // block 0: threads 0 .. kIcpBarSpread-1 poll one counter each
-    int good = 1;
-    if (threadIdx.x < kIcpBarSpread) {
-      const unsigned want =
-          k * ((nb + kIcpBarSpread - 1 - threadIdx.x) / kIcpBarSpread);
-      volatile unsigned* c = bar_counter(bar, (int)threadIdx.x);
-      const unsigned long long t0 = global_ns();
-      while (*c < want) {
-        if (*(volatile int*)abort || global_ns() - t0 > kBarrierWaitNs) {
-          good = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
-      __threadfence();  // the arrivals' partial sums before the release
-    }
-    good = __syncthreads_and(good);
-    if (threadIdx.x == 0) {
-      if (good)
-        for (int i = 0; i < kIcpBarSpread; ++i) *(volatile unsigned*)bar_flag(bar, i) = k;
-      else
-        atomicExch(abort, 1);
-      ok = good;
-    }
-  } else if (threadIdx.x == 0) {
-    volatile unsigned* flag = bar_flag(bar, (int)(me % kIcpBarSpread));
-    const unsigned long long t0 = global_ns();
-    int good = 1;
-    while (*flag < k) {
-      if (*(volatile int*)abort || global_ns() - t0 > kBarrierWaitNs) {
-        good = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    if (!good) atomicExch(abort, 1);
-    __threadfence();  // the other blocks' partial sums after the release
-    ok = good;
-  }
-  __syncthreads();
-  return ok != 0;
+};
+
+__device__ inline uint2 load_word(const uint2* p) {
+  unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+  return make_uint2((unsigned)w, (unsigned)(w >> 32));
+}
+__device__ inline void store_word(uint2* p, unsigned data, unsigned tag) {
+  const unsigned long long w = ((unsigned long long)tag << 32) | data;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+// Value k of a row: words k and 32 + k.
+__device__ inline void put_value(uint2* row, int k, double x, unsigned tag) {
+  store_word(row + k, (unsigned)__double2loint(x), tag);
+  store_word(row + 32 + k, (unsigned)__double2hiint(x), tag);
 }
 
-// Blocks of a session in a persistent launch of 'budget' blocks over a table
-// whose sessions have sum_tiles level-0 tiles in all.
-__host__ __device__ inline int icp_share(int tiles, long long sum_tiles, int budget) {
-  long long b = (long long)budget * tiles / (sum_tiles > 0 ? sum_tiles : 1);
+// Lane k's values of this warp's rows (w, w + 16, ... below ntiles) once they
+// carry 'tag'; false when the wait ran out.  All rows are asked for at once,
+// then those that are not there yet again.
+__device__ inline bool wait_rows(const uint2* rows, int ntiles, unsigned tag,
+                                 unsigned* abort_word, double (&v)[kWarpRows]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned missing = 0;
+#pragma unroll
+  for (int i = 0; i < kWarpRows; ++i) {
+    v[i] = 0.0;
+    if (w + i * kFrameWarps < ntiles) missing |= 1u << i;
+  }
+  BoundedWait wait;
+  while (missing) {
+    uint2 lo[kWarpRows], hi[kWarpRows];
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i)
+      if (missing >> i & 1u) {
+        const uint2* r = rows + (size_t)(w + i * kFrameWarps) * kIcpRowWords + lane;
+        lo[i] = load_word(r);
+        hi[i] = load_word(r + 32);
+      }
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i)
+      if (missing >> i & 1u) {
+        const bool here = lane >= kIcpVals || (lo[i].y == tag && hi[i].y == tag);
+        if (__all_sync(0xffffffffu, here)) {
+          missing &= ~(1u << i);
+          if (lane < kIcpVals) v[i] = __hiloint2double((int)hi[i].x, (int)lo[i].x);
+        }
+      }
+    if (missing && __any_sync(0xffffffffu, lane == 0 && wait.expired(abort_word))) return false;
+  }
+  return true;
+}
+
+// The persistent kernel's per-block solver state.
+struct FrameState {
+  double tot[kIcpVals];
+  double inc[6], prev[6];
+  M4f T;  // the transform of the iteration
+  int conv, have, par, iters[3], inliers[3];
+  float rms[3];
+  unsigned epoch;
+};
+
+// The rows of the level, then the iteration's update; false when the wait ran
+// out (block-uniform).  Out of line: its registers are not the sums'.
+template <bool KAHAN>
+__device__ __noinline__ bool finish_iteration(const uint2* rows, const FrameLevel& L,
+                                              unsigned tag, unsigned* abort_word, int pl, int it,
+                                              FrameState& F, double* red) {
+  double v[kWarpRows];
+  const bool good = wait_rows(rows, L.ntiles, tag, abort_word, v);
+  if (!__syncthreads_and(good)) return false;
+  level_update<KAHAN>(v, L.P, pl, it, F.tot, red, F.inc, F.prev, F.T.m, &F.conv, F.iters,
+                      F.inliers, F.rms);
+  return true;
+}
+
+// Blocks of a session of npx pixels in a persistent launch of 'budget' blocks
+// over a table whose sessions weigh 'sum' in all.
+__host__ __device__ inline int icp_share(int npx, int kahan, long long sum, int budget) {
+  const int tiles = icp_tiles(npx, kahan);
+  long long b = (long long)budget * icp_weight(npx, kahan) / (sum > 0 ? sum : 1);
   if (b > tiles) b = tiles;
   if (b < 1) b = 1;
   return (int)b;
 }
 
+// This block's session among the table's sessions of its kind, its index
+// among the session's blocks and their number, in shared memory (out[3]).
+template <bool KAHAN>
+__device__ inline void find_session(const SessDev* __restrict__ tab, int n, int budget, int* out) {
+  __shared__ long long sum_s;
+  __shared__ int part[kFrameWarps], carry;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    sum_s = 0;
+    carry = 0;
+    out[0] = out[1] = out[2] = 0;
+  }
+  __syncthreads();
+  long long mine = 0;
+  for (int j = tid; j < n; j += kIcpFrameThreads)
+    if ((tab[j].icpp.kahan != 0) == KAHAN) mine += icp_weight(tab[j].npx, KAHAN);
+  if (mine) atomicAdd(reinterpret_cast<unsigned long long*>(&sum_s), (unsigned long long)mine);
+  __syncthreads();
+  for (int j0 = 0; j0 < n; j0 += kIcpFrameThreads) {
+    const int j = j0 + tid;
+    int b = 0;
+    if (j < n && (tab[j].icpp.kahan != 0) == KAHAN) b = icp_share(tab[j].npx, KAHAN, sum_s, budget);
+    int sum = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += u;
+    }
+    if (lane == 31) part[warp] = sum;
+    __syncthreads();
+    int before = carry;
+    for (int w = 0; w < warp; ++w) before += part[w];
+    const int first = before + sum - b;
+    if (b > 0 && (int)blockIdx.x >= first && (int)blockIdx.x < first + b) {
+      out[0] = j;
+      out[1] = (int)blockIdx.x - first;
+      out[2] = b;
+    }
+    __syncthreads();
+    if (tid == kIcpFrameThreads - 1) carry = before + sum;
+    __syncthreads();
+  }
+}
+
 // One instantiation per summation kind: a table whose sessions sum both
 // ways gets one launch per kind, each over that kind's sessions only.
 template <bool KAHAN>
-__global__ void __launch_bounds__(kIcpThreads, 2)
+__global__ void __launch_bounds__(kIcpFrameThreads, 1)
     fused_icp_persistent_kernel(const SessDev* __restrict__ tab, int n, int budget,
-                                int it0, int it1, int it2, unsigned* __restrict__ bar) {
-  // this block's session and its index among the session's blocks
-  __shared__ int z_s, local_s, nblk_s;
-  if (threadIdx.x == 0) {
-    long long sum = 0;
-    for (int j = 0; j < n; ++j)
-      if ((tab[j].icpp.kahan != 0) == KAHAN) sum += icp_tiles(tab[j].npx);
-    int first = 0, z = n - 1, nb = 1;
-    for (int j = 0; j < n; ++j) {
-      if ((tab[j].icpp.kahan != 0) != KAHAN) continue;
-      nb = icp_share(icp_tiles(tab[j].npx), sum, budget);
-      if ((int)blockIdx.x < first + nb) {
-        z = j;
-        break;
-      }
-      first += nb;
+                                int it0, int it1, int it2) {
+  // this block's session, its index among the session's blocks, their number
+  __shared__ int who[3];
+  if (n == 1) {
+    if (threadIdx.x == 0) {
+      who[0] = 0;
+      who[1] = blockIdx.x;
+      who[2] = gridDim.x;
     }
-    z_s = z;
-    local_s = (int)blockIdx.x - first;
-    nblk_s = nb;
+    __syncthreads();
+  } else {
+    find_session<KAHAN>(tab, n, budget, who);
   }
-  __syncthreads();
-  const SessDev& S = tab[z_s];
-  const int local = local_s, nblk = nblk_s;
-  const bool own = local >= 0 && local < nblk;  // spare blocks only pass the barriers
+  const SessDev& S = tab[who[0]];
+  const int local = who[1], nblk = who[2];
+  if (nblk == 0) return;  // (the grid is the sum of the shares)
   // the session's solver state, one copy per block
-  __shared__ double red[(kIcpThreads / 32) * kIcpVals];
-  __shared__ double tot[kIcpVals];
-  __shared__ double inc[6], prev[6];
-  __shared__ M4f Tm;                      // the transform of the iteration
-  __shared__ IcpLevel Ls;                 // the iteration's level
-  float* const Tf = Tm.m;
-  __shared__ int conv, have, iters[3], inliers[3];
-  __shared__ float rms[3];
+  __shared__ double red[kTileBatch * kFrameWarps * kIcpVals];
+  __shared__ FrameState F;
+  __shared__ FrameLevel Ls;  // the iteration's level
+  float* const Tf = F.T.m;
   if (threadIdx.x < 6) {
-    inc[threadIdx.x] = S.icp->inc[threadIdx.x];
-    prev[threadIdx.x] = S.icp->prev[threadIdx.x];
+    F.inc[threadIdx.x] = S.icp->inc[threadIdx.x];
+    F.prev[threadIdx.x] = S.icp->prev[threadIdx.x];
   }
   if (threadIdx.x < 16) Tf[threadIdx.x] = S.icp->T[threadIdx.x];
   if (threadIdx.x < 3) {
-    iters[threadIdx.x] = S.icp->iters[threadIdx.x];
-    inliers[threadIdx.x] = S.icp->inliers[threadIdx.x];
-    rms[threadIdx.x] = S.icp->rms[threadIdx.x];
+    F.iters[threadIdx.x] = S.icp->iters[threadIdx.x];
+    F.inliers[threadIdx.x] = S.icp->inliers[threadIdx.x];
+    F.rms[threadIdx.x] = S.icp->rms[threadIdx.x];
   }
   if (threadIdx.x == 0) {
-    conv = S.icp->converged;
-    have = S.icp->have_target;
+    F.conv = S.icp->converged;
+    F.have = S.icp->have_target;
+    F.par = 0;
+    F.epoch = S.icp_bar[0];
   }
   __syncthreads();
   const int maxit[3] = {it0, it1, it2};
-  const size_t row = (size_t)icp_tiles(S.npx) * kIcpVals;
-  unsigned nbar = 0;
-  int parity = 0;
+  const unsigned epoch = F.epoch;
+  unsigned* const abort_word = S.icp_bar + kIcpAbort;
+  uint2* const rows =
+      reinterpret_cast<uint2*>(reinterpret_cast<char*>(S.partials) + icp_rows_offset());
+  // the last level this block has a tile of
+  int last = -1;
   for (int pl = 0; pl < 3; ++pl)
-    for (int it = 1; it < maxit[pl]; ++it) {
-      const bool sess_active = it < S.slot_iters[pl] && have && !(it > 1 && conv);
-      // a lone session's blocks all hold its state: once it has converged
-      // (or has no target) they skip the level's remaining barriers together
-      if (n == 1 && !sess_active) continue;
-      const bool active = own && sess_active;
-      const int l = S.slot_level[pl];
-      const int ntiles = icp_tiles(S.ls[l].rows * S.ls[l].cols);
-      double* part = S.partials + (size_t)parity * row;
-      if (active) {
-        // level and transform stay in shared memory (registers go to the sums)
-        if (threadIdx.x == 0) Ls = level_of(S, l);
-        __syncthreads();
-        for (int tile = local; tile < ntiles; tile += nblk)
-          tile_partial<KAHAN>(Ls, S.icpp, Tm, tile, red, part + (size_t)tile * kIcpVals);
+    if (min(maxit[pl], S.slot_iters[pl]) > 1 &&
+        local < icp_tiles(S.ls[S.slot_level[pl]].rows * S.ls[S.slot_level[pl]].cols, KAHAN))
+      last = pl;
+  if (local == 0) last = 2;
+  bool good = true;
+  for (int pl = 0; pl <= last; ++pl) {
+    const int l = S.slot_level[pl], iters_pl = min(maxit[pl], S.slot_iters[pl]);
+    if (!F.have || iters_pl <= 1) continue;  // (alike in every block of the session)
+    const int ntiles = icp_tiles(S.ls[l].rows * S.ls[l].cols, KAHAN);
+    const unsigned tag0 = epoch + (unsigned)pl * 1024u;  // iterations 1 .. 999, then the state
+    uint2* const state = rows + (size_t)(2 * kIcpMaxTiles + pl) * kIcpRowWords;
+    if (local < ntiles) {
+      // level and transform stay in shared memory (registers go to the sums)
+      if (threadIdx.x == 0) Ls = level_of(S, l);
+      __syncthreads();
+      int parity = F.par;
+      for (int it = 1; it < iters_pl; ++it) {
+        // every block at the level holds the state: they leave it together
+        if (it > 1 && F.conv) break;
+        uint2* const part = rows + (size_t)parity * kIcpMaxTiles * kIcpRowWords;
+        const unsigned tag = tag0 + (unsigned)it;
+        tile_partials<KAHAN>(Ls, F.T, local, nblk, red,
+                             [&](int tile, int k, double x) {
+                               put_value(part + (size_t)tile * kIcpRowWords, k, x, tag);
+                             });
+        good = finish_iteration<KAHAN>(part, Ls, tag, abort_word, pl, it, F, red);
+        if (!good) break;
+        parity ^= 1;
       }
-      ++nbar;
-      if (!grid_barrier(bar, nbar, gridDim.x)) {
-        if (threadIdx.x == 0) atomicExch(&S.vol.cnt->icp_timeout, 1);
-        return;
+      if (!good) break;  // (block-uniform)
+      __syncthreads();
+      if (threadIdx.x == 0) F.par = parity;
+      if (local == 0 && nblk > ntiles) {  // for the blocks without a tile here
+        const unsigned tag = tag0 + 1023u;
+        const int k = threadIdx.x;
+        if (k < 12) put_value(state, k, k < 6 ? F.inc[k] : F.prev[k - 6], tag);
+        else if (k < 28) store_word(state + k, __float_as_uint(Tf[k - 12]), tag);
+        else if (k == 28) store_word(state + 28, (unsigned)parity, tag);
       }
-      if (active) {
-        level_update<KAHAN>(part, ntiles, S.icpp, pl, it, tot, red, inc, prev, Tf, &conv, iters,
-                            inliers, rms);
-        __syncthreads();
+      __syncthreads();
+    } else {
+      if (threadIdx.x < 32) {
+        const unsigned tag = tag0 + 1023u;
+        const int k = threadIdx.x;
+        uint2 a = make_uint2(0u, 0u), b = a;
+        BoundedWait wait;
+        for (;;) {
+          bool here = true;
+          if (k < 29) {
+            a = load_word(state + k);
+            here = a.y == tag;
+          }
+          if (k < 12) {
+            b = load_word(state + 32 + k);
+            here = here && b.y == tag;
+          }
+          if (__all_sync(0xffffffffu, here)) break;
+          if (__any_sync(0xffffffffu, k == 0 && wait.expired(abort_word))) {
+            good = false;
+            break;
+          }
+          __nanosleep(200);  // (leave L2 to the level's blocks)
+        }
+        if (k < 12) (k < 6 ? F.inc[k] : F.prev[k - 6]) = __hiloint2double((int)b.x, (int)a.x);
+        else if (k < 28) Tf[k - 12] = __uint_as_float(a.x);
+        else if (k == 28) F.par = (int)a.x;
       }
-      parity ^= 1;
+      if (!__syncthreads_and(good)) {
+        good = false;
+        break;
+      }
     }
-  // the session's first block hands the state on (pose finalisation)
-  if (own && local == 0) {
+  }
+  if (!good && threadIdx.x == 0) atomicExch(&S.vol.cnt->icp_timeout, 1);
+  __syncthreads();
+  // the session's first block hands the state on to the pose finalisation
+  // (after a timeout it stays as the frame found it)
+  if (local == 0 && good) {
     if (threadIdx.x < 6) {
-      S.icp->inc[threadIdx.x] = inc[threadIdx.x];
-      S.icp->prev[threadIdx.x] = prev[threadIdx.x];
+      S.icp->inc[threadIdx.x] = F.inc[threadIdx.x];
+      S.icp->prev[threadIdx.x] = F.prev[threadIdx.x];
     }
     if (threadIdx.x < 16) S.icp->T[threadIdx.x] = Tf[threadIdx.x];
     if (threadIdx.x < 3) {
-      S.icp->iters[threadIdx.x] = iters[threadIdx.x];
-      S.icp->inliers[threadIdx.x] = inliers[threadIdx.x];
-      S.icp->rms[threadIdx.x] = rms[threadIdx.x];
+      S.icp->iters[threadIdx.x] = F.iters[threadIdx.x];
+      S.icp->inliers[threadIdx.x] = F.inliers[threadIdx.x];
+      S.icp->rms[threadIdx.x] = F.rms[threadIdx.x];
     }
-    if (threadIdx.x == 0) {
-      S.icp->converged = conv;
-      S.icp->ticket = 0;
-    }
+    if (threadIdx.x == 0) S.icp->converged = F.conv;
   }
 }
 
-// A barrier self-test: the launch's blocks meet at barrier 1 expecting
-// 'expect' blocks (more than were launched: a wait that cannot complete,
-// which must end in the bounded timeout).
+// The bounded wait run alone: each block adds one to the counter and waits
+// until it holds 'expect' (more than were launched: a wait that cannot
+// complete, which must end in the timeout).
 __global__ void barrier_selftest_kernel(unsigned* bar, unsigned expect) {
-  grid_barrier(bar, 1u, expect);
+  if (threadIdx.x != 0) return;
+  atomicAdd(bar, 1u);
+  BoundedWait wait;
+  while (*(volatile unsigned*)bar < expect)
+    if (wait.expired(bar + kIcpAbort)) return;
 }
 
 // Normal equations only (stage entry point): no solver state.
-template <bool KAHAN>
 __global__ void __launch_bounds__(kIcpThreads)
     icp_reduce_kernel(IcpLevel L, IcpParams P, const float* __restrict__ Tdev,
                       double* __restrict__ partials, unsigned int* ticket_ctr,
@@ -1002,8 +1273,8 @@ __global__ void __launch_bounds__(kIcpThreads)
   const int n = L.s.rows * L.s.cols;
   for (int idx = blockIdx.x * kIcpThreads + threadIdx.x; idx < n;
        idx += gridDim.x * kIcpThreads)
-    pixel_terms<KAHAN>(L, P, T, idx, a);
-  block_reduce<KAHAN>(a, red);
+    pixel_terms<false>(L, P, T, idx, a);
+  block_reduce<false, kIcpThreads / 32>(a, red);
   if (threadIdx.x < kIcpVals) partials[(size_t)blockIdx.x * kIcpVals + threadIdx.x] = red[threadIdx.x];
   __threadfence();
   __shared__ unsigned int ticket;
@@ -1012,7 +1283,7 @@ __global__ void __launch_bounds__(kIcpThreads)
   if (ticket != gridDim.x - 1) return;
   __threadfence();
   __shared__ double tot[kIcpVals];
-  final_reduce<KAHAN>(partials, gridDim.x, tot, red);
+  final_reduce(partials, gridDim.x, tot, red);
   if (threadIdx.x < kIcpVals) out[threadIdx.x] = tot[threadIdx.x];
   if (threadIdx.x == 0) *ticket_ctr = 0;
 }
@@ -1059,12 +1330,15 @@ __global__ void pose_finalize_kernel(IcpParams P, IcpState* st, PoseState* ps) {
   pose_finalize_body(P, st, ps);
 }
 
-// one thread per session; bump != 0 also advances the frame counter
+// one thread per session; bump != 0 also advances the frame counter (within the
+// persistent kernel it measured 4 us slower)
 __global__ void fused_pose_finalize_kernel(const SessDev* __restrict__ tab, int n, int bump) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const SessDev& S = tab[s];
   pose_finalize_body(S.icpp, S.icp, S.pose);
+  S.icp_bar[0] += kIcpEpochStep;  // the next launch's tags
+  S.icp_bar[kIcpAbort] = 0;
   if (bump) S.pose->frame += 1;
 }
 
@@ -1150,11 +1424,6 @@ __global__ void pose_set_kernel(PoseState* ps, const double* pose) {
 
 size_t icp_scratch_bytes() { return sizeof(double) * (size_t)kIcpMaxBlocks * kIcpVals; }
 
-size_t icp_frame_scratch_bytes(size_t npx) {
-  const size_t rows = 2 * (size_t)icp_tiles((int)npx) * kIcpVals * sizeof(double);
-  return rows > icp_scratch_bytes() ? rows : icp_scratch_bytes();
-}
-
 int icp_persistent_capacity(int device) {
   static std::mutex mu;
   static int cap[64] = {};
@@ -1165,9 +1434,9 @@ int icp_persistent_capacity(int device) {
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_icp_persistent_kernel<false>,
-                                                      kIcpThreads, 0) != cudaSuccess ||
+                                                      kIcpFrameThreads, 0) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_k, fused_icp_persistent_kernel<true>,
-                                                      kIcpThreads, 0) != cudaSuccess) {
+                                                      kIcpFrameThreads, 0) != cudaSuccess) {
       cudaGetLastError();
       coop = 0;
     }
@@ -1183,10 +1452,10 @@ int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int
   for (int kind = 0; kind < 2; ++kind) {
     long long sum = 0;
     for (int j = 0; j < n; ++j)
-      if ((kahan[j] != 0) == (kind == 1)) sum += icp_tiles(npx[j]);
+      if ((kahan[j] != 0) == (kind == 1)) sum += icp_weight(npx[j], kind);
     long long g = 0;
     for (int j = 0; j < n; ++j)
-      if ((kahan[j] != 0) == (kind == 1)) g += icp_share(icp_tiles(npx[j]), sum, budget);
+      if ((kahan[j] != 0) == (kind == 1)) g += icp_share(npx[j], kind, sum, budget);
     if (g > budget) {
       grid_k[0] = grid_k[1] = 0;
       return 0;
@@ -1198,11 +1467,9 @@ int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int
 
 template <bool KAHAN>
 static void launch_persistent(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  // the barrier's counters, flags and abort word start at zero every launch
-  cudaMemsetAsync(b.icp_bar, 0, kIcpBarWords * sizeof(unsigned), st);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(b.icp_grid_k[KAHAN ? 1 : 0]);
-  cfg.blockDim = dim3(kIcpThreads);
+  cfg.blockDim = dim3(kIcpFrameThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -1210,7 +1477,7 @@ static void launch_persistent(const SessDev* tab, const BatchShape& b, cudaStrea
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, fused_icp_persistent_kernel<KAHAN>, tab, b.n, b.icp_budget,
-                     b.max_slot_iters[0], b.max_slot_iters[1], b.max_slot_iters[2], b.icp_bar);
+                     b.max_slot_iters[0], b.max_slot_iters[1], b.max_slot_iters[2]);
 }
 
 void fused_icp_persistent(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
@@ -1247,7 +1514,7 @@ dyn_status icp_barrier_selftest(int blocks, int missing, unsigned* bar_dev, cuda
     return e == cudaErrorCooperativeLaunchTooLarge ? DYN_ERR_INVALID_ARG : DYN_ERR_CUDA;
   }
   int abort_h = 0;
-  if (cudaMemcpyAsync(&abort_h, bar_dev + 32 * (2 * kIcpBarSpread), sizeof(int),
+  if (cudaMemcpyAsync(&abort_h, bar_dev + kIcpAbort, sizeof(int),
                       cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return DYN_ERR_CUDA;
@@ -1270,22 +1537,14 @@ void launch_pose_set(PoseState* ps, const double* pose_dev, cudaStream_t stream)
 void launch_icp_reduce_only(const IcpLevel& L, const IcpParams& P, const float* T_dev,
                             double* partials, unsigned int* ticket, double* out_dev,
                             cudaStream_t stream) {
-  int g = icp_grid(L.s.rows * L.s.cols);
-  if (P.kahan)
-    icp_reduce_kernel<true><<<g, kIcpThreads, 0, stream>>>(L, P, T_dev, partials, ticket, out_dev);
-  else
-    icp_reduce_kernel<false><<<g, kIcpThreads, 0, stream>>>(L, P, T_dev, partials, ticket, out_dev);
+  launch_icp_reduce_grid(L, P, T_dev, partials, ticket, out_dev,
+                         icp_stage_grid(L.s.rows * L.s.cols), stream);
 }
 
 void launch_icp_reduce_grid(const IcpLevel& L, const IcpParams& P, const float* T_dev,
                             double* partials, unsigned int* ticket, double* out_dev, int grid,
                             cudaStream_t stream) {
-  if (P.kahan)
-    icp_reduce_kernel<true><<<grid, kIcpThreads, 0, stream>>>(L, P, T_dev, partials, ticket,
-                                                               out_dev);
-  else
-    icp_reduce_kernel<false><<<grid, kIcpThreads, 0, stream>>>(L, P, T_dev, partials, ticket,
-                                                                out_dev);
+  icp_reduce_kernel<<<grid, kIcpThreads, 0, stream>>>(L, P, T_dev, partials, ticket, out_dev);
 }
 
 // 'chained': launched with programmatic stream serialization, so that the
@@ -1296,8 +1555,9 @@ void fused_icp_iteration(const SessDev* tab, const BatchShape& b, int slot, int 
                          cudaStream_t st) {
   if (it >= b.max_slot_iters[slot]) return;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(icp_grid(b.max_slot_px[slot]), 1, b.n);
-  cfg.blockDim = dim3(kIcpThreads);
+  // (a smaller level may have more tiles than the largest: 148 at most)
+  cfg.gridDim = dim3(kIcpMaxTiles, 1, b.n);
+  cfg.blockDim = dim3(kIcpFrameThreads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

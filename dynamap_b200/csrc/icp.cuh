@@ -47,31 +47,58 @@ struct IcpParams {
   int kahan;           // compensated FP32 per-thread sums (mixed precision)
 };
 
+constexpr int kIcpVals = 29;
+// The stage entry points' reduction (icp_reduce_kernel).
 constexpr int kIcpThreads = 256;
 constexpr int kIcpMaxBlocks = 148 * 8;
-constexpr int kIcpVals = 29;
-// The per-frame ICP sums its normal equations per pixel tile: tile j holds
-// pixels [j * t, (j + 1) * t) of a level of n pixels, t = icp_tile_px(n)
-// (256, 512 or 1024 pixels: one, two or four per thread, smaller tiles on
-// the coarse levels so that more blocks share their short work), and its
-// partial sums are the same whichever block computes them; the level's
-// total adds the tiles in index order.  So the result does not depend on
-// how many blocks work on a level, nor on the sessions that share the
-// launch.  A level never has more tiles than the session's finest one.
-inline __host__ __device__ int icp_tile_px(int npx) {
-  return npx <= 8192 ? kIcpThreads : (npx <= 65536 ? 2 * kIcpThreads : 4 * kIcpThreads);
+// The per-frame ICP: one 512-thread block per SM, and its normal equations
+// summed per tile of a level; a tile's partial sums are the same whichever
+// block computes them, and the level's total adds the tiles in a fixed order.
+// So the result does not depend on how many blocks work on a level, nor on the
+// sessions that share the launch.  A tile is a run of icp_tile_slots(n, kahan)
+// slots: 256 (half of a block's warps, so that a level of 19,200 pixels still
+// spreads over 75 SMs) or a whole number per thread, the least that gives at
+// most 160 tiles -- about one per SM; every block reads every tile's row.  A
+// slot of the plain form is a pixel; of the compensated form a group of
+// icp_group(n) pixels 256 apart (of runs of 256 times as many pixels), which
+// one thread sums in plain FP32.
+constexpr int kIcpFrameThreads = 512;
+constexpr int kIcpMaxTiles = 160;
+inline __host__ __device__ int icp_group(int npx) { return npx <= 8192 ? 1 : (npx <= 65536 ? 2 : 4); }
+inline __host__ __device__ int icp_slots(int npx, int kahan) {
+  if (!kahan) return npx;
+  const int run = icp_group(npx) * 256;
+  return (npx + run - 1) / run * 256;
 }
-inline __host__ __device__ int icp_tiles(int npx) {
-  const int t = icp_tile_px(npx);
-  return (npx + t - 1) / t;
+inline __host__ __device__ int icp_tile_slots(int npx, int kahan) {
+  const int n = icp_slots(npx, kahan);
+  if (n <= 148 * 256) return 256;
+  return (n + kIcpMaxTiles * kIcpFrameThreads - 1) / (kIcpMaxTiles * kIcpFrameThreads) *
+         kIcpFrameThreads;
+}
+inline __host__ __device__ int icp_tiles(int npx, int kahan) {
+  const int t = icp_tile_slots(npx, kahan);
+  return (icp_slots(npx, kahan) + t - 1) / t;
 }
 
-// Scratch a reduction needs: per-block partial sums (kIcpMaxBlocks*29 doubles).
+// Weight of a session in the shares of a table's blocks: its level-0 pixels and
+// two pixels' worth per slot for the warps' sums.
+inline __host__ __device__ long long icp_weight(int npx, int kahan) {
+  return npx + (kahan ? 2ll * icp_slots(npx, kahan) : 0ll);
+}
+
+// Scratch of a stage reduction: per-block partial sums (kIcpMaxBlocks*29 doubles).
 size_t icp_scratch_bytes();
-// Scratch of the per-frame ICP of a session whose largest level has npx
-// pixels: two rows of per-tile partial sums (iterations alternate rows) and
-// at least icp_scratch_bytes().
-size_t icp_frame_scratch_bytes(size_t npx);
+// Scratch of a session's per-frame ICP: the chained kernels' row of partial
+// sums per tile, then the persistent kernel's rows (kIcpRowWords tagged words
+// each): two per tile (iterations alternate) and the state's of each level.
+constexpr int kIcpRowWords = 64;
+inline __host__ __device__ size_t icp_rows_offset() {  // bytes
+  return ((size_t)kIcpMaxTiles * kIcpVals * sizeof(double) + 255) / 256 * 256;
+}
+inline size_t icp_frame_scratch_bytes() {
+  return icp_rows_offset() + (size_t)(2 * kIcpMaxTiles + 3) * kIcpRowWords * 8;
+}
 
 // The persistent ICP (one cooperative launch per frame and summation kind):
 // the blocks that can be resident at once on 'device' (0: cooperative
@@ -82,15 +109,16 @@ size_t icp_frame_scratch_bytes(size_t npx);
 // chained kernels run the table, with the same results).
 int icp_persistent_capacity(int device);
 int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int* grid_k);
-// The persistent ICP's grid barrier words (a launch's arrival counters,
-// release flags and abort word, each on its own 128-byte line): a launch's
-// barrier buffer holds kIcpBarWords unsigned words.
-constexpr int kIcpBarSpread = 8;
-constexpr int kIcpBarWords = (2 * kIcpBarSpread + 1) * 32;
-// A bounded grid barrier run alone: 'blocks' blocks wait for blocks +
-// missing arrivals (bar_dev: kIcpBarWords words).  DYN_OK when it completes,
-// DYN_ERR_TIMEOUT when the bounded wait ran out, DYN_ERR_INVALID_ARG when
-// the blocks cannot all be resident.
+// The persistent ICP's words of a session: the epoch of the next launch's tags
+// (advanced by kIcpEpochStep by the pose finalisation that follows a launch;
+// never 0) and, on a line of its own, the abort word (zero before a launch).
+constexpr int kIcpAbort = 32;
+constexpr int kIcpBarWords = 64;
+constexpr unsigned kIcpEpochStep = 4096;
+// The bounded wait of the persistent ICP's blocks, as a barrier run alone:
+// 'blocks' blocks wait for blocks + missing arrivals (bar_dev: kIcpBarWords
+// words).  DYN_OK when it completes, DYN_ERR_TIMEOUT when the wait ran out,
+// DYN_ERR_INVALID_ARG when the blocks cannot all be resident.
 dyn_status icp_barrier_selftest(int blocks, int missing, unsigned* bar_dev, cudaStream_t st);
 // After the last level: guards, pose composition, float pose + inverse, reset
 // of the solver state.  Runs with one thread.

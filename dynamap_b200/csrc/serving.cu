@@ -19,19 +19,20 @@ extern "C" {
 // ---------------------------------------------------------------- batches
 
 // Resident blocks of group g's persistent ICP out of 'cap': in proportion
-// to the group's level-0 pixel tiles among all groups' (at least one).
+// to the group's work among all groups' (at least one per session).
 static int group_budget(const std::vector<dyn_session*>& sorted, const std::vector<int>& start,
                         int g, int cap) {
   long long all = 0, mine = 0;
   const int k = (int)start.size() - 1;
   for (int h = 0; h < k; ++h)
     for (int j = start[h]; j < start[h + 1]; ++j) {
-      const long long t = icp_tiles((int)sorted[j]->npx);
+      const long long t = icp_weight((int)sorted[j]->npx, sorted[j]->icp_params().kahan);
       all += t;
       if (h == g) mine += t;
     }
   if (all <= 0) return 0;
-  return std::max(1, (int)((long long)cap * mine / all));
+  const int n = start[g + 1] - start[g];
+  return cap > 0 ? std::max(n, (int)((long long)cap * mine / all)) : 0;
 }
 
 dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch** out) {
@@ -103,7 +104,6 @@ dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch**
   if (r == DYN_OK) r = dalloc((void**)&b->d_map, sizeof(int) * (size_t)n);
   if (r == DYN_OK) r = dalloc((void**)&b->d_gvis, sizeof(int2) * (size_t)cap);
   if (r == DYN_OK) r = dalloc((void**)&b->d_gcount, sizeof(int) * kMaxGroups);
-  if (r == DYN_OK) r = dalloc((void**)&b->d_icp_bar, kIcpBarWords * sizeof(unsigned) * kMaxGroups);
   if (r == DYN_OK) r = dalloc((void**)&b->d_res, sizeof(ResultBlock) * (size_t)n);
   for (int g = 1; g < k && r == DYN_OK; ++g)
     if (cudaStreamCreateWithFlags(&b->groups.st[g], cudaStreamNonBlocking) != cudaSuccess ||
@@ -148,7 +148,7 @@ dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch**
                             (int)cap_g);
     // the groups' persistent ICP launches may run at once: each takes a
     // share of the resident blocks in proportion to its pixel tiles
-    set_icp_persistent(G.shape[g], sorted.data() + start[g], n_g, b->d_icp_bar + kIcpBarWords * g,
+    set_icp_persistent(G.shape[g], sorted.data() + start[g], n_g,
                        group_budget(sorted, start, g, icp_persistent_capacity(b->device)));
     voff += cap_g;
   }
@@ -160,7 +160,7 @@ dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch**
   b->sorted = sorted;
   b->gstart.assign(start.begin(), start.end());
   one.shape[0] = make_shape(sorted.data(), n, b->d_gvis, b->d_gcount, (int)cap);
-  set_icp_persistent(one.shape[0], sorted.data(), n, b->d_icp_bar, icp_persistent_capacity(b->device));
+  set_icp_persistent(one.shape[0], sorted.data(), n, icp_persistent_capacity(b->device));
   b->shape = one.shape[0];
   for (int i = 0; i < n; ++i) sessions[i]->batch = b;
   *out = b;
@@ -206,7 +206,7 @@ static void apply_shape(dyn_batch* b, const TuneCandidate& c) {
     const int share = group_budget(b->sorted, b->gstart, g, cap);
     const int budget = c.icp == 2 ? 0 : (c.icp == 1 ? share / 2 : share);
     set_icp_persistent(sh, b->sorted.data() + b->gstart[g], b->gstart[g + 1] - b->gstart[g],
-                       sh.icp_bar, budget);
+                       budget);
   }
   b->single.shape[0].integrate_ctas = c.integrate_ctas;
   b->single.shape[0].ray_tile = c.ray_tile;
@@ -508,7 +508,6 @@ struct dyn_server {
   int64_t frames = 0;
   int2* d_gvis = nullptr;  // the start of the budget: one entry per block admissible
   int* d_gcount = nullptr;
-  unsigned* d_icp_bar = nullptr;  // the persistent ICP's barrier words
   int64_t gvis_cap = 0;
   // streams and events lent to admitted sessions (created ahead of the
   // serving loop: stream creation can block for tens of milliseconds while
@@ -546,7 +545,6 @@ void release(dyn_server* sv) {
   }
   cudaFree(sv->d_arena);
   cudaFree(sv->d_gcount);
-  cudaFree(sv->d_icp_bar);
   cudaFree(sv->d_res);
   if (sv->h_res) cudaFreeHost(sv->h_res);
   if (sv->stream) cudaStreamDestroy(sv->stream);
@@ -623,7 +621,6 @@ dyn_status dyn_server_create(const dyn_server_params* p, dyn_server** out) {
   bool ok = cudaMalloc(&sv->d_arena, sv->budget) == cudaSuccess &&
             cudaStreamCreateWithFlags(&sv->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaMalloc(&sv->d_gcount, 256) == cudaSuccess &&
-            cudaMalloc(&sv->d_icp_bar, kIcpBarWords * sizeof(unsigned)) == cudaSuccess &&
             cudaMalloc(&sv->d_res, sizeof(ResultBlock) * (size_t)cap) == cudaSuccess &&
             cudaMallocHost(&sv->h_res, sizeof(ResultBlock) * (size_t)cap) == cudaSuccess;
   for (StepBuf& r : sv->ring)
@@ -792,7 +789,7 @@ dyn_status dyn_server_step(dyn_server* sv, int32_t* n_out) {
     DYN_CUDA(cudaEventRecord(s->h2d_done, st));
   }
   BatchShape b = make_shape(sv->act.data(), n, sv->d_gvis, sv->d_gcount, (int)cap);
-  set_icp_persistent(b, sv->act.data(), n, sv->d_icp_bar, icp_persistent_capacity(sv->device));
+  set_icp_persistent(b, sv->act.data(), n, icp_persistent_capacity(sv->device));
   enqueue_frame(rb.d_tab, b, rb.d_map, sv->d_res, sv->h_res, sv->capacity, st, Marks());
   DYN_CUDA(cudaGetLastError());
   DYN_CUDA(cudaEventRecord(rb.done, st));

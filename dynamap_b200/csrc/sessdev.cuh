@@ -69,7 +69,8 @@ struct SessDev {
   // solver
   IcpState* icp;
   PoseState* pose;
-  double* partials;
+  double* partials;    // icp_frame_scratch_bytes
+  unsigned* icp_bar;   // kIcpBarWords: the persistent ICP's epoch and abort word
   IcpParams icpp;
   int slot_level[3];  // pyramid level of each ICP level slot
   int slot_iters[3];  // lvl_iteration_num of each slot (runs N-1 iterations)
@@ -103,13 +104,11 @@ struct BatchShape {
   int* gcount;             // its length (device)
   int gvis_cap;
   // the persistent ICP: blocks of its cooperative launches (0: the chained
-  // kernels instead) in all and per summation kind (plain, compensated),
-  // the budget each launch's shares are taken from, and the barrier's
-  // counters, flags and abort word (kIcpBarWords, device)
+  // kernels instead) in all and per summation kind (plain, compensated), and
+  // the budget each launch's shares are taken from
   int icp_grid;
   int icp_grid_k[2];
   int icp_budget;
-  unsigned* icp_bar;
 };
 
 // image.cu

@@ -279,11 +279,10 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
   return b;
 }
 
-// The persistent ICP for a table of sessions: its grid within 'budget'
-// blocks (0: chained kernels) and its barrier words.  DYN_ICP_CHAINED=1 in
-// the environment keeps every table on the chained kernels (the same
-// results; for comparisons).
-void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, unsigned* bar, int budget) {
+// The persistent ICP for a table of sessions: its grid within 'budget' blocks
+// (0: chained kernels).  DYN_ICP_CHAINED=1 in the environment keeps every
+// table on the chained kernels (the same results; for comparisons).
+void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget) {
   static const bool chained_only = [] {
     const char* e = std::getenv("DYN_ICP_CHAINED");
     return e && e[0] == '1';
@@ -295,10 +294,9 @@ void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, unsigned* 
   }
   b.icp_budget = budget;
   b.icp_grid_k[0] = b.icp_grid_k[1] = 0;
-  b.icp_grid = (chained_only || !bar)
+  b.icp_grid = chained_only
                    ? 0
                    : icp_persistent_grid(npx.data(), kahan.data(), n, budget, b.icp_grid_k);
-  b.icp_bar = bar;
 }
 
 // The session's descriptor (device buffers, sensor levels, parameters).
@@ -339,6 +337,7 @@ void fill_sessdev(dyn_session* s) {
   d.icp = s->d_icp;
   d.pose = s->d_pose;
   d.partials = s->d_partials;
+  d.icp_bar = s->d_icp_bar;
   d.icpp = s->icp_params();
   for (int pl = 0; pl < 3; ++pl) {
     d.slot_level[pl] = level_of_scale(s->gp.lvl_scale[pl]);
@@ -561,6 +560,10 @@ void fill_stats(const dyn_session* s, const ResultBlock& r, dyn_frame_stats* st)
 dyn_status reset_state(dyn_session* s, bool sync = true) {
   cudaStream_t st = s->stream;
   launch_volume_clear(s->vol, st);
+  // no row carries a tag of the first epoch
+  DYN_CUDA(cudaMemsetAsync(s->d_partials, 0, icp_frame_scratch_bytes(), st));
+  unsigned bar[kIcpBarWords] = {kIcpEpochStep};
+  DYN_CUDA(cudaMemcpyAsync(s->d_icp_bar, bar, sizeof(bar), cudaMemcpyHostToDevice, st));
   IcpState z;
   std::memset(&z, 0, sizeof(z));
   for (int k = 0; k < 16; ++k) z.T[k] = (k % 5 == 0) ? 1.0f : 0.0f;
@@ -605,7 +608,7 @@ size_t session_bytes(const dyn_tsdf_params& t, const dyn_sensor& s, int precisio
     b += 4 * (size_t)(ray_bounds_words(tx, ty) + free_tile_words(tx, ty)) + 512;
   }
   b += 2 * n * (4 + 16 + 16 + 4) * 4 / 3;  // source + target pyramids
-  b += icp_frame_scratch_bytes(n) + sizeof(SessDev) + sizeof(BilateralTable) + sizeof(ResultBlock) +
+  b += icp_frame_scratch_bytes() + sizeof(SessDev) + sizeof(BilateralTable) + sizeof(ResultBlock) +
        8192;
   return b;
 }
@@ -693,7 +696,7 @@ dyn_status alloc_device_buffers(dyn_session* s) {
   }
   DYN_TRY(s->dalloc(&s->d_pose_override, 64));
   DYN_TRY(s->dalloc(&s->d_pose_in, 128));
-  DYN_TRY(s->dalloc(&s->d_partials, icp_frame_scratch_bytes(s->npx)));
+  DYN_TRY(s->dalloc(&s->d_partials, icp_frame_scratch_bytes()));
   DYN_TRY(s->dalloc(&s->d_icp_bar, kIcpBarWords * sizeof(unsigned)));
   DYN_TRY(s->dalloc(&s->d_icp, sizeof(IcpState)));
   DYN_TRY(s->dalloc(&s->d_pose, sizeof(PoseState)));
@@ -860,7 +863,7 @@ dyn_status create_session(const dyn_tsdf_params* tsdf, const dyn_gn_params* gn,
   s->hsd_1.rgb_flag = s->d_rgb_flag_1;
   dyn_session* self = s;
   s->shape = make_shape(&self, 1, s->d_gvis, s->d_gcount, tsdf->num_blocks);
-  set_icp_persistent(s->shape, &self, 1, s->d_icp_bar, icp_persistent_capacity(device));
+  set_icp_persistent(s->shape, &self, 1, icp_persistent_capacity(device));
   if (cudaMemcpyAsync(s->d_btab, &s->btab, sizeof(BilateralTable), cudaMemcpyHostToDevice,
                       s->stream) != cudaSuccess ||
       cudaMemcpyAsync(s->d_sd, &s->hsd, sizeof(SessDev), cudaMemcpyHostToDevice, s->stream) !=

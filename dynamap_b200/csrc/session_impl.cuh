@@ -276,7 +276,6 @@ struct dyn_batch {
   SessDev* d_tab = nullptr;
   int2* d_gvis = nullptr;
   int* d_gcount = nullptr;
-  unsigned* d_icp_bar = nullptr;  // kIcpBarWords per group (persistent ICP barrier)
   ResultBlock* d_res = nullptr;
   ResultBlock* h_res = nullptr;  // pinned, n entries
   BatchShape shape;
@@ -341,8 +340,8 @@ dyn_status quiesce(dyn_session* s);
 // grid).
 BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, int gvis_cap);
 // The persistent ICP of a table: its grid within 'budget' blocks (0 when it
-// does not fit: the chained kernels, same results) and its barrier words.
-void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, unsigned* bar, int budget);
+// does not fit: the chained kernels, same results).
+void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget);
 // Marks whether this frame of 's' carries RGB (stream-ordered).
 dyn_status set_rgb_flag(dyn_session* s, bool has_rgb, cudaStream_t st);
 // Host frame into the session's device input buffers on 'st'.
