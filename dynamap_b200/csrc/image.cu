@@ -308,23 +308,43 @@ __global__ void target_prepare_kernel(const float* __restrict__ ray, float* __re
 }
 
 // ---------------------------------------------------------------- fused
-// ingest (+ the unfiltered copy when the bilateral filter is off), and the
-// distance from the camera centre to each pixel's back-projected point
-// (IntegrateScanKernel's per-voxel |getPoint3d(pixel, depth)|,
-// tsdf.cu:316-317): it depends only on the pixel, so integration reads it
-// instead of recomputing it (two divisions and a square root) for every
-// voxel that projects there -- the same operations, so the same bits
+// ingest (+ the unfiltered copy when the bilateral filter is off), and what
+// integration reads per voxel that projects to a pixel: the distance from the
+// camera centre to the pixel's back-projected point (IntegrateScanKernel's
+// |getPoint3d(pixel, depth)|, tsdf.cu:316-317 -- it depends only on the pixel,
+// the same operations so the same bits; by the band form's approximate
+// operations for band sessions), NaN where the depth is outside the sensor
+// range (every comparison then fails, as the reference's range test does) and
+// negative where it is the range's end (the reference's band test excludes it);
+// and the packed colour.
+__device__ inline float pixel_distance(int x, int y, float d, const DSensor& s, const DTsdf& t) {
+  if (d < t.dmin || d > t.dmax) return __int_as_float(0x7fffffff);
+  float sd;
+  if (t.band) {
+    const F3 p = f3(__fdividef(((float)x - s.cx) * d, s.fx), __fdividef(((float)y - s.cy) * d, s.fy), d);
+    const float q = __fmaf_rn(p.x, p.x, __fmaf_rn(p.y, p.y, p.z * p.z));
+    sd = q > 0.0f ? q * rsqrtf(q) : 0.0f;
+  } else {
+    sd = norm3(point3d_uv(x, y, d, s));
+  }
+  return d < t.dmax ? sd : -sd;
+}
+
 __global__ void fused_ingest_kernel(const SessDev* __restrict__ tab) {
   const SessDev& S = tab[blockIdx.z];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= S.npx) return;
-  ingest_px(S.u16, *S.rgb_flag ? S.rgb : nullptr, S.depth_scaler, S.raw,
-            S.use_color ? S.sint[0] : nullptr, i);
+  const uint8_t* rgb = *S.rgb_flag ? S.rgb : nullptr;
+  ingest_px(S.u16, rgb, S.depth_scaler, S.raw, S.use_color ? S.sint[0] : nullptr, i);
+  if (rgb) {
+    const uint8_t* c = rgb + 3 * (size_t)i;
+    S.rgb4[i] = (unsigned)c[0] | ((unsigned)c[1] << 8) | ((unsigned)c[2] << 16);
+  }
   const float d = S.raw[i];
   if (!S.bil_enabled) S.filt[i] = d;
   const DSensor& s0 = S.ls[0];
   const int y = i / s0.cols;
-  S.sdist[i] = norm3(point3d_uv(i - y * s0.cols, y, d, s0));
+  S.sdist[i] = pixel_distance(i - y * s0.cols, y, d, s0, S.vol.t);
 }
 
 // The free-space tile map of a depth-only frame of a carving session (one
@@ -345,7 +365,7 @@ __global__ void fused_free_tiles_kernel(const SessDev* __restrict__ tab) {
     for (int x = x0; x < x1; ++x) {
       const float d = S.raw[y * s.cols + x];
       if (!(d >= t.dmin && d <= t.dmax)) ok = false;
-      else mn = fminf(mn, S.sdist[y * s.cols + x] - t.trunc);
+      else mn = fminf(mn, fabsf(S.sdist[y * s.cols + x]) - t.trunc);
     }
   const unsigned v = __float_as_uint(ok ? fmaxf(mn, 0.0f) : 0.0f);
   S.ftile[i] = v;

@@ -50,7 +50,8 @@ struct SessDev {
   const uint8_t* rgb;
   // images
   float* raw;
-  float* sdist;         // |point3d_uv(x, y, raw)| per pixel (integration)
+  float* sdist;         // |point3d_uv(x, y, raw)| per pixel (integration; see fused_ingest_kernel)
+  unsigned* rgb4;       // the frame's colours, packed (when it carries RGB)
   float* filt;
   float* sdep[kLevels];
   float4* snrm[kLevels];

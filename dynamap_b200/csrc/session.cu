@@ -316,6 +316,7 @@ void fill_sessdev(dyn_session* s) {
   d.rgb = s->d_rgb;
   d.raw = s->d_raw;
   d.sdist = s->d_sdist;
+  d.rgb4 = s->d_rgb4;
   d.filt = s->d_filt;
   for (int l = 0; l < s->nlev; ++l) {
     d.sdep[l] = s->d_sdep[l];
@@ -602,7 +603,7 @@ size_t session_bytes(const dyn_tsdf_params& t, const dyn_sensor& s, int precisio
     const DSensor ds = dsensor(s);
     b += sizeof(unsigned) * (size_t)grid_entries(ds, dtsdf(t, precision));  // raycast block grid
   }
-  b += n * (2 + 3 + 4 + 4 + 4 + 3);  // inputs, raw, filtered, ray depth, target rgb
+  b += n * (2 + 3 + 4 + 4 + 4 + 4 + 3);  // inputs, packed rgb, raw, filtered, ray depth, target rgb
   {  // ray depth bounds and the free-space tile map
     const int tx = ((int)s.cols + 7) / 8, ty = ((int)s.rows + 7) / 8;
     b += 4 * (size_t)(ray_bounds_words(tx, ty) + free_tile_words(tx, ty)) + 512;
@@ -678,6 +679,7 @@ dyn_status alloc_device_buffers(dyn_session* s) {
   DYN_TRY(s->dalloc(&s->d_rgb, n * 3));
   DYN_TRY(s->dalloc(&s->d_raw, n * 4));
   DYN_TRY(s->dalloc(&s->d_sdist, n * 4));
+  DYN_TRY(s->dalloc(&s->d_rgb4, n * 4));
   DYN_TRY(s->dalloc(&s->d_filt, n * 4));
   DYN_TRY(s->dalloc(&s->d_ray, n * 4));
   DYN_TRY(s->dalloc(&s->d_trgb, n * 3));

@@ -123,6 +123,7 @@ struct dyn_session {
   uint8_t* d_rgb = nullptr;
   float* d_raw = nullptr;
   float* d_sdist = nullptr;
+  unsigned* d_rgb4 = nullptr;
   float* d_filt = nullptr;
   float* d_sdep[kLevels] = {};
   float4* d_snrm[kLevels] = {};

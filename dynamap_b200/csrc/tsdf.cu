@@ -26,6 +26,23 @@ namespace dyn {
 
 namespace {
 
+// ------------------------------------------------------------ exact shortcuts
+// Rounding by adding and subtracting 1.5 * 2^23: two additions and no
+// conversion (the conversions run at an eighth of the FP32 rate); the sum's
+// low bits are the integer.
+constexpr float kRint = 12582912.0f;   // 1.5 * 2^23
+constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
+
+// a / b by b's hoisted reciprocal: yh = fl(1/b), yl the rest of 1/b;
+// q = fl(a * yh + fl(a * yl)) is within an ulp of a / b, and
+// fma(fma(-b, q, a), yh, q) is then the correctly rounded quotient (Markstein,
+// IBM J. Res. Dev. 34, 1990) unless a step under- or overflows.  A zero
+// dividend gives zero (of either sign).
+__device__ inline float div_by(float a, float b, float yh, float yl) {
+  const float q = __fmaf_rn(a, yh, __fmul_rn(a, yl));
+  return __fmaf_rn(__fmaf_rn(-b, q, a), yh, q);
+}
+
 // ------------------------------------------------------------ the block grid
 // The raycast looks blocks up by their coordinates far more often than
 // anything else (every sample, up to eight blocks), so each frame's blocks are
@@ -568,31 +585,45 @@ __global__ void fused_surface_bound_kernel(const SessDev* __restrict__ tab) {
 
 // ------------------------------------------------------------ integration
 // IntegrateScanKernel voxel loop (tsdf.cu:301-341) + Voxel::mergeVoxel
-// (geom_Types.h:79-103) for voxel 'lin' of block 'ptr'.  The voxel updated
-// is the thread's own: the reference's camera->world round trip through
-// UpdateVoxel lands on the same voxel (the oracle checks this).
+// (geom_Types.h:79-103).  The voxel updated is the thread's own: the
+// reference's camera->world round trip through UpdateVoxel lands on the same
+// voxel (the oracle checks this).
+//
+// One warp per block: lane (y, z pair) walks x, so that a step is 64 voxels in
+// 512 contiguous bytes (256 in the mixed form), two per lane in one vector,
+// and the products of the camera transform that depend on y and z alone are
+// taken once per block -- the reference's sums, with their terms computed
+// once.  A voxel gathers one word of its pixel (sdist, which carries the
+// depth's validity, image.cu) and, when it is updated, the pixel's packed
+// colour.  Three of the reference's IEEE operations only decide something for
+// few voxels, which alone compute them:
+//  * the pixel: an approximate quotient within a margin of its rounding;
+//  * the distance from the camera: its approximation tells free space and
+//    behind the surface apart, the band takes the square root;
+//  * the merge's division by weight + 1: by the tabulated reciprocal with an
+//    exact correction (div_by), the colours' by a tabulated multiplier.
+// A 640x480 RGB frame (32,000 blocks): the CTA-per-block kernel before it took
+// 106 M warp instructions and waited on its barriers and on gathers of five
+// words per voxel (L1 at 76 %); this one takes 75 M and issues in 70 % of the
+// cycles (80 registers and 24 warps per SM: 57 %).  Live stage before -> now:
+// 640x480 RGB FP32 156 -> 112 us, mixed with its free-cell passes 195 -> 141,
+// 320x240 FP32 41 -> 36, 32-session band batch 357 -> 194; reading and writing
+// the blocks once would take 45 us of the first.
+//
 // FAST (band sessions, whose allocation already departs from the
 // reference's): fused multiply-adds and hardware-approximate division and
 // square root throughout.
-__device__ inline F3 xform_fma(const M4f& T, F3 v) {
-  return f3(__fmaf_rn(T.m[0], v.x, __fmaf_rn(T.m[1], v.y, __fmaf_rn(T.m[2], v.z, T.m[3]))),
-            __fmaf_rn(T.m[4], v.x, __fmaf_rn(T.m[5], v.y, __fmaf_rn(T.m[6], v.z, T.m[7]))),
-            __fmaf_rn(T.m[8], v.x, __fmaf_rn(T.m[9], v.y, __fmaf_rn(T.m[10], v.z, T.m[11]))));
-}
-__device__ inline float norm3_fast(F3 v) {
-  const float q = __fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z));
-  return q > 0.0f ? q * rsqrtf(q) : 0.0f;
-}
 
-// Whether this frame updates voxel 'lin' of block 'ptr', and with which
-// sdf and colour (the per-voxel test of IntegrateScanKernel).
-// The world position of a block's first voxel (its key times the block's
-// extent, as the reference computes it per voxel).
-__device__ inline F3 block_origin(const VolumeDev& v, int ptr) {
-  const float vs = v.t.vs;
-  const unsigned long long key = v.block_keys[ptr];
-  return f3((float)key_x(key) * vs * (float)kBlockSize, (float)key_y(key) * vs * (float)kBlockSize,
-            (float)key_z(key) * vs * (float)kBlockSize);
+// The tabulated divisors of the merge, for weights 0 .. 255 (divisor w + 1).
+struct MergeTable {
+  float2 rcp[256];    // 1 / (w + 1) as yh, yl of div_by
+  unsigned mul[256];  // ceil(2^24 / (w + 1))
+};
+__device__ inline void make_merge_table(MergeTable& t, int k) {
+  const float b = (float)(k + 1);
+  const float yh = 1.0f / b;
+  t.rcp[k] = make_float2(yh, __fmaf_rn(-b, yh, 1.0f) * yh);
+  t.mul[k] = (0x1000000u + (unsigned)k) / (unsigned)(k + 1);
 }
 
 // Voxel::mergeVoxelColor (geom_Types.h:87-91) of an observation of weight 1
@@ -601,199 +632,287 @@ __device__ inline F3 block_origin(const VolumeDev& v, int ptr) {
 // rounded quotient truncates to the floor of the exact one: below an
 // integer k <= 255 the quotient is at least 1 / (w + 1) >= 2^-16 away,
 // more than the half ulp (at most 2^-17) it would take to round up to k.
-// So the integer quotient gives the same byte; it comes from an estimate
-// by the reciprocal rcp_d of w + 1 (relative error a few 2^-24, under one
-// unit off) corrected by one step.
-__device__ inline uint8_t colour_merge(unsigned old, unsigned obs, unsigned w, float rcp_d) {
-  const int n = (int)(old * w + obs), d = (int)w + 1;
-  int q = __float2int_rz(__int2float_rn(n) * rcp_d);
-  const int r = n - q * d;
-  q += (int)(r >= d) - (int)(r < 0);
-  return (uint8_t)q;
+// So the integer quotient gives the same byte; for w <= 255 (n <= 65280) it is
+// the high part of n * ceil(2^24 / (w + 1)): the multiplier is less than 1 too
+// large by (w + 1) parts in 2^24, and n (w + 1) < 2^24.
+__device__ inline unsigned colour_merge(unsigned old, unsigned obs, unsigned w, unsigned mul) {
+  const unsigned n = old * w + obs;
+  return (unsigned)(((unsigned long long)n * mul) >> 24);
+}
+// the three channels of packed colours (byte 3 zero)
+__device__ inline unsigned colours_merge(unsigned old, unsigned obs, unsigned w,
+                                         const MergeTable& tb) {
+  unsigned r = 0;
+  if (w <= 255u) {
+    const unsigned m = tb.mul[w];
+#pragma unroll
+    for (int k = 0; k < 24; k += 8)
+      r |= colour_merge((old >> k) & 255u, (obs >> k) & 255u, w, m) << k;
+  } else {  // mixed form
+#pragma unroll
+    for (int k = 0; k < 24; k += 8)
+      r |= ((((old >> k) & 255u) * w + ((obs >> k) & 255u)) / (w + 1u)) << k;
+  }
+  return r;
 }
 
+struct FrameView {
+  const float* __restrict__ sdist;
+  int cols, rows;
+  float fx, fy, cx, cy, trunc;
+  float mx, my;  // a half less the margin of the approximate pixel coordinate
+};
+
+__device__ inline float norm3_fast(F3 v) {
+  const float q = __fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z));
+  return q > 0.0f ? q * rsqrtf(q) : 0.0f;
+}
+
+// roundf(x) as an integer biased by kRintBits, for |x| < 2^22 (other values
+// give integers outside 0 .. 8191, as do NaNs: the addition is monotone).
+__device__ inline int round_biased(float x) {
+  const float t = x + kRint;
+  const float d = x - (t - kRint);  // ties went to even: away from zero instead
+  return __float_as_int(t) + (d == 0.5f && x > 0.0f ? 1 : 0) - (d == -0.5f && x < 0.0f ? 1 : 0);
+}
+
+// The pixel that camera-frame point p projects to, or -1.
 template <bool FAST>
-__device__ inline bool observe_voxel(const VolumeDev& v, const float* __restrict__ depth,
-                                     const float* __restrict__ sdist,
-                                     const uint8_t* __restrict__ rgb, const DSensor& s,
-                                     const M4f& invT, F3 position, int lin, float& sdf,
-                                     uint8_t& c0, uint8_t& c1, uint8_t& c2) {
-  const DTsdf& t = v.t;
-  const float vs = t.vs;
-  const int bx = lin >> 6, by = (lin >> 3) & 7, bz = lin & 7;
-  F3 vp = f3(position.x + (float)bx * vs, position.y + (float)by * vs,
-             position.z + (float)bz * vs);
-  // pixel, depth gate and band decide which voxels a frame updates: IEEE
-  // arithmetic in the FP32 and mixed forms, so that the mixed form's
-  // weights stay exact
+__device__ inline int observed_pixel(const FrameView& f, F3 p) {
   int px, py;
-  float sd, vd, d;
+  bool ok = true;
   if (FAST) {
-    vp = xform_fma(invT, vp);
-    if (!(vp.z > 0.0f)) return false;
-    const float rz = __fdividef(1.0f, vp.z);
-    const float xf = __fmaf_rn(s.fx * vp.x, rz, s.cx), yf = __fmaf_rn(s.fy * vp.y, rz, s.cy);
-    if (!(fabsf(xf) < 2e9f) || !(fabsf(yf) < 2e9f)) return false;
-    px = (int)roundf(xf);
-    py = (int)roundf(yf);
-    if (!(px >= 0 && py >= 0 && px < s.cols && py < s.rows)) return false;
-    d = __ldg(depth + py * s.cols + px);
-    if (d < t.dmin) return false;
-    if (d > t.dmax) return false;
-    const F3 p3 = f3(__fdividef(((float)px - s.cx) * d, s.fx),
-                     __fdividef(((float)py - s.cy) * d, s.fy), d);
-    sd = norm3_fast(p3);
-    vd = norm3_fast(vp);
+    ok = p.z > 0.0f;
+    const float rz = __fdividef(1.0f, p.z);
+    px = round_biased(__fmaf_rn(f.fx * p.x, rz, f.cx)) - kRintBits;
+    py = round_biased(__fmaf_rn(f.fy * p.y, rz, f.cy)) - kRintBits;
   } else {
-    vp = xform(invT, vp);
-    if (!project(vp, s, &px, &py)) return false;
-    if (!(px >= 0 && py >= 0 && px < s.cols && py < s.rows)) return false;
-    d = __ldg(depth + py * s.cols + px);
-    if (d < t.dmin) return false;
-    if (d > t.dmax) return false;
-    sd = __ldg(sdist + py * s.cols + px);  // norm3(point3d_uv(px, py, d, s))
-    vd = norm3(vp);
-  }
-  const int idx = py * s.cols + px;
-  if (vd > sd - t.trunc && vd < sd + t.trunc && d < t.dmax) sdf = sd - vd;
-  else if (vd < sd - t.trunc) sdf = t.trunc;
-  else return false;
-  c0 = c1 = c2 = 0;
-  if (rgb) {
-    c0 = __ldg(rgb + 3 * (size_t)idx);
-    c1 = __ldg(rgb + 3 * (size_t)idx + 1);
-    c2 = __ldg(rgb + 3 * (size_t)idx + 2);
-  }
-  return true;
-}
-
-// Voxel::mergeVoxel (geom_Types.h:79-103) of one observation into voxel vi.
-// Returns the change of the block's count of observed, non-saturated voxels
-// (-1, 0 or +1) that the update makes (FP16 form; the FP32 form keeps no
-// free-space summaries and returns 0).
-template <bool FP16>
-__device__ inline int merge_voxel(const VolumeDev& v, size_t vi, float sdf, bool has_rgb,
-                                  uint8_t c0, uint8_t c1, uint8_t c2) {
-  const DTsdf& t = v.t;
-  if (FP16) {
-    // mixed form: the same FP32 merge, stored as f16 sdf / truncation
-    // (|value| <= 1, free space exactly 1) and a u16 weight
-    const unsigned raw = v.vox16[vi];
-    const float osdf =
-        __half2float(__ushort_as_half((unsigned short)(raw & 0xffffu))) * t.trunc;
-    const int w = (int)(raw >> 16);
-    const float fw = (float)w;
-    const float nsdf = __fdividef(osdf * fw + sdf, fw + 1.0f);
-    int nw = w + 1;
-    if (nw > t.max_w) nw = t.max_w;
-    const unsigned short nh = __half_as_ushort(__float2half_rn(__fdividef(nsdf, t.trunc)));
-    v.vox16[vi] = (unsigned)nh | ((unsigned)nw << 16);
-    if (v.colors) {
-      uchar4 c = v.colors[vi];
-      // colour exactly as the FP32 form (truncated to bytes)
-      const float rd = __fdividef(1.0f, fw + 1.0f);
-      c.x = colour_merge(c.x, c0, (unsigned)w, rd);
-      c.y = colour_merge(c.y, c1, (unsigned)w, rd);
-      c.z = colour_merge(c.z, c2, (unsigned)w, rd);
-      v.colors[vi] = c;
+    const float ax = f.fx * p.x, ay = f.fy * p.y;
+    float rz;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(rz) : "f"(p.z));
+    const float x = __fmaf_rn(ax, rz, f.cx), y = __fmaf_rn(ay, rz, f.cy);
+    const float tx = x + kRint, ty = y + kRint;
+    px = __float_as_int(tx) - kRintBits;
+    py = __float_as_int(ty) - kRintBits;
+    if (!(fabsf(x - (tx - kRint)) < f.mx && fabsf(y - (ty - kRint)) < f.my)) {
+      // Project, utils.h:114-119
+      const float rx = roundf(ax / p.z + f.cx), ry = roundf(ay / p.z + f.cy);
+      ok = fabsf(rx) < 2e9f && fabsf(ry) < 2e9f;
+      px = ok ? (int)rx : 0;
+      py = ok ? (int)ry : 0;
     }
-    // saturated: f16 value exactly 1 (free space); unobserved before
-    const bool was = w == 0 || (raw & 0xffffu) == 0x3C00u, now = nh == 0x3C00u;
-    return (int)was - (int)now;
   }
-  dyn_voxel* vox = v.voxels + vi;
-  uint2 raw = *reinterpret_cast<const uint2*>(vox);
-  uint8_t r0 = raw.x & 0xff, r1 = (raw.x >> 8) & 0xff, r2 = (raw.x >> 16) & 0xff,
-          w = raw.x >> 24;
-  float osdf = __uint_as_float(raw.y);
-  float fw = (float)w;
-  float nsdf = (osdf * fw + sdf * 1.0f) / (fw + 1.0f);
-  // colour merge (geom_Types.h:87-91); a zero colour merged with a zero
-  // colour stays exactly zero, so depth-only frames skip the divisions
-  if (has_rgb || (raw.x & 0x00ffffffu)) {
-    const float rd = __fdividef(1.0f, fw + 1.0f);
-    r0 = colour_merge(r0, c0, w, rd);
-    r1 = colour_merge(r1, c1, w, rd);
-    r2 = colour_merge(r2, c2, w, rd);
+  ok = ok && (unsigned)px < (unsigned)f.cols && (unsigned)py < (unsigned)f.rows;
+  return ok ? py * f.cols + px : -1;
+}
+
+// Whether the voxel at camera-frame point p is updated by its pixel's sdist
+// word, and with which sdf.
+template <bool FAST>
+__device__ inline bool observed_sdf(const FrameView& f, F3 p, float sd, float& sdf) {
+  const float s = fabsf(sd), lo = s - f.trunc, hi = s + f.trunc;  // (NaN: no depth in range)
+  float vd;
+  sdf = f.trunc;
+  if (FAST) {
+    vd = norm3_fast(p);
+  } else {
+    const float q = p.x * p.x + p.y * p.y + p.z * p.z;
+    const float va = q * rsqrtf(q);  // |p| to within 4e-7
+    if (va * 1.000002f < lo) return true;
+    if (va > hi * 1.000002f) return false;
+    vd = sqrtf(q);
   }
+  if (vd > lo && vd < hi && __float_as_int(sd) >= 0) {  // sign: depth at the range's end
+    sdf = s - vd;
+    return true;
+  }
+  return vd < lo;
+}
+
+// Voxel::mergeVoxel (geom_Types.h:79-103) of one observation into an FP32-form
+// voxel {r, g, b, w | sdf}.
+__device__ inline uint2 merge_fp32(uint2 raw, float sdf, bool has_rgb, unsigned rgb, int max_w,
+                                   const MergeTable& tb) {
+  const unsigned w = raw.x >> 24;
+  const float fw = (float)w, d = fw + 1.0f;
+  const float a = __uint_as_float(raw.y) * fw + sdf * 1.0f;
+  const float2 r = tb.rcp[w];
+  float nsdf = div_by(a, d, r.x, r.y);
+  if (!(fabsf(a) > 1e-18f && fabsf(a) < 1e18f)) nsdf = a / d;  // div_by's range
+  // a zero colour merged with a zero colour stays exactly zero
+  unsigned c = raw.x & 0x00ffffffu;
+  if (has_rgb || c) c = colours_merge(c, rgb, w, tb);
   int nw = (uint8_t)(w + 1);
-  if (nw > t.max_w) nw = t.max_w;
-  uint2 out;
-  out.x = (unsigned)r0 | ((unsigned)r1 << 8) | ((unsigned)r2 << 16) | ((unsigned)nw << 24);
-  out.y = __float_as_uint(nsdf);
-  *reinterpret_cast<uint2*>(vox) = out;
-  return 0;
+  if (nw > max_w) nw = max_w;
+  return make_uint2(c | ((unsigned)nw << 24), __float_as_uint(nsdf));
 }
 
-// IntegrateScanKernel voxel loop (tsdf.cu:301-341) + Voxel::mergeVoxel for
-// voxel 'lin' of block 'ptr': the nonsat change (merge_voxel), 0 when the
-// voxel is not updated.
+// The same into a mixed-form voxel {f16 sdf / truncation | u16 weight}: the
+// FP32 merge, stored as f16 (|value| <= 1, free space exactly 1).  'delta':
+// the change of the block's count of observed, non-saturated voxels.
+__device__ inline unsigned merge_mixed(unsigned raw, float sdf, float trunc, int max_w, int& delta) {
+  const float osdf = __half2float(__ushort_as_half((unsigned short)(raw & 0xffffu))) * trunc;
+  const int w = (int)(raw >> 16);
+  const float fw = (float)w;
+  const float nsdf = __fdividef(osdf * fw + sdf, fw + 1.0f);
+  int nw = w + 1;
+  if (nw > max_w) nw = max_w;
+  const unsigned short nh = __half_as_ushort(__float2half_rn(__fdividef(nsdf, trunc)));
+  // saturated: f16 value exactly 1 (free space); unobserved before
+  const bool was = w == 0 || (raw & 0xffffu) == 0x3C00u, now = nh == 0x3C00u;
+  delta += (int)was - (int)now;
+  return (unsigned)nh | ((unsigned)nw << 16);
+}
+
+// The frame's update of block 'ptr' by one warp; free: a free-space block
+// (every voxel's sdf is the truncation, no colours).
 template <bool FP16, bool FAST>
-__device__ inline int integrate_voxel(const VolumeDev& v, const float* __restrict__ depth,
-                                       const float* __restrict__ sdist,
-                                       const uint8_t* __restrict__ rgb, const DSensor& s,
-                                       const M4f& invT, F3 origin, int ptr, int lin) {
-  float sdf;
-  uint8_t c0, c1, c2;
-  if (!observe_voxel<FAST>(v, depth, sdist, rgb, s, invT, origin, lin, sdf, c0, c1, c2)) return 0;
-  return merge_voxel<FP16>(v, (size_t)ptr * kBlockVox + lin, sdf, rgb != nullptr, c0, c1, c2);
+__device__ inline void integrate_block(const SessDev& S, int ptr, bool free,
+                                       const MergeTable& tb) {
+  const VolumeDev& v = S.vol;
+  const DTsdf& t = v.t;
+  const int lane = threadIdx.x & 31, y = lane >> 2, z0 = (lane & 3) * 2;
+  const unsigned* __restrict__ rgb = (!free && *S.rgb_flag) ? S.rgb4 : nullptr;
+  const int max_w = t.max_w;
+  const float vs = t.vs, trunc = t.trunc;
+  FrameView f;
+  f.sdist = S.sdist;
+  f.cols = S.ls[0].cols;
+  f.rows = S.ls[0].rows;
+  f.fx = S.ls[0].fx;
+  f.fy = S.ls[0].fy;
+  f.cx = S.ls[0].cx;
+  f.cy = S.ls[0].cy;
+  f.trunc = trunc;
+  // the coordinate's error: two roundings of x - cx (2^-22 of it), one of x
+  f.mx = 0.5f - 6e-7f * ((float)f.cols + fabsf(f.cx) + 1.0f);
+  f.my = 0.5f - 6e-7f * ((float)f.rows + fabsf(f.cy) + 1.0f);
+  M4f T;
+  const float4* inv = reinterpret_cast<const float4*>(S.pose->invf);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float4 r = __ldg(inv + k);
+    T.m[4 * k] = r.x;
+    T.m[4 * k + 1] = r.y;
+    T.m[4 * k + 2] = r.z;
+    T.m[4 * k + 3] = r.w;
+  }
+  // the block's first voxel and the lane's two, as the reference computes
+  // them: key * extent + index * voxel
+  const unsigned long long key = v.block_keys[ptr];
+  const float ox = (float)key_x(key) * vs * (float)kBlockSize;
+  const float vy = (float)key_y(key) * vs * (float)kBlockSize + (float)y * vs;
+  const float oz = (float)key_z(key) * vs * (float)kBlockSize;
+  const float vz[2] = {oz + (float)z0 * vs, oz + (float)(z0 + 1) * vs};
+  float py[3], pz[2][3];  // the transform's terms in y and z
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    py[a] = T.m[4 * a + 1] * vy;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      pz[k][a] = FAST ? __fmaf_rn(T.m[4 * a + 1], vy, __fmaf_rn(T.m[4 * a + 2], vz[k], T.m[4 * a + 3]))
+                      : T.m[4 * a + 2] * vz[k];
+  }
+  const size_t base = (size_t)ptr * kBlockVox + y * 8 + z0;
+  int delta = 0;
+#pragma unroll 1
+  for (int x = 0; x < 8; ++x) {
+    const size_t i = base + (size_t)x * 64;
+    bool up[2] = {true, true};
+    float sdf[2] = {trunc, trunc};
+    unsigned col[2] = {0u, 0u};
+    if (!free) {
+      const float vx = ox + (float)x * vs;
+      F3 c[2];
+      {
+        float e[2][3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (FAST) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) e[k][a] = __fmaf_rn(T.m[4 * a], vx, pz[k][a]);
+          } else {
+            const float xy = T.m[4 * a] * vx + py[a];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) e[k][a] = xy + pz[k][a] + T.m[4 * a + 3] * 1.0f;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) c[k] = f3(e[k][0], e[k][1], e[k][2]);
+      }
+      int px[2];
+      float sd[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) px[k] = observed_pixel<FAST>(f, c[k]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        sd[k] = px[k] >= 0 ? __ldg(f.sdist + px[k]) : __int_as_float(0x7fffffff);
+      if (rgb) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          if (px[k] >= 0) col[k] = __ldg(rgb + px[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) up[k] = observed_sdf<FAST>(f, c[k], sd[k], sdf[k]);
+      if (!up[0] && !up[1]) continue;
+    }
+    if (FP16) {
+      uint2* vp = reinterpret_cast<uint2*>(v.vox16 + i);
+      uint2 r = *vp;
+      if (v.colors) {
+        uint2* cp = reinterpret_cast<uint2*>(v.colors + i);
+        uint2 c = *cp;
+        // colour exactly as the FP32 form (truncated to bytes)
+        if (up[0]) c.x = (c.x & 0xff000000u) | colours_merge(c.x & 0x00ffffffu, col[0], r.x >> 16, tb);
+        if (up[1]) c.y = (c.y & 0xff000000u) | colours_merge(c.y & 0x00ffffffu, col[1], r.y >> 16, tb);
+        *cp = c;
+      }
+      if (up[0]) r.x = merge_mixed(r.x, sdf[0], trunc, max_w, delta);
+      if (up[1]) r.y = merge_mixed(r.y, sdf[1], trunc, max_w, delta);
+      *vp = r;
+    } else {
+      uint4* vp = reinterpret_cast<uint4*>(v.voxels + i);
+      uint4 r = *vp;
+      if (up[0]) {
+        const uint2 n = merge_fp32(make_uint2(r.x, r.y), sdf[0], rgb != nullptr, col[0], max_w, tb);
+        r.x = n.x;
+        r.y = n.y;
+      }
+      if (up[1]) {
+        const uint2 n = merge_fp32(make_uint2(r.z, r.w), sdf[1], rgb != nullptr, col[1], max_w, tb);
+        r.z = n.x;
+        r.w = n.y;
+      }
+      *vp = r;
+    }
+  }
+  // the block's non-saturated count follows its voxels exactly (the block is
+  // this warp's alone)
+  if (FP16 && v.nonsat) {
+    const int net = __reduce_add_sync(0xffffffffu, delta);
+    if (lane == 0 && net != 0) v.nonsat[ptr] += net;
+  }
 }
 
-// the batch-wide visible list: each item (session, block) by one CTA
-__global__ void __launch_bounds__(kBlockVox)
+// the batch-wide visible list: each item (session, block) by one warp
+constexpr int kIntThreads = 256;
+__global__ void __launch_bounds__(kIntThreads, 4)
     fused_integrate_kernel(const SessDev* __restrict__ tab, const int2* __restrict__ gvis,
                            const int* __restrict__ gcount) {
-  __shared__ M4f invT;
-  __shared__ int cur_s;
-  __shared__ float org[2][3];  // the block's origin, by iteration parity
-  const int n = *gcount;
-  if (threadIdx.x == 0) cur_s = -1;
+  __shared__ MergeTable tb;
+  static_assert(kIntThreads == 256, "a table entry per thread");
+  make_merge_table(tb, threadIdx.x);
   __syncthreads();
-  int par = 0;
-  for (int b = blockIdx.x; b < n; b += gridDim.x, par ^= 1) {
+  const int n = *gcount;
+  const int warps = gridDim.x * (kIntThreads / 32);
+  for (int b = blockIdx.x * (kIntThreads / 32) + (threadIdx.x >> 5); b < n; b += warps) {
     const int2 entry = gvis[b];
-    const int2 item = make_int2(entry.x & ~kVisFree, entry.y);
-    if (item.x != cur_s) {  // uniform across the CTA
-      __syncthreads();
-      if (threadIdx.x < 16) invT.m[threadIdx.x] = tab[item.x].pose->invf[threadIdx.x];
-      if (threadIdx.x == 0) cur_s = item.x;
-      __syncthreads();
-    }
-    const SessDev& S = tab[item.x];
-    // one thread computes the block's origin (the same expression every
-    // voxel would evaluate); the barrier also keeps every thread within one
-    // iteration of the others, so the other parity's slot is free
-    if (threadIdx.x == 0 && !(entry.x & kVisFree)) {
-      const F3 o = block_origin(S.vol, item.y);
-      org[par][0] = o.x;
-      org[par][1] = o.y;
-      org[par][2] = o.z;
-    }
-    __syncthreads();
-    const F3 origin = f3(org[par][0], org[par][1], org[par][2]);
-    const uint8_t* rgb = *S.rgb_flag ? S.rgb : nullptr;
-    int d;
-    if (entry.x & kVisFree) {  // a free-space block: every voxel's sdf is the truncation
-      const size_t vi = (size_t)item.y * kBlockVox + threadIdx.x;
-      d = S.vol.fp16 ? merge_voxel<true>(S.vol, vi, S.vol.t.trunc, false, 0, 0, 0)
-                     : merge_voxel<false>(S.vol, vi, S.vol.t.trunc, false, 0, 0, 0);
-    } else if (!S.vol.fp16)
-      d = integrate_voxel<false, false>(S.vol, S.raw, S.sdist, rgb, S.ls[0], invT, origin,
-                                        item.y, threadIdx.x);
-    else if (S.vol.t.band)
-      d = integrate_voxel<true, true>(S.vol, S.raw, S.sdist, rgb, S.ls[0], invT, origin,
-                                      item.y, threadIdx.x);
-    else
-      d = integrate_voxel<true, false>(S.vol, S.raw, S.sdist, rgb, S.ls[0], invT, origin,
-                                       item.y, threadIdx.x);
-    // the block's non-saturated count follows its voxels exactly: each warp
-    // adds its voxels' changes (mixed sessions only; most warps change
-    // nothing, and no barrier holds the CTA's warps together)
-    if (S.vol.nonsat) {
-      const unsigned up = __ballot_sync(0xffffffffu, d > 0), dn = __ballot_sync(0xffffffffu, d < 0);
-      const int net = __popc(up) - __popc(dn);
-      if ((threadIdx.x & 31) == 0 && net != 0) atomicAdd(S.vol.nonsat + item.y, net);
-    }
+    const SessDev& S = tab[entry.x & ~kVisFree];
+    const bool free = (entry.x & kVisFree) != 0;
+    if (!S.vol.fp16) integrate_block<false, false>(S, entry.y, free, tb);
+    else if (S.vol.t.band) integrate_block<true, true>(S, entry.y, free, tb);
+    else integrate_block<true, false>(S, entry.y, free, tb);
+    __syncwarp();
   }
 }
 
@@ -1066,16 +1185,9 @@ __device__ __noinline__ bool raycast_exact_hash_px(const VolumeDev& v, const DSe
 // every multiple of one half the indices are the reference's; else
 // (exact_axis) they are computed with its own expressions.
 //
-// (x - cx) * z / fx by the hoisted reciprocal: yh = fl(1/b), yl the rest of
-// 1/b; q = fl(a * yh + fl(a * yl)) is within an ulp of a / b, and
-// fma(fma(-b, q, a), yh, q) is then the correctly rounded quotient (Markstein,
-// IBM J. Res. Dev. 34, 1990) unless a step under- or overflows, which the
-// ranges of march_setup exclude.  A zero dividend gives zero (of either sign:
-// the sign reaches only sums with the pose's translation, and a zero's sign
-// changes no index, weight or depth).
-constexpr float kRint = 12582912.0f;   // 1.5 * 2^23
-constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
-
+// (x - cx) * z / fx by the hoisted reciprocal (div_by), whose range march_setup
+// checks; a zero's sign reaches only sums with the pose's translation, where it
+// changes no index, weight or depth.
 // v rounded to the nearest integer (|v| < 2^22): its integer biased by
 // kRintBits, the integer of floor(v) likewise, and v - round(v).
 struct Rounded {
@@ -1224,11 +1336,6 @@ struct MarchRange {
     return false;
   }
 };
-
-__device__ inline float div_by(float a, float b, float yh, float yl) {
-  const float q = __fmaf_rn(a, yh, __fmul_rn(a, yl));
-  return __fmaf_rn(__fmaf_rn(-b, q, a), yh, q);
-}
 
 // One axis by the reference's expressions: (low corner, voxel - low corner),
 // or a second value of 2 where the high corner is not low + 1 or the voxel is
@@ -1850,7 +1957,7 @@ void fused_visible(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
 }
 
 void fused_integrate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  fused_integrate_kernel<<<b.integrate_ctas > 0 ? b.integrate_ctas : 148 * 8, kBlockVox, 0,
+  fused_integrate_kernel<<<b.integrate_ctas > 0 ? b.integrate_ctas : 148 * 8, kIntThreads, 0,
                            st>>>(tab, b.gvis, b.gcount);
 }
 

@@ -65,3 +65,46 @@ def test_indices_from_the_rounded_product(vs):
         assert np.array_equal(low[sure] + 1, g1[sure])
         used += int(sure.sum())
     assert used > 1_000_000
+
+
+def test_division_by_merge_weights_is_exact(host):
+    """The merge's quotient by weight + 1 through its tabulated reciprocal."""
+    for d in list(range(1, 67)) + [100, 127, 128, 129, 200, 251, 255, 256]:
+        assert host.march_div_mismatches(float(d), 2.0 ** -60) == 0
+        assert host.march_div_mismatches(float(d), 0.0078125) == 0
+
+
+def test_colour_quotient_by_multiplication_is_exact():
+    """(old * w + obs) / (w + 1) as the high part of a product, every weight
+    and numerator."""
+    for d in range(1, 257):
+        n = np.arange(0, 255 * (d - 1) + 256, dtype=np.uint64)
+        m = np.uint64((0x1000000 + d - 1) // d)
+        assert np.array_equal((n * m) >> np.uint64(24), n // np.uint64(d)), d
+
+
+@pytest.mark.parametrize("cols,cx,fx", [(160, 79.5, 131.25), (640, 319.5, 525.0), (1280, 639.5, 910.0),
+                                        (8192, 4000.0, 5000.0), (633, 316.0, 519.25)])
+def test_pixels_from_the_approximate_quotient(cols, cx, fx):
+    """The voxel's pixel from (fx x) * rcp(z) + cx equals round(fx x / z + cx)
+    outside the margin, for reciprocals an ulp either way."""
+    rng = np.random.default_rng(11)
+    n = 500_000
+    z = rng.uniform(0.1, 8.0, n).astype(f)
+    u = np.concatenate([rng.uniform(-2, cols + 2, n // 2),
+                        rng.integers(-1, cols + 1, n // 2) + 0.5 + rng.normal(0, 1e-4, n // 2)])
+    x = ((u - cx) * z / fx).astype(f)
+    ax = (f(fx) * x).astype(f)
+    ref = ((ax / z).astype(f) + f(cx)).astype(f)
+    want = np.trunc(ref.astype(np.float64) + np.copysign(0.5, ref)).astype(np.int64)
+    margin = 0.5 - 6e-7 * (cols + abs(cx) + 1.0)
+    for k in (-1, 0, 1):
+        rz = ((f(1.0) / z).astype(np.float64) * (1 + k * 2.0 ** -23)).astype(f)
+        a = (ax.astype(np.float64) * rz.astype(np.float64) + cx).astype(f)  # one rounding
+        t = np.rint(a)
+        sure = np.abs(a - t) < margin
+        inside = (want >= 0) & (want < cols)
+        assert np.array_equal(t[sure & inside].astype(np.int64), want[sure & inside])
+        out = sure & ~inside
+        assert not ((t[out] >= 0) & (t[out] < cols)).any()
+        assert sure.mean() > 0.45
