@@ -26,6 +26,27 @@ struct DSensor {
   float fx, fy, cx, cy;
 };
 
+// A level's intrinsics with the reciprocals of its focal lengths (fl(1/f) and
+// the rest, for div_by).
+constexpr float kModerateMin = 9.5367431640625e-7f, kModerateMax = 1048576.0f;  // 2^-20, 2^20
+struct LevelCamera {
+  DSensor s;
+  float yhx, ylx, yhy, yly;
+  int ok;  // the quotients of depths in kModerateMin .. Max stay in div_by's range
+};
+inline LevelCamera level_camera(const DSensor& s) {
+  const auto moderate = [](float x) { return x >= kModerateMin && x <= kModerateMax; };
+  LevelCamera c;
+  c.s = s;
+  c.yhx = 1.0f / s.fx;
+  c.yhy = 1.0f / s.fy;
+  c.ylx = fmaf(-s.fx, c.yhx, 1.0f) * c.yhx;
+  c.yly = fmaf(-s.fy, c.yhy, 1.0f) * c.yhy;
+  c.ok = moderate(s.fx) && moderate(s.fy) && (s.cx == 0.0f || moderate(fabsf(s.cx))) &&
+         (s.cy == 0.0f || moderate(fabsf(s.cy)));
+  return c;
+}
+
 struct DTsdf {
   float vs;          // voxelSize
   float bsm;         // blockSize * voxelSize (metres), tsdf.cu:437-438
@@ -74,6 +95,16 @@ __host__ __device__ inline F3 f3(float x, float y, float z) {
   r.z = z;
   return r;
 }
+// a / b by b's hoisted reciprocal: yh = fl(1/b), yl the rest of 1/b;
+// q = fl(a * yh + fl(a * yl)) is within an ulp of a / b, and
+// fma(fma(-b, q, a), yh, q) is then the correctly rounded quotient (Markstein,
+// IBM J. Res. Dev. 34, 1990) unless a step under- or overflows.  A zero
+// dividend gives zero (of either sign).
+__device__ inline float div_by(float a, float b, float yh, float yl) {
+  const float q = __fmaf_rn(a, yh, __fmul_rn(a, yl));
+  return __fmaf_rn(__fmaf_rn(-b, q, a), yh, q);
+}
+
 __device__ inline F3 operator+(F3 a, F3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ inline F3 operator-(F3 a, F3 b) { return f3(a.x - b.x, a.y - b.y, a.z - b.z); }
 __device__ inline F3 operator*(F3 a, float s) { return f3(a.x * s, a.y * s, a.z * s); }

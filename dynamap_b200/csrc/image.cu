@@ -28,21 +28,6 @@ __device__ inline float intensity_u8(const uint8_t* c) {
 }
 
 // u16 sensor units -> metres (builder.cu:111, utils_Dataset.cpp:233-235)
-__device__ inline void ingest_px(const uint16_t* __restrict__ raw, const uint8_t* __restrict__ rgb,
-                                 float scaler, float* __restrict__ depth,
-                                 float* __restrict__ inten, int i) {
-  depth[i] = (float)raw[i] / scaler;
-  if (inten) inten[i] = rgb ? intensity_u8(rgb + 3 * (size_t)i) : 0.0f;
-}
-
-__global__ void ingest_kernel(const uint16_t* __restrict__ raw,
-                              const uint8_t* __restrict__ rgb, int n, float scaler,
-                              float* __restrict__ depth, float* __restrict__ inten) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  ingest_px(raw, rgb, scaler, depth, inten, i);
-}
-
 // pyramid::applyBilateralFilter, pyramid.cu:213-233, window rows x-r..x+r-1,
 // cols y-r..y+r-1, summed row-major.  The depth tile plus halo is staged in
 // shared memory (0 where outside the image or not > 0: such taps are skipped,
@@ -207,11 +192,8 @@ __global__ void bilateral_kernel(const float* __restrict__ src, float* __restric
 
 // One 2x pyramid step: mean of the valid depths of each 2x2 cell (fix of
 // pyramid.cu:49-82, which scatters into a fixed 640x480 window).
-__device__ inline void downsample_depth_px(const float* __restrict__ src, int cols, int c2,
-                                           float* __restrict__ dst, int i) {
-  int y = i / c2, x = i - (i / c2) * c2;
-  const float* a = src + (2 * y) * cols + 2 * x;
-  float v[4] = {a[0], a[1], a[cols], a[cols + 1]};
+__device__ inline float mean_valid(float a, float b, float c, float d) {
+  const float v[4] = {a, b, c, d};
   float s = 0.0f;
   int n = 0;
 #pragma unroll
@@ -220,29 +202,16 @@ __device__ inline void downsample_depth_px(const float* __restrict__ src, int co
       s += v[k];
       n++;
     }
-  dst[i] = n ? s / (float)n : 0.0f;
+  // s / n: a half and a quarter are exact as products, a third by its reciprocal
+  if (n == 3) {
+    const float yh = 1.0f / 3.0f;
+    return s >= kModerateMin && s <= kModerateMax ? div_by(s, 3.0f, yh, fmaf(-3.0f, yh, 1.0f) * yh)
+                                                  : s / 3.0f;
+  }
+  return s * (n == 4 ? 0.25f : (n == 2 ? 0.5f : 1.0f));
 }
-__device__ inline void downsample_intensity_px(const float* __restrict__ src, int cols, int c2,
-                                               float* __restrict__ dst, int i) {
-  int y = i / c2, x = i - (i / c2) * c2;
-  const float* a = src + (2 * y) * cols + 2 * x;
-  dst[i] = (((a[0] + a[1]) + a[cols]) + a[cols + 1]) * 0.25f;
-}
-
-__global__ void downsample_depth_kernel(const float* __restrict__ src, int rows, int cols,
-                                        float* __restrict__ dst) {
-  int c2 = cols / 2, r2 = rows / 2;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r2 * c2) return;
-  downsample_depth_px(src, cols, c2, dst, i);
-}
-
-__global__ void downsample_intensity_kernel(const float* __restrict__ src, int rows, int cols,
-                                            float* __restrict__ dst) {
-  int c2 = cols / 2, r2 = rows / 2;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r2 * c2) return;
-  downsample_intensity_px(src, cols, c2, dst, i);
+__device__ inline float mean4(float a, float b, float c, float d) {
+  return (((a + b) + c) + d) * 0.25f;
 }
 
 // creatPointCloudKernel (rgbdImage.cu:23-38) and vertextoNormal
@@ -250,61 +219,64 @@ __global__ void downsample_intensity_kernel(const float* __restrict__ src, int r
 // Vertices are recomputed from depth, so neighbours need no vertex map.  A
 // normal is 0 when the centre or a neighbour is invalid or outside the
 // row/image.
-__device__ inline void maps_px(const float* __restrict__ depth, float4* __restrict__ normal,
-                               float4* __restrict__ vertex, const DSensor& s, int i) {
-  const int y = i / s.cols, x = i - y * s.cols;
-  float d = depth[i];
-  float4 nrm = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (!(d > 0.0f)) {
-    normal[i] = nrm;
-    if (vertex) vertex[i] = nrm;
-    return;
-  }
-  F3 p = point3d_uv(x, y, d, s);
-  if (vertex) vertex[i] = make_float4(p.x, p.y, p.z, 1.0f);
-  if (x - 2 >= 0 && x + 2 < s.cols && y - 1 >= 0 && y + 1 < s.rows) {
-    int il = i - 2, ir = i + 2, iu = i - s.cols, id = i + s.cols;
-    float dl = depth[il], dr = depth[ir], du = depth[iu], dd = depth[id];
-    if (dl > 0.0f && dr > 0.0f && du > 0.0f && dd > 0.0f) {
-      F3 left = point3d_uv(x - 2, y, dl, s), right = point3d_uv(x + 2, y, dr, s);
-      F3 up = point3d_uv(x, y - 1, du, s), down = point3d_uv(x, y + 1, dd, s);
-      F3 c = cross3(right - left, down - up);
-      float dd2 = dot3(c, c);
-      if (dd2 > 0.0f) {
-        F3 n = c * (1.0f / sqrtf(dd2));
-        nrm = make_float4(n.x, n.y, n.z, 0.0f);
-      }
+//
+// The quotients by the focal lengths go through their reciprocals with an exact
+// correction (div_by) where no step can leave the normal range, else through
+// IEEE division.
+// (LevelCamera::ok: an offset u - cx is 0 or at least 2^-24 then.)
+__device__ inline bool moderate(float x) { return x >= kModerateMin && x <= kModerateMax; }
+__device__ inline F3 camera_point(const LevelCamera& c, int u, int v, float d, bool fast) {
+  if (!fast) return point3d_uv(u, v, d, c.s);
+  const float a = ((float)u - c.s.cx) * d, b = ((float)v - c.s.cy) * d;
+  return f3(div_by(a, c.s.fx, c.yhx, c.ylx), div_by(b, c.s.fy, c.yhy, c.yly), d);
+}
+
+// The normal of pixel (x, y), whose depth is d[0] in rows of 'pitch' floats
+// (neighbours are read only inside the level).
+__device__ inline float4 normal_at(const float* d, int pitch, const LevelCamera& c, int x, int y) {
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!(d[0] > 0.0f) || x < 2 || x + 2 >= c.s.cols || y < 1 || y + 1 >= c.s.rows) return none;
+  const float dl = d[-2], dr = d[2], du = d[-pitch], dd = d[pitch];
+  if (!(dl > 0.0f && dr > 0.0f && du > 0.0f && dd > 0.0f)) return none;
+  const bool fast = c.ok && fminf(fminf(dl, dr), fminf(du, dd)) >= kModerateMin &&
+                    fmaxf(fmaxf(dl, dr), fmaxf(du, dd)) <= kModerateMax;
+  const F3 left = camera_point(c, x - 2, y, dl, fast), right = camera_point(c, x + 2, y, dr, fast);
+  const F3 up = camera_point(c, x, y - 1, du, fast), down = camera_point(c, x, y + 1, dd, fast);
+  const F3 k = cross3(right - left, down - up);
+  const float k2 = dot3(k, k);
+  if (!(k2 > 0.0f)) return none;
+  const F3 n = k * (1.0f / sqrtf(k2));
+  return make_float4(n.x, n.y, n.z, 0.0f);
+}
+
+// one level, a 32x8 tile of pixels per CTA (the stage entry points: little
+// more than a launch, 6.1 us at 640x480 as without the tiles)
+constexpr int kMapTX = 32, kMapTY = 8;
+__global__ void __launch_bounds__(kMapTX * kMapTY)
+    maps_kernel(const float* __restrict__ depth, float4* __restrict__ normal,
+                float4* __restrict__ vertex, const LevelCamera c) {
+  const int x = blockIdx.x * kMapTX + threadIdx.x, y = blockIdx.y * kMapTY + threadIdx.y;
+  if (x >= c.s.cols || y >= c.s.rows) return;
+  const int i = y * c.s.cols + x;
+  if (vertex) {
+    const float d = depth[i];
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d > 0.0f) {
+      const F3 p = camera_point(c, x, y, d, c.ok && moderate(d));
+      v = make_float4(p.x, p.y, p.z, 1.0f);
     }
+    vertex[i] = v;
   }
-  normal[i] = nrm;
+  normal[i] = normal_at(depth + i, c.s.cols, c, x, y);
 }
 
-// all pyramid levels of one image in one launch
-__global__ void maps_kernel(MapsArgs a) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= a.total) return;
-  int l = 0;
-#pragma unroll
-  for (int k = 1; k < kLevels; ++k)
-    if (k < a.nlev && g >= a.lv[k].offset) l = k;
-  const LevelMaps& L = a.lv[l];
-  maps_px(L.depth, L.normal, L.vertex, L.s, g - L.offset);
-}
-
-__device__ inline void target_prepare_px(const float* __restrict__ ray, float* __restrict__ d0,
-                                         float dmax, const uint8_t* __restrict__ rgb,
-                                         float* __restrict__ inten, int i) {
-  float d = ray[i];
-  d0[i] = (d < dmax) ? d : 0.0f;
-  if (inten) inten[i] = rgb ? intensity_u8(rgb + 3 * (size_t)i) : 0.0f;
-}
-
-__global__ void target_prepare_kernel(const float* __restrict__ ray, float* __restrict__ d0,
-                                      float dmax, const uint8_t* __restrict__ rgb,
-                                      float* __restrict__ inten, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// raycast depth with its misses invalid
+__global__ void miss_to_zero_kernel(const float* __restrict__ ray, float* __restrict__ d0,
+                                    float dmax, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  target_prepare_px(ray, d0, dmax, rgb, inten, i);
+  const float d = ray[i];
+  d0[i] = (d < dmax) ? d : 0.0f;
 }
 
 // ---------------------------------------------------------------- fused
@@ -330,47 +302,91 @@ __device__ inline float pixel_distance(int x, int y, float d, const DSensor& s, 
   return d < t.dmax ? sd : -sd;
 }
 
-__global__ void fused_ingest_kernel(const SessDev* __restrict__ tab) {
+// A 32x8 pixel tile per CTA (four fine tiles of the ray bounds), which also
+//  * resets the frame's counters, its visible list and its ray depth bounds
+//    (near: no block, or 0 where unused; far: no block);
+//  * builds the free-space tile map of a depth-only frame of a carving session:
+//    per fine tile the least (sdist - truncation), 0 where a pixel's depth is
+//    outside the sensor range, and its minimum per coarse tile.  The coarse map
+//    is one of two by the frame's parity; each frame empties the other one.
+// Bound by latency (the pointers, a pixel's load, a division).  As three
+// kernels, the map's with a thread per tile, this took 31 us of a 320x240
+// frame, now 12-15; 19.4 -> 15 of a 640x480 one with colours.
+__global__ void __launch_bounds__(256) fused_ingest_kernel(const SessDev* __restrict__ tab,
+                                                           int* __restrict__ gcount) {
   const SessDev& S = tab[blockIdx.z];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= S.npx) return;
-  const uint8_t* rgb = *S.rgb_flag ? S.rgb : nullptr;
-  ingest_px(S.u16, rgb, S.depth_scaler, S.raw, S.use_color ? S.sint[0] : nullptr, i);
-  if (rgb) {
-    const uint8_t* c = rgb + 3 * (size_t)i;
-    S.rgb4[i] = (unsigned)c[0] | ((unsigned)c[1] << 8) | ((unsigned)c[2] << 16);
-  }
-  const float d = S.raw[i];
-  if (!S.bil_enabled) S.filt[i] = d;
   const DSensor& s0 = S.ls[0];
-  const int y = i / s0.cols;
-  S.sdist[i] = pixel_distance(i - y * s0.cols, y, d, s0, S.vol.t);
-}
-
-// The free-space tile map of a depth-only frame of a carving session (one
-// thread per fine tile; its value also enters its coarse tile's minimum).
-__global__ void fused_free_tiles_kernel(const SessDev* __restrict__ tab) {
-  const SessDev& S = tab[blockIdx.z];
-  if (!S.ftile || S.vol.t.band || *S.rgb_flag) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= S.rb_tx * S.rb_ty) return;
-  const DSensor& s = S.ls[0];
   const DTsdf& t = S.vol.t;
-  const int tx = i % S.rb_tx, ty = i / S.rb_tx;
-  const int x0 = tx * kRbTile, y0 = ty * kRbTile;
-  const int x1 = min(x0 + kRbTile, s.cols), y1 = min(y0 + kRbTile, s.rows);
-  float mn = 3.0e38f;
-  bool ok = true;
-  for (int y = y0; y < y1; ++y)
-    for (int x = x0; x < x1; ++x) {
-      const float d = S.raw[y * s.cols + x];
-      if (!(d >= t.dmin && d <= t.dmax)) ok = false;
-      else mn = fminf(mn, fabsf(S.sdist[y * s.cols + x]) - t.trunc);
+  if ((int)blockIdx.x * 32 >= s0.cols || (int)blockIdx.y * 8 >= s0.rows) return;
+  __shared__ unsigned least[4];
+  const int lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int x = blockIdx.x * 32 + lane, y = blockIdx.y * 8 + (tid >> 5);
+  const bool in = x < s0.cols && y < s0.rows;
+  const int i = y * s0.cols + x;
+  const unsigned raw = in ? S.u16[i] : 0u;
+  const uint8_t* rgb = *S.rgb_flag ? S.rgb : nullptr;
+  const bool free_map = S.ftile && !t.band && !rgb;
+  const int parity = S.pose->frame & 1;
+  if (tid < 4) least[tid] = 0x7f7f7f7fu;
+  unsigned word = 0x7f7f7f7fu;
+  if (in) {
+    const float d = (float)raw / S.depth_scaler;
+    const float sd = pixel_distance(x, y, d, s0, t);
+    if (S.use_color) S.sint[0][i] = rgb ? intensity_u8(rgb + 3 * (size_t)i) : 0.0f;
+    if (rgb) {
+      const uint8_t* c = rgb + 3 * (size_t)i;
+      S.rgb4[i] = (unsigned)c[0] | ((unsigned)c[1] << 8) | ((unsigned)c[2] << 16);
     }
-  const unsigned v = __float_as_uint(ok ? fmaxf(mn, 0.0f) : 0.0f);
-  S.ftile[i] = v;
-  const int cx = (S.rb_tx + kRbCoarse - 1) / kRbCoarse;
-  atomicMin(S.ftile + S.rb_tx * S.rb_ty + (ty / kRbCoarse) * cx + tx / kRbCoarse, v);
+    S.raw[i] = d;
+    if (!S.bil_enabled) S.filt[i] = d;
+    S.sdist[i] = sd;
+    const float room = fabsf(sd) - t.trunc;  // NaN: outside the range
+    word = room > 0.0f ? __float_as_uint(room) : 0u;
+  }
+  const int tx0 = blockIdx.x * 4, ty = blockIdx.y;
+  const int cx = (S.rb_tx + kRbCoarse - 1) / kRbCoarse, cy = (S.rb_ty + kRbCoarse - 1) / kRbCoarse;
+  unsigned* const coarse = S.ftile ? S.ftile + S.rb_tx * S.rb_ty : nullptr;
+  if (free_map) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) word = min(word, __shfl_xor_sync(0xffffffffu, word, o));
+    __syncthreads();
+    if ((lane & 7) == 0) atomicMin(&least[lane >> 3], word);
+    __syncthreads();
+  }
+  if (tid < 4 && tx0 + tid < S.rb_tx) {
+    const int tx = tx0 + tid, i = ty * S.rb_tx + tx;
+    const bool near_used = t.band || (S.vol.nonsat && S.vol.free_ok);
+    const unsigned nb = near_used ? 0x7f7f7f7fu : 0u;
+    const int c = (ty / kRbCoarse) * cx + tx / kRbCoarse;
+    const bool first = tx % kRbCoarse == 0 && ty % kRbCoarse == 0;
+    if (S.rbound) {
+      unsigned* const n8 = S.rbound;
+      unsigned* const n64 = n8 + 2 * S.rb_tx * S.rb_ty;
+      n8[i] = nb;
+      n8[S.rb_tx * S.rb_ty + i] = 0u;
+      if (first) {
+        n64[c] = nb;
+        n64[cx * cy + c] = 0u;
+      }
+    }
+    if (free_map) {
+      S.ftile[i] = least[tid];
+      atomicMin(coarse + parity * cx * cy + c, least[tid]);
+    }
+    if (coarse && first) coarse[(parity ^ 1) * cx * cy + c] = 0x7f7f7f7fu;
+  }
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 4) {
+    if (blockIdx.z == 0) *gcount = 0;
+    Counters* c = S.vol.cnt;  // all but nalloc, the heap top
+    c->new_blocks = 0;
+    c->bucket_full = 0;
+    c->heap_exhausted = 0;
+    c->dda_overruns = 0;
+    c->raycast_overruns = 0;
+    c->visible = 0;
+    c->unique_probed = 0;
+    c->icp_timeout = 0;
+  }
 }
 
 __global__ void fused_bilateral_kernel(const SessDev* __restrict__ tab) {
@@ -386,59 +402,194 @@ __global__ void fused_bilateral_kernel(const SessDev* __restrict__ tab) {
     bilateral_tile<false>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
 }
 
-// level l of the source (target == 0) or target pyramid from level l-1
-__global__ void fused_downsample_kernel(const SessDev* __restrict__ tab, int l, int target) {
+// ---- pyramid and normals of an image in one launch
+// A CTA owns 32x16 pixels of level 0 and what lies over them on levels 1 and 2.
+// It stages the level-0 depths with the halo that the level-2 normals need (8
+// columns, 4 rows), computes the upper levels of the halo again in shared
+// memory, and writes its own part of every level and its normals.  A tile this
+// small, because the chain of a CTA (loads, three levels, normals) is what a
+// frame waits for; six CTAs an SM hide each other's.  With a launch per level
+// and one for the normals (four or five per image) a 640x480 frame took 16.4 us
+// for the source and 20.6 for the target, now 12.3 and 15; 32 frames of 320x240
+// in four groups 80 and 110 us, now 62 and 67.  A fourth level (scale 8) is
+// made from level 2 by the two kernels below.
+//
+// what: 0 the frame's source (filtered depth and intensity are there); 1 the
+// frame's target: the raycast, misses invalid (mode 1), or the source (mode 0);
+// 2, 3 dyn_solver_solve's source (S.raw, colours S.rgb) and target (S.ray,
+// S.trgb), colours only with has_rgb.
+constexpr int kPyrX = 32, kPyrY = 16, kPyrHX = 8, kPyrHY = 4;
+constexpr int kP0W = kPyrX + 2 * kPyrHX, kP0H = kPyrY + 2 * kPyrHY;
+constexpr int kP1W = kP0W / 2, kP1H = kP0H / 2, kP2W = kP0W / 4, kP2H = kP0H / 4;
+__global__ void __launch_bounds__(256, 6)
+    fused_pyramid_kernel(const SessDev* __restrict__ tab, int what, int has_rgb) {
   const SessDev& S = tab[blockIdx.z];
-  if (l >= S.nlev) return;
-  const DSensor& sp = S.ls[l - 1];
-  const int c2 = sp.cols / 2, n = (sp.rows / 2) * c2;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  downsample_depth_px(target ? S.tdep[l - 1] : S.sdep[l - 1], sp.cols, c2,
-                      target ? S.tdep[l] : S.sdep[l], i);
-  if (S.use_color)
-    downsample_intensity_px(target ? S.tint[l - 1] : S.sint[l - 1], sp.cols, c2,
-                            target ? S.tint[l] : S.sint[l], i);
-}
-
-__global__ void fused_maps_kernel(const SessDev* __restrict__ tab, int target) {
-  const SessDev& S = tab[blockIdx.z];
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int l = 0; l < S.nlev; ++l) {
-    const int n = S.ls[l].rows * S.ls[l].cols;
-    if (g < n) {
-      float4* vtx = S.debug_maps ? (target ? S.tvtx[l] : S.svtx[l]) : nullptr;
-      maps_px(target ? S.tdep[l] : S.sdep[l], target ? S.tnrm[l] : S.snrm[l], vtx, S.ls[l], g);
-      return;
+  const DSensor& s0 = S.ls[0];
+  const int X0 = blockIdx.x * kPyrX, Y0 = blockIdx.y * kPyrY;
+  if (X0 >= s0.cols || Y0 >= s0.rows) return;
+  __shared__ float d0[kP0H * kP0W], d1[kP1H * kP1W], d2[kP2H * kP2W];
+  __shared__ float i0[kPyrY * kPyrX], i1[kPyrY * kPyrX / 4];
+  const int tid = threadIdx.x;
+  const bool target = (what & 1) != 0, frame = what < 2;
+  const bool copy = what == 1 && S.mode != 1;  // frame-to-frame: the source is the target
+  const float* in = what == 0 ? S.sdep[0] : (what == 1 ? (copy ? S.sdep[0] : S.ray)
+                                                       : (what == 2 ? S.raw : S.ray));
+  const float limit = what == 1 && !copy ? S.vol.t.dmax : 3.402823466e+38f;
+  float* const out0 = what == 0 ? nullptr : (target ? S.tdep[0] : S.sdep[0]);
+  const int nlev = min(S.nlev, 3);
+  if (target && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) S.icp->have_target = 1;
+  // all loads before the first store (a store could be to what they read)
+  // (a warp per row of the staged depths: 24 rows of 48)
+  constexpr int kOwn = kPyrY * kPyrX / 256, kRows = kP0H / 8;
+  static_assert(kP0H % 8 == 0 && kP0W > 32 && kP0W <= 64 && kPyrX == 32, "row mapping");
+  const int lane = tid & 31, warp = tid >> 5;
+  const bool colour = S.use_color != 0, gray = what == 0 || copy;
+  const uint8_t* rgb = colour && !gray && (frame || has_rgb) ? (target ? S.trgb : S.rgb) : nullptr;
+  float dv[kRows][2], iv[kOwn];
+  const int xa = X0 - kPyrHX + lane, xb = xa + 32;
+  const bool ina = xa >= 0 && xa < s0.cols, inb = lane < kP0W - 32 && xb < s0.cols;
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int y = Y0 - kPyrHY + warp + j * 8;
+    const bool iny = y >= 0 && y < s0.rows;
+    const float* a = in + y * s0.cols + xa;
+    dv[j][0] = ina && iny ? a[0] : 0.0f;
+    dv[j][1] = inb && iny ? a[32] : 0.0f;
+  }
+#pragma unroll
+  for (int j = 0; j < kOwn; ++j) {
+    const int y = Y0 + warp + j * 8, x = X0 + lane, i = y * s0.cols + x;
+    iv[j] = 0.0f;
+    if (colour && x < s0.cols && y < s0.rows)
+      iv[j] = gray ? S.sint[0][i] : (rgb ? intensity_u8(rgb + 3 * (size_t)i) : 0.0f);
+  }
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int r = warp + j * 8, y = Y0 - kPyrHY + r;
+    float a = dv[j][0], b = dv[j][1];
+    if (what != 0 && !copy) {
+      a = a < limit ? a : 0.0f;
+      b = b < limit ? b : 0.0f;
     }
-    g -= n;
+    d0[r * kP0W + lane] = a;
+    if (lane < kP0W - 32) d0[r * kP0W + 32 + lane] = b;
+    if (out0 && r >= kPyrHY && r < kPyrHY + kPyrY && y < s0.rows) {
+      if (lane >= kPyrHX && xa < s0.cols) out0[y * s0.cols + xa] = a;
+      if (lane < kPyrHX && xb < s0.cols) out0[y * s0.cols + xb] = b;
+    }
+  }
+  if (colour) {
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      const int k = tid + j * 256, y = Y0 + k / kPyrX, x = X0 + k % kPyrX;
+      i0[k] = iv[j];
+      if (what != 0 && x < s0.cols && y < s0.rows)
+        (target ? S.tint[0] : S.sint[0])[y * s0.cols + x] = iv[j];
+    }
+  }
+  __syncthreads();
+  if (nlev > 1) {
+    const DSensor& s = S.ls[1];
+    for (int r = warp, c = lane; r < kP1H && c < kP1W; r += 8) {
+      const int y = Y0 / 2 - kPyrHY / 2 + r, x = X0 / 2 - kPyrHX / 2 + c;
+      float d = 0.0f;
+      if (x >= 0 && y >= 0 && x < s.cols && y < s.rows) {
+        const float* a = d0 + 2 * r * kP0W + 2 * c;
+        d = mean_valid(a[0], a[1], a[kP0W], a[kP0W + 1]);
+        if (r >= kPyrHY / 2 && r < (kPyrHY + kPyrY) / 2 && c >= kPyrHX / 2 && c < (kPyrHX + kPyrX) / 2)
+          (target ? S.tdep[1] : S.sdep[1])[y * s.cols + x] = d;
+      }
+      d1[r * kP1W + c] = d;
+    }
+    if (colour && tid < kPyrY * kPyrX / 4) {
+      const int r = tid / (kPyrX / 2), c = tid % (kPyrX / 2), y = Y0 / 2 + r, x = X0 / 2 + c;
+      const float* a = i0 + 2 * r * kPyrX + 2 * c;
+      const float v = mean4(a[0], a[1], a[kPyrX], a[kPyrX + 1]);
+      i1[tid] = v;
+      if (x < s.cols && y < s.rows) (target ? S.tint[1] : S.sint[1])[y * s.cols + x] = v;
+    }
+    __syncthreads();
+  }
+  if (nlev > 2) {
+    const DSensor& s = S.ls[2];
+    if (tid < kP2H * kP2W) {
+      const int r = tid / kP2W, c = tid - r * kP2W;
+      const int y = Y0 / 4 - kPyrHY / 4 + r, x = X0 / 4 - kPyrHX / 4 + c;
+      float d = 0.0f;
+      if (x >= 0 && y >= 0 && x < s.cols && y < s.rows) {
+        const float* a = d1 + 2 * r * kP1W + 2 * c;
+        d = mean_valid(a[0], a[1], a[kP1W], a[kP1W + 1]);
+        if (r >= kPyrHY / 4 && r < (kPyrHY + kPyrY) / 4 && c >= kPyrHX / 4 && c < (kPyrHX + kPyrX) / 4)
+          (target ? S.tdep[2] : S.sdep[2])[y * s.cols + x] = d;
+      }
+      d2[tid] = d;
+    } else if (colour && tid >= 128 && tid < 128 + kPyrY * kPyrX / 16) {
+      const int k = tid - 128, r = k / (kPyrX / 4), c = k % (kPyrX / 4);
+      const int y = Y0 / 4 + r, x = X0 / 4 + c;
+      const float* a = i1 + 2 * r * (kPyrX / 2) + 2 * c;
+      if (x < s.cols && y < s.rows)
+        (target ? S.tint[2] : S.sint[2])[y * s.cols + x] =
+            mean4(a[0], a[1], a[kPyrX / 2], a[kPyrX / 2 + 1]);
+    }
+    __syncthreads();
+  }
+  // normals: level 0, then the upper levels by the threads it leaves
+  float4* const* nrm = target ? S.tnrm : S.snrm;
+  {
+    const LevelCamera& c = S.cam[0];
+#pragma unroll
+    for (int k = 0; k < kPyrY * kPyrX; k += 256) {
+      const int r = (k + tid) / kPyrX, q = (k + tid) % kPyrX, y = Y0 + r, x = X0 + q;
+      if (x < s0.cols && y < s0.rows)
+        nrm[0][y * s0.cols + x] =
+            normal_at(d0 + (r + kPyrHY) * kP0W + q + kPyrHX, kP0W, c, x, y);
+    }
+  }
+  if (nlev > 1 && tid < kPyrY * kPyrX / 4) {
+    const LevelCamera& c = S.cam[1];
+    const int r = tid / (kPyrX / 2), q = tid % (kPyrX / 2), y = Y0 / 2 + r, x = X0 / 2 + q;
+    if (x < c.s.cols && y < c.s.rows)
+      nrm[1][y * c.s.cols + x] =
+          normal_at(d1 + (r + kPyrHY / 2) * kP1W + q + kPyrHX / 2, kP1W, c, x, y);
+  } else if (nlev > 2 && tid >= 128 && tid < 128 + kPyrY * kPyrX / 16) {
+    const LevelCamera& c = S.cam[2];
+    const int k = tid - 128, r = k / (kPyrX / 4), q = k % (kPyrX / 4);
+    const int y = Y0 / 4 + r, x = X0 / 4 + q;
+    if (x < c.s.cols && y < c.s.rows)
+      nrm[2][y * c.s.cols + x] =
+          normal_at(d2 + (r + kPyrHY / 4) * kP2W + q + kPyrHX / 4, kP2W, c, x, y);
   }
 }
 
-// next frame's target level 0: the raycast (mode 1, misses -> 0) or the
-// source itself (mode 0); flags the target as present
-__global__ void fused_target_prepare_kernel(const SessDev* __restrict__ tab) {
+// level 3 of the sessions that have it, from level 2; then its normals
+__global__ void fused_level3_kernel(const SessDev* __restrict__ tab, int target) {
   const SessDev& S = tab[blockIdx.z];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) S.icp->have_target = 1;
-  if (i >= S.npx) return;
-  if (S.mode == 1) {
-    target_prepare_px(S.ray, S.tdep[0], S.vol.t.dmax, S.use_color ? S.trgb : nullptr,
-                      S.use_color ? S.tint[0] : nullptr, i);
-  } else {
-    S.tdep[0][i] = S.sdep[0][i];
-    if (S.use_color) S.tint[0][i] = S.sint[0][i];
+  if (S.nlev < 4) return;
+  const DSensor &s = S.ls[3], &p = S.ls[2];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.rows * s.cols) return;
+  const int y = i / s.cols, x = i - y * s.cols, j = 2 * y * p.cols + 2 * x;
+  const float* a = (target ? S.tdep[2] : S.sdep[2]) + j;
+  (target ? S.tdep[3] : S.sdep[3])[i] = mean_valid(a[0], a[1], a[p.cols], a[p.cols + 1]);
+  if (S.use_color) {
+    const float* b = (target ? S.tint[2] : S.sint[2]) + j;
+    (target ? S.tint[3] : S.sint[3])[i] = mean4(b[0], b[1], b[p.cols], b[p.cols + 1]);
   }
+}
+__global__ void fused_level3_normals_kernel(const SessDev* __restrict__ tab, int target) {
+  const SessDev& S = tab[blockIdx.z];
+  if (S.nlev < 4) return;
+  const LevelCamera& c = S.cam[3];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.s.rows * c.s.cols) return;
+  const int y = i / c.s.cols, x = i - y * c.s.cols;
+  (target ? S.tnrm[3] : S.snrm[3])[i] =
+      normal_at((target ? S.tdep[3] : S.sdep[3]) + i, c.s.cols, c, x, y);
 }
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
-
-void launch_ingest(const uint16_t* raw, const uint8_t* rgb, int n, float scaler,
-                   float* depth_out, float* intensity_out, cudaStream_t st) {
-  ingest_kernel<<<nblk(n, 256), 256, 0, st>>>(raw, rgb, n, scaler, depth_out, intensity_out);
-}
 
 // pyramid::gaussian, pyramid.cu:208-211, in double.
 static double gaussian_d(double x, double sigma) {
@@ -487,31 +638,20 @@ void launch_bilateral(const float* src, float* dst, int rows, int cols, const Bi
                      bilateral_smem(tb.radius, ty), st>>>(src, dst, rows, cols, tb);
 }
 
-void launch_downsample_depth(const float* src, int rows, int cols, float* dst, cudaStream_t st) {
-  int n = (rows / 2) * (cols / 2);
-  if (n > 0) downsample_depth_kernel<<<nblk(n, 256), 256, 0, st>>>(src, rows, cols, dst);
+void launch_maps(const float* depth, const DSensor& s, float4* normal, float4* vertex,
+                 cudaStream_t st) {
+  maps_kernel<<<dim3(nblk(s.cols, kMapTX), nblk(s.rows, kMapTY)), dim3(kMapTX, kMapTY), 0, st>>>(
+      depth, normal, vertex, level_camera(s));
 }
-void launch_downsample_intensity(const float* src, int rows, int cols, float* dst,
-                                 cudaStream_t st) {
-  int n = (rows / 2) * (cols / 2);
-  if (n > 0) downsample_intensity_kernel<<<nblk(n, 256), 256, 0, st>>>(src, rows, cols, dst);
-}
-void launch_maps(const MapsArgs& a, cudaStream_t st) {
-  if (a.total > 0) maps_kernel<<<nblk(a.total, 256), 256, 0, st>>>(a);
-}
-void launch_target_prepare(const float* ray_depth, float* depth0, float dmax, const uint8_t* rgb,
-                           float* intensity0, int n, cudaStream_t st) {
-  target_prepare_kernel<<<nblk(n, 256), 256, 0, st>>>(ray_depth, depth0, dmax, rgb, intensity0,
-                                                      n);
-}
-void launch_copy_f(const float* src, float* dst, size_t n, cudaStream_t st) {
-  if (n) cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, st);
+void launch_miss_to_zero(const float* ray_depth, float* depth0, float dmax, int n,
+                         cudaStream_t st) {
+  miss_to_zero_kernel<<<nblk(n, 256), 256, 0, st>>>(ray_depth, depth0, dmax, n);
 }
 
 // ---- fused stages
 void fused_ingest(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  fused_ingest_kernel<<<dim3(nblk(b.max_npx, 256), 1, b.n), 256, 0, st>>>(tab);
-  fused_free_tiles_kernel<<<dim3(nblk(b.max_rb_tiles, 128), 1, b.n), 128, 0, st>>>(tab);
+  fused_ingest_kernel<<<dim3(nblk(b.max_cols, 32), nblk(b.max_rows, 8), b.n), 256, 0, st>>>(
+      tab, b.gcount);
 }
 
 void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
@@ -521,18 +661,15 @@ void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
                            bilateral_smem(b.max_bil_radius, ty), st>>>(tab);
 }
 
-void fused_pyramid(const SessDev* tab, const BatchShape& b, int target, cudaStream_t st) {
-  for (int l = 1; l < b.max_nlev; ++l)
-    if (b.max_level_px[l] > 0)
-      fused_downsample_kernel<<<dim3(nblk(b.max_level_px[l], 256), 1, b.n), 256, 0, st>>>(
-          tab, l, target);
-  int tot = 0;
-  for (int l = 0; l < b.max_nlev; ++l) tot += b.max_level_px[l];
-  fused_maps_kernel<<<dim3(nblk(tot, 256), 1, b.n), 256, 0, st>>>(tab, target);
-}
-
-void fused_target_prepare(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  fused_target_prepare_kernel<<<dim3(nblk(b.max_npx, 256), 1, b.n), 256, 0, st>>>(tab);
+void fused_pyramid(const SessDev* tab, const BatchShape& b, int what, int has_rgb,
+                   cudaStream_t st) {
+  fused_pyramid_kernel<<<dim3(nblk(b.max_cols, kPyrX), nblk(b.max_rows, kPyrY), b.n), 256, 0,
+                         st>>>(tab, what, has_rgb);
+  if (b.max_nlev > 3 && b.max_level_px[3] > 0) {
+    const dim3 grid(nblk(b.max_level_px[3], 256), 1, b.n);
+    fused_level3_kernel<<<grid, 256, 0, st>>>(tab, what & 1);
+    fused_level3_normals_kernel<<<grid, 256, 0, st>>>(tab, what & 1);
+  }
 }
 
 }  // namespace dyn

@@ -30,13 +30,17 @@ constexpr int kVisFree = 1 << 30;
 // Free-space tile map of a depth-only frame: per fine 8x8-pixel tile, then
 // per coarse tile, the least (sdist - truncation) over its pixels as float
 // bits, 0 where a pixel's depth is outside the sensor range (negative
-// values count as 0).
+// values count as 0).  Two coarse maps, by the frame's parity.
+inline __host__ __device__ int coarse_tiles(int tiles_x, int tiles_y) {
+  return ((tiles_x + kRbCoarse - 1) / kRbCoarse) * ((tiles_y + kRbCoarse - 1) / kRbCoarse);
+}
 inline __host__ __device__ int free_tile_words(int tiles_x, int tiles_y) {
-  return ray_bounds_words(tiles_x, tiles_y) / 2;
+  return tiles_x * tiles_y + 2 * coarse_tiles(tiles_x, tiles_y);
 }
 
 struct SessDev {
   DSensor ls[kLevels];  // level sensors (scale 1, 2, 4, 8)
+  LevelCamera cam[kLevels];
   int nlev;             // levels in use
   int npx;              // level-0 pixels
   float depth_scaler;
@@ -44,7 +48,6 @@ struct SessDev {
   int use_color;        // photometric term on (intensity / colour images kept)
   int bil_enabled;
   int mode;             // 0 frame-to-frame, 1 frame-to-model
-  int debug_maps;       // also write vertex maps
   // frame input (device copies)
   const uint16_t* u16;
   const uint8_t* rgb;
@@ -55,11 +58,9 @@ struct SessDev {
   float* filt;
   float* sdep[kLevels];
   float4* snrm[kLevels];
-  float4* svtx[kLevels];
   float* sint[kLevels];
   float* tdep[kLevels];
   float4* tnrm[kLevels];
-  float4* tvtx[kLevels];
   float* tint[kLevels];
   float* ray;
   uint8_t* trgb;
@@ -115,15 +116,15 @@ struct BatchShape {
 // image.cu
 void fused_ingest(const SessDev* tab, const BatchShape& b, cudaStream_t st);
 void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st);
-void fused_pyramid(const SessDev* tab, const BatchShape& b, int target, cudaStream_t st);
-void fused_target_prepare(const SessDev* tab, const BatchShape& b, cudaStream_t st);
+// what: 0, 1 the frame's source and target; 2, 3 dyn_solver_solve's
+void fused_pyramid(const SessDev* tab, const BatchShape& b, int what, int has_rgb,
+                   cudaStream_t st);
 // icp.cu
 void fused_icp_iteration(const SessDev* tab, const BatchShape& b, int slot, int it, bool chained,
                          cudaStream_t st);
 void fused_pose_finalize(const SessDev* tab, const BatchShape& b, int bump, cudaStream_t st);
 void fused_icp_persistent(const SessDev* tab, const BatchShape& b, cudaStream_t st);
 // tsdf.cu
-void fused_reset_counters(const SessDev* tab, const BatchShape& b, cudaStream_t st);
 void fused_allocate(const SessDev* tab, const BatchShape& b, cudaStream_t st);
 void fused_visible(const SessDev* tab, const BatchShape& b, cudaStream_t st);
 void fused_integrate(const SessDev* tab, const BatchShape& b, cudaStream_t st);

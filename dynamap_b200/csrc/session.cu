@@ -85,25 +85,6 @@ void release(dyn_session* s) {
   delete s;
 }
 
-MapsArgs maps_args(dyn_session* s, bool target) {
-  MapsArgs a;
-  int off = 0;
-  for (int l = 0; l < s->nlev; ++l) {
-    a.lv[l].depth = target ? s->d_tdep[l] : s->d_sdep[l];
-    a.lv[l].normal = target ? s->d_tnrm[l] : s->d_snrm[l];
-    a.lv[l].vertex = s->debug_maps ? (target ? s->d_tvtx[l] : s->d_svtx[l]) : nullptr;
-    a.lv[l].s = s->ls[l];
-    a.lv[l].offset = off;
-    off += s->ls[l].rows * s->ls[l].cols;
-  }
-  a.nlev = s->nlev;
-  a.total = off;
-  return a;
-}
-
-__global__ void mark_target_kernel(IcpState* st) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) st->have_target = 1;
-}
 __global__ void bump_frame_kernel(PoseState* ps) {
   if (threadIdx.x == 0 && blockIdx.x == 0) ps->frame += 1;
 }
@@ -129,12 +110,11 @@ __global__ void gather_results_kernel(const SessDev* __restrict__ tab, int n,
 // Source side of a frame: ingest, bilateral filter, pyramid, normal maps.
 void enqueue_source(const SessDev* tab, const BatchShape& b, cudaStream_t st, const Marks& m) {
   m(DYN_STAGE_FRAME);
-  fused_reset_counters(tab, b, st);
   fused_ingest(tab, b, st);
   m(DYN_STAGE_INGEST);
   fused_bilateral(tab, b, st);
   m(DYN_STAGE_BILATERAL);
-  fused_pyramid(tab, b, 0, st);
+  fused_pyramid(tab, b, 0, 0, st);
   m(DYN_STAGE_SOURCE_MAPS);
 }
 
@@ -166,8 +146,7 @@ void enqueue_map_update(const SessDev* tab, const BatchShape& b, cudaStream_t st
   m(DYN_STAGE_INTEGRATE);
   fused_raycast(tab, b, st);
   m(DYN_STAGE_RAYCAST);
-  fused_target_prepare(tab, b, st);
-  fused_pyramid(tab, b, 1, st);
+  fused_pyramid(tab, b, 1, 0, st);
   m(DYN_STAGE_TARGET_MAPS);
 }
 
@@ -303,7 +282,10 @@ void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget
 void fill_sessdev(dyn_session* s) {
   SessDev& d = s->hsd;
   std::memset(&d, 0, sizeof(d));
-  for (int l = 0; l < kLevels; ++l) d.ls[l] = s->ls[l];
+  for (int l = 0; l < kLevels; ++l) {
+    d.ls[l] = s->ls[l];
+    d.cam[l] = level_camera(s->ls[l]);
+  }
   d.nlev = s->nlev;
   d.npx = (int)s->npx;
   d.depth_scaler = s->sensor.depth_scaler;
@@ -311,7 +293,6 @@ void fill_sessdev(dyn_session* s) {
   d.use_color = s->use_color() ? 1 : 0;
   d.bil_enabled = s->bp.enabled ? 1 : 0;
   d.mode = s->gp.mode;
-  d.debug_maps = 0;
   d.u16 = s->d_u16;
   d.rgb = s->d_rgb;
   d.raw = s->d_raw;
@@ -321,11 +302,9 @@ void fill_sessdev(dyn_session* s) {
   for (int l = 0; l < s->nlev; ++l) {
     d.sdep[l] = s->d_sdep[l];
     d.snrm[l] = s->d_snrm[l];
-    d.svtx[l] = s->d_svtx[l];
     d.sint[l] = s->d_sint[l];
     d.tdep[l] = s->d_tdep[l];
     d.tnrm[l] = s->d_tnrm[l];
-    d.tvtx[l] = s->d_tvtx[l];
     d.tint[l] = s->d_tint[l];
   }
   d.ray = s->d_ray;
@@ -561,6 +540,9 @@ void fill_stats(const dyn_session* s, const ResultBlock& r, dyn_frame_stats* st)
 dyn_status reset_state(dyn_session* s, bool sync = true) {
   cudaStream_t st = s->stream;
   launch_volume_clear(s->vol, st);
+  // both coarse free-space maps: no tile yet
+  DYN_CUDA(cudaMemsetAsync(s->d_ftile, 0x7f,
+                           sizeof(unsigned) * (size_t)free_tile_words(s->rb_tx, s->rb_ty), st));
   // no row carries a tag of the first epoch
   DYN_CUDA(cudaMemsetAsync(s->d_partials, 0, icp_frame_scratch_bytes(), st));
   unsigned bar[kIcpBarWords] = {kIcpEpochStep};
@@ -1027,7 +1009,6 @@ dyn_status dyn_solver_solve(dyn_session* s, const float* target_depth_host,
   cudaStream_t st = s->stream;
   const size_t n = s->npx;
   const bool col = s->use_color();
-  const float inf = 3.402823466e+38f;
   dyn_status r = dyn_session_set_pose(s, pose_inout);
   if (r != DYN_OK) return r;
   // target: images as given (the reference solves on raw images,
@@ -1035,27 +1016,12 @@ dyn_status dyn_solver_solve(dyn_session* s, const float* target_depth_host,
   DYN_CUDA(cudaMemcpyAsync(s->d_ray, target_depth_host, n * 4, cudaMemcpyHostToDevice, st));
   if (col && target_rgb_host)
     DYN_CUDA(cudaMemcpyAsync(s->d_trgb, target_rgb_host, n * 3, cudaMemcpyHostToDevice, st));
-  launch_target_prepare(s->d_ray, s->d_tdep[0], inf, (col && target_rgb_host) ? s->d_trgb : nullptr,
-                        col ? s->d_tint[0] : nullptr, (int)n, st);
   // source
   DYN_CUDA(cudaMemcpyAsync(s->d_raw, source_depth_host, n * 4, cudaMemcpyHostToDevice, st));
   if (col && source_rgb_host)
     DYN_CUDA(cudaMemcpyAsync(s->d_rgb, source_rgb_host, n * 3, cudaMemcpyHostToDevice, st));
-  launch_target_prepare(s->d_raw, s->d_sdep[0], inf, (col && source_rgb_host) ? s->d_rgb : nullptr,
-                        col ? s->d_sint[0] : nullptr, (int)n, st);
-  for (int l = 1; l < s->nlev; ++l) {
-    launch_downsample_depth(s->d_tdep[l - 1], s->ls[l - 1].rows, s->ls[l - 1].cols, s->d_tdep[l], st);
-    launch_downsample_depth(s->d_sdep[l - 1], s->ls[l - 1].rows, s->ls[l - 1].cols, s->d_sdep[l], st);
-    if (col) {
-      launch_downsample_intensity(s->d_tint[l - 1], s->ls[l - 1].rows, s->ls[l - 1].cols,
-                                  s->d_tint[l], st);
-      launch_downsample_intensity(s->d_sint[l - 1], s->ls[l - 1].rows, s->ls[l - 1].cols,
-                                  s->d_sint[l], st);
-    }
-  }
-  launch_maps(maps_args(s, true), st);
-  launch_maps(maps_args(s, false), st);
-  mark_target_kernel<<<1, 32, 0, st>>>(s->d_icp);
+  fused_pyramid(s->d_sd, s->shape, 3, col && target_rgb_host ? 1 : 0, st);
+  fused_pyramid(s->d_sd, s->shape, 2, col && source_rgb_host ? 1 : 0, st);
   enqueue_icp(s->d_sd, s->shape, st);
   fused_pose_finalize(s->d_sd, s->shape, 0, st);
   gather_results_kernel<<<1, 128, 0, st>>>(s->d_sd, 1, nullptr, s->d_res);
@@ -1104,17 +1070,8 @@ dyn_status dyn_raycast_maps(dyn_session* s, const float pose[16], const dyn_sens
                  rgb_host ? s->d_trgb : nullptr, raycast_grid_fits(s, vs), st);
   // misses (at max_sensor_depth or beyond) become invalid depth, then the
   // maps of that depth in the raycast camera's frame
-  launch_target_prepare(s->d_ray, s->d_filt, s->tp.max_sensor_depth, nullptr, nullptr, (int)n,
-                        st);
-  MapsArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.lv[0].depth = s->d_filt;
-  a.lv[0].normal = s->d_snrm[0];
-  a.lv[0].vertex = s->d_svtx[0];
-  a.lv[0].s = dsensor(vs);
-  a.nlev = 1;
-  a.total = (int)n;
-  launch_maps(a, st);
+  launch_miss_to_zero(s->d_ray, s->d_filt, s->tp.max_sensor_depth, (int)n, st);
+  launch_maps(s->d_filt, dsensor(vs), s->d_snrm[0], s->d_svtx[0], st);
   DYN_CUDA(cudaGetLastError());
   if (depth_host)
     DYN_CUDA(cudaMemcpyAsync(depth_host, s->d_ray, n * 4, cudaMemcpyDeviceToHost, st));
@@ -1248,11 +1205,11 @@ dyn_status dyn_debug_image(dyn_session* s, int32_t which, int32_t level, void* h
     default: return DYN_ERR_INVALID_ARG;
   }
   if (bytes < nb) return DYN_ERR_INVALID_ARG;
-  if ((which == 3 || which == 6) && !s->debug_maps) {
-    // vertex maps are only written in debug mode: recompute them now
-    s->debug_maps = true;
-    launch_maps(maps_args(s, which == 6), s->stream);
-    s->debug_maps = false;
+  if (which == 3 || which == 6) {  // vertex maps are not kept: made now
+    const bool t = which == 6;
+    launch_maps(t ? s->d_tdep[level] : s->d_sdep[level], s->ls[level],
+                t ? s->d_tnrm[level] : s->d_snrm[level], t ? s->d_tvtx[level] : s->d_svtx[level],
+                s->stream);
   }
   DYN_CUDA(cudaMemcpyAsync(host_out, src, nb, cudaMemcpyDeviceToHost, s->stream));
   DYN_CUDA(cudaStreamSynchronize(s->stream));
@@ -1353,16 +1310,8 @@ dyn_status dyn_depth_to_maps_host(const float* depth_host, const dyn_sensor* lev
 dyn_status dyn_depth_to_maps(const float* depth_dev, const dyn_sensor* level, float* vertex4_dev,
                              float* normal4_dev, void* stream) {
   if (!depth_dev || !valid_sensor(level) || !normal4_dev) return DYN_ERR_INVALID_ARG;
-  MapsArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.lv[0].depth = depth_dev;
-  a.lv[0].normal = reinterpret_cast<float4*>(normal4_dev);
-  a.lv[0].vertex = reinterpret_cast<float4*>(vertex4_dev);
-  a.lv[0].s = dsensor(*level);
-  a.lv[0].offset = 0;
-  a.nlev = 1;
-  a.total = (int)(level->rows * level->cols);
-  launch_maps(a, (cudaStream_t)stream);
+  launch_maps(depth_dev, dsensor(*level), reinterpret_cast<float4*>(normal4_dev),
+              reinterpret_cast<float4*>(vertex4_dev), (cudaStream_t)stream);
   DYN_CUDA(cudaGetLastError());
   return DYN_OK;
 }

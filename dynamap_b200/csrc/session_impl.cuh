@@ -170,7 +170,6 @@ struct dyn_session {
   double stage_ms[DYN_NUM_STAGES] = {};
   int64_t prof_frames = 0;
   int kernels_per_frame = 0;
-  bool debug_maps = false;
   int frames = 0;
   bool pending = false;  // a frame submitted whose result has not been read
   // Two frames in flight (dyn_frame_submit before the previous frame's

@@ -33,16 +33,6 @@ namespace {
 constexpr float kRint = 12582912.0f;   // 1.5 * 2^23
 constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
 
-// a / b by b's hoisted reciprocal: yh = fl(1/b), yl the rest of 1/b;
-// q = fl(a * yh + fl(a * yl)) is within an ulp of a / b, and
-// fma(fma(-b, q, a), yh, q) is then the correctly rounded quotient (Markstein,
-// IBM J. Res. Dev. 34, 1990) unless a step under- or overflows.  A zero
-// dividend gives zero (of either sign).
-__device__ inline float div_by(float a, float b, float yh, float yl) {
-  const float q = __fmaf_rn(a, yh, __fmul_rn(a, yl));
-  return __fmaf_rn(__fmaf_rn(-b, q, a), yh, q);
-}
-
 // ------------------------------------------------------------ the block grid
 // The raycast looks blocks up by their coordinates far more often than
 // anything else (every sample, up to eight blocks), so each frame's blocks are
@@ -458,7 +448,7 @@ __device__ inline void bound_block(unsigned long long key, const DTsdf& t, const
 // more than 16 coarse tiles (close to the camera) take the per-voxel test.
 __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, const DSensor& s,
                                         const M4f& invT, const unsigned* __restrict__ ftile,
-                                        int tiles_x, int tiles_y) {
+                                        int tiles_x, int tiles_y, int parity) {
   const float vs = t.vs, e = 7.0f * vs;
   const float ox = (float)key_x(key) * vs * (float)kBlockSize,
               oy = (float)key_y(key) * vs * (float)kBlockSize,
@@ -485,7 +475,7 @@ __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, 
   const unsigned* m = ftile;
   int tw = tiles_x;
   if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > 16) {
-    m = ftile + tiles_x * tiles_y;
+    m = ftile + tiles_x * tiles_y + parity * coarse_tiles(tiles_x, tiles_y);
     tw = (tiles_x + kRbCoarse - 1) / kRbCoarse;
     tx0 /= kRbCoarse;
     tx1 /= kRbCoarse;
@@ -540,7 +530,9 @@ __global__ void fused_visible_kernel(const SessDev* __restrict__ tab, int2* __re
     }
     bool fr = false;
     if (vis && S.ftile && !v.t.band && !*S.rgb_flag)
-      fr = free_space_block(v.block_keys[i], v.t, S.ls[0], invT, S.ftile, S.rb_tx, S.rb_ty);
+      // (the frame counter has advanced since the ingest made the map)
+      fr = free_space_block(v.block_keys[i], v.t, S.ls[0], invT, S.ftile, S.rb_tx, S.rb_ty,
+                            (S.pose->frame - 1) & 1);
     unsigned m = __ballot_sync(0xffffffffu, vis);
     int off = 0;
     if (lane == 0 && m) {
@@ -1828,42 +1820,6 @@ void launch_fused_raycast(const SessDev* tab, const BatchShape& b, cudaStream_t 
   if (b.fp16_mask & 2) fused_raycast_kernel<true, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
 }
 
-// per-frame counters of every session (all but nalloc, the heap top) and
-// the batch visible list
-// (and the ray depth bounds to "no block")
-__global__ void fused_reset_counters_kernel(const SessDev* __restrict__ tab,
-                                            int* __restrict__ gcount) {
-  const SessDev& S = tab[blockIdx.z];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (S.rbound) {
-    // near: no block (3.4e38), or 0 where unused; far: no block (0)
-    const bool near_used = S.vol.t.band || (S.vol.nonsat && S.vol.free_ok);
-    const unsigned nb = near_used ? 0x7f7f7f7fu : 0u;
-    const RayBounds B = ray_bounds(S.rbound, S.rb_tx, S.rb_ty);
-    if (i < S.rb_tx * S.rb_ty) {
-      B.near8[i] = nb;
-      B.far8[i] = 0u;
-    }
-    if (i < B.cx * B.cy) {
-      B.near64[i] = nb;
-      B.far64[i] = 0u;
-    }
-  }
-  if (S.ftile && i < ((S.rb_tx + kRbCoarse - 1) / kRbCoarse) * ((S.rb_ty + kRbCoarse - 1) / kRbCoarse))
-    S.ftile[S.rb_tx * S.rb_ty + i] = 0x7f7f7f7fu;  // coarse free-space tiles: min of none
-  if (i != 0) return;
-  if (blockIdx.z == 0) *gcount = 0;
-  Counters* c = S.vol.cnt;
-  c->new_blocks = 0;
-  c->bucket_full = 0;
-  c->heap_exhausted = 0;
-  c->dda_overruns = 0;
-  c->raycast_overruns = 0;
-  c->visible = 0;
-  c->unique_probed = 0;
-  c->icp_timeout = 0;
-}
-
 __global__ void clear_entries_kernel(Entry* e, size_t n) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1935,11 +1891,6 @@ void launch_find_blocks(const VolumeDev& v, const int* coords, int n, int* ptr_o
 }
 
 // ---- fused stages
-void fused_reset_counters(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  fused_reset_counters_kernel<<<dim3(nblk(b.max_rb_tiles, 256), 1, b.n), 256, 0, st>>>(
-      tab, b.gcount);
-}
-
 void fused_allocate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   const int tx = nblk(b.max_cols, kAllocT), ty = nblk(b.max_rows, kAllocT);
   // about two CTAs per SM for the grids (enough for their writes)
