@@ -38,7 +38,7 @@ inline __host__ __device__ int free_tile_words(int tiles_x, int tiles_y) {
   return tiles_x * tiles_y + 2 * coarse_tiles(tiles_x, tiles_y);
 }
 
-struct SessDev {
+struct alignas(16) SessDev {
   DSensor ls[kLevels];  // level sensors (scale 1, 2, 4, 8)
   LevelCamera cam[kLevels];
   int nlev;             // levels in use
@@ -79,6 +79,17 @@ struct SessDev {
   // map
   VolumeDev vol;
 };
+static_assert(sizeof(SessDev) % 16 == 0, "copied in 16-byte words");
+
+#ifdef __CUDACC__
+// A CTA's own copy of its session's record, in one round trip to L2 instead of
+// one per line and branch; a barrier follows before its use.
+__device__ inline void stage_session(const SessDev* __restrict__ tab, SessDev* own) {
+  const uint4* src = reinterpret_cast<const uint4*>(tab);
+  uint4* dst = reinterpret_cast<uint4*>(own);
+  for (int i = threadIdx.x; i < (int)(sizeof(SessDev) / 16); i += blockDim.x) dst[i] = __ldg(src + i);
+}
+#endif
 
 // Launch helpers of the fused stages (image.cu, icp.cu, tsdf.cu).  'tab' is
 // a device array of n descriptors; the grid of each launch is sized for the

@@ -102,18 +102,51 @@ __device__ inline void grid_put(const VolumeDev& v, const GridBox& b, unsigned l
     v.grid[(x * b.ny + y) * b.nz + z] = ((unsigned)ptr * (unsigned)kBlockVox) | flag;
 }
 // ------------------------------------------------------------ allocation
-constexpr int kAllocT = 16;          // 16x16 pixel tile per CTA
-constexpr int kSetSlots = 2048;      // CTA-local dedup set (16 KB)
+constexpr int kAllocX = 16, kAllocY = 16, kAllocN = kAllocX * kAllocY;  // pixel tile per CTA
+constexpr int kSetBits = 11, kSetSlots = 1 << kSetBits;                 // CTA-local dedup set
 constexpr int kSetProbes = 32;
 
-__device__ inline unsigned set_hash(unsigned long long k) {
-  return (unsigned)((k * 0x9E3779B97F4A7C15ull) >> 53) & (kSetSlots - 1);
+// A block in a CTA's set: its offset from the camera's block, biased fields of
+// BITS bits an axis, so that a step is one addition and the 32-bit form of it
+// (10 bits) one multiplication away from its slot.  The 64-bit form (21 bits,
+// as wide as the volume's own keys) serves sessions whose rays may take more
+// steps than 10 bits hold.
+template <class K>
+struct NearKey;
+template <>
+struct NearKey<unsigned> {
+  static constexpr int kBits = 10;
+  static __device__ unsigned slot(unsigned k) { return (k * 0x9E3779B1u) >> (32 - kSetBits); }
+};
+template <>
+struct NearKey<unsigned long long> {
+  static constexpr int kBits = 21;
+  static __device__ unsigned slot(unsigned long long k) {
+    return (unsigned)((k * 0x9E3779B97F4A7C15ull) >> (64 - kSetBits));
+  }
+};
+template <class K>
+__device__ inline K near_key(int dx, int dy, int dz) {
+  constexpr int B = NearKey<K>::kBits, half = 1 << (B - 1);
+  return ((K)(unsigned)(dx + half) << (2 * B)) + ((K)(unsigned)(dy + half) << B) +
+         (K)(unsigned)(dz + half);
 }
+template <class K>
+__device__ inline unsigned long long volume_key(K k, const int (&cam)[3]) {
+  constexpr int B = NearKey<K>::kBits, half = 1 << (B - 1), mask = (1 << B) - 1;
+  return pack_key((int)((k >> (2 * B)) & mask) - half + cam[0],
+                  (int)((k >> B) & mask) - half + cam[1], (int)(k & mask) - half + cam[2]);
+}
+__device__ inline int apart_of(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
 
-struct AllocSmem {
-  unsigned long long set[kSetSlots];
-  int claim_entry[kSetSlots];
-  int nclaims;
+struct alignas(16) AllocSmem {
+  unsigned long long set[kSetSlots];  // keys; all bits set: none; later the claimed entries
+  unsigned short list[kSetSlots];     // the keys' slots in order of arrival
+  unsigned short claim[kSetSlots];    // the claimed ones'
+  M4f T;       // the frame's pose
+  int cam[3];  // the camera's block
+  int stamp;
+  int nkeys, nclaims;
   int base;
   int new_blocks, bucket_full, heap_exhausted, unique, overruns;
 };
@@ -123,130 +156,218 @@ struct AllocSmem {
 // AllocateFromDepthKernel (tsdf.cu:346-453) for one pixel: the reference's
 // DDA over blocks, exact FP32 (this file is built with -fmad=false), with
 // the 'diff' pre-step for negative directions and the step cap.
-template <class F>
-__device__ inline bool dda_ray(F3 start_pt, F3 point, float trunc, float block_size, int cap,
-                               F&& visit) {
+struct RayWalk {
+  int bx, by, bz;  // first block
+  int nx, ny, nz;  // pre-step (0 or -1)
+  int ex, ey, ez;  // last block
+  int sx, sy, sz;
+  float mx, my, mz, dtx, dty, dtz;
+};
+__device__ inline RayWalk ray_walk(F3 start_pt, F3 point, float trunc, float block_size) {
+  RayWalk w;
   F3 dir = normalize3(point - start_pt);
   float surface_distance = norm3(start_pt - point);
   F3 ray_start = start_pt;
   F3 ray_end = start_pt + dir * (surface_distance + trunc);
-  int bpx = (int)floorf(ray_start.x / block_size);
-  int bpy = (int)floorf(ray_start.y / block_size);
-  int bpz = (int)floorf(ray_start.z / block_size);
-  int ebx = (int)floorf(ray_end.x / block_size);
-  int eby = (int)floorf(ray_end.y / block_size);
-  int ebz = (int)floorf(ray_end.z / block_size);
-  int sx = (dir.x > 0) - (dir.x < 0), sy = (dir.y > 0) - (dir.y < 0),
-      sz = (dir.z > 0) - (dir.z < 0);
+  w.bx = (int)floorf(ray_start.x / block_size);
+  w.by = (int)floorf(ray_start.y / block_size);
+  w.bz = (int)floorf(ray_start.z / block_size);
+  w.ex = (int)floorf(ray_end.x / block_size);
+  w.ey = (int)floorf(ray_end.y / block_size);
+  w.ez = (int)floorf(ray_end.z / block_size);
+  w.sx = (dir.x > 0) - (dir.x < 0);
+  w.sy = (dir.y > 0) - (dir.y < 0);
+  w.sz = (dir.z > 0) - (dir.z < 0);
   const float FMAX = 3.402823466e+38f;
-  float dtx = dir.x != 0 ? fabsf(block_size / dir.x) : FMAX;
-  float dty = dir.y != 0 ? fabsf(block_size / dir.y) : FMAX;
-  float dtz = dir.z != 0 ? fabsf(block_size / dir.z) : FMAX;
-  float bdx = ((float)bpx + (float)sx) * block_size;
-  float bdy = ((float)bpy + (float)sy) * block_size;
-  float bdz = ((float)bpz + (float)sz) * block_size;
-  float mx = dir.x != 0 ? (bdx - ray_start.x) / dir.x : FMAX;
-  float my = dir.y != 0 ? (bdy - ray_start.y) / dir.y : FMAX;
-  float mz = dir.z != 0 ? (bdz - ray_start.z) / dir.z : FMAX;
-  int dx = 0, dy = 0, dz = 0;
-  bool neg = false;
-  if (bpx != ebx && dir.x < 0) { dx--; neg = true; }
-  if (bpy != eby && dir.y < 0) { dy--; neg = true; }
-  if (bpz != ebz && dir.z < 0) { dz--; neg = true; }
-  visit(bpx, bpy, bpz);
-  if (neg) {
-    bpx += dx;
-    bpy += dy;
-    bpz += dz;
-    visit(bpx, bpy, bpz);
-  }
-  int steps = 0;
-  while (bpx != ebx || bpy != eby || bpz != ebz) {
-    if (steps++ >= cap) return false;
-    if (mx < my) {
-      if (mx < mz) { bpx += sx; mx += dtx; }
-      else { bpz += sz; mz += dtz; }
-    } else {
-      if (my < mz) { bpy += sy; my += dty; }
-      else { bpz += sz; mz += dtz; }
-    }
-    visit(bpx, bpy, bpz);
-  }
+  w.dtx = dir.x != 0 ? fabsf(block_size / dir.x) : FMAX;
+  w.dty = dir.y != 0 ? fabsf(block_size / dir.y) : FMAX;
+  w.dtz = dir.z != 0 ? fabsf(block_size / dir.z) : FMAX;
+  float bdx = ((float)w.bx + (float)w.sx) * block_size;
+  float bdy = ((float)w.by + (float)w.sy) * block_size;
+  float bdz = ((float)w.bz + (float)w.sz) * block_size;
+  w.mx = dir.x != 0 ? (bdx - ray_start.x) / dir.x : FMAX;
+  w.my = dir.y != 0 ? (bdy - ray_start.y) / dir.y : FMAX;
+  w.mz = dir.z != 0 ? (bdz - ray_start.z) / dir.z : FMAX;
+  w.nx = w.bx != w.ex && dir.x < 0 ? -1 : 0;
+  w.ny = w.by != w.ey && dir.y < 0 ? -1 : 0;
+  w.nz = w.bz != w.ez && dir.z < 0 ? -1 : 0;
+  return w;
+}
+
+// The ray of a pixel; false: none (tsdf.cu:442-444)
+__device__ inline bool pixel_ray(const float* __restrict__ depth, const DSensor& s, const DTsdf& t,
+                                 const M4f& T, int x, int y, RayWalk& w) {
+  if (x >= s.cols || y >= s.rows) return false;
+  const float d = depth[y * s.cols + x];
+  if (d < t.dmin || d > t.dmax) return false;
+  const F3 point = xform(T, point3d_uv(x, y, d, s));
+  if (point.x == 0 && point.y == 0 && point.z == 0) return false;
+  F3 start_pt = f3(T.m[3], T.m[7], T.m[11]);
+  // band allocation: the ray starts a truncation distance before the
+  // surface point instead of at the camera
+  if (t.band) start_pt = point - normalize3(point - start_pt) * t.trunc;
+  w = ray_walk(start_pt, point, t.trunc, t.bsm);
   return true;
 }
 
-// One 16x16 pixel tile (tx, ty) of AllocateFromDepthKernel.
-__device__ inline void allocate_tile(const float* __restrict__ depth, const DSensor& s,
-                                     const VolumeDev& v, const PoseState* __restrict__ ps,
-                                     int tx, int ty) {
-  __shared__ AllocSmem sm;
-  __shared__ M4f T;
-  __shared__ int stamp_s;
-  const int tid = threadIdx.y * kAllocT + threadIdx.x;
-  for (int k = tid; k < kSetSlots; k += kAllocT * kAllocT) sm.set[k] = kEmptyKey;
-  if (tid < 16) T.m[tid] = ps->posef[tid];
-  if (tid == 0) {
-    sm.nclaims = 0;
-    sm.new_blocks = sm.bucket_full = sm.heap_exhausted = sm.unique = sm.overruns = 0;
-    stamp_s = ps->frame;
+// One block into the global table, its heap index from the volume's counter.
+__device__ __noinline__ void insert_block(const VolumeDev& v, unsigned long long key,
+                                          AllocSmem& sm) {
+  const int r = bucket_insert(v.entries, v.t, key, sm.stamp, &sm.unique);
+  if (r >= 0) {
+    const int ptr = atomicAdd(&v.cnt->nalloc, 1);
+    if (ptr < v.t.num_blocks) {
+      v.entries[r].ptr = ptr;
+      v.block_keys[ptr] = key;
+      atomicAdd(&sm.new_blocks, 1);
+    } else {
+      atomicAdd(&sm.heap_exhausted, 1);
+    }
+  } else if (r == -2) {
+    atomicAdd(&sm.bucket_full, 1);
   }
-  __syncthreads();
-  const int stamp = stamp_s;
-  const DTsdf& t = v.t;
-  const int x = tx * kAllocT + threadIdx.x;
-  const int y = ty * kAllocT + threadIdx.y;
-  if (x < s.cols && y < s.rows) {
-    const int i = y * s.cols + x;
-    const float d = depth[i];
-    if (!(d < t.dmin || d > t.dmax)) {  // tsdf.cu:442-444
-      F3 point = xform(T, point3d_uv(x, y, d, s));
-      if (!(point.x == 0 && point.y == 0 && point.z == 0)) {
-        F3 start_pt = f3(T.m[3], T.m[7], T.m[11]);
-        // band allocation: the ray starts a truncation distance before the
-        // surface point instead of at the camera
-        if (t.band) start_pt = point - normalize3(point - start_pt) * t.trunc;
-        bool ok = dda_ray(start_pt, point, t.trunc, t.bsm, t.dda_cap, [&](int bx, int by, int bz) {
-          unsigned long long key = pack_key(bx, by, bz);
-          unsigned h = set_hash(key);
-          for (int p = 0; p < kSetProbes; ++p) {
-            unsigned slot = (h + p) & (kSetSlots - 1);
-            // neighbouring rays visit the same blocks: most visits find
-            // their key already in the set with a plain read
-            unsigned long long old = *(volatile unsigned long long*)&sm.set[slot];
-            if (old == key) return;
-            if (old == kEmptyKey) {
-              old = atomicCAS(&sm.set[slot], kEmptyKey, key);
-              if (old == kEmptyKey || old == key) return;
-            }
-          }
-          // set saturated: insert directly
-          int r = bucket_insert(v.entries, t, key, stamp, &sm.unique);
-          if (r >= 0) {
-            int ptr = atomicAdd(&v.cnt->nalloc, 1);
-            if (ptr < t.num_blocks) {
-              v.entries[r].ptr = ptr;
-              v.block_keys[ptr] = key;
-              atomicAdd(&sm.new_blocks, 1);
-            } else {
-              atomicAdd(&sm.heap_exhausted, 1);
-            }
-          } else if (r == -2) {
-            atomicAdd(&sm.bucket_full, 1);
-          }
-        });
-        if (!ok) atomicAdd(&sm.overruns, 1);
+}
+
+// A pixel's whole ray without the set (anywhere; blocks that other rays enter
+// as well are found or claimed once).
+__device__ __noinline__ void walk_far(const SessDev& S, int x, int y, AllocSmem& sm) {
+  const VolumeDev& v = S.vol;
+  RayWalk w;
+  if (!pixel_ray(S.raw, S.ls[0], v.t, sm.T, x, y, w)) return;
+  int bx = w.bx, by = w.by, bz = w.bz;
+  insert_block(v, pack_key(bx, by, bz), sm);
+  if (w.nx | w.ny | w.nz) {
+    bx += w.nx;
+    by += w.ny;
+    bz += w.nz;
+    insert_block(v, pack_key(bx, by, bz), sm);
+  }
+  int left = v.t.dda_cap;
+  while (bx != w.ex || by != w.ey || bz != w.ez) {
+    if (left-- <= 0) {
+      atomicAdd(&sm.overruns, 1);
+      return;
+    }
+    const bool xy = w.mx < w.my, xz = w.mx < w.mz, yz = w.my < w.mz;
+    const bool gx = xy && xz, gy = !xy && yz;
+    if (gx) { bx += w.sx; w.mx += w.dtx; }
+    else if (gy) { by += w.sy; w.my += w.dty; }
+    else { bz += w.sz; w.mz += w.dtz; }
+    insert_block(v, pack_key(bx, by, bz), sm);
+  }
+}
+
+// One block of a ray into the CTA's set.  Neighbouring rays visit the same
+// blocks: most visits find their key with a plain read; of a run of lanes that
+// miss the same key together the first enters it (their compare-and-swaps would
+// queue at the slot: half of this kernel's shared memory cycles).
+template <class K>
+__device__ inline void visit_block(K key, const VolumeDev& v, AllocSmem& sm) {
+  K* const set = reinterpret_cast<K*>(sm.set);
+  constexpr K none = ~(K)0;
+  unsigned slot = NearKey<K>::slot(key);
+  for (int p = 0; p < kSetProbes; ++p) {
+    K old = *(volatile K*)&set[slot];
+    if (old == none) {
+      const unsigned here = __activemask(), lane = threadIdx.x & 31;
+      const K left = __shfl_up_sync(here, key, 1);
+      const bool follows = lane > 0 && (here >> (lane - 1) & 1u) && left == key;
+      if (!follows) {
+        old = atomicCAS(&set[slot], none, key);
+        if (old == none) {
+          sm.list[atomicAdd(&sm.nkeys, 1)] = (unsigned short)slot;
+          old = key;
+        }
       }
+      __syncwarp(here);
+      if (follows) old = *(volatile K*)&set[slot];
+    }
+    if (old == key) return;
+    slot = (slot + 1) & (kSetSlots - 1);
+  }
+  insert_block(v, volume_key(key, sm.cam), sm);  // set saturated
+}
+
+// The rays of one pixel tile (tx, ty) of AllocateFromDepthKernel.
+template <class K>
+__device__ inline void walk_rays(const SessDev& S, int tx, int ty, AllocSmem& sm) {
+  constexpr int B = NearKey<K>::kBits;
+  const VolumeDev& v = S.vol;
+  const int tid = threadIdx.x;
+  // (a warp's rays are 8x4 pixels)
+  const int x = tx * kAllocX + (tid & 7) + (tid >> 2 & (kAllocX - 8)),
+            y = ty * kAllocY + (tid >> 3 & 3) + tid / (kAllocX * 4) * 4;
+  RayWalk w;
+  if (!pixel_ray(S.raw, S.ls[0], v.t, sm.T, x, y, w)) return;
+  const int ox = apart_of(w.bx, sm.cam[0]), oy = apart_of(w.by, sm.cam[1]),
+            oz = apart_of(w.bz, sm.cam[2]);
+  // (a last block beyond the fields is beyond the cap as well)
+  const int lx = apart_of(w.ex, sm.cam[0]), ly = apart_of(w.ey, sm.cam[1]),
+            lz = apart_of(w.ez, sm.cam[2]);
+  constexpr unsigned half = 1u << (B - 1);
+  const bool ends = (unsigned)lx + half < 2 * half && (unsigned)ly + half < 2 * half &&
+                    (unsigned)lz + half < 2 * half;
+  const K last = ends ? near_key<K>(lx, ly, lz) : ~(K)0;
+  int left = v.t.dda_cap;
+  if (B == 10) {
+    // band rays start at the surface: none that could leave the fields is
+    // walked with them (poses that are not rigid)
+    const int start = max(max(abs(ox), abs(oy)), abs(oz));
+    if (start < 0 || start + left + 2 > (int)half) {
+      walk_far(S, x, y, sm);
+      return;
     }
   }
+  const K ix = (K)(long long)w.sx << (2 * B), iy = (K)(long long)w.sy << B, iz = (K)(long long)w.sz;
+  K key = near_key<K>(ox, oy, oz);
+  visit_block<K>(key, v, sm);
+  if (w.nx | w.ny | w.nz) {
+    key = near_key<K>(ox + w.nx, oy + w.ny, oz + w.nz);
+    visit_block<K>(key, v, sm);
+  }
+  while (key != last) {
+    if (left-- <= 0) {
+      atomicAdd(&sm.overruns, 1);
+      break;
+    }
+    const bool xy = w.mx < w.my, xz = w.mx < w.mz, yz = w.my < w.mz;
+    const bool gx = xy && xz, gy = !xy && yz;
+    key += gx ? ix : (gy ? iy : iz);
+    if (gx) w.mx += w.dtx;
+    else if (gy) w.my += w.dty;
+    else w.mz += w.dtz;
+    visit_block<K>(key, v, sm);
+  }
+}
+
+template <class K>
+__device__ inline void allocate_tile(const SessDev& S, int tx, int ty, AllocSmem& sm) {
+  K* const set = reinterpret_cast<K*>(sm.set);
+  const VolumeDev& v = S.vol;
+  const DTsdf& t = v.t;
+  const int tid = threadIdx.x;
+  for (int k = tid; k < kSetSlots * (int)sizeof(K) / 16; k += kAllocN)
+    reinterpret_cast<uint4*>(sm.set)[k] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  if (tid < 16) {
+    const float m = S.pose->posef[tid];
+    sm.T.m[tid] = m;
+    if ((tid & 3) == 3 && tid < 12) sm.cam[tid >> 2] = (int)floorf(m / t.bsm);
+  }
+  if (tid == 0) {
+    sm.nkeys = sm.nclaims = 0;
+    sm.new_blocks = sm.bucket_full = sm.heap_exhausted = sm.unique = sm.overruns = 0;
+    sm.stamp = S.pose->frame;
+  }
+  __syncthreads();
+  walk_rays<K>(S, tx, ty, sm);
   __syncthreads();
   // drain the set into the global table
-  for (int k = tid; k < kSetSlots; k += kAllocT * kAllocT) {
-    unsigned long long key = sm.set[k];
-    if (key == kEmptyKey) continue;
-    int r = bucket_insert(v.entries, t, key, stamp, &sm.unique);
+  for (int k = tid; k < sm.nkeys; k += kAllocN) {
+    const int slot = sm.list[k];
+    const int r = bucket_insert(v.entries, t, volume_key(set[slot], sm.cam), sm.stamp, &sm.unique);
     if (r >= 0) {
-      int c = atomicAdd(&sm.nclaims, 1);
-      sm.claim_entry[c] = r;
+      set[slot] = (K)(unsigned)r;
+      sm.claim[atomicAdd(&sm.nclaims, 1)] = (unsigned short)slot;
     } else if (r == -2) {
       atomicAdd(&sm.bucket_full, 1);
     }
@@ -254,9 +375,9 @@ __device__ inline void allocate_tile(const float* __restrict__ depth, const DSen
   __syncthreads();
   if (tid == 0 && sm.nclaims > 0) sm.base = atomicAdd(&v.cnt->nalloc, sm.nclaims);
   __syncthreads();
-  for (int c = tid; c < sm.nclaims; c += kAllocT * kAllocT) {
+  for (int c = tid; c < sm.nclaims; c += kAllocN) {
     int ptr = sm.base + c;
-    int e = sm.claim_entry[c];
+    const int e = (int)set[sm.claim[c]];
     if (ptr < t.num_blocks) {
       v.entries[e].ptr = ptr;
       v.block_keys[ptr] = v.entries[e].key;
@@ -275,24 +396,39 @@ __device__ inline void allocate_tile(const float* __restrict__ depth, const DSen
   }
 }
 
-// (8 CTAs per SM -- at most 32 registers, 24.7 KB of shared memory each --
-// so that a 640x480 frame's 1,200 tiles run in one wave instead of 1.35)
+// 8 CTAs per SM -- at most 32 registers, 25.5 KB of shared memory each -- so
+// that a 640x480 frame's 1,200 tiles run in about one wave instead of 1.35.
+// Bound by the walks (a frame without the drain: 63 of 69 us): about 30
+// instructions a step, and a wait at each block that the tile meets for the
+// first time.  Smaller tiles meet more of them (16x8 98 us, 8x8 134), sets twice
+// as large, two to four steps looked up together or warps held together at each
+// step are no faster (70 to 118).  640x480, 5 mm voxels: 92 us with 64-bit keys
+// packed at each step and a compare-and-swap by every lane, now 69; a frame of
+// ten 640x480 streams 3664 us before this work, 2733 before this, now 2306.
 // The tiles' rows of CTAs are followed by rows that empty the raycast's grid at
 // the frame's pose (memory-bound work beside the rays' latency-bound one).
-__global__ void __launch_bounds__(kAllocT* kAllocT, 8)
+__global__ void __launch_bounds__(kAllocN, 8)
     fused_allocate_kernel(const SessDev* __restrict__ tab, int tile_rows) {
-  const SessDev& S = tab[blockIdx.z];
+  __shared__ SessDev S;
+  stage_session(tab + blockIdx.z, &S);
+  __syncthreads();
   const DSensor& s = S.ls[0];
   if ((int)blockIdx.y >= tile_rows) {
     if (S.vol.grid && S.mode == 1)
       grid_clear(S.vol, S.pose->posef, s,
-                 (((int)blockIdx.y - tile_rows) * (int)gridDim.x + (int)blockIdx.x) * kAllocT * kAllocT +
-                     (int)threadIdx.y * kAllocT + (int)threadIdx.x,
-                 ((int)gridDim.y - tile_rows) * (int)gridDim.x * kAllocT * kAllocT);
+                 (((int)blockIdx.y - tile_rows) * (int)gridDim.x + (int)blockIdx.x) * kAllocN +
+                     (int)threadIdx.x,
+                 ((int)gridDim.y - tile_rows) * (int)gridDim.x * kAllocN);
     return;
   }
-  if ((int)blockIdx.x * kAllocT >= s.cols || (int)blockIdx.y * kAllocT >= s.rows) return;
-  allocate_tile(S.raw, s, S.vol, S.pose, blockIdx.x, blockIdx.y);
+  if ((int)blockIdx.x * kAllocX >= s.cols || (int)blockIdx.y * kAllocY >= s.rows) return;
+  // 10 bits hold a ray of the cap's steps from the camera; a band ray's start as
+  // well, up to twice the sensor range away
+  __shared__ AllocSmem sm;
+  if (S.vol.t.dda_cap <= (S.vol.t.band ? 300 : 509))
+    allocate_tile<unsigned>(S, blockIdx.x, blockIdx.y, sm);
+  else
+    allocate_tile<unsigned long long>(S, blockIdx.x, blockIdx.y, sm);
 }
 
 // ------------------------------------------------------------ visibility
@@ -372,8 +508,11 @@ __device__ inline void bound_block(unsigned long long key, const DTsdf& t, const
   }
   if (!(zmax >= znear)) return;  // wholly nearer than the near distance
   float umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
-  auto add = [&](float X, float Y, float Z) {
-    const float u = s.fx * X / Z + s.cx, w = s.fy * Y / Z + s.cy;
+  // (approximate reciprocals: their error is far below the rectangle's margin
+  // of a pixel wherever it lies in the image)
+  const float rnear = 1.0f / znear;
+  auto add = [&](float X, float Y, float rz) {
+    const float u = s.fx * X * rz + s.cx, w = s.fy * Y * rz + s.cy;
     umin = fminf(umin, u);
     umax = fmaxf(umax, u);
     vmin = fminf(vmin, w);
@@ -381,19 +520,20 @@ __device__ inline void bound_block(unsigned long long key, const DTsdf& t, const
   };
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    if (c[k].z >= znear) add(c[k].x, c[k].y, c[k].z);
+    if (c[k].z >= znear) add(c[k].x, c[k].y, __fdividef(1.0f, c[k].z));
   // the 12 box edges (corner pairs differing in one bit) cut by z = znear
+  if (zmin < znear)
 #pragma unroll
-  for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < 8; ++k)
 #pragma unroll
-    for (int bit = 1; bit < 8; bit <<= 1) {
-      if (k & bit) continue;
-      const F3 a = c[k], b = c[k | bit];
-      if ((a.z < znear) != (b.z < znear)) {
-        const float f = (znear - a.z) / (b.z - a.z);
-        add(a.x + f * (b.x - a.x), a.y + f * (b.y - a.y), znear);
+      for (int bit = 1; bit < 8; bit <<= 1) {
+        if (k & bit) continue;
+        const F3 a = c[k], b = c[k | bit];
+        if ((a.z < znear) != (b.z < znear)) {
+          const float f = (znear - a.z) / (b.z - a.z);
+          add(a.x + f * (b.x - a.x), a.y + f * (b.y - a.y), rnear);
+        }
       }
-    }
   umin -= 1.0f;
   vmin -= 1.0f;
   umax += 1.0f;
@@ -459,13 +599,15 @@ __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, 
     const F3 c = xform(invT, f3(ox + ((k & 1) ? e : 0.0f), oy + ((k & 2) ? e : 0.0f),
                                 oz + ((k & 4) ? e : 0.0f)));
     if (!(c.z > 0.01f)) return false;
-    const float u = s.fx * c.x / c.z + s.cx, w = s.fy * c.y / c.z + s.cy;
+    const float rz = __fdividef(1.0f, c.z);  // far more exact than the pixel of margin
+    const float u = s.fx * c.x * rz + s.cx, w = s.fy * c.y * rz + s.cy;
     u0 = fminf(u0, u);
     u1 = fmaxf(u1, u);
     v0 = fminf(v0, w);
     v1 = fmaxf(v1, w);
-    dm = fmaxf(dm, norm3(c));
+    dm = fmaxf(dm, dot3(c, c));
   }
+  dm = sqrtf(dm);
   if (!(u0 >= 1.0f && v0 >= 1.0f && u1 <= (float)(s.cols - 2) && v1 <= (float)(s.rows - 2)))
     return false;
   const int x0 = (int)floorf(u0) - 1, x1 = (int)ceilf(u1) + 1;
@@ -483,9 +625,18 @@ __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, 
     ty1 /= kRbCoarse;
     if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) > 16) return false;
   }
+  // at most 16 tiles, four loads in flight (the last one repeated)
+  const int w = tx1 - tx0 + 1, n = w * (ty1 - ty0 + 1);
   unsigned mn = 0xffffffffu;
-  for (int ty = ty0; ty <= ty1; ++ty)
-    for (int tx = tx0; tx <= tx1; ++tx) mn = min(mn, __ldg(m + ty * tw + tx));
+  for (int k = 0; k < n; k += 4) {
+    unsigned q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = min(k + j, n - 1), r = i / w;
+      q[j] = __ldg(m + (ty0 + r) * tw + tx0 + (i - r * w));
+    }
+    mn = min(min(mn, min(q[0], q[1])), min(q[2], q[3]));
+  }
   return dm * (1.0f + 1e-5f) + 1e-5f < __uint_as_float(mn);
 }
 
@@ -506,44 +657,67 @@ __global__ void grid_fill_kernel(const __grid_constant__ VolumeDev v) {
 // Every session's visible blocks appended to one batch-wide list of
 // (session, heap index), so integration balances across sessions; the
 // session index carries kVisFree for free-space blocks.
-__global__ void fused_visible_kernel(const SessDev* __restrict__ tab, int2* __restrict__ gvis,
+// Bound by latency: a thread's chain (three sets of corners and the tile
+// minima), and the list's one counter, which takes an atomic per CTA and step
+// (per warp, 1100 of them at 640x480, and with IEEE quotients, 27 us of a
+// frame, now 24.6; 27 -> 18.4 at 320x240; more with a CTA's look at the
+// bounds before their atomics).  CTAs this small, so that a few thousand blocks reach every
+// SM.
+constexpr int kVisThreads = 128;
+__global__ void __launch_bounds__(kVisThreads) fused_visible_kernel(const SessDev* __restrict__ tab, int2* __restrict__ gvis,
                                      int* __restrict__ gcount) {
-  const SessDev& S = tab[blockIdx.z];
+  __shared__ SessDev S;
+  stage_session(tab + blockIdx.z, &S);
+  __syncthreads();
   const VolumeDev& v = S.vol;
   __shared__ M4f invT;
+  __shared__ int seen[2][kVisThreads / 32], base_s[2];
   if (threadIdx.x < 16) invT.m[threadIdx.x] = S.pose->invf[threadIdx.x];
-  __syncthreads();
   int n = v.cnt->nalloc;
   if (n > v.t.num_blocks) n = v.t.num_blocks;
-  const int lane = threadIdx.x & 31;
-  // (mixed carving sessions enter their blocks after the free-cell pass)
-  const bool put = v.grid && S.mode == 1 && !v.nonsat && v.gbox->ok;
+  if ((int)(blockIdx.x * blockDim.x) >= n) return;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int total = 0, step = 0;
+  // (mixed carving sessions' entries get their free-cell flags afterwards)
+  GridBox box;
+  box.ok = 0;
+  if (v.grid && S.mode == 1) box = *v.gbox;
+  const bool carve = S.ftile && !v.t.band && !*S.rgb_flag;
+  // (the frame counter has advanced since the ingest made the map)
+  const int parity = (S.pose->frame - 1) & 1;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     int i = base + threadIdx.x;
     bool vis = false;
+    unsigned long long key = 0;
     if (i < n) {
-      const unsigned long long key = v.block_keys[i];
-      if (put) grid_put(v, *v.gbox, key, i, 0u);
+      key = v.block_keys[i];
+      if (box.ok) grid_put(v, box, key, i, 0u);
       vis = block_visible(key, v.t, S.ls[0], invT);
       // every allocated block (visible or not) enters the ray-start bound
       if (S.rbound) bound_block(key, v.t, S.ls[0], invT, S.rbound, S.rb_tx, S.rb_ty, v.t.band, true);
     }
     bool fr = false;
-    if (vis && S.ftile && !v.t.band && !*S.rgb_flag)
-      // (the frame counter has advanced since the ingest made the map)
-      fr = free_space_block(v.block_keys[i], v.t, S.ls[0], invT, S.ftile, S.rb_tx, S.rb_ty,
-                            (S.pose->frame - 1) & 1);
-    unsigned m = __ballot_sync(0xffffffffu, vis);
-    int off = 0;
-    if (lane == 0 && m) {
-      atomicAdd(&v.cnt->visible, __popc(m));
-      off = atomicAdd(gcount, __popc(m));
+    if (vis && carve)
+      fr = free_space_block(key, v.t, S.ls[0], invT, S.ftile, S.rb_tx, S.rb_ty, parity);
+    const unsigned m = __ballot_sync(0xffffffffu, vis);
+    if (lane == 0) seen[step][warp] = __popc(m);
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kVisThreads / 32; ++w) {
+      if (w < warp) before += seen[step][w];
+      all += seen[step][w];
     }
-    off = __shfl_sync(0xffffffffu, off, 0);
+    if (threadIdx.x == 0 && all) base_s[step] = atomicAdd(gcount, all);
+    total += all;
+    __syncthreads();
     if (vis)
-      gvis[off + __popc(m & ((1u << lane) - 1))] =
+      gvis[base_s[step] + before + __popc(m & ((1u << lane) - 1))] =
           make_int2((int)blockIdx.z | (fr ? kVisFree : 0), i);
+    step ^= 1;  // (the other buffer: no barrier before its next use)
   }
+  if (threadIdx.x == 0 && total) atomicAdd(&v.cnt->visible, total);
 }
 
 // The near ray bound of mixed carving sessions, after integration.  A
@@ -555,7 +729,7 @@ __global__ void fused_visible_kernel(const SessDev* __restrict__ tab, int2* __re
 // tile is the nearest depth of the boxes of the blocks that hold such
 // voxels (VolumeDev::nonsat > 0), widened as bound_block widens every box.
 // Every block also enters the raycast's grid here, with its free-cell flag.
-__global__ void fused_surface_bound_kernel(const SessDev* __restrict__ tab) {
+__global__ void __launch_bounds__(kVisThreads) fused_surface_bound_kernel(const SessDev* __restrict__ tab) {
   const SessDev& S = tab[blockIdx.z];
   const VolumeDev& v = S.vol;
   if (!v.nonsat) return;
@@ -908,6 +1082,31 @@ __global__ void __launch_bounds__(kIntThreads, 4)
   }
 }
 
+// Heap indices (or -1) of the seven neighbours of a block to one side: from the
+// frame's block grid where it covers them, else from the hash.
+__device__ inline void neighbours(const VolumeDev& v, bool grid, int x, int y, int z, int sg,
+                                  int (&p)[8]) {
+  if (grid) {
+    const GridBox b = *v.gbox;
+    const int gx = x - b.x0, gy = y - b.y0, gz = z - b.z0;
+    const int ux = gx + sg, uy = gy + sg, uz = gz + sg;
+    if (min(min(gx, ux), min(min(gy, uy), min(gz, uz))) >= 0 && max(gx, ux) < b.nx &&
+        max(gy, uy) < b.ny && max(gz, uz) < b.nz) {
+#pragma unroll
+      for (int k = 1; k < 8; ++k) {
+        const unsigned e = v.grid[((k & 1 ? ux : gx) * b.ny + (k & 2 ? uy : gy)) * b.nz +
+                                  (k & 4 ? uz : gz)];
+        p[k] = (int)(e / kBlockVox) < v.t.num_blocks ? (int)(e / kBlockVox) : -1;
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int k = 1; k < 8; ++k)
+    p[k] = find_block(v.entries, v.t, x + (k & 1 ? sg : 0), y + (k & 2 ? sg : 0),
+                      z + (k & 4 ? sg : 0));
+}
+
 // Free-cell flags of the visible blocks (after their integration): a block's
 // flag is set when it and its seven upper neighbours (+x, +y, +z and their
 // combinations; missing ones count as free) hold no observed non-saturated
@@ -930,17 +1129,22 @@ __global__ void fused_free_cells_kernel(const SessDev* __restrict__ tab,
     const int x = key_x(key), y = key_y(key), z = key_z(key);
     const bool own = v.nonsat[item.y] == 0;
     bool free = own && v.free_ok;
+    if (own && !free) {
+      v.freecell[item.y] = 0;
+      continue;
+    }
+    // the upper neighbours of a block without such a voxel, the lower ones of
+    // one with
+    const int sg = own ? 1 : -1;
+    int p[8];
+    neighbours(v, tab[item.x].mode == 1 && v.grid && v.gbox->ok, x, y, z, sg, p);
 #pragma unroll
     for (int k = 1; k < 8; ++k) {
-      const int dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
-      if (free) {
-        const int p = find_block(v.entries, v.t, x + dx, y + dy, z + dz);
-        if (p >= 0 && v.nonsat[p] != 0) free = false;
-      }
-      if (!own) {
-        const int q = find_block(v.entries, v.t, x - dx, y - dy, z - dz);
-        if (q >= 0) v.freecell[q] = 0;
-      }
+      if (p[k] < 0) continue;
+      if (own)
+        free = free && v.nonsat[p[k]] == 0;
+      else
+        v.freecell[p[k]] = 0;
     }
     v.freecell[item.y] = free ? 1 : 0;
   }
@@ -1892,19 +2096,18 @@ void launch_find_blocks(const VolumeDev& v, const int* coords, int n, int* ptr_o
 
 // ---- fused stages
 void fused_allocate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  const int tx = nblk(b.max_cols, kAllocT), ty = nblk(b.max_rows, kAllocT);
+  const int tx = nblk(b.max_cols, kAllocX), ty = nblk(b.max_rows, kAllocY);
   // about two CTAs per SM for the grids (enough for their writes)
   const int extra = b.max_grid > 0 ? nblk(std::max(8, 148 * 2 / b.n), tx) : 0;
-  fused_allocate_kernel<<<dim3(tx, ty + extra, b.n), dim3(kAllocT, kAllocT), 0, st>>>(tab, ty);
+  fused_allocate_kernel<<<dim3(tx, ty + extra, b.n), kAllocN, 0, st>>>(tab, ty);
 }
 
+// grid-stride over each session's heap; a wave of CTAs in all
+static dim3 visible_grid(const BatchShape& b) {
+  return dim3(std::min(nblk(b.max_blocks, kVisThreads), std::max(148 * 12 / b.n, 32)), 1, b.n);
+}
 void fused_visible(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  // grid-stride over each session's heap; about 600 CTAs in all
-  int cap = 592 / b.n;
-  if (cap < 8) cap = 8;
-  int g = nblk(b.max_blocks, 256);
-  if (g > cap) g = cap;
-  fused_visible_kernel<<<dim3(g, 1, b.n), 256, 0, st>>>(tab, b.gvis, b.gcount);
+  fused_visible_kernel<<<visible_grid(b), kVisThreads, 0, st>>>(tab, b.gvis, b.gcount);
 }
 
 void fused_integrate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
@@ -1913,13 +2116,9 @@ void fused_integrate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
 }
 
 void fused_free_cells(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  fused_free_cells_kernel<<<148 * 2, 256, 0, st>>>(tab, b.gvis, b.gcount);
+  fused_free_cells_kernel<<<148 * 8, 64, 0, st>>>(tab, b.gvis, b.gcount);
   if (b.fp16_mask & 2) {  // mixed sessions: the near ray bound from their summaries
-    int cap = 592 / b.n;
-    if (cap < 8) cap = 8;
-    int g = nblk(b.max_blocks, 256);
-    if (g > cap) g = cap;
-    fused_surface_bound_kernel<<<dim3(g, 1, b.n), 256, 0, st>>>(tab);
+    fused_surface_bound_kernel<<<visible_grid(b), kVisThreads, 0, st>>>(tab);
   }
 }
 
