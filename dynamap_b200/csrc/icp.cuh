@@ -131,11 +131,12 @@ void launch_pose_hint(PoseState* ps, IcpState* st, const double* hint_dev, int c
                       cudaStream_t stream);
 // Set the pose from the host (double[16]); recomputes posef/invf.
 void launch_pose_set(PoseState* ps, const double* pose_dev, cudaStream_t stream);
-// Normal equations only (no solve): out[29] doubles on the device.
-void launch_icp_reduce_only(const IcpLevel& L, const IcpParams& P, const float* T_dev,
-                            double* partials, unsigned int* ticket, double* out_dev,
+// Normal equations only (no solve): out[29] doubles on the device or in pinned
+// host memory.
+void launch_icp_reduce_only(const IcpLevel& L, const IcpParams& P, const M4f& T,
+                            double* partials, unsigned int* ticket, double* out,
                             cudaStream_t stream);
-// The same reduction on an explicit grid ('partials' holds grid * 29
+// The same reduction on an explicit grid, T on the device ('partials' holds grid * 29
 // doubles; pixels beyond grid * kIcpThreads are covered by the grid-stride
 // loop).
 void launch_icp_reduce_grid(const IcpLevel& L, const IcpParams& P, const float* T_dev,

@@ -600,8 +600,7 @@ size_t session_bytes(const dyn_tsdf_params& t, const dyn_sensor& s, int precisio
 struct StageScratch {
   double* partials = nullptr;
   unsigned int* ticket = nullptr;
-  double* out = nullptr;
-  float* T = nullptr;
+  double* out = nullptr;  // pinned: the kernel writes it, the call reads it
 };
 std::mutex g_stage_mu;
 StageScratch g_stage[64];
@@ -1332,11 +1331,12 @@ dyn_status dyn_icp_normal_equations(const float* src_depth_dev, const float* src
   std::lock_guard<std::mutex> lk(g_stage_mu);
   StageScratch& sc = g_stage[dev];
   if (!sc.partials) {
+    if (!sc.out) DYN_CUDA(cudaHostAlloc(&sc.out, 256, cudaHostAllocMapped));
+    if (!sc.ticket) {
+      DYN_CUDA(cudaMalloc(&sc.ticket, 256));
+      DYN_CUDA(cudaMemset(sc.ticket, 0, 256));
+    }
     DYN_CUDA(cudaMalloc(&sc.partials, icp_scratch_bytes()));
-    DYN_CUDA(cudaMalloc(&sc.ticket, 256));
-    DYN_CUDA(cudaMemset(sc.ticket, 0, 256));
-    DYN_CUDA(cudaMalloc(&sc.out, 256));
-    DYN_CUDA(cudaMalloc(&sc.T, 64));
   }
   cudaStream_t st = (cudaStream_t)stream;
   IcpLevel L;
@@ -1357,11 +1357,12 @@ dyn_status dyn_icp_normal_equations(const float* src_depth_dev, const float* src
   P.reg = gn->regularization;
   P.compose_left = gn->compose_left;
   P.kahan = 0;
-  DYN_CUDA(cudaMemcpyAsync(sc.T, T, 64, cudaMemcpyHostToDevice, st));
-  launch_icp_reduce_only(L, P, sc.T, sc.partials, sc.ticket, sc.out, st);
+  M4f pose;
+  std::memcpy(pose.m, T, sizeof(pose.m));
+  launch_icp_reduce_only(L, P, pose, sc.partials, sc.ticket, sc.out, st);
   DYN_CUDA(cudaGetLastError());
-  DYN_CUDA(cudaMemcpyAsync(out_host, sc.out, sizeof(double) * kIcpVals, cudaMemcpyDeviceToHost, st));
   DYN_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(out_host, sc.out, sizeof(double) * kIcpVals);
   return DYN_OK;
 }
 
