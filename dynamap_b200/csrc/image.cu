@@ -55,7 +55,8 @@ __device__ inline float intensity_u8(const uint8_t* c) {
 // A call at diameter 8, before -> now: 160x120 43.3 -> 12.4 us (the kernel 8),
 // 320x240 45 -> 14, 640x480 80 -> 33, 1280x720 146 -> 71.  Two pixels of a
 // column per thread, each staged depth read once for both, measured 16, 37 and
-// 72 us: the shared-memory reads are not what it waits for.
+// 72 us: the shared-memory reads are not what it waits for.  (They are in the
+// mixed form, whose taps are six operations and an exponential: bilateral_pair.)
 constexpr int BTX = 32;
 
 __device__ __host__ inline int bil_pitch(int D) { return BTX + D - 1; }
@@ -118,16 +119,61 @@ __device__ inline float bilateral_sum(const float* __restrict__ t, const float* 
   return acc / wp;
 }
 
-// One tile of 32 x blockDim.y pixels, tile column bx and row by.
-template <bool FAST>
+// The mixed form's sums of two pixels of a column, each staged depth read once
+// for both (window 16 only; each pixel's taps in the same order as above).
+template <bool MASK>
+__device__ inline void bilateral_pair(const float* __restrict__ t, const float* __restrict__ gs,
+                                      int pitch, float inv2s2, const float (&c)[2],
+                                      float (&out)[2]) {
+  constexpr int D = 16;
+  const float c2 = inv2s2 * 1.4426950408889634f;
+  float acc[2] = {0.0f, 0.0f}, wp[2] = {0.0f, 0.0f};
+  auto tap = [&](float nv, float g, int n) {
+    const float dn = nv - c[n];
+    float w;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(__fmaf_rn(-(dn * dn), c2, g)));
+    if (MASK) w = nv > 0.0f ? w : 0.0f;
+    acc[n] = __fmaf_rn(nv, w, acc[n]);
+    wp[n] += w;
+  };
+  // tile row r holds window row r of the first pixel and r - 1 of the second
+#pragma unroll 4
+  for (int j = 0; j < D; ++j) tap(t[j], gs[j], 0);
+#pragma unroll 1
+  for (int r = 1; r < D; ++r) {
+    const float* tr = t + r * pitch;
+    const float* gr = gs + r * D;
+#pragma unroll
+    for (int j = 0; j < D; j += 4) {
+      const float4 g0 = *reinterpret_cast<const float4*>(gr + j);
+      const float4 g1 = *reinterpret_cast<const float4*>(gr - D + j);
+      const float v[4] = {tr[j], tr[j + 1], tr[j + 2], tr[j + 3]};
+      tap(v[0], g0.x, 0);
+      tap(v[0], g1.x, 1);
+      tap(v[1], g0.y, 0);
+      tap(v[1], g1.y, 1);
+      tap(v[2], g0.z, 0);
+      tap(v[2], g1.z, 1);
+      tap(v[3], g0.w, 0);
+      tap(v[3], g1.w, 1);
+    }
+  }
+#pragma unroll 4
+  for (int j = 0; j < D; ++j) tap(t[D * pitch + j], gs[(D - 1) * D + j], 1);
+#pragma unroll
+  for (int n = 0; n < 2; ++n) out[n] = acc[n] / wp[n];
+}
+
+// One tile of 32 x (blockDim.y * NR) pixels, tile column bx and row by.
+template <bool FAST, int NR>
 __device__ inline void bilateral_tile(const float* __restrict__ src, float* __restrict__ dst,
                                       int rows, int cols, const BilateralTable& tb, int bx,
                                       int by, float* tile) {
   __shared__ unsigned lo_s, hi_s;
-  const int D = 2 * tb.radius, half = tb.radius, TY = blockDim.y;
+  const int D = 2 * tb.radius, half = tb.radius, TY = blockDim.y * NR;
   const int TW = bil_pitch(D), TH = TY + D - 1;
   float* gs = tile + bil_tile_floats(D, TY);  // the spatial weights, staged once per CTA
-  const int tid = threadIdx.y * BTX + threadIdx.x, threads = TY * BTX;
+  const int tid = threadIdx.y * BTX + threadIdx.x, threads = blockDim.y * BTX;
   if (tid == 0) {
     lo_s = 0xffffffffu;
     hi_s = 0u;
@@ -136,7 +182,7 @@ __device__ inline void bilateral_tile(const float* __restrict__ src, float* __re
   const int row0 = by * TY - half, col0 = bx * BTX - half;
   unsigned lo = 0xffffffffu, hi = 0u;  // valid depths as bits (positive floats order as theirs)
   bool hole = false;
-  for (int tr = threadIdx.y; tr < TH; tr += TY) {
+  for (int tr = threadIdx.y; tr < TH; tr += blockDim.y) {
     const int gr = row0 + tr;
     const bool in = gr >= 0 && gr < rows;
     for (int tc = threadIdx.x; tc < TW; tc += BTX) {
@@ -161,32 +207,52 @@ __device__ inline void bilateral_tile(const float* __restrict__ src, float* __re
   }
   const bool mask = __syncthreads_or(hole) != 0;
   const int y = bx * BTX + threadIdx.x;  // column
-  const int x = by * TY + threadIdx.y;   // row (the reference's x)
-  if (x >= rows || y >= cols) return;
-  const float* t = tile + (int)threadIdx.y * TW + threadIdx.x;
-  const float c = t[half * TW + half];
-  float out = 0.0f;
-  if (c > 0.0f) {
-    // the largest |exponent| of the tile's taps, by the taps' own (monotone)
-    // operations
-    const float span = __uint_as_float(hi_s) - __uint_as_float(lo_s);
-    const float i2 = tb.inv2s2, nm = tb.norm;
-    if (!FAST && !(span * span * i2 * 1.44269504088896341f <= 0.5f))
-      out = bilateral_sum<FAST, false, true, 0>(t, gs, TW, D, i2, nm, c);
-    else if (D != 16)
-      out = bilateral_sum<FAST, true, true, 0>(t, gs, TW, D, i2, nm, c);
-    else if (mask)
-      out = bilateral_sum<FAST, true, true, 16>(t, gs, TW, D, i2, nm, c);
-    else
-      out = bilateral_sum<FAST, true, false, 16>(t, gs, TW, D, i2, nm, c);
+  if (y >= cols) return;
+  if (NR == 2 && D == 16) {
+    const int x = by * TY + 2 * threadIdx.y;
+    const float* t = tile + 2 * (int)threadIdx.y * TW + threadIdx.x;
+    const float c[2] = {t[half * TW + half], t[(half + 1) * TW + half]};
+    float out[2] = {0.0f, 0.0f};
+    if (c[0] > 0.0f || c[1] > 0.0f) {
+      if (mask)
+        bilateral_pair<true>(t, gs, TW, tb.inv2s2, c, out);
+      else
+        bilateral_pair<false>(t, gs, TW, tb.inv2s2, c, out);
+    }
+    if (x < rows) dst[x * cols + y] = c[0] > 0.0f ? out[0] : 0.0f;
+    if (x + 1 < rows) dst[(x + 1) * cols + y] = c[1] > 0.0f ? out[1] : 0.0f;
+    return;
   }
-  dst[x * cols + y] = out;
+#pragma unroll 1
+  for (int n = 0; n < NR; ++n) {
+    const int row = (int)threadIdx.y + n * blockDim.y;
+    const int x = by * TY + row;  // row (the reference's x)
+    if (x >= rows) return;
+    const float* t = tile + row * TW + threadIdx.x;
+    const float c = t[half * TW + half];
+    float out = 0.0f;
+    if (c > 0.0f) {
+      // the largest |exponent| of the tile's taps, by the taps' own (monotone)
+      // operations
+      const float span = __uint_as_float(hi_s) - __uint_as_float(lo_s);
+      const float i2 = tb.inv2s2, nm = tb.norm;
+      if (!FAST && !(span * span * i2 * 1.44269504088896341f <= 0.5f))
+        out = bilateral_sum<FAST, false, true, 0>(t, gs, TW, D, i2, nm, c);
+      else if (D != 16)
+        out = bilateral_sum<FAST, true, true, 0>(t, gs, TW, D, i2, nm, c);
+      else if (mask)
+        out = bilateral_sum<FAST, true, true, 16>(t, gs, TW, D, i2, nm, c);
+      else
+        out = bilateral_sum<FAST, true, false, 16>(t, gs, TW, D, i2, nm, c);
+    }
+    dst[x * cols + y] = out;
+  }
 }
 
 __global__ void bilateral_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                  int rows, int cols, const __grid_constant__ BilateralTable tb) {
   extern __shared__ float4 smem4[];
-  bilateral_tile<false>(src, dst, rows, cols, tb, blockIdx.x, blockIdx.y,
+  bilateral_tile<false, 1>(src, dst, rows, cols, tb, blockIdx.x, blockIdx.y,
                         reinterpret_cast<float*>(smem4));
 }
 
@@ -249,9 +315,9 @@ __device__ inline float4 normal_at(const float* d, int pitch, const LevelCamera&
   return make_float4(n.x, n.y, n.z, 0.0f);
 }
 
-// one level, a 32x8 tile of pixels per CTA (the stage entry points: little
+// one level, a 128x2 tile of pixels per CTA (the stage entry points: little
 // more than a launch, 6.1 us at 640x480 as without the tiles)
-constexpr int kMapTX = 32, kMapTY = 8;
+constexpr int kMapTX = 128, kMapTY = 2;
 __global__ void __launch_bounds__(kMapTX * kMapTY)
     maps_kernel(const float* __restrict__ depth, float4* __restrict__ normal,
                 float4* __restrict__ vertex, const LevelCamera c) {
@@ -389,17 +455,19 @@ __global__ void __launch_bounds__(256) fused_ingest_kernel(const SessDev* __rest
   }
 }
 
+template <int NR>  // rows a thread of the mixed form
 __global__ void fused_bilateral_kernel(const SessDev* __restrict__ tab) {
   extern __shared__ float4 smem4[];
   float* tile = reinterpret_cast<float*>(smem4);
   const SessDev& S = tab[blockIdx.z];
   if (!S.bil_enabled) return;
   const int rows = S.ls[0].rows, cols = S.ls[0].cols;
-  if ((int)blockIdx.x * BTX >= cols || (int)(blockIdx.y * blockDim.y) >= rows) return;
+  const int ty = blockDim.y * (S.vol.fp16 ? NR : 1);
+  if ((int)blockIdx.x * BTX >= cols || (int)blockIdx.y * ty >= rows) return;
   if (S.vol.fp16)  // mixed-precision session
-    bilateral_tile<true>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
+    bilateral_tile<true, NR>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
   else
-    bilateral_tile<false>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
+    bilateral_tile<false, 1>(S.raw, S.filt, rows, cols, *S.btab, blockIdx.x, blockIdx.y, tile);
 }
 
 // ---- pyramid and normals of an image in one launch
@@ -627,6 +695,7 @@ static size_t bilateral_smem(int radius, int rows) {
 }
 // Rows of a CTA's tile: 8 stage less halo per pixel, 4 balance small images
 // over the SMs (453x340: 20.2 us with 4, 23.4 with 8; 640x480: 35.1 and 32.6).
+constexpr int kPairCtas = 4 * 148;
 static int bilateral_rows(long long cols, long long rows, int n) {
   return (cols + BTX - 1) / BTX * ((rows + 7) / 8) * n >= 6 * 148 ? 8 : 4;
 }
@@ -657,8 +726,20 @@ void fused_ingest(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
 void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   if (b.max_bil_radius <= 0) return;
   const int ty = bilateral_rows(b.max_cols, b.max_rows, b.n);
-  fused_bilateral_kernel<<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, ty), b.n), dim3(BTX, ty),
-                           bilateral_smem(b.max_bil_radius, ty), st>>>(tab);
+  // Two pixels a thread for tables of mixed sessions alone that still fill the
+  // SMs with half the CTAs (600 of them for one 640x480 frame: 28.3 -> 26.7 us;
+  // 1280x720 51.7 -> 47.4; 32 frames of 320x240 in four groups 213 -> 177, where
+  // their exponentials alone take 140).  An FP32 session's tile has no use for
+  // it, so a table with one keeps the rows of its own.
+  const dim3 threads(BTX, ty);
+  if (ty == 8 && b.fp16_mask == 2 &&
+      (long long)nblk(b.max_cols, BTX) * nblk(b.max_rows, 16) * b.n >= kPairCtas) {
+    fused_bilateral_kernel<2><<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, 2 * ty), b.n), threads,
+                                bilateral_smem(b.max_bil_radius, 2 * ty), st>>>(tab);
+    return;
+  }
+  fused_bilateral_kernel<1><<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, ty), b.n), threads,
+                              bilateral_smem(b.max_bil_radius, ty), st>>>(tab);
 }
 
 void fused_pyramid(const SessDev* tab, const BatchShape& b, int what, int has_rgb,
