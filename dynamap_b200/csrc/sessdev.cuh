@@ -104,7 +104,6 @@ struct BatchShape {
   int max_slot_px[3];      // largest pixel count of each ICP level slot
   int max_slot_iters[3];   // largest lvl_iteration_num of each slot
   int max_bil_radius;      // 0: no session filters
-  int max_rb_tiles;        // largest ray-start bound (tiles; at least 1)
   int max_grid;            // largest block grid (entries; 0: none)
   int kahan_mask;          // bit 0: some session sums plainly, bit 1: some use Kahan sums
   int fp16_mask;           // bit 0: some session keeps FP32 voxels, bit 1: some mixed

@@ -250,7 +250,6 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
       b.max_slot_iters[pl] = std::max(b.max_slot_iters[pl], s->gp.lvl_iteration_num[pl]);
     }
     if (s->bp.enabled) b.max_bil_radius = std::max(b.max_bil_radius, s->btab.radius);
-    b.max_rb_tiles = std::max(b.max_rb_tiles, std::max(1, s->rb_tx * s->rb_ty));
     if (s->vol.grid) b.max_grid = std::max(b.max_grid, s->vol.grid_cap);
     b.kahan_mask |= s->icp_params().kahan ? 2 : 1;
     b.fp16_mask |= s->vol.fp16 ? 2 : 1;
