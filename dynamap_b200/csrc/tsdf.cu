@@ -20,6 +20,7 @@
 
 #include <algorithm>
 
+#include "ray_grid.cuh"
 #include "sessdev.cuh"
 
 namespace dyn {
@@ -33,74 +34,6 @@ namespace {
 constexpr float kRint = 12582912.0f;   // 1.5 * 2^23
 constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
 
-// ------------------------------------------------------------ the block grid
-// The raycast looks blocks up by their coordinates far more often than
-// anything else (every sample, up to eight blocks), so each frame's blocks are
-// also laid out in a dense grid over the box the frame's rays can reach
-// (GridBox; z fastest): entry = first voxel of the block (512 x heap index),
-// or of the empty block after the heap.  A lookup is one multiply-add chain
-// and one load without branches, where the hash takes a bucket scan in a
-// divergent branch for every lane that changes block: with the exact march
-// below and hash lookups a 640x480 FP32 target took 257 M warp instructions at
-// 20 of 32 lanes (485 us, as before it); with the grid 138 M at 28 lanes
-// (260 us; 320x240 225 -> 98 us).  The mixed march, whose arithmetic did not
-// change: 640x480 136 -> 61 us, 1280x720 band 200 -> 100 us, and a 32-session
-// band batch 667 -> 351 us.
-__device__ inline GridBox grid_box(const float* __restrict__ T, const DSensor& s, const DTsdf& t,
-                                   int cap) {
-  GridBox b;
-  float lo[3], hi[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) lo[a] = hi[a] = T[4 * a + 3];
-  const float u0 = (0.0f - s.cx) / s.fx, u1 = ((float)(s.cols - 1) - s.cx) / s.fx;
-  const float v0 = (0.0f - s.cy) / s.fy, v1 = ((float)(s.rows - 1) - s.cy) / s.fy;
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float e = (T[4 * a] * ((k & 1) ? u1 : u0) + T[4 * a + 1] * ((k & 2) ? v1 : v0) +
-                       T[4 * a + 2]) * t.dmax + T[4 * a + 3];
-      lo[a] = fminf(lo[a], e);
-      hi[a] = fmaxf(hi[a], e);
-    }
-  int n[3], o[3];
-  bool ok = cap > 0;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    // a block of margin below, two above (a cell's high corners); 2^20 blocks
-    // is the key's range
-    const float l = floorf(lo[a] / t.bsm) - 1.0f, h = floorf(hi[a] / t.bsm) + 2.0f;
-    ok = ok && l > -1048576.0f && h < 1048576.0f;
-    o[a] = ok ? (int)l : 0;
-    n[a] = ok ? (int)h - (int)l + 1 : 0;
-  }
-  ok = ok && (double)n[0] * (double)n[1] * (double)n[2] <= (double)cap;
-  b.x0 = o[0];
-  b.y0 = o[1];
-  b.z0 = o[2];
-  b.nx = n[0];
-  b.ny = n[1];
-  b.nz = n[2];
-  b.ok = ok ? 1 : 0;
-  return b;
-}
-// The grid emptied at pose T by 'threads' threads, this one number 'thread'.
-__device__ inline void grid_clear(const VolumeDev& v, const float* __restrict__ T,
-                                  const DSensor& s, int thread, int threads) {
-  const GridBox b = grid_box(T, s, v.t, v.grid_cap);
-  if (thread == 0) *v.gbox = b;
-  if (!b.ok) return;
-  const int n4 = (b.nx * b.ny * b.nz + 3) / 4;  // (the buffer holds whole vectors)
-  const unsigned e = (unsigned)v.t.num_blocks * (unsigned)kBlockVox;
-  for (int i = thread; i < n4; i += threads)
-    reinterpret_cast<uint4*>(v.grid)[i] = make_uint4(e, e, e, e);
-}
-__device__ inline void grid_put(const VolumeDev& v, const GridBox& b, unsigned long long key,
-                                int ptr, unsigned flag) {
-  const int x = key_x(key) - b.x0, y = key_y(key) - b.y0, z = key_z(key) - b.z0;
-  if ((unsigned)x < (unsigned)b.nx && (unsigned)y < (unsigned)b.ny && (unsigned)z < (unsigned)b.nz)
-    v.grid[(x * b.ny + y) * b.nz + z] = ((unsigned)ptr * (unsigned)kBlockVox) | flag;
-}
 // ------------------------------------------------------------ allocation
 constexpr int kAllocX = 16, kAllocY = 16, kAllocN = kAllocX * kAllocY;  // pixel tile per CTA
 constexpr int kSetBits = 11, kSetSlots = 1 << kSetBits;                 // CTA-local dedup set
@@ -608,7 +541,9 @@ __device__ inline bool free_space_block(unsigned long long key, const DTsdf& t, 
     dm = fmaxf(dm, dot3(c, c));
   }
   dm = sqrtf(dm);
-  if (!(u0 >= 1.0f && v0 >= 1.0f && u1 <= (float)(s.cols - 2) && v1 <= (float)(s.rows - 2)))
+  // (u0 <= u1 fails where every corner's projection is NaN)
+  if (!(u0 >= 1.0f && v0 >= 1.0f && u1 <= (float)(s.cols - 2) && v1 <= (float)(s.rows - 2) &&
+        u0 <= u1 && v0 <= v1))
     return false;
   const int x0 = (int)floorf(u0) - 1, x1 = (int)ceilf(u1) + 1;
   const int y0 = (int)floorf(v0) - 1, y1 = (int)ceilf(v1) + 1;
@@ -1459,50 +1394,6 @@ __device__ inline void cell_corners(const GridView& G, unsigned g, unsigned e0, 
   i[7] = b[7] + (xh + yh) + zh;
 }
 
-struct MarchRay {
-  float yhx, ylx, yhy, yly;  // reciprocals of fx and fy
-};
-
-__device__ inline bool recip_ok(float x) {
-  return fabsf(x) >= 9.5367431640625e-7f && fabsf(x) <= 1048576.0f;  // 2^-20 .. 2^20
-}
-
-// The largest |coordinate| in voxels of the samples of pixel offset (px, py)
-// (per unit depth) from pose T, up to dmax; NaN for a pose that is not finite.
-__device__ inline float march_extent(const DTsdf& t, const M4f& T, float px, float py,
-                                     float inv_vs) {
-  float far = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float e = (fabsf(T.m[4 * i]) * fabsf(px) + fabsf(T.m[4 * i + 1]) * fabsf(py) +
-                     fabsf(T.m[4 * i + 2])) * t.dmax + fabsf(T.m[4 * i + 3]);
-    far = e > far ? e : (e <= far ? far : e);  // NaN passes on
-  }
-  return far * inv_vs * 1.001f + 2.0f;
-}
-
-// Every step of a march is at least min(voxel, truncation): below 4096 of them
-// up to dmax the roundings of cur add up to less than a step, so the march
-// ends within the step cap (rc_cap, four steps more) and needs no count.
-__device__ inline bool march_bounded(const DTsdf& t) {
-  return t.dmax <= 4096.0f * fminf(t.vs, t.trunc);
-}
-
-// Whether the fast indices and divisions hold along the whole ray of pixel
-// offset (ax, ay) from pose T, with their constants.
-__device__ inline bool march_setup(const DTsdf& t, const DSensor& s, const M4f& T, float ax,
-                                   float ay, float inv_vs, MarchRay& m) {
-  const bool ok = recip_ok(s.fx) && recip_ok(s.fy) && (ax == 0.0f || recip_ok(ax)) &&
-                  (ay == 0.0f || recip_ok(ay)) && recip_ok(t.vs) && recip_ok(t.trunc) &&
-                  recip_ok(t.dmax) && march_bounded(t);
-  m.yhx = 1.0f / s.fx;
-  m.yhy = 1.0f / s.fy;
-  m.ylx = __fmaf_rn(-s.fx, m.yhx, 1.0f) * m.yhx;
-  m.yly = __fmaf_rn(-s.fy, m.yhy, 1.0f) * m.yhy;
-  const float far = march_extent(t, T, ax * m.yhx, ay * m.yhy, inv_vs);
-  return ok && far < 131072.0f;
-}
-
 // The depths of a march: samples below the near distance, then steps without a
 // lookup up to the tile's near bound (no allocated block there, so each sample
 // would step by the truncation), samples up to the far bound, and steps
@@ -1883,8 +1774,7 @@ __device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4
   const DTsdf& t = v.t;
   const float inv_vs = 1.0f / t.vs;
   const float axf = ((float)x - s.cx) / s.fx, ayf = ((float)y - s.cy) / s.fy;
-  if (!v.grid || !v.gbox->ok || !march_bounded(t) ||
-      !(march_extent(t, T, axf, ayf, inv_vs) < 131072.0f))
+  if (!v.grid || !v.gbox->ok || !march_bounded(t) || !march_within(t, T, axf, ayf, inv_vs))
     return raycast_hash_px<true, FREE>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
   const F3 o = f3(T.m[3] * inv_vs, T.m[7] * inv_vs, T.m[11] * inv_vs);
   const F3 d = f3((T.m[0] * axf + T.m[1] * ayf + T.m[2]) * inv_vs,
