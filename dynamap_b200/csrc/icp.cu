@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "last_block.cuh"
 #include "sessdev.cuh"
 
 namespace dyn {
@@ -849,12 +850,7 @@ __device__ inline void icp_iteration_body(const FrameLevel& L, int pl, int it, I
   tile_partials<KAHAN>(L, Ts, bid, nb, red, [&](int tile, int k, double x) {
     partials[(size_t)tile * kIcpVals + k] = x;
   });
-  __threadfence();
-  __shared__ unsigned int ticket;
-  if (threadIdx.x == 0) ticket = atomicAdd(&st->ticket, 1u);
-  __syncthreads();
-  if (ticket != (unsigned)nb - 1) return;
-  __threadfence();
+  if (!last_block(&st->ticket, (unsigned)nb)) return;
   __shared__ double tot[kIcpVals];
   double v[kWarpRows];
 #pragma unroll
@@ -1280,12 +1276,7 @@ __global__ void __launch_bounds__(kIcpThreads)
     pixel_terms<false>(L, P, T, idx, a);
   block_reduce<false, kIcpThreads / 32>(a, red);
   if (threadIdx.x < kIcpVals) partials[(size_t)blockIdx.x * kIcpVals + threadIdx.x] = red[threadIdx.x];
-  __threadfence();
-  __shared__ unsigned int ticket;
-  if (threadIdx.x == 0) ticket = atomicAdd(ticket_ctr, 1u);
-  __syncthreads();
-  if (ticket != gridDim.x - 1) return;
-  __threadfence();
+  if (!last_block(ticket_ctr, gridDim.x)) return;
   __shared__ double tot[kIcpVals];
   final_reduce(partials, gridDim.x, tot, red);
   if (threadIdx.x < kIcpVals) out[threadIdx.x] = tot[threadIdx.x];
