@@ -902,15 +902,19 @@ template <bool KAHAN>
 __global__ void __launch_bounds__(kIcpFrameThreads, 1)
     fused_icp_iteration_kernel(const SessDev* __restrict__ tab, int pl, int it) {
   const SessDev& S = tab[blockIdx.z];
-  if ((S.icpp.kahan != 0) != KAHAN) return;
-  if (it >= S.slot_iters[pl]) return;  // the reference runs iterations 1 .. N-1
   const int l = S.slot_level[pl];
   const int nb = icp_tiles(S.ls[l].rows * S.ls[l].cols, KAHAN);
-  if ((int)blockIdx.x >= nb) return;
+  // (the reference runs iterations 1 .. N-1)
+  const bool mine = (S.icpp.kahan != 0) == KAHAN && it < S.slot_iters[pl] && (int)blockIdx.x < nb;
   __shared__ FrameLevel L;  // shared: registers go to the sums
-  if (threadIdx.x == 0) L = level_of(S, l);
-  wait_predecessor();  // the solver state and partials of the previous iteration
+  if (mine && threadIdx.x == 0) L = level_of(S, l);
+  // The solver state and partials of the previous iteration.  Every block waits,
+  // those without work too: a launch waits for the one before it alone, so one
+  // whose blocks all left at once (no session of its kind has that many
+  // iterations) would let the next start beside the last but one.
+  wait_predecessor();
   release_successor();
+  if (!mine) return;
   icp_iteration_body<KAHAN>(L, pl, it, S.icp, S.partials, blockIdx.x, nb);
 }
 
