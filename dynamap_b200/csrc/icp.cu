@@ -932,11 +932,12 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
 // themselves until they carry the iteration's tag -- one store's and one
 // load's way through L2 between two blocks, with no fence (whose acquire side
 // also empties L1, where the images stay from iteration to iteration).
-// Iterations alternate between two rows per tile: a block writes its row of an
-// iteration only after reading every row of the one before, so the rows it
-// overwrites have been read.  Blocks without a tile of a level wait for the
-// state that the session's first block leaves at the level's end; those
-// without a tile of a later level return.
+// A level's iterations alternate between two rows per tile: a block writes its
+// row of an iteration only after reading every row of the one before, which the
+// others wrote after reading the rows that it overwrites.  Each level has its own
+// rows (icp_row).  Blocks without a tile of a level wait for the state that the
+// session's first block leaves at the level's end; those without a tile of a
+// later level return.
 //
 // The coarse levels are a chain of latencies, about six iterations of a
 // frame's nine: the block's sums 2,500 (sky) to 6,000 cycles, the rows 2,000,
@@ -1027,7 +1028,7 @@ struct FrameState {
   double tot[kIcpVals];
   double inc[6], prev[6];
   M4f T;  // the transform of the iteration
-  int conv, have, par, iters[3], inliers[3];
+  int conv, have, iters[3], inliers[3];
   float rms[3];
   unsigned epoch;
 };
@@ -1139,7 +1140,6 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
   if (threadIdx.x == 0) {
     F.conv = S.icp->converged;
     F.have = S.icp->have_target;
-    F.par = 0;
     F.epoch = S.icp_bar[0];
   }
   __syncthreads();
@@ -1161,16 +1161,15 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
     if (!F.have || iters_pl <= 1) continue;  // (alike in every block of the session)
     const int ntiles = icp_tiles(S.ls[l].rows * S.ls[l].cols, KAHAN);
     const unsigned tag0 = epoch + (unsigned)pl * 1024u;  // iterations 1 .. 999, then the state
-    uint2* const state = rows + (size_t)(2 * kIcpMaxTiles + pl) * kIcpRowWords;
+    uint2* const state = rows + (size_t)icp_state_row(pl) * kIcpRowWords;
     if (local < ntiles) {
       // level and transform stay in shared memory (registers go to the sums)
       if (threadIdx.x == 0) Ls = level_of(S, l);
       __syncthreads();
-      int parity = F.par;
       for (int it = 1; it < iters_pl; ++it) {
         // every block at the level holds the state: they leave it together
         if (it > 1 && F.conv) break;
-        uint2* const part = rows + (size_t)parity * kIcpMaxTiles * kIcpRowWords;
+        uint2* const part = rows + (size_t)icp_row(pl, it, 0) * kIcpRowWords;
         const unsigned tag = tag0 + (unsigned)it;
         tile_partials<KAHAN>(Ls, F.T, local, nblk, red,
                              [&](int tile, int k, double x) {
@@ -1178,17 +1177,14 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
                              });
         good = finish_iteration<KAHAN>(part, Ls, tag, abort_word, pl, it, F, red);
         if (!good) break;
-        parity ^= 1;
       }
       if (!good) break;  // (block-uniform)
       __syncthreads();
-      if (threadIdx.x == 0) F.par = parity;
       if (local == 0 && nblk > ntiles) {  // for the blocks without a tile here
         const unsigned tag = tag0 + 1023u;
         const int k = threadIdx.x;
         if (k < 12) put_value(state, k, k < 6 ? F.inc[k] : F.prev[k - 6], tag);
         else if (k < 28) store_word(state + k, __float_as_uint(Tf[k - 12]), tag);
-        else if (k == 28) store_word(state + 28, (unsigned)parity, tag);
       }
       __syncthreads();
     } else {
@@ -1199,7 +1195,7 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
         BoundedWait wait;
         for (;;) {
           bool here = true;
-          if (k < 29) {
+          if (k < 28) {
             a = load_word(state + k);
             here = a.y == tag;
           }
@@ -1216,7 +1212,6 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
         }
         if (k < 12) (k < 6 ? F.inc[k] : F.prev[k - 6]) = __hiloint2double((int)b.x, (int)a.x);
         else if (k < 28) Tf[k - 12] = __uint_as_float(a.x);
-        else if (k == 28) F.par = (int)a.x;
       }
       if (!__syncthreads_and(good)) {
         good = false;

@@ -91,13 +91,23 @@ inline __host__ __device__ long long icp_weight(int npx, int kahan) {
 size_t icp_scratch_bytes();
 // Scratch of a session's per-frame ICP: the chained kernels' row of partial
 // sums per tile, then the persistent kernel's rows (kIcpRowWords tagged words
-// each): two per tile (iterations alternate) and the state's of each level.
+// each): per level slot two per tile, by the iteration's parity, and the level's
+// state.  A level has rows of its own: a block that leaves after its last level
+// still reads that level's last rows, and says nothing to the others, who may be
+// two iterations into the next level by then (as with two rows per tile for all
+// levels; 161 KB per session, now 481).
 constexpr int kIcpRowWords = 64;
 inline __host__ __device__ size_t icp_rows_offset() {  // bytes
   return ((size_t)kIcpMaxTiles * kIcpVals * sizeof(double) + 255) / 256 * 256;
 }
+// The row of tile 'tile' in iteration 'it' of level slot pl.
+inline __host__ __device__ int icp_row(int pl, int it, int tile) {
+  return (2 * pl + (it & 1)) * kIcpMaxTiles + tile;
+}
+// The row that level slot pl's state is left in.
+inline __host__ __device__ int icp_state_row(int pl) { return 6 * kIcpMaxTiles + pl; }
 inline size_t icp_frame_scratch_bytes() {
-  return icp_rows_offset() + (size_t)(2 * kIcpMaxTiles + 3) * kIcpRowWords * 8;
+  return icp_rows_offset() + (size_t)(6 * kIcpMaxTiles + 3) * kIcpRowWords * 8;
 }
 
 // The persistent ICP (one cooperative launch per frame and summation kind):

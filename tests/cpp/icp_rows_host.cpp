@@ -1,0 +1,49 @@
+// The rows of the persistent ICP (dynamap_b200/csrc/icp.cuh) in the order that
+// lets a block fall behind: one that has left after its last level's rows were
+// complete, but has not read them yet, while the others run every later level.
+#include "cuda_emu.h"
+
+#include <set>
+
+#include "../../dynamap_b200/csrc/icp.cuh"
+
+extern "C" int icp_tiles_of(int npx, int kahan) { return dyn::icp_tiles(npx, kahan); }
+
+// Level slots of npx[0..2] pixels, iters[0..2] executed iterations each, a block
+// per tile.  Returns the rows of some block's last level that a later level
+// overwrites (of *leavers levels that some block leaves after).
+extern "C" int icp_rows_overwritten(const int* npx, const int* iters, int kahan, int* leavers) {
+  using namespace dyn;
+  int nt[3], bad = 0;
+  *leavers = 0;
+  for (int pl = 0; pl < 3; ++pl) nt[pl] = iters[pl] > 0 ? icp_tiles(npx[pl], kahan) : 0;
+  for (int pl = 0; pl < 3; ++pl) {
+    int later = 0;
+    for (int q = pl + 1; q < 3; ++q) later = nt[q] > later ? nt[q] : later;
+    if (nt[pl] <= later || nt[pl] == 0) continue;  // every block goes on
+    ++*leavers;
+    std::set<int> rows;  // what a block that leaves reads last
+    for (int t = 0; t < nt[pl]; ++t) rows.insert(icp_row(pl, iters[pl], t));
+    for (int q = pl + 1; q < 3; ++q) {
+      for (int it = 1; it <= iters[q]; ++it)
+        for (int t = 0; t < nt[q]; ++t) bad += rows.count(icp_row(q, it, t)) != 0;
+      bad += rows.count(icp_state_row(q)) != 0;
+    }
+  }
+  return bad;
+}
+
+// Every row and state word lies in the scratch; rows of one level and parity
+// are distinct.
+extern "C" int icp_rows_in_scratch() {
+  using namespace dyn;
+  std::set<int> seen;
+  for (int pl = 0; pl < 3; ++pl) {
+    for (int par = 0; par < 2; ++par)
+      for (int t = 0; t < kIcpMaxTiles; ++t) seen.insert(icp_row(pl, 2 + par, t));
+    seen.insert(icp_state_row(pl));
+  }
+  const size_t end = icp_rows_offset() + ((size_t)*seen.rbegin() + 1) * kIcpRowWords * 8;
+  return *seen.begin() == 0 && (int)seen.size() == 6 * kIcpMaxTiles + 3 &&
+         end <= icp_frame_scratch_bytes();
+}

@@ -1,6 +1,6 @@
 """The chained ICP (a launch per iteration) and the persistent one (one launch
 per frame) give the same bits: tables of both summation kinds with different
-iteration counts."""
+iteration counts, and sessions whose levels differ in the shape of their tiles."""
 import json
 import os
 import subprocess
@@ -92,3 +92,23 @@ def test_kinds_of_different_iteration_counts(tmp_path, gpu_lib):
         [member(120, 160, fp32, few), member(120, 160, mixed, many)],
         [member(120, 160, fp32, many), member(120, 160, mixed, few),
          member(96, 128, mixed, many, rgb=True)]])
+
+
+FP32, MIXED = abi.PRECISION_FP32, abi.PRECISION_MIXED
+
+
+def test_tile_shapes(tmp_path, gpu_lib):
+    """Levels where the tiles change shape: a level of 256-slot tiles at its
+    largest and one pixel row beyond, blocks that leave before the last level
+    (more tiles on a coarser level, levels from fine to coarse), pixel groups of
+    one, two and four in the compensated form, ragged levels."""
+    it = (5, 4, 4)
+    tables = [member(497, 661, FP32, it),                   # 41, 160, 129 tiles
+              member(148, 256, FP32, it), member(149, 256, FP32, it), member(147, 257, FP32, it),
+              member(120, 160, FP32, it, (1, 2, 4)), member(497, 661, FP32, it, (1, 2, 4)),
+              member(120, 160, MIXED, it, (1, 2, 4), rgb=True), member(240, 320, FP32, it, (2, 4, 1)),
+              member(64, 128, MIXED, it), member(65, 127, MIXED, it),
+              member(256, 256, MIXED, it), member(257, 255, MIXED, it, rgb=True),
+              member(133, 177, FP32, it, rgb=True), member(133, 177, MIXED, it, (8, 4, 1)),
+              member(24, 40, FP32, it, (8, 2, 1)), member(24, 40, MIXED, it, (8, 2, 1))]
+    assert_forms_agree(tmp_path, [[m] for m in tables])
