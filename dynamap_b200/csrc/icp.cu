@@ -1331,7 +1331,7 @@ __global__ void fused_pose_finalize_kernel(const SessDev* __restrict__ tab, int 
   if (s >= n) return;
   const SessDev& S = tab[s];
   pose_finalize_body(S.icpp, S.icp, S.pose);
-  S.icp_bar[0] += kIcpEpochStep;  // the next launch's tags
+  advance_epoch(S.icp_bar, S.partials);  // the next launch's tags
   S.icp_bar[kIcpAbort] = 0;
   if (bump) S.pose->frame += 1;
 }

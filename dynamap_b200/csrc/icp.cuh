@@ -106,8 +106,9 @@ inline __host__ __device__ int icp_row(int pl, int it, int tile) {
 }
 // The row that level slot pl's state is left in.
 inline __host__ __device__ int icp_state_row(int pl) { return 6 * kIcpMaxTiles + pl; }
+constexpr int kIcpRows = 6 * kIcpMaxTiles + 3;
 inline size_t icp_frame_scratch_bytes() {
-  return icp_rows_offset() + (size_t)(6 * kIcpMaxTiles + 3) * kIcpRowWords * 8;
+  return icp_rows_offset() + (size_t)kIcpRows * kIcpRowWords * 8;
 }
 
 // The persistent ICP (one cooperative launch per frame and summation kind):
@@ -120,11 +121,25 @@ inline size_t icp_frame_scratch_bytes() {
 int icp_persistent_capacity(int device);
 int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int* grid_k);
 // The persistent ICP's words of a session: the epoch of the next launch's tags
-// (advanced by kIcpEpochStep by the pose finalisation that follows a launch;
-// never 0) and, on a line of its own, the abort word (zero before a launch).
+// (advance_epoch) and, on a line of its own, the abort word (zero before a launch).
 constexpr int kIcpAbort = 32;
 constexpr int kIcpBarWords = 64;
 constexpr unsigned kIcpEpochStep = 4096;
+// Called by one thread after a launch: the next launch's epoch.  Tags are 32
+// bits, so an epoch comes again after 2^20 launches; a row that none of them
+// wrote would then pass for this launch's, so the rows are emptied where the
+// epochs start again (481 KB by one thread, once in 9.7 hours at 30 Hz).  0 is no
+// epoch: an empty row carries no tag of any launch.
+inline __host__ __device__ void advance_epoch(unsigned* bar, void* scratch) {
+  unsigned e = bar[0] + kIcpEpochStep;
+  if (e < kIcpEpochStep) {
+    uint4* const rows = reinterpret_cast<uint4*>(static_cast<char*>(scratch) + icp_rows_offset());
+    const int n = kIcpRows * kIcpRowWords / 2;
+    for (int i = 0; i < n; ++i) rows[i] = make_uint4(0u, 0u, 0u, 0u);
+    e = kIcpEpochStep;
+  }
+  bar[0] = e;
+}
 // The bounded wait of the persistent ICP's blocks, as a barrier run alone:
 // 'blocks' blocks wait for blocks + missing arrivals (bar_dev: kIcpBarWords
 // words).  DYN_OK when it completes, DYN_ERR_TIMEOUT when the wait ran out,

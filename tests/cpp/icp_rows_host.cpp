@@ -3,7 +3,9 @@
 // complete, but has not read them yet, while the others run every later level.
 #include "cuda_emu.h"
 
+#include <cstdint>
 #include <set>
+#include <vector>
 
 #include "../../dynamap_b200/csrc/icp.cuh"
 
@@ -46,4 +48,20 @@ extern "C" int icp_rows_in_scratch() {
   const size_t end = icp_rows_offset() + ((size_t)*seen.rbegin() + 1) * kIcpRowWords * 8;
   return *seen.begin() == 0 && (int)seen.size() == 6 * kIcpMaxTiles + 3 &&
          end <= icp_frame_scratch_bytes();
+}
+
+// The epoch after the one given, over a scratch filled with 'fill': returns the
+// new epoch; *rows the bytes of the rows that still hold the fill, *before those
+// of what lies before the rows.
+extern "C" unsigned icp_next_epoch(unsigned epoch, int fill, int64_t* rows, int64_t* before) {
+  using namespace dyn;
+  std::vector<unsigned char> scratch(icp_frame_scratch_bytes() + 16, (unsigned char)fill);
+  unsigned bar[kIcpBarWords] = {epoch};
+  unsigned char* base = scratch.data();
+  while (reinterpret_cast<uintptr_t>(base) & 15) ++base;
+  advance_epoch(bar, base);
+  *rows = *before = 0;
+  for (size_t i = 0; i < icp_frame_scratch_bytes(); ++i)
+    (i < icp_rows_offset() ? *before : *rows) += base[i] == (unsigned char)fill;
+  return bar[0];
 }

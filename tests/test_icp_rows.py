@@ -48,3 +48,16 @@ def test_no_level_overwrites_rows_of_another(lib, scales, kahan):
                 left += n.value
     if scales[0] < scales[2]:
         assert left > 0
+
+
+def test_rows_are_empty_when_the_epochs_start_again(lib):
+    """Tags repeat after 2^20 launches: no row of the round before survives that."""
+    f = lib.icp_next_epoch
+    f.restype, f.argtypes = C.c_uint, [C.c_uint, C.c_int, C.c_void_p, C.c_void_p]
+    rows, before = C.c_int64(0), C.c_int64(0)
+    row_bytes = (6 * 160 + 3) * 512
+    for epoch in (4096, 8192, 0x7ffff000, 0xffffe000):
+        assert f(epoch, 0xab, C.byref(rows), C.byref(before)) == epoch + 4096
+        assert rows.value == row_bytes
+    assert f(0xfffff000, 0xab, C.byref(rows), C.byref(before)) == 4096
+    assert rows.value == 0 and before.value >= 160 * 29 * 8
