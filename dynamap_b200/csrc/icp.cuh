@@ -120,6 +120,42 @@ inline size_t icp_frame_scratch_bytes() {
 // chained kernels run the table, with the same results).
 int icp_persistent_capacity(int device);
 int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int* grid_k);
+// Resident blocks that each of k groups of sessions may take for its persistent
+// ICP, out[g], when the groups run at once: 'weight' a group's icp_weight in all,
+// 'count' its sessions.  The shares never add up to more than 'cap', so that all
+// launches can be resident together (their blocks wait for one another: a launch
+// that is resident in part beside another such would wait out its bound); a
+// group has a block per session or none (the chained kernels).  Shares follow the
+// weights, except that a group whose part would be less than a block per session
+// is given just that while there are blocks for every session.
+inline void icp_group_budgets(const long long* weight, const int* count, int k, int cap,
+                              int* out) {
+  long long sessions = 0;
+  for (int g = 0; g < k; ++g) {
+    sessions += count[g];
+    out[g] = 0;
+  }
+  if (cap <= 0) return;
+  const bool all_fit = sessions <= cap;
+  long long left = cap, rest = 0;  // blocks and weight of the groups not yet settled
+  for (int g = 0; g < k; ++g) rest += weight[g];
+  for (bool again = all_fit; again;) {
+    again = false;
+    for (int g = 0; g < k; ++g)
+      if (out[g] == 0 && count[g] > 0 && left * weight[g] < rest * count[g]) {
+        out[g] = count[g];
+        left -= count[g];
+        rest -= weight[g];
+        again = true;
+      }
+  }
+  for (int g = 0; g < k; ++g)
+    if (out[g] == 0 && count[g] > 0 && rest > 0) {
+      const int share = (int)(left * weight[g] / rest);
+      out[g] = share >= count[g] ? share : 0;
+    }
+}
+
 // The persistent ICP's words of a session: the epoch of the next launch's tags
 // (advance_epoch) and, on a line of its own, the abort word (zero before a launch).
 constexpr int kIcpAbort = 32;

@@ -18,21 +18,19 @@ extern "C" {
 
 // ---------------------------------------------------------------- batches
 
-// Resident blocks of group g's persistent ICP out of 'cap': in proportion
-// to the group's work among all groups' (at least one per session).
-static int group_budget(const std::vector<dyn_session*>& sorted, const std::vector<int>& start,
-                        int g, int cap) {
-  long long all = 0, mine = 0;
+// Each group's share of the 'cap' blocks that can be resident (icp_group_budgets).
+static std::vector<int> group_budgets(const std::vector<dyn_session*>& sorted,
+                                      const std::vector<int>& start, int cap) {
   const int k = (int)start.size() - 1;
-  for (int h = 0; h < k; ++h)
-    for (int j = start[h]; j < start[h + 1]; ++j) {
-      const long long t = icp_weight((int)sorted[j]->npx, sorted[j]->icp_params().kahan);
-      all += t;
-      if (h == g) mine += t;
-    }
-  if (all <= 0) return 0;
-  const int n = start[g + 1] - start[g];
-  return cap > 0 ? std::max(n, (int)((long long)cap * mine / all)) : 0;
+  std::vector<long long> weight((size_t)k, 0);
+  std::vector<int> count((size_t)k), out((size_t)k);
+  for (int g = 0; g < k; ++g) {
+    count[g] = start[g + 1] - start[g];
+    for (int j = start[g]; j < start[g + 1]; ++j)
+      weight[g] += icp_weight((int)sorted[j]->npx, sorted[j]->icp_params().kahan);
+  }
+  icp_group_budgets(weight.data(), count.data(), k, cap, out.data());
+  return out;
 }
 
 dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch** out) {
@@ -137,6 +135,8 @@ dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch**
   FrameGroups& G = b->groups;
   G.k = k;
   G.st[0] = b->stream;
+  // the groups' persistent ICP launches may run at once: together they fit
+  const std::vector<int> budget = group_budgets(sorted, start, icp_persistent_capacity(b->device));
   int64_t voff = 0;
   for (int g = 0; g < k; ++g) {
     const int n_g = start[g + 1] - start[g];
@@ -146,10 +146,7 @@ dyn_status dyn_batch_create(dyn_session* const* sessions, int32_t n, dyn_batch**
     G.map[g] = b->d_map + start[g];
     G.shape[g] = make_shape(sorted.data() + start[g], n_g, b->d_gvis + voff, b->d_gcount + g,
                             (int)cap_g);
-    // the groups' persistent ICP launches may run at once: each takes a
-    // share of the resident blocks in proportion to its pixel tiles
-    set_icp_persistent(G.shape[g], sorted.data() + start[g], n_g,
-                       group_budget(sorted, start, g, icp_persistent_capacity(b->device)));
+    set_icp_persistent(G.shape[g], sorted.data() + start[g], n_g, budget[g]);
     voff += cap_g;
   }
   FrameGroups& one = b->single;
@@ -197,14 +194,14 @@ constexpr int kNumTune = (int)(sizeof(kTune) / sizeof(kTune[0]));
 constexpr int kNumIcpShapes = 3;
 
 static void apply_shape(dyn_batch* b, const TuneCandidate& c) {
-  const int cap = icp_persistent_capacity(b->device);
+  const std::vector<int> shares =
+      group_budgets(b->sorted, b->gstart, icp_persistent_capacity(b->device));
   const int k = b->groups.k;
   for (int g = 0; g < k; ++g) {
     BatchShape& sh = b->groups.shape[g];
     sh.integrate_ctas = c.integrate_ctas;
     sh.ray_tile = c.ray_tile;
-    const int share = group_budget(b->sorted, b->gstart, g, cap);
-    const int budget = c.icp == 2 ? 0 : (c.icp == 1 ? share / 2 : share);
+    const int budget = c.icp == 2 ? 0 : (c.icp == 1 ? shares[g] / 2 : shares[g]);
     set_icp_persistent(sh, b->sorted.data() + b->gstart[g], b->gstart[g + 1] - b->gstart[g],
                        budget);
   }

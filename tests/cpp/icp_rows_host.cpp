@@ -1,4 +1,4 @@
-// The rows of the persistent ICP (dynamap_b200/csrc/icp.cuh) in the order that
+// The persistent ICP's host arithmetic (dynamap_b200/csrc/icp.cuh).  Its rows, in the order that
 // lets a block fall behind: one that has left after its last level's rows were
 // complete, but has not read them yet, while the others run every later level.
 #include "cuda_emu.h"
@@ -65,3 +65,8 @@ extern "C" unsigned icp_next_epoch(unsigned epoch, int fill, int64_t* rows, int6
     (i < icp_rows_offset() ? *before : *rows) += base[i] == (unsigned char)fill;
   return bar[0];
 }
+
+extern "C" void icp_budgets(const long long* weight, const int* count, int k, int cap, int* out) {
+  dyn::icp_group_budgets(weight, count, k, cap, out);
+}
+extern "C" long long icp_weight_of(int npx, int kahan) { return dyn::icp_weight(npx, kahan); }

@@ -112,3 +112,12 @@ def test_tile_shapes(tmp_path, gpu_lib):
               member(133, 177, FP32, it, rgb=True), member(133, 177, MIXED, it, (8, 4, 1)),
               member(24, 40, FP32, it, (8, 2, 1)), member(24, 40, MIXED, it, (8, 2, 1))]
     assert_forms_agree(tmp_path, [[m] for m in tables])
+
+
+def test_batches_of_many_sessions(tmp_path, gpu_lib):
+    """More sessions than a group's part of the device has blocks: 66 members of
+    three sizes and both kinds, their groups' launches running at once."""
+    it = (4, 3, 3)
+    sizes = [(48, 64), (48, 64), (48, 64), (120, 160), (48, 64), (240, 320)]
+    assert_forms_agree(tmp_path, [[member(*sizes[i % 6], (FP32, MIXED)[i % 4 == 1], it)
+                                   for i in range(66)]])
