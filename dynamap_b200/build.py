@@ -23,7 +23,7 @@ SOURCES = ["image.cu", "icp.cu", "tsdf.cu", "session.cu", "serving.cu", "noalloc
            "mesh.cu", "evict.cu", "config.cpp"]
 HEADERS = ["common.cuh", "image.cuh", "icp.cuh", "tsdf.cuh", "sessdev.cuh", "session_impl.cuh",
            "dyn_exp.h", "mesh_cell.h", "mc_tables.h", "evict_ops.h", "mesh_kernels.cuh",
-           "evict_kernels.cuh", "ray_grid.cuh", "last_block.cuh"]
+           "evict_kernels.cuh", "ray_grid.cuh", "last_block.cuh", "near_key.cuh"]
 
 # -fmad=false: no FMA contraction, IEEE div/sqrt: every float operation
 # rounds once, in source order (the bit-exact parity with the oracle relies

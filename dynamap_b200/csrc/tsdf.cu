@@ -20,6 +20,7 @@
 
 #include <algorithm>
 
+#include "near_key.cuh"
 #include "ray_grid.cuh"
 #include "sessdev.cuh"
 
@@ -36,41 +37,7 @@ constexpr int kRintBits = 0x4B400000;  // its bits: a multiple of 8
 
 // ------------------------------------------------------------ allocation
 constexpr int kAllocX = 16, kAllocY = 16, kAllocN = kAllocX * kAllocY;  // pixel tile per CTA
-constexpr int kSetBits = 11, kSetSlots = 1 << kSetBits;                 // CTA-local dedup set
 constexpr int kSetProbes = 32;
-
-// A block in a CTA's set: its offset from the camera's block, biased fields of
-// BITS bits an axis, so that a step is one addition and the 32-bit form of it
-// (10 bits) one multiplication away from its slot.  The 64-bit form (21 bits,
-// as wide as the volume's own keys) serves sessions whose rays may take more
-// steps than 10 bits hold.
-template <class K>
-struct NearKey;
-template <>
-struct NearKey<unsigned> {
-  static constexpr int kBits = 10;
-  static __device__ unsigned slot(unsigned k) { return (k * 0x9E3779B1u) >> (32 - kSetBits); }
-};
-template <>
-struct NearKey<unsigned long long> {
-  static constexpr int kBits = 21;
-  static __device__ unsigned slot(unsigned long long k) {
-    return (unsigned)((k * 0x9E3779B97F4A7C15ull) >> (64 - kSetBits));
-  }
-};
-template <class K>
-__device__ inline K near_key(int dx, int dy, int dz) {
-  constexpr int B = NearKey<K>::kBits, half = 1 << (B - 1);
-  return ((K)(unsigned)(dx + half) << (2 * B)) + ((K)(unsigned)(dy + half) << B) +
-         (K)(unsigned)(dz + half);
-}
-template <class K>
-__device__ inline unsigned long long volume_key(K k, const int (&cam)[3]) {
-  constexpr int B = NearKey<K>::kBits, half = 1 << (B - 1), mask = (1 << B) - 1;
-  return pack_key((int)((k >> (2 * B)) & mask) - half + cam[0],
-                  (int)((k >> B) & mask) - half + cam[1], (int)(k & mask) - half + cam[2]);
-}
-__device__ inline int apart_of(int a, int b) { return (int)((unsigned)a - (unsigned)b); }
 
 struct alignas(16) AllocSmem {
   unsigned long long set[kSetSlots];  // keys; all bits set: none; later the claimed entries
@@ -242,14 +209,11 @@ __device__ inline void walk_rays(const SessDev& S, int tx, int ty, AllocSmem& sm
                     (unsigned)lz + half < 2 * half;
   const K last = ends ? near_key<K>(lx, ly, lz) : ~(K)0;
   int left = v.t.dda_cap;
-  if (B == 10) {
-    // band rays start at the surface: none that could leave the fields is
-    // walked with them (poses that are not rigid)
-    const int start = max(max(abs(ox), abs(oy)), abs(oz));
-    if (start < 0 || start + left + 2 > (int)half) {
-      walk_far(S, x, y, sm);
-      return;
-    }
+  // (none that could leave the fields is walked with them: band rays of poses
+  // that are not rigid start anywhere)
+  if (!near_walk<K>(ox, oy, oz, left)) {
+    walk_far(S, x, y, sm);
+    return;
   }
   const K ix = (K)(long long)w.sx << (2 * B), iy = (K)(long long)w.sy << B, iz = (K)(long long)w.sz;
   K key = near_key<K>(ox, oy, oz);
