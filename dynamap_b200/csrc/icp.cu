@@ -1550,8 +1550,8 @@ void fused_icp_iteration(const SessDev* tab, const BatchShape& b, int slot, int 
                          cudaStream_t st) {
   if (it >= b.max_slot_iters[slot]) return;
   cudaLaunchConfig_t cfg = {};
-  // (a smaller level may have more tiles than the largest: 148 at most)
-  cfg.gridDim = dim3(kIcpMaxTiles, 1, b.n);
+  // (the table's most tiles, not its largest level's: a smaller level may have more)
+  cfg.gridDim = dim3(b.max_slot_tiles[slot], 1, b.n);
   cfg.blockDim = dim3(kIcpFrameThreads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;

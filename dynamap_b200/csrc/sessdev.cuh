@@ -101,7 +101,7 @@ struct BatchShape {
   int max_nlev;
   int max_blocks;          // largest num_blocks
   int max_level_px[kLevels];
-  int max_slot_px[3];      // largest pixel count of each ICP level slot
+  int max_slot_tiles[3];   // most tiles (icp_tiles) of each ICP level slot
   int max_slot_iters[3];   // largest lvl_iteration_num of each slot
   int max_bil_radius;      // 0: no session filters
   int max_grid;            // largest block grid (entries; 0: none)

@@ -246,7 +246,9 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
       b.max_level_px[l] = std::max(b.max_level_px[l], s->ls[l].rows * s->ls[l].cols);
     for (int pl = 0; pl < 3; ++pl) {
       const int l = level_of_scale(s->gp.lvl_scale[pl]);
-      b.max_slot_px[pl] = std::max(b.max_slot_px[pl], s->ls[l].rows * s->ls[l].cols);
+      b.max_slot_tiles[pl] =
+          std::max(b.max_slot_tiles[pl],
+                   icp_tiles(s->ls[l].rows * s->ls[l].cols, s->icp_params().kahan));
       b.max_slot_iters[pl] = std::max(b.max_slot_iters[pl], s->gp.lvl_iteration_num[pl]);
     }
     if (s->bp.enabled) b.max_bil_radius = std::max(b.max_bil_radius, s->btab.radius);
