@@ -1047,20 +1047,11 @@ __device__ __noinline__ bool finish_iteration(const uint2* rows, const FrameLeve
   return true;
 }
 
-// Blocks of a session of npx pixels in a persistent launch of 'budget' blocks
-// over a table whose sessions weigh 'sum' in all.
-__host__ __device__ inline int icp_share(int npx, int kahan, long long sum, int budget) {
-  const int tiles = icp_tiles(npx, kahan);
-  long long b = (long long)budget * icp_weight(npx, kahan) / (sum > 0 ? sum : 1);
-  if (b > tiles) b = tiles;
-  if (b < 1) b = 1;
-  return (int)b;
-}
-
 // This block's session among the table's sessions of its kind, its index
 // among the session's blocks and their number, in shared memory (out[3]).
 template <bool KAHAN>
-__device__ inline void find_session(const SessDev* __restrict__ tab, int n, int budget, int* out) {
+__device__ inline void find_session(const SessDev* __restrict__ tab, int n, int pool, int base,
+                                    int* out) {
   __shared__ long long sum_s;
   __shared__ int part[kFrameWarps], carry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1078,7 +1069,8 @@ __device__ inline void find_session(const SessDev* __restrict__ tab, int n, int 
   for (int j0 = 0; j0 < n; j0 += kIcpFrameThreads) {
     const int j = j0 + tid;
     int b = 0;
-    if (j < n && (tab[j].icpp.kahan != 0) == KAHAN) b = icp_share(tab[j].npx, KAHAN, sum_s, budget);
+    if (j < n && (tab[j].icpp.kahan != 0) == KAHAN)
+      b = icp_share(tab[j].npx, KAHAN, sum_s, pool, base);
     int sum = b;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1105,7 +1097,7 @@ __device__ inline void find_session(const SessDev* __restrict__ tab, int n, int 
 // ways gets one launch per kind, each over that kind's sessions only.
 template <bool KAHAN>
 __global__ void __launch_bounds__(kIcpFrameThreads, 1)
-    fused_icp_persistent_kernel(const SessDev* __restrict__ tab, int n, int budget,
+    fused_icp_persistent_kernel(const SessDev* __restrict__ tab, int n, int pool, int base,
                                 int it0, int it1, int it2) {
   // this block's session, its index among the session's blocks, their number
   __shared__ int who[3];
@@ -1117,7 +1109,7 @@ __global__ void __launch_bounds__(kIcpFrameThreads, 1)
     }
     __syncthreads();
   } else {
-    find_session<KAHAN>(tab, n, budget, who);
+    find_session<KAHAN>(tab, n, pool, base, who);
   }
   const SessDev& S = tab[who[0]];
   const int local = who[1], nblk = who[2];
@@ -1440,29 +1432,13 @@ int icp_persistent_capacity(int device) {
   return cap[device] > 0 ? cap[device] : 0;
 }
 
-int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int* grid_k) {
-  grid_k[0] = grid_k[1] = 0;
-  if (budget <= 0 || n <= 0) return 0;
-  for (int kind = 0; kind < 2; ++kind) {
-    long long sum = 0;
-    for (int j = 0; j < n; ++j)
-      if ((kahan[j] != 0) == (kind == 1)) sum += icp_weight(npx[j], kind);
-    long long g = 0;
-    for (int j = 0; j < n; ++j)
-      if ((kahan[j] != 0) == (kind == 1)) g += icp_share(npx[j], kind, sum, budget);
-    if (g > budget) {
-      grid_k[0] = grid_k[1] = 0;
-      return 0;
-    }
-    grid_k[kind] = (int)g;
-  }
-  return grid_k[0] + grid_k[1];
-}
-
 template <bool KAHAN>
-static void launch_persistent(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
+static void launch_persistent(const SessDev* tab, const BatchShape& b, int part, cudaStream_t st) {
+  const int grid = b.icp.grid[part][KAHAN];
+  if (grid == 0) return;
+  const int first = icp_part_first(b.n, b.icp.parts, part);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(b.icp_grid_k[KAHAN ? 1 : 0]);
+  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kIcpFrameThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -1470,13 +1446,17 @@ static void launch_persistent(const SessDev* tab, const BatchShape& b, cudaStrea
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, fused_icp_persistent_kernel<KAHAN>, tab, b.n, b.icp_budget,
-                     b.max_slot_iters[0], b.max_slot_iters[1], b.max_slot_iters[2]);
+  cudaLaunchKernelEx(&cfg, fused_icp_persistent_kernel<KAHAN>, tab + first,
+                     icp_part_first(b.n, b.icp.parts, part + 1) - first, b.icp.pool[part][KAHAN],
+                     b.icp.base[part][KAHAN], b.max_slot_iters[0], b.max_slot_iters[1],
+                     b.max_slot_iters[2]);
 }
 
 void fused_icp_persistent(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  if (b.icp_grid_k[0] > 0) launch_persistent<false>(tab, b, st);
-  if (b.icp_grid_k[1] > 0) launch_persistent<true>(tab, b, st);
+  for (int part = 0; part < b.icp.parts; ++part) {
+    launch_persistent<false>(tab, b, part, st);
+    launch_persistent<true>(tab, b, part, st);
+  }
 }
 
 dyn_status icp_barrier_selftest(int blocks, int missing, unsigned* bar_dev, cudaStream_t st) {

@@ -111,23 +111,73 @@ inline size_t icp_frame_scratch_bytes() {
   return icp_rows_offset() + (size_t)kIcpRows * kIcpRowWords * 8;
 }
 
-// The persistent ICP (one cooperative launch per frame and summation kind):
-// the blocks that can be resident at once on 'device' (0: cooperative
-// launches unavailable), and the grids of a table whose sessions' largest
-// levels have npx[j] pixels and sum plainly (kahan[j] == 0) or with
-// compensation: grid_k[kind] blocks within 'budget' each (0: no session of
-// that kind).  Returns their total, or 0 when a kind does not fit (the
-// chained kernels run the table, with the same results).
+// The persistent ICP (one cooperative launch per frame and summation kind, or
+// one per part of a large table): the blocks that can be resident at once on
+// 'device' (0: cooperative launches unavailable).
 int icp_persistent_capacity(int device);
-int icp_persistent_grid(const int* npx, const int* kahan, int n, int budget, int* grid_k);
+// Blocks of a session of npx pixels in a persistent launch over sessions that
+// weigh 'sum' in all: its part of 'pool' blocks beside 'base', at least one.
+__host__ __device__ inline int icp_share(int npx, int kahan, long long sum, int pool, int base) {
+  const int tiles = icp_tiles(npx, kahan);
+  long long b = base + (long long)pool * icp_weight(npx, kahan) / (sum > 0 ? sum : 1);
+  if (b > tiles) b = tiles;
+  if (b < 1) b = 1;
+  return (int)b;
+}
+
+// The launches of a table of n sessions within 'budget' blocks: the table in
+// 'parts' runs one after another (0: the chained kernels run it, with the same
+// results), each with a launch per summation kind of grid[part][kind] blocks (0:
+// no session of that kind).  Every session needs a block: a table of more
+// sessions than blocks takes the fewest parts that give them one.  (160 sessions
+// of 64x48 in two parts: 266 us of ICP, in the chained kernels 459; 580 in four:
+// 550 and 1349; 200 of 320x240 in two: 2281 and 4671.)  Blocks follow the
+// sessions' weights; where that leaves small sessions less than one each, all get
+// one first and the weights share out the rest.
+constexpr int kIcpMaxParts = 4;
+struct IcpLaunches {
+  int parts;
+  int grid[kIcpMaxParts][2], pool[kIcpMaxParts][2], base[kIcpMaxParts][2];
+};
+inline __host__ __device__ int icp_part_first(int n, int parts, int part) {
+  return (int)((long long)n * part / parts);
+}
+inline IcpLaunches icp_launches(const int* npx, const int* kahan, int n, int budget) {
+  IcpLaunches L = {};
+  if (budget <= 0 || n <= 0 || n > (long long)kIcpMaxParts * budget) return L;
+  L.parts = (n + budget - 1) / budget;
+  for (int part = 0; part < L.parts; ++part) {
+    const int first = icp_part_first(n, L.parts, part), end = icp_part_first(n, L.parts, part + 1);
+    for (int kind = 0; kind < 2; ++kind) {
+      long long sum = 0;
+      int members = 0;
+      for (int j = first; j < end; ++j)
+        if ((kahan[j] != 0) == (kind == 1)) {
+          sum += icp_weight(npx[j], kind);
+          ++members;
+        }
+      for (int base = 0; base < 2; ++base) {
+        const int pool = budget - base * members;
+        long long g = 0;
+        for (int j = first; j < end; ++j)
+          if ((kahan[j] != 0) == (kind == 1)) g += icp_share(npx[j], kind, sum, pool, base);
+        L.grid[part][kind] = (int)g;
+        L.pool[part][kind] = pool;
+        L.base[part][kind] = base;
+        if (g <= budget) break;
+      }
+    }
+  }
+  return L;
+}
 // Resident blocks that each of k groups of sessions may take for its persistent
 // ICP, out[g], when the groups run at once: 'weight' a group's icp_weight in all,
 // 'count' its sessions.  The shares never add up to more than 'cap', so that all
 // launches can be resident together (their blocks wait for one another: a launch
 // that is resident in part beside another such would wait out its bound); a
-// group has a block per session or none (the chained kernels).  Shares follow the
-// weights, except that a group whose part would be less than a block per session
-// is given just that while there are blocks for every session.
+// group without a block runs the chained kernels.  Shares follow the weights,
+// except that a group whose share would be less than a block per session is given
+// just that while there are blocks for every session.
 inline void icp_group_budgets(const long long* weight, const int* count, int k, int cap,
                               int* out) {
   long long sessions = 0;
@@ -150,10 +200,7 @@ inline void icp_group_budgets(const long long* weight, const int* count, int k, 
       }
   }
   for (int g = 0; g < k; ++g)
-    if (out[g] == 0 && count[g] > 0 && rest > 0) {
-      const int share = (int)(left * weight[g] / rest);
-      out[g] = share >= count[g] ? share : 0;
-    }
+    if (out[g] == 0 && rest > 0) out[g] = (int)(left * weight[g] / rest);
 }
 
 // The persistent ICP's words of a session: the epoch of the next launch's tags

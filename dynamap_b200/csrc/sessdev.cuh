@@ -115,12 +115,7 @@ struct BatchShape {
   int2* gvis;              // batch-wide visible list (session, heap index)
   int* gcount;             // its length (device)
   int gvis_cap;
-  // the persistent ICP: blocks of its cooperative launches (0: the chained
-  // kernels instead) in all and per summation kind (plain, compensated), and
-  // the budget each launch's shares are taken from
-  int icp_grid;
-  int icp_grid_k[2];
-  int icp_budget;
+  IcpLaunches icp;         // the persistent ICP's launches
 };
 
 // image.cu

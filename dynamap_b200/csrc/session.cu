@@ -122,7 +122,7 @@ void enqueue_source(const SessDev* tab, const BatchShape& b, cudaStream_t st, co
 // of each level slot; every launch after the first overlaps its
 // predecessor's tail (programmatic dependent launch).
 void enqueue_icp(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
-  if (b.icp_grid > 0) {  // one persistent launch for every level and iteration
+  if (b.icp.parts > 0) {  // a persistent launch for every level and iteration
     fused_icp_persistent(tab, b, st);
     return;
   }
@@ -259,7 +259,7 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
   return b;
 }
 
-// The persistent ICP for a table of sessions: its grid within 'budget' blocks
+// The persistent ICP for a table of sessions: its launches within 'budget' blocks
 // (0: chained kernels).  DYN_ICP_CHAINED=1 in the environment keeps every
 // table on the chained kernels (the same results; for comparisons).
 void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget) {
@@ -272,11 +272,7 @@ void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget
     npx[i] = (int)ss[i]->npx;
     kahan[i] = ss[i]->icp_params().kahan;
   }
-  b.icp_budget = budget;
-  b.icp_grid_k[0] = b.icp_grid_k[1] = 0;
-  b.icp_grid = chained_only
-                   ? 0
-                   : icp_persistent_grid(npx.data(), kahan.data(), n, budget, b.icp_grid_k);
+  b.icp = icp_launches(npx.data(), kahan.data(), n, chained_only ? 0 : budget);
 }
 
 // The session's descriptor (device buffers, sensor levels, parameters).

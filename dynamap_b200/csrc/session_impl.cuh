@@ -339,8 +339,8 @@ dyn_status quiesce(dyn_session* s);
 // The launch shape of a table of sessions (the largest member bounds every
 // grid).
 BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, int gvis_cap);
-// The persistent ICP of a table: its grid within 'budget' blocks (0 when it
-// does not fit: the chained kernels, same results).
+// The persistent ICP of a table: its launches within 'budget' blocks (none when
+// it does not fit: the chained kernels, same results).
 void set_icp_persistent(BatchShape& b, dyn_session* const* ss, int n, int budget);
 // Marks whether this frame of 's' carries RGB (stream-ordered).
 dyn_status set_rgb_flag(dyn_session* s, bool has_rgb, cudaStream_t st);

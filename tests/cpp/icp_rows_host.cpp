@@ -70,3 +70,13 @@ extern "C" void icp_budgets(const long long* weight, const int* count, int k, in
   dyn::icp_group_budgets(weight, count, k, cap, out);
 }
 extern "C" long long icp_weight_of(int npx, int kahan) { return dyn::icp_weight(npx, kahan); }
+
+// The parts of a table (0: chained): their grids per kind and first sessions.
+extern "C" int icp_table(const int* npx, const int* kahan, int n, int budget, int* grid,
+                         int* first) {
+  const dyn::IcpLaunches L = dyn::icp_launches(npx, kahan, n, budget);
+  for (int p = 0; p < L.parts; ++p)
+    for (int k = 0; k < 2; ++k) grid[2 * p + k] = L.grid[p][k];
+  for (int p = 0; p <= L.parts && L.parts > 0; ++p) first[p] = dyn::icp_part_first(n, L.parts, p);
+  return L.parts;
+}

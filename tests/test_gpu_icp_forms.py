@@ -121,3 +121,11 @@ def test_batches_of_many_sessions(tmp_path, gpu_lib):
     sizes = [(48, 64), (48, 64), (48, 64), (120, 160), (48, 64), (240, 320)]
     assert_forms_agree(tmp_path, [[member(*sizes[i % 6], (FP32, MIXED)[i % 4 == 1], it)
                                    for i in range(66)]])
+
+
+def test_tables_in_parts(tmp_path, gpu_lib):
+    """More sessions than the device has resident blocks: the persistent form runs
+    the table in parts."""
+    it = (4, 3, 3)
+    assert_forms_agree(tmp_path, [[member(32, 48, (FP32, MIXED)[i % 3 == 1], it)
+                                   for i in range(170)]])

@@ -1,6 +1,7 @@
 """The shares of the device that a batch's groups take for their persistent ICP
 (icp_group_budgets, dynamap_b200/csrc/icp.cuh), on the CPU: all launches fit on
-the device together, for the library's own mixes and random ones."""
+the device together, for the library's own mixes and random ones; and the parts
+that a table of more sessions than blocks is run in (icp_launches)."""
 import ctypes as C
 import os
 import random
@@ -54,7 +55,6 @@ def groups(px):
 def check(lib, weights, counts, cap):
     b = budgets(lib, weights, counts, cap)
     assert sum(b) <= max(cap, 0)
-    assert all(x == 0 or x >= c for x, c in zip(b, counts))
     if sum(counts) <= cap:
         assert all(x >= c for x, c in zip(b, counts))
         plain = [cap * w // sum(weights) for w in weights]
@@ -83,4 +83,29 @@ def test_random_groups(lib):
 def test_small_groups_are_given_a_block_per_session(lib):
     assert budgets(lib, [1000000, 10], [1, 20], 148) == [128, 20]
     assert budgets(lib, [1000000, 10], [1, 200], 148) == [147, 0]  # chained kernels
+    assert budgets(lib, [10, 10], [100, 100], 148) == [74, 74]     # in parts of a table
     assert budgets(lib, [5, 5], [1, 1], 0) == [0, 0]
+
+
+@pytest.mark.parametrize("budget", [1, 7, 18, 74, 148, 296])
+def test_parts_of_a_table(lib, budget):
+    """Every launch has a block per session and fits the budget; a table is split
+    only where it has to be."""
+    rng = random.Random(budget)
+    lib.icp_table.restype = C.c_int
+    for n in list(range(1, 30)) + [37, 74, 80, 147, 148, 149, 160, 280, 296, 297, 400, 592, 700]:
+        for kinds in (lambda: 0, lambda: 1, lambda: rng.randint(0, 1)):
+            for sizes in ([3072], [19200], [3072, 19200, 307200]):
+                px = [rng.choice(sizes) for _ in range(n)]
+                kahan = [kinds() for _ in range(n)]
+                grid, first = (C.c_int * 8)(), (C.c_int * 5)()
+                parts = lib.icp_table((C.c_int * n)(*px), (C.c_int * n)(*kahan), n, budget, grid, first)
+                assert parts == (0 if n > 4 * budget else -(-n // budget))
+                if parts == 0:
+                    continue
+                assert first[0] == 0 and first[parts] == n
+                for p in range(parts):
+                    for kind in (0, 1):
+                        members = sum(k == kind for k in kahan[first[p]:first[p + 1]])
+                        assert members <= grid[2 * p + kind] <= budget
+                        assert (grid[2 * p + kind] == 0) == (members == 0)
