@@ -255,6 +255,7 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
     if (s->vol.grid) b.max_grid = std::max(b.max_grid, s->vol.grid_cap);
     b.kahan_mask |= s->icp_params().kahan ? 2 : 1;
     b.fp16_mask |= s->vol.fp16 ? 2 : 1;
+    if (s->gp.mode == 1) b.ray_mask |= (s->vol.fp16 ? 2 : 1) << (s->vol.grid ? 2 : 0);
   }
   return b;
 }
@@ -740,10 +741,15 @@ size_t session_device_bytes(const dyn_tsdf_params* tsdf, const dyn_gn_params* gn
   return b;
 }
 
-// Whether the session's block grid covers the rays of sensor 'virt'.
-static bool raycast_grid_fits(const dyn_session* s, const dyn_sensor& virt) {
+// Whether a render of sensor 'virt' goes through the session's block grid: where
+// the grid covers the sensor's rays, except for views of the mixed forms of so few
+// rays that filling the grid costs more than it saves.  (Band session, 3 m and 6 m
+// of range at 5 mm, grid / hash: 8x6 131 / 111 and 207 / 193 us a call, 32x24 122
+// / 149 and 202 / 222; FP32 gains at 8x6 already: 182 / 321.)
+static bool raycast_uses_grid(const dyn_session* s, const dyn_sensor& virt) {
+  if (!s->vol.grid || (s->vol.fp16 && (long long)virt.rows * virt.cols < 256)) return false;
   const long long n = grid_entries(dsensor(virt), s->vol.t);
-  return s->vol.grid && n > 0 && n <= s->vol.grid_cap;
+  return n > 0 && n <= s->vol.grid_cap;
 }
 
 dyn_status ensure_staging(dyn_session* s) {
@@ -1042,7 +1048,7 @@ dyn_status dyn_raycast(dyn_session* s, const float pose[16], const dyn_sensor* v
   DYN_CUDA(cudaMemcpyAsync(s->d_pose_override, pose, 64, cudaMemcpyHostToDevice, s->stream));
   size_t n = (size_t)vs.rows * vs.cols;
   launch_raycast(s->vol, dsensor(vs), s->d_pose, s->d_pose_override, s->d_ray,
-                 rgb_host ? s->d_trgb : nullptr, raycast_grid_fits(s, vs), s->stream);
+                 rgb_host ? s->d_trgb : nullptr, raycast_uses_grid(s, vs), s->stream);
   DYN_CUDA(cudaGetLastError());
   DYN_CUDA(cudaMemcpyAsync(depth_host, s->d_ray, n * 4, cudaMemcpyDeviceToHost, s->stream));
   if (rgb_host)
@@ -1063,7 +1069,7 @@ dyn_status dyn_raycast_maps(dyn_session* s, const float pose[16], const dyn_sens
   DYN_CUDA(cudaMemcpyAsync(s->d_pose_override, pose, 64, cudaMemcpyHostToDevice, st));
   const size_t n = (size_t)vs.rows * vs.cols;
   launch_raycast(s->vol, dsensor(vs), s->d_pose, s->d_pose_override, s->d_ray,
-                 rgb_host ? s->d_trgb : nullptr, raycast_grid_fits(s, vs), st);
+                 rgb_host ? s->d_trgb : nullptr, raycast_uses_grid(s, vs), st);
   // misses (at max_sensor_depth or beyond) become invalid depth, then the
   // maps of that depth in the raycast camera's frame
   launch_miss_to_zero(s->d_ray, s->d_filt, s->tp.max_sensor_depth, (int)n, st);

@@ -1216,7 +1216,7 @@ __device__ inline VoxelSample get_interpolated(const VolumeDev& v, F3 position, 
 // skip_to or after skip_far (the tile's ray depth bounds: no allocated block
 // there) step by the truncation without a lookup -- what the lookup would
 // have returned.  Returns true when the march hit the step cap.
-__device__ __noinline__ bool raycast_exact_hash_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
+__device__ inline bool exact_hash_march(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
                                         int y, float skip_to, float skip_far,
                                         float* __restrict__ depth_out,
                                         uint8_t* __restrict__ rgb_out) {
@@ -1263,6 +1263,15 @@ __device__ __noinline__ bool raycast_exact_hash_px(const VolumeDev& v, const DSe
     rgb_out[3 * (size_t)i + 2] = b;
   }
   return over;
+}
+
+// The same out of line, for the rays of a grid session that its grid does not
+// take.
+__device__ __noinline__ bool raycast_exact_hash_px(const VolumeDev& v, const DSensor& s,
+                                                   const M4f& T, int x, int y, float skip_to,
+                                                   float skip_far, float* __restrict__ depth_out,
+                                                   uint8_t* __restrict__ rgb_out) {
+  return exact_hash_march(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
 }
 
 // ---- the exact march over the block grid
@@ -1412,10 +1421,9 @@ __device__ __noinline__ float2 interpolated_generic(const VolumeDev& v, float x,
   return make_float2(s.sdf, s.w ? 1.0f : 0.0f);
 }
 
-// The march of raycast_exact_hash_px, its blocks looked up in the grid: every
-// sample reads the entry of its voxel's block, an observed one those of its
-// cell's blocks.  Rays outside march_setup's ranges, and volumes without a
-// grid, take raycast_exact_hash_px.
+// exact_hash_march over the block grid (which the volume has): every sample
+// reads the entry of its voxel's block, an observed one those of its cell's
+// blocks.  Rays outside march_setup's ranges take raycast_exact_hash_px.
 __device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
                                         int y, float skip_to, float skip_far,
                                         float* __restrict__ depth_out,
@@ -1425,7 +1433,7 @@ __device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, co
   // getPoint3d (utils.h:104-112) with the pixel's (u - cx), (v - cy) hoisted
   const float ax = (float)x - s.cx, ay = (float)y - s.cy;
   MarchRay R;
-  if (!v.grid || !v.gbox->ok || !march_setup(t, s, T, ax, ay, inv_vs, R))
+  if (!v.gbox->ok || !march_setup(t, s, T, ax, ay, inv_vs, R))
     return raycast_exact_hash_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
   const GridView G = grid_view(v);
   const uint2* __restrict__ vox = reinterpret_cast<const uint2*>(v.voxels);
@@ -1658,12 +1666,12 @@ __device__ inline int cell_block_free(const VolumeDev& v, int bx, int by, int bz
 // Returns true when the march hit the step cap.  FREE: the session keeps
 // free-cell flags (mixed form with carving); without them (band sessions)
 // the cell's and the centre voxel's blocks share one lookup cache.
-template <bool FP16, bool FREE>
-__device__ __noinline__ bool raycast_hash_px(const VolumeDev& v, const DSensor& s, const M4f& T,
-                                             int x, int y, float skip_to, float skip_far,
-                                             float* __restrict__ depth_out,
-                                             uint8_t* __restrict__ rgb_out) {
-  using V = Vox<FP16>;
+template <bool FREE>
+__device__ inline bool mixed_hash_march(const VolumeDev& v, const DSensor& s, const M4f& T, int x,
+                                        int y, float skip_to, float skip_far,
+                                        float* __restrict__ depth_out,
+                                        uint8_t* __restrict__ rgb_out) {
+  using V = Vox<true>;
   const int i = y * s.cols + x;
   const DTsdf& t = v.t;
   const float inv_vs = 1.0f / t.vs;
@@ -1713,7 +1721,7 @@ __device__ __noinline__ bool raycast_hash_px(const VolumeDev& v, const DSensor& 
       cur += t.trunc;
       continue;
     }
-    const VoxelSample vx = interp<FP16, false>(v, q, raw, ptr, lin, bc);
+    const VoxelSample vx = interp<true, false>(v, q, raw, ptr, lin, bc);
     cur += vx.sdf;
     if (vx.sdf < t.vs) break;
   }
@@ -1728,7 +1736,16 @@ __device__ __noinline__ bool raycast_hash_px(const VolumeDev& v, const DSensor& 
   return over;
 }
 
-// raycast_hash_px over the block grid: the same samples, each with the entries
+// The same out of line (raycast_exact_hash_px).
+template <bool FREE>
+__device__ __noinline__ bool raycast_hash_px(const VolumeDev& v, const DSensor& s, const M4f& T,
+                                             int x, int y, float skip_to, float skip_far,
+                                             float* __restrict__ depth_out,
+                                             uint8_t* __restrict__ rgb_out) {
+  return mixed_hash_march<FREE>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+}
+
+// mixed_hash_march over the block grid: the same samples, each with the entries
 // of its cell's blocks read from the grid.  FREE: bit 0 of a block's entry is
 // its free-cell flag.
 template <bool FREE>
@@ -1738,8 +1755,8 @@ __device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4
   const DTsdf& t = v.t;
   const float inv_vs = 1.0f / t.vs;
   const float axf = ((float)x - s.cx) / s.fx, ayf = ((float)y - s.cy) / s.fy;
-  if (!v.grid || !v.gbox->ok || !march_bounded(t) || !march_within(t, T, axf, ayf, inv_vs))
-    return raycast_hash_px<true, FREE>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  if (!v.gbox->ok || !march_bounded(t) || !march_within(t, T, axf, ayf, inv_vs))
+    return raycast_hash_px<FREE>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
   const F3 o = f3(T.m[3] * inv_vs, T.m[7] * inv_vs, T.m[11] * inv_vs);
   const F3 d = f3((T.m[0] * axf + T.m[1] * ayf + T.m[2]) * inv_vs,
                   (T.m[4] * axf + T.m[5] * ayf + T.m[6]) * inv_vs,
@@ -1804,8 +1821,8 @@ __device__ inline bool raycast_px(const VolumeDev& v, const DSensor& s, const M4
 
 // One pixel's ray of a TX x TY pixel tile (bx, by) from pose16 (a float 4x4);
 // warps cover 8x4 pixel sub-tiles for coherent rays.  Step-cap overruns are
-// counted.
-template <bool MIXED, int TX, int TY>
+// counted.  GRID: the volume has a block grid.
+template <bool MIXED, bool GRID, int TX, int TY>
 __device__ inline void raycast_tile(const VolumeDev& v, const DSensor& s,
                                     const float* __restrict__ pose16, float* __restrict__ depth_out,
                                     uint8_t* __restrict__ rgb_out, int bx, int by,
@@ -1833,49 +1850,60 @@ __device__ inline void raycast_tile(const VolumeDev& v, const DSensor& s,
     skip_to = fminf(__uint_as_float(B.near8[f]), __uint_as_float(B.near64[c]));
     skip_far = fmaxf(__uint_as_float(B.far8[f]), __uint_as_float(B.far64[c]));
   }
-  const bool over = MIXED ? (v.freecell ? raycast_px<true>(v, s, T, x, y, skip_to, skip_far,
-                                                           depth_out, rgb_out)
-                                        : raycast_px<false>(v, s, T, x, y, skip_to, skip_far,
-                                                            depth_out, rgb_out))
-                          : raycast_exact_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  bool over;
+  if (MIXED) {
+    const bool free = v.freecell != nullptr;
+    if (GRID)
+      over = free ? raycast_px<true>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out)
+                  : raycast_px<false>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+    else
+      over = free ? mixed_hash_march<true>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out)
+                  : mixed_hash_march<false>(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  } else {
+    over = GRID ? raycast_exact_px(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out)
+                : exact_hash_march(v, s, T, x, y, skip_to, skip_far, depth_out, rgb_out);
+  }
   if (over) atomicAdd(&v.cnt->raycast_overruns, 1);
 }
 
-template <bool MIXED>
+template <bool MIXED, bool GRID>
 __global__ void __launch_bounds__(256)
     raycast_kernel(const __grid_constant__ VolumeDev v, const __grid_constant__ DSensor s,
                    const PoseState* __restrict__ ps, const float* __restrict__ pose_override,
                    float* __restrict__ depth_out, uint8_t* __restrict__ rgb_out) {
-  raycast_tile<MIXED, 16, 16>(v, s, pose_override ? pose_override : ps->posef, depth_out, rgb_out,
-                              blockIdx.x, blockIdx.y, nullptr, 0);
+  raycast_tile<MIXED, GRID, 16, 16>(v, s, pose_override ? pose_override : ps->posef, depth_out, rgb_out,
+                                    blockIdx.x, blockIdx.y, nullptr, 0);
 }
 
 // next frame's target of every mode-1 session (blockIdx.z) at its new pose;
-// one instantiation per voxel form (sessions of the other form return) and
-// per tile shape (every pixel's march is independent of the tiling)
+// one instantiation per voxel form and march, through the block grid or the
+// hash (other sessions return), and per tile shape (every pixel's march is
+// independent of the tiling)
 // (at least 1024 threads resident per SM: the march waits on its own loads --
 // grid entry, voxel, corners -- and issues in 60 % of the cycles, and 4 CTAs of
 // 256 hide more of it than the 3 that 76 registers allow.  A persistent launch
 // whose warps fetch 8x4 tiles from an even sample of the image balanced the
 // SMs but spilled in the loop: 272 against 253 us.  All nine loads of a sample
 // issued together: 275 against 265 us, the weight test saves more.)
-template <bool MIXED, int TX, int TY>
+template <bool MIXED, bool GRID, int TX, int TY>
 __global__ void __launch_bounds__(TX* TY, 1024 / (TX * TY))
     fused_raycast_kernel(const SessDev* __restrict__ tab) {
   const SessDev& S = tab[blockIdx.z];
-  if (S.mode != 1 || (S.vol.fp16 != 0) != MIXED) return;
+  if (S.mode != 1 || (S.vol.fp16 != 0) != MIXED || (S.vol.grid != nullptr) != GRID) return;
   const DSensor& s = S.ls[0];
   if ((int)blockIdx.x * TX >= s.cols || (int)blockIdx.y * TY >= s.rows) return;
   uint8_t* rgb_out = S.use_color ? S.trgb : nullptr;
-  raycast_tile<MIXED, TX, TY>(S.vol, s, S.pose->posef, S.ray, rgb_out, blockIdx.x, blockIdx.y,
-                              S.rbound, S.rb_tx);
+  raycast_tile<MIXED, GRID, TX, TY>(S.vol, s, S.pose->posef, S.ray, rgb_out, blockIdx.x,
+                                    blockIdx.y, S.rbound, S.rb_tx);
 }
 
 template <int TX, int TY>
 void launch_fused_raycast(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   dim3 grid((b.max_cols + TX - 1) / TX, (b.max_rows + TY - 1) / TY, b.n);
-  if (b.fp16_mask & 1) fused_raycast_kernel<false, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
-  if (b.fp16_mask & 2) fused_raycast_kernel<true, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
+  if (b.ray_mask & 1) fused_raycast_kernel<false, false, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
+  if (b.ray_mask & 2) fused_raycast_kernel<true, false, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
+  if (b.ray_mask & 4) fused_raycast_kernel<false, true, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
+  if (b.ray_mask & 8) fused_raycast_kernel<true, true, TX, TY><<<grid, TX * TY, 0, st>>>(tab);
 }
 
 __global__ void clear_entries_kernel(Entry* e, size_t n) {
@@ -1928,15 +1956,10 @@ void launch_raycast(const VolumeDev& v, const DSensor& s, const PoseState* ps,
     grid_clear_kernel<<<148 * 4, 256, 0, st>>>(v, s, pose_override ? pose_override : ps->posef);
     grid_fill_kernel<<<148 * 4, 256, 0, st>>>(v);
   }
-  VolumeDev w = v;
-  if (!use_grid) w.grid = nullptr;
   const dim3 grid(nblk(s.cols, 16), nblk(s.rows, 16));
-  if (v.fp16)
-    raycast_kernel<true><<<grid, 256, 0, st>>>(w, s, ps, pose_override,
-                                                                depth_out, rgb_out);
-  else
-    raycast_kernel<false><<<grid, 256, 0, st>>>(w, s, ps, pose_override,
-                                                                 depth_out, rgb_out);
+  const auto kernel = v.fp16 ? (use_grid ? raycast_kernel<true, true> : raycast_kernel<true, false>)
+                             : (use_grid ? raycast_kernel<false, true> : raycast_kernel<false, false>);
+  kernel<<<grid, 256, 0, st>>>(v, s, ps, pose_override, depth_out, rgb_out);
 }
 
 void launch_block_coords(const VolumeDev& v, int n, int* coords, cudaStream_t st) {

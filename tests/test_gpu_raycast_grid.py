@@ -57,3 +57,27 @@ def test_grid_and_hash_marches_agree(gpu_lib, oracle, prec, rows, cols, shift):
                 od, oc, _ = ovol.raycast(q, s, rgb=True)
                 np.testing.assert_array_equal(gd.view(np.uint32), od.view(np.uint32))
                 np.testing.assert_array_equal(gc, oc)
+
+
+@pytest.mark.parametrize("prec", [abi.PRECISION_FP32, abi.PRECISION_MIXED,
+                                  abi.PRECISION_MIXED_BAND])
+def test_small_views_agree(gpu_lib, prec):
+    """Views on either side of the size from which the mixed forms take the grid."""
+    p = configs.preset("cfg1")
+    p["sensor"].update(rows=120, cols=160, fx=131.25, fy=131.25, cx=79.5, cy=59.5)
+    p["tsdf"].update(num_blocks=1 << 14, num_buckets=1 << 15, voxel_size=0.01,
+                     truncation_distance=0.04)
+    p["gn"].update(lvl_scale=[1, 1, 1])
+    seq = configs.sequence(p, seed=23, n_frames=2)
+    frames = [(seq.depth[k], None, seq.poses[k].astype(np.float32)) for k in range(2)]
+    near, _, _ = session(p, 6.0, prec, frames)
+    far, _, _ = session(p, 60.0, prec, frames)
+    with near, far:
+        for rows, cols in ((15, 17), (16, 16), (6, 8), (1, 1), (24, 32)):
+            f = 131.25 * cols / 160.0
+            v = abi.Sensor(rows=rows, cols=cols, fx=f, fy=f, cx=(cols - 1) / 2, cy=(rows - 1) / 2,
+                           depth_scaler=1000.0)
+            a, b = near.raycast(frames[1][2], v)[0], far.raycast(frames[1][2], v)[0]
+            hit = a < 6.0
+            np.testing.assert_array_equal(hit, b < 6.0)
+            np.testing.assert_array_equal(a[hit].view(np.uint32), b[hit].view(np.uint32))
