@@ -9,7 +9,7 @@ namespace {
 constexpr int kSetBits = 11, kSetSlots = 1 << kSetBits;  // the set's slots
 
 // A block in a CTA's set: its offset from the camera's block, biased fields of
-// BITS bits an axis, so that a step is one addition and the 32-bit form of it
+// kBits bits an axis, so that a step is one addition and the 32-bit form of it
 // (10 bits) one multiplication away from its slot.  The 64-bit form (21 bits,
 // as wide as the volume's own keys) serves sessions whose rays may take more
 // steps than 10 bits hold.

@@ -107,6 +107,7 @@ struct BatchShape {
   int max_grid;            // largest block grid (entries; 0: none)
   int kahan_mask;          // bit 0: some session sums plainly, bit 1: some use Kahan sums
   int fp16_mask;           // bit 0: some session keeps FP32 voxels, bit 1: some mixed
+  int close_mask;          // bit 0: some session's rays are apart, bit 1: some close (close_rays)
   int ray_mask;            // of the sessions that raycast, likewise: bits 0, 1 without a block
                            // grid, bits 2, 3 with one
   // launch shapes that leave every result unchanged (chosen by a batch's

@@ -255,6 +255,7 @@ BatchShape make_shape(dyn_session* const* ss, int n, int2* gvis, int* gcount, in
     if (s->vol.grid) b.max_grid = std::max(b.max_grid, s->vol.grid_cap);
     b.kahan_mask |= s->icp_params().kahan ? 2 : 1;
     b.fp16_mask |= s->vol.fp16 ? 2 : 1;
+    b.close_mask |= close_rays(s->vol.t, s->ls[0]) ? 2 : 1;
     if (s->gp.mode == 1) b.ray_mask |= (s->vol.fp16 ? 2 : 1) << (s->vol.grid ? 2 : 0);
   }
   return b;

@@ -111,8 +111,8 @@ __device__ inline bool pixel_ray(const float* __restrict__ depth, const DSensor&
 }
 
 // One block into the global table, its heap index from the volume's counter.
-__device__ __noinline__ void insert_block(const VolumeDev& v, unsigned long long key,
-                                          AllocSmem& sm) {
+__device__ __forceinline__ void insert_block_inline(const VolumeDev& v, unsigned long long key,
+                                                    AllocSmem& sm) {
   const int r = bucket_insert(v.entries, v.t, key, sm.stamp, &sm.unique);
   if (r >= 0) {
     const int ptr = atomicAdd(&v.cnt->nalloc, 1);
@@ -126,6 +126,11 @@ __device__ __noinline__ void insert_block(const VolumeDev& v, unsigned long long
   } else if (r == -2) {
     atomicAdd(&sm.bucket_full, 1);
   }
+}
+
+__device__ __noinline__ void insert_block(const VolumeDev& v, unsigned long long key,
+                                          AllocSmem& sm) {
+  insert_block_inline(v, key, sm);
 }
 
 // A pixel's whole ray without the set (anywhere; blocks that other rays enter
@@ -157,11 +162,13 @@ __device__ __noinline__ void walk_far(const SessDev& S, int x, int y, AllocSmem&
   }
 }
 
-// One block of a ray into the CTA's set.  Neighbouring rays visit the same
-// blocks: most visits find their key with a plain read; of a run of lanes that
-// miss the same key together the first enters it (their compare-and-swaps would
-// queue at the slot: half of this kernel's shared memory cycles).
-template <class K>
+// One block of a ray into the CTA's set.  Most visits find their key with a plain
+// read.  CLOSE (close_rays): of a run of lanes that miss the same key together the first
+// enters it (their compare-and-swaps would queue at the slot: half of the shared
+// memory cycles there), and the entered slots are listed.  Else nearly every lane
+// misses another key, the set fills up, and holding the lanes together for each
+// other is what costs; the set is then scanned as a whole.
+template <class K, bool CLOSE>
 __device__ inline void visit_block(K key, const VolumeDev& v, AllocSmem& sm) {
   K* const set = reinterpret_cast<K*>(sm.set);
   constexpr K none = ~(K)0;
@@ -169,27 +176,36 @@ __device__ inline void visit_block(K key, const VolumeDev& v, AllocSmem& sm) {
   for (int p = 0; p < kSetProbes; ++p) {
     K old = *(volatile K*)&set[slot];
     if (old == none) {
-      const unsigned here = __activemask(), lane = threadIdx.x & 31;
-      const K left = __shfl_up_sync(here, key, 1);
-      const bool follows = lane > 0 && (here >> (lane - 1) & 1u) && left == key;
-      if (!follows) {
-        old = atomicCAS(&set[slot], none, key);
-        if (old == none) {
-          sm.list[atomicAdd(&sm.nkeys, 1)] = (unsigned short)slot;
-          old = key;
+      if (CLOSE) {
+        const unsigned here = __activemask(), lane = threadIdx.x & 31;
+        const K left = __shfl_up_sync(here, key, 1);
+        const bool follows = lane > 0 && (here >> (lane - 1) & 1u) && left == key;
+        if (!follows) {
+          old = atomicCAS(&set[slot], none, key);
+          if (old == none) {
+            sm.list[atomicAdd(&sm.nkeys, 1)] = (unsigned short)slot;
+            old = key;
+          }
         }
+        __syncwarp(here);
+        if (follows) old = *(volatile K*)&set[slot];
+      } else {
+        old = atomicCAS(&set[slot], none, key);
+        if (old == none) old = key;
       }
-      __syncwarp(here);
-      if (follows) old = *(volatile K*)&set[slot];
     }
     if (old == key) return;
     slot = (slot + 1) & (kSetSlots - 1);
   }
-  insert_block(v, volume_key(key, sm.cam), sm);  // set saturated
+  // set saturated
+  if (CLOSE)
+    insert_block(v, volume_key(key, sm.cam), sm);
+  else
+    insert_block_inline(v, volume_key(key, sm.cam), sm);
 }
 
 // The rays of one pixel tile (tx, ty) of AllocateFromDepthKernel.
-template <class K>
+template <class K, bool CLOSE>
 __device__ inline void walk_rays(const SessDev& S, int tx, int ty, AllocSmem& sm) {
   constexpr int B = NearKey<K>::kBits;
   const VolumeDev& v = S.vol;
@@ -217,10 +233,10 @@ __device__ inline void walk_rays(const SessDev& S, int tx, int ty, AllocSmem& sm
   }
   const K ix = (K)(long long)w.sx << (2 * B), iy = (K)(long long)w.sy << B, iz = (K)(long long)w.sz;
   K key = near_key<K>(ox, oy, oz);
-  visit_block<K>(key, v, sm);
+  visit_block<K, CLOSE>(key, v, sm);
   if (w.nx | w.ny | w.nz) {
     key = near_key<K>(ox + w.nx, oy + w.ny, oz + w.nz);
-    visit_block<K>(key, v, sm);
+    visit_block<K, CLOSE>(key, v, sm);
   }
   while (key != last) {
     if (left-- <= 0) {
@@ -233,11 +249,11 @@ __device__ inline void walk_rays(const SessDev& S, int tx, int ty, AllocSmem& sm
     if (gx) w.mx += w.dtx;
     else if (gy) w.my += w.dty;
     else w.mz += w.dtz;
-    visit_block<K>(key, v, sm);
+    visit_block<K, CLOSE>(key, v, sm);
   }
 }
 
-template <class K>
+template <class K, bool CLOSE>
 __device__ inline void allocate_tile(const SessDev& S, int tx, int ty, AllocSmem& sm) {
   K* const set = reinterpret_cast<K*>(sm.set);
   const VolumeDev& v = S.vol;
@@ -256,11 +272,13 @@ __device__ inline void allocate_tile(const SessDev& S, int tx, int ty, AllocSmem
     sm.stamp = S.pose->frame;
   }
   __syncthreads();
-  walk_rays<K>(S, tx, ty, sm);
+  walk_rays<K, CLOSE>(S, tx, ty, sm);
   __syncthreads();
   // drain the set into the global table
-  for (int k = tid; k < sm.nkeys; k += kAllocN) {
-    const int slot = sm.list[k];
+  const int listed = CLOSE ? sm.nkeys : kSetSlots;
+  for (int k = tid; k < listed; k += kAllocN) {
+    const int slot = CLOSE ? sm.list[k] : k;
+    if (!CLOSE && set[slot] == ~(K)0) continue;
     const int r = bucket_insert(v.entries, t, volume_key(set[slot], sm.cam), sm.stamp, &sm.unique);
     if (r >= 0) {
       set[slot] = (K)(unsigned)r;
@@ -293,23 +311,26 @@ __device__ inline void allocate_tile(const SessDev& S, int tx, int ty, AllocSmem
   }
 }
 
-// 8 CTAs per SM -- at most 32 registers, 25.5 KB of shared memory each -- so
-// that a 640x480 frame's 1,200 tiles run in about one wave instead of 1.35.
-// Bound by the walks (a frame without the drain: 63 of 69 us): about 30
-// instructions a step, and a wait at each block that the tile meets for the
-// first time.  Smaller tiles meet more of them (16x8 98 us, 8x8 134), sets twice
-// as large, two to four steps looked up together or warps held together at each
-// step are no faster (70 to 118).  640x480, 5 mm voxels: 92 us with 64-bit keys
-// packed at each step and a compare-and-swap by every lane, now 69; a frame of
-// ten 640x480 streams 3664 us before this work, 2733 before this, now 2306.
+// One kernel per form (sessions of the other form return).  Bound by the walks: a
+// 640x480 frame at 5 mm without the drain takes 63 of 69 us, about 30 instructions
+// a step and a wait at each block that the tile meets for the first time.  Smaller
+// tiles meet more of them (16x8 98 us, 8x8 134), sets twice as large, two to four
+// steps looked up together or warps held together at each step are no faster (70
+// to 118).  CLOSE: 5 CTAs per SM, 48 registers and nothing spilled in the walk: 63
+// us, with 8 CTAs and 32 registers 73, with 64-bit keys packed at each step and a
+// compare-and-swap by every lane 85.  Otherwise 8 CTAs (32 registers): rays that
+// share no blocks wait on more of them, 640x480 at 4 mm and 8 m 819 us, with 6
+// CTAs 942.
 // The tiles' rows of CTAs are followed by rows that empty the raycast's grid at
 // the frame's pose (memory-bound work beside the rays' latency-bound one).
-__global__ void __launch_bounds__(kAllocN, 8)
+template <bool CLOSE>
+__global__ void __launch_bounds__(kAllocN, CLOSE ? 5 : 8)
     fused_allocate_kernel(const SessDev* __restrict__ tab, int tile_rows) {
   __shared__ SessDev S;
   stage_session(tab + blockIdx.z, &S);
   __syncthreads();
   const DSensor& s = S.ls[0];
+  if (close_rays(S.vol.t, s) != CLOSE) return;
   if ((int)blockIdx.y >= tile_rows) {
     if (S.vol.grid && S.mode == 1)
       grid_clear(S.vol, S.pose->posef, s,
@@ -319,13 +340,11 @@ __global__ void __launch_bounds__(kAllocN, 8)
     return;
   }
   if ((int)blockIdx.x * kAllocX >= s.cols || (int)blockIdx.y * kAllocY >= s.rows) return;
-  // 10 bits hold a ray of the cap's steps from the camera; a band ray's start as
-  // well, up to twice the sensor range away
   __shared__ AllocSmem sm;
-  if (S.vol.t.dda_cap <= (S.vol.t.band ? 300 : 509))
-    allocate_tile<unsigned>(S, blockIdx.x, blockIdx.y, sm);
+  if (CLOSE || narrow_keys(S.vol.t))
+    allocate_tile<unsigned, CLOSE>(S, blockIdx.x, blockIdx.y, sm);
   else
-    allocate_tile<unsigned long long>(S, blockIdx.x, blockIdx.y, sm);
+    allocate_tile<unsigned long long, CLOSE>(S, blockIdx.x, blockIdx.y, sm);
 }
 
 // ------------------------------------------------------------ visibility
@@ -1976,7 +1995,9 @@ void fused_allocate(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   const int tx = nblk(b.max_cols, kAllocX), ty = nblk(b.max_rows, kAllocY);
   // about two CTAs per SM for the grids (enough for their writes)
   const int extra = b.max_grid > 0 ? nblk(std::max(8, 148 * 2 / b.n), tx) : 0;
-  fused_allocate_kernel<<<dim3(tx, ty + extra, b.n), kAllocN, 0, st>>>(tab, ty);
+  const dim3 grid(tx, ty + extra, b.n);
+  if (b.close_mask & 1) fused_allocate_kernel<false><<<grid, kAllocN, 0, st>>>(tab, ty);
+  if (b.close_mask & 2) fused_allocate_kernel<true><<<grid, kAllocN, 0, st>>>(tab, ty);
 }
 
 // grid-stride over each session's heap; a wave of CTAs in all

@@ -74,6 +74,24 @@ inline long long grid_entries(const DSensor& s, const DTsdf& t) {
   return n <= kGridMax ? n : 0;
 }
 
+// Allocation's form of a session (walk_rays).  The tile-local keys' 10 bits an axis
+// hold a ray of the step cap from the camera; a band ray's start as well, up to
+// twice the sensor range away.
+inline __host__ __device__ bool narrow_keys(const DTsdf& t) {
+  return t.dda_cap <= (t.band ? 300 : 509);
+}
+// Whether neighbouring rays run through the same blocks: a block spans at least
+// four of them at the sensor range.  Allocation in us with CLOSE / without:
+// 640x480, 5 mm, 3 m and 5 m of range (7 and 4.2 rays) 63 / 108 and 78 / 141;
+// 1280x720, 4 mm, 5 m (6.7) 424 / 688; 320x240, 5 mm, 3 m (3.5) 72 / 66, 4 m (2.6)
+// 123 / 89; 160x120, 5 mm, 3 m (1.8) 274 / 151; 640x480, 4 mm, 8 m (2.1) 1505 / 819.
+// Rays of more steps than the narrow keys hold fill the set either way: 1280x720,
+// 2 mm, 3 m (5.6) 491 / 406, 3 mm, 6 m (4.2) 1376 / 1081, 4 mm, 8 m (4.2) 813 / 824.
+// A band ray's few blocks do not: 160x120, 5 mm, 3 m 14 / 20, and the sessions of
+// a batch stay in one launch.
+inline __host__ __device__ bool close_rays(const DTsdf& t, const DSensor& s) {
+  return narrow_keys(t) && (t.band || t.bsm * (s.fx < s.fy ? s.fx : s.fy) >= 4.0f * t.dmax);
+}
 
 void launch_volume_clear(const VolumeDev& v, cudaStream_t st);
 // GenerateDepthKernel / GenerateRgbKernel (tsdf.cu:471-526).  pose_override
