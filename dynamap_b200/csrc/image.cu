@@ -315,13 +315,13 @@ __device__ inline float4 normal_at(const float* d, int pitch, const LevelCamera&
   return make_float4(n.x, n.y, n.z, 0.0f);
 }
 
-// one level, a 128x2 tile of pixels per CTA (the stage entry points: little
-// more than a launch, 6.1 us at 640x480 as without the tiles)
-constexpr int kMapTX = 128, kMapTY = 2;
-__global__ void __launch_bounds__(kMapTX * kMapTY)
+// one level, a tile of 256 pixels per CTA (launch_maps; the stage entry points:
+// little more than a launch, 6.1 us at 640x480 as without the tiles)
+constexpr int kMapThreads = 256;
+__global__ void __launch_bounds__(kMapThreads)
     maps_kernel(const float* __restrict__ depth, float4* __restrict__ normal,
                 float4* __restrict__ vertex, const LevelCamera c) {
-  const int x = blockIdx.x * kMapTX + threadIdx.x, y = blockIdx.y * kMapTY + threadIdx.y;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= c.s.cols || y >= c.s.rows) return;
   const int i = y * c.s.cols + x;
   if (vertex) {
@@ -707,9 +707,14 @@ void launch_bilateral(const float* src, float* dst, int rows, int cols, const Bi
                      bilateral_smem(tb.radius, ty), st>>>(src, dst, rows, cols, tb);
 }
 
+// Tiles as wide as leave at most a quarter of the threads' columns outside the
+// image: 128x2 (a row's vectors in one piece), 32x8 or 8x32.
 void launch_maps(const float* depth, const DSensor& s, float4* normal, float4* vertex,
                  cudaStream_t st) {
-  maps_kernel<<<dim3(nblk(s.cols, kMapTX), nblk(s.rows, kMapTY)), dim3(kMapTX, kMapTY), 0, st>>>(
+  int tx = 128;
+  while (tx > 8 && 4 * (nblk(s.cols, tx) * tx - s.cols) > s.cols) tx /= 4;
+  const int ty = kMapThreads / tx;
+  maps_kernel<<<dim3(nblk(s.cols, tx), nblk(s.rows, ty)), dim3(tx, ty), 0, st>>>(
       depth, normal, vertex, level_camera(s));
 }
 void launch_miss_to_zero(const float* ray_depth, float* depth0, float dmax, int n,
