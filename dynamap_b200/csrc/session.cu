@@ -589,7 +589,7 @@ size_t session_bytes(const dyn_tsdf_params& t, const dyn_sensor& s, int precisio
     const int tx = ((int)s.cols + 7) / 8, ty = ((int)s.rows + 7) / 8;
     b += 4 * (size_t)(ray_bounds_words(tx, ty) + free_tile_words(tx, ty)) + 512;
   }
-  b += 2 * n * (4 + 16 + 16 + 4) * 4 / 3;  // source + target pyramids
+  b += n * (2 * (4 + 16 + 4) + 16) * 4 / 3;  // source + target pyramids, vertices on demand
   b += icp_frame_scratch_bytes() + sizeof(SessDev) + sizeof(BilateralTable) + sizeof(ResultBlock) +
        8192;
   return b;
@@ -673,7 +673,6 @@ dyn_status alloc_device_buffers(dyn_session* s) {
     DYN_TRY(s->dalloc(&s->d_sint[l], m4 * 4));
     DYN_TRY(s->dalloc(&s->d_tdep[l], m4 * 4));
     DYN_TRY(s->dalloc(&s->d_tnrm[l], m * 16));
-    DYN_TRY(s->dalloc(&s->d_tvtx[l], m * 16));
     DYN_TRY(s->dalloc(&s->d_tint[l], m4 * 4));
   }
   DYN_TRY(s->dalloc(&s->d_pose_override, 64));
@@ -1200,7 +1199,7 @@ dyn_status dyn_debug_image(dyn_session* s, int32_t which, int32_t level, void* h
     case 3: src = s->d_svtx[level]; nb = m * 16; break;
     case 4: src = s->d_snrm[level]; nb = m * 16; break;
     case 5: src = s->d_tdep[level]; nb = m * 4; break;
-    case 6: src = s->d_tvtx[level]; nb = m * 16; break;
+    case 6: src = s->d_svtx[level]; nb = m * 16; break;
     case 7: src = s->d_tnrm[level]; nb = m * 16; break;
     case 8: src = s->d_trgb; nb = s->npx * 3; break;
     case 9: src = s->d_sint[level]; nb = m * 4; break;
@@ -1211,7 +1210,7 @@ dyn_status dyn_debug_image(dyn_session* s, int32_t which, int32_t level, void* h
   if (which == 3 || which == 6) {  // vertex maps are not kept: made now
     const bool t = which == 6;
     launch_maps(t ? s->d_tdep[level] : s->d_sdep[level], s->ls[level],
-                t ? s->d_tnrm[level] : s->d_snrm[level], t ? s->d_tvtx[level] : s->d_svtx[level],
+                t ? s->d_tnrm[level] : s->d_snrm[level], s->d_svtx[level],
                 s->stream);
   }
   DYN_CUDA(cudaMemcpyAsync(host_out, src, nb, cudaMemcpyDeviceToHost, s->stream));

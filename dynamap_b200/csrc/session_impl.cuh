@@ -127,11 +127,10 @@ struct dyn_session {
   float* d_filt = nullptr;
   float* d_sdep[kLevels] = {};
   float4* d_snrm[kLevels] = {};
-  float4* d_svtx[kLevels] = {};
+  float4* d_svtx[kLevels] = {};  // vertex maps of either pyramid, made when asked for
   float* d_sint[kLevels] = {};
   float* d_tdep[kLevels] = {};
   float4* d_tnrm[kLevels] = {};
-  float4* d_tvtx[kLevels] = {};
   float* d_tint[kLevels] = {};
   float* d_ray = nullptr;
   uint8_t* d_trgb = nullptr;

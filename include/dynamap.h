@@ -172,7 +172,8 @@ dyn_status dyn_default_params(dyn_tsdf_params* tsdf, dyn_gn_params* gn,
 dyn_status dyn_load_yaml(const char* path, dyn_tsdf_params* tsdf,
                          dyn_gn_params* gn, dyn_bilateral_params* bil,
                          dyn_sensor* sensor);
-/* Bytes of device memory a session with these parameters holds. */
+/* Bytes of device memory a session with these parameters holds (the raycast's
+ * block grid, up to 64 MB, among them). */
 dyn_status dyn_session_bytes(const dyn_tsdf_params* tsdf,
                              const dyn_sensor* sensor, int32_t precision,
                              size_t* bytes_out);
