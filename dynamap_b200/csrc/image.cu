@@ -695,7 +695,6 @@ static size_t bilateral_smem(int radius, int rows) {
 }
 // Rows of a CTA's tile: 8 stage less halo per pixel, 4 balance small images
 // over the SMs (453x340: 20.2 us with 4, 23.4 with 8; 640x480: 35.1 and 32.6).
-constexpr int kPairCtas = 4 * 148;
 static int bilateral_rows(long long cols, long long rows, int n) {
   return (cols + BTX - 1) / BTX * ((rows + 7) / 8) * n >= 6 * 148 ? 8 : 4;
 }
@@ -731,14 +730,14 @@ void fused_ingest(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
 void fused_bilateral(const SessDev* tab, const BatchShape& b, cudaStream_t st) {
   if (b.max_bil_radius <= 0) return;
   const int ty = bilateral_rows(b.max_cols, b.max_rows, b.n);
-  // Two pixels a thread for tables of mixed sessions alone that still fill the
-  // SMs with half the CTAs (600 of them for one 640x480 frame: 28.3 -> 26.7 us;
-  // 1280x720 51.7 -> 47.4; 32 frames of 320x240 in four groups 213 -> 177, where
-  // their exponentials alone take 140).  An FP32 session's tile has no use for
-  // it, so a table with one keeps the rows of its own.
+  // Two pixels a thread for tables of mixed sessions alone of that size (one frame,
+  // with / without: 560x420 24.5 / 26.1 us, 592x444 26.4 / 27.9, 640x480 26.7 /
+  // 28.6, 720x540 32.7 / 30.4, 1280x720 47.2 / 52.3; a batch of 32, 8 of 160x120, 16
+  // of 320x240 and 8 of 640x480, 177 / 213, where the exponentials take 211 were
+  // every pixel valid).  An FP32 session's tile has no use for it, so a table with
+  // one keeps the rows of its own.
   const dim3 threads(BTX, ty);
-  if (ty == 8 && b.fp16_mask == 2 &&
-      (long long)nblk(b.max_cols, BTX) * nblk(b.max_rows, 16) * b.n >= kPairCtas) {
+  if (ty == 8 && b.fp16_mask == 2) {
     fused_bilateral_kernel<2><<<dim3(nblk(b.max_cols, BTX), nblk(b.max_rows, 2 * ty), b.n), threads,
                                 bilateral_smem(b.max_bil_radius, 2 * ty), st>>>(tab);
     return;

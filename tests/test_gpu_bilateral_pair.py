@@ -38,3 +38,9 @@ def test_pair_and_single_agree(gpu_lib, rows, cols, diameter, holes):
         np.testing.assert_array_equal(a.view(np.uint32), r.view(np.uint32))
         assert np.count_nonzero(a) == np.count_nonzero(depth)
         batch.close()
+
+
+@pytest.mark.parametrize("rows,cols", [(420, 560), (425, 575)])
+def test_pair_from_the_smallest_size(gpu_lib, rows, cols):
+    """The smallest images with two pixels a thread (tiles of eight rows)."""
+    test_pair_and_single_agree(gpu_lib, rows, cols, 8, True)
