@@ -29,13 +29,13 @@ struct DSensor {
 // A level's intrinsics with the reciprocals of its focal lengths (fl(1/f) and
 // the rest, for div_by).
 constexpr float kModerateMin = 9.5367431640625e-7f, kModerateMax = 1048576.0f;  // 2^-20, 2^20
+__host__ __device__ inline bool moderate(float x) { return x >= kModerateMin && x <= kModerateMax; }
 struct LevelCamera {
   DSensor s;
   float yhx, ylx, yhy, yly;
   int ok;  // the quotients of depths in kModerateMin .. Max stay in div_by's range
 };
 inline LevelCamera level_camera(const DSensor& s) {
-  const auto moderate = [](float x) { return x >= kModerateMin && x <= kModerateMax; };
   LevelCamera c;
   c.s = s;
   c.yhx = 1.0f / s.fx;

@@ -5,17 +5,17 @@
 // gnSolver::solve (:317-438).  The reference adds 42 FP32 atomics per
 // correspondence into one 6x6 system and round-trips to the host (Eigen LDLT)
 // every iteration.  Here each thread accumulates its pixels' 21 upper-
-// triangle JtJ terms, 6 Jtr terms, r^2 and a count in registers (FP64 sums
-// of the FP32 terms; compensated FP32 sums in the mixed form), the block
-// reduces them with warp shuffles into a partial per pixel tile, and the
-// tiles' partials are summed in FP64 in tile order -- a fixed reduction
-// order, so results are run-to-run deterministic and do not depend on the
-// grid -- before the GN update (scale by 1/max(A), damping, 6x6 LDL^T,
-// convergence test) and the SE(3) exponential for the next iteration, in
-// FP64, with no host round trip.  Per frame this runs either as one chained
-// launch per iteration (the last block to finish a level's tiles updates
-// the solver) or as one persistent cooperative launch for all levels and
-// iterations (below); both give the same bits.
+// triangle JtJ terms, 6 Jtr terms, r^2 and a count in registers (FP64 sums of
+// the FP32 terms; in the mixed form FP32 sums of a few pixels, from there on
+// compensated FP32 pairs), warps and blocks reduce them with shuffles into a
+// partial per pixel tile, and the tiles' partials are added in a fixed order:
+// rows w, w + 16, ... by warp w, then the 16 warps' sums (level_total).  So
+// results are run-to-run deterministic and do not depend on the grid.  The GN
+// update (scale by 1/max(A), damping, 6x6 LDL^T, convergence test) and the SE(3)
+// exponential for the next iteration follow in FP64, with no host round trip.
+// Per frame this runs either as one chained launch per iteration (the last block
+// to finish a level's tiles updates the solver) or as one persistent cooperative
+// launch for all levels and iterations (below); both give the same bits.
 #include "icp.cuh"
 
 #include <algorithm>

@@ -11,7 +11,6 @@
 
 #include <cmath>
 #include <cstdlib>
-#include <cstring>
 
 #include "dyn_exp.h"
 #include "sessdev.cuh"
@@ -27,7 +26,6 @@ __device__ inline float intensity_u8(const uint8_t* c) {
   return (float)(0.2126 * (double)r + 0.7152 * (double)g + 0.0722 * (double)b);
 }
 
-// u16 sensor units -> metres (builder.cu:111, utils_Dataset.cpp:233-235)
 // pyramid::applyBilateralFilter, pyramid.cu:213-233, window rows x-r..x+r-1,
 // cols y-r..y+r-1, summed row-major.  The depth tile plus halo is staged in
 // shared memory (0 where outside the image or not > 0: such taps are skipped,
@@ -271,8 +269,7 @@ __device__ inline float mean_valid(float a, float b, float c, float d) {
   // s / n: a half and a quarter are exact as products, a third by its reciprocal
   if (n == 3) {
     const float yh = 1.0f / 3.0f;
-    return s >= kModerateMin && s <= kModerateMax ? div_by(s, 3.0f, yh, fmaf(-3.0f, yh, 1.0f) * yh)
-                                                  : s / 3.0f;
+    return moderate(s) ? div_by(s, 3.0f, yh, fmaf(-3.0f, yh, 1.0f) * yh) : s / 3.0f;
   }
   return s * (n == 4 ? 0.25f : (n == 2 ? 0.5f : 1.0f));
 }
@@ -290,7 +287,6 @@ __device__ inline float mean4(float a, float b, float c, float d) {
 // correction (div_by) where no step can leave the normal range, else through
 // IEEE division.
 // (LevelCamera::ok: an offset u - cx is 0 or at least 2^-24 then.)
-__device__ inline bool moderate(float x) { return x >= kModerateMin && x <= kModerateMax; }
 __device__ inline F3 camera_point(const LevelCamera& c, int u, int v, float d, bool fast) {
   if (!fast) return point3d_uv(u, v, d, c.s);
   const float a = ((float)u - c.s.cx) * d, b = ((float)v - c.s.cy) * d;
@@ -346,7 +342,8 @@ __global__ void miss_to_zero_kernel(const float* __restrict__ ray, float* __rest
 }
 
 // ---------------------------------------------------------------- fused
-// ingest (+ the unfiltered copy when the bilateral filter is off), and what
+// ingest: u16 sensor units -> metres (builder.cu:111, utils_Dataset.cpp:233-235;
+// + the unfiltered copy when the bilateral filter is off), and what
 // integration reads per voxel that projects to a pixel: the distance from the
 // camera centre to the pixel's back-projected point (IntegrateScanKernel's
 // |getPoint3d(pixel, depth)|, tsdf.cu:316-317 -- it depends only on the pixel,
@@ -478,8 +475,8 @@ __global__ void fused_bilateral_kernel(const SessDev* __restrict__ tab) {
 // small, because the chain of a CTA (loads, three levels, normals) is what a
 // frame waits for; six CTAs an SM hide each other's.  With a launch per level
 // and one for the normals (four or five per image) a 640x480 frame took 16.4 us
-// for the source and 20.6 for the target, now 12.3 and 15; 32 frames of 320x240
-// in four groups 80 and 110 us, now 62 and 67.  A fourth level (scale 8) is
+// for the source and 20.6 for the target, now 12.3 and 15; a batch of 32 (8 of
+// 160x120, 16 of 320x240, 8 of 640x480) 80 and 110 us, now 62 and 67.  A fourth level (scale 8) is
 // made from level 2 by the two kernels below.
 //
 // what: 0 the frame's source (filtered depth and intensity are there); 1 the

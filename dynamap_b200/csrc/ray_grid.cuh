@@ -88,9 +88,7 @@ struct MarchRay {
   float yhx, ylx, yhy, yly;  // reciprocals of fx and fy
 };
 
-__device__ inline bool recip_ok(float x) {
-  return fabsf(x) >= kModerateMin && fabsf(x) <= kModerateMax;
-}
+__device__ inline bool recip_ok(float x) { return moderate(fabsf(x)); }
 
 // Whether the samples of pixel offset (px, py) (per unit depth) from pose T, up
 // to dmax, stay within 131072 voxels of the origin on every axis: the range of

@@ -1579,20 +1579,15 @@ __device__ inline bool raycast_exact_px(const VolumeDev& v, const DSensor& s, co
 // frames on the parity sequences, through the solver's discrete
 // convergence test (an extra or a missing iteration moves a pose by up to
 // the 1e-3 increment threshold).
-template <bool FP16>
-struct Vox;
-template <>
-struct Vox<true> {
-  using raw_t = unsigned;
-  static __device__ raw_t load(const VolumeDev& v, int ptr, int lin) {
+struct MixedVox {
+  static __device__ unsigned load(const VolumeDev& v, int ptr, int lin) {
     return ptr < 0 ? 0u : __ldg(v.vox16 + (size_t)ptr * kBlockVox + lin);
   }
-  static __device__ int w(raw_t r) { return (int)(r >> 16); }
-  static __device__ float val(raw_t r) {
+  static __device__ int w(unsigned r) { return (int)(r >> 16); }
+  static __device__ float val(unsigned r) {
     return __half2float(__ushort_as_half((unsigned short)(r & 0xffffu)));
   }
-  static __device__ float unit(const DTsdf& t) { return t.trunc; }
-  static __device__ uchar4 color(const VolumeDev& v, raw_t, int ptr, int lin) {
+  static __device__ uchar4 color(const VolumeDev& v, int ptr, int lin) {
     return (v.colors && ptr >= 0) ? v.colors[(size_t)ptr * kBlockVox + lin]
                                   : make_uchar4(0, 0, 0, 0);
   }
@@ -1601,10 +1596,10 @@ struct Vox<true> {
 // The interpolated sample at q (voxel units) whose centre voxel raw0 (heap
 // index ptr0, local index lin0) is observed.  Sums by fused multiply-adds
 // in the reference's corner order.
-template <bool FP16, bool COLOR>
-__device__ inline VoxelSample interp(const VolumeDev& v, F3 q, typename Vox<FP16>::raw_t raw0,
-                                     int ptr0, int lin0, BlockCache& bc) {
-  using V = Vox<FP16>;
+template <bool COLOR>
+__device__ inline VoxelSample interp(const VolumeDev& v, F3 q, unsigned raw0, int ptr0, int lin0,
+                                     BlockCache& bc) {
+  using V = MixedVox;
   VoxelSample out;
   const float fx = floorf(q.x), fy = floorf(q.y), fz = floorf(q.z);
   const float wx = q.x - fx, wy = q.y - fy, wz = q.z - fz;
@@ -1617,7 +1612,7 @@ __device__ inline VoxelSample interp(const VolumeDev& v, F3 q, typename Vox<FP16
   // into the next block where the cell crosses)
   const int base = (lx << 6) | (ly << 3) | lz;
   const int dx = cx ? -448 : 64, dy = cy ? -56 : 8, dz = cz ? -7 : 1;
-  const uchar4 c0 = COLOR ? V::color(v, raw0, ptr0, lin0) : make_uchar4(0, 0, 0, 0);
+  const uchar4 c0 = COLOR ? V::color(v, ptr0, lin0) : make_uchar4(0, 0, 0, 0);
   const float n0 = V::val(raw0);
   const float ax[2] = {1.0f - wx, wx}, ay[2] = {1.0f - wy, wy}, az[2] = {1.0f - wz, wz};
   float dist = 0.0f, cr = 0.0f, cg = 0.0f, cbl = 0.0f;
@@ -1628,18 +1623,18 @@ __device__ inline VoxelSample interp(const VolumeDev& v, F3 q, typename Vox<FP16
     const int ox = off[k][0], oy = off[k][1], oz = off[k][2];
     const int ptr = corner_block(cb, cx, cy, cz, ox, oy, oz);
     const int lin = base + (ox ? dx : 0) + (oy ? dy : 0) + (oz ? dz : 0);
-    const typename V::raw_t r = V::load(v, ptr, lin);
+    const unsigned r = V::load(v, ptr, lin);
     const bool use0 = V::w(r) == 0;
     const float coef = (ax[ox] * ay[oy]) * az[oz];
     dist = __fmaf_rn(coef, use0 ? n0 : V::val(r), dist);
     if (COLOR) {
-      const uchar4 cc = use0 ? c0 : V::color(v, r, ptr, lin);
+      const uchar4 cc = use0 ? c0 : V::color(v, ptr, lin);
       cr = __fmaf_rn((float)cc.x, coef, cr);
       cg = __fmaf_rn((float)cc.y, coef, cg);
       cbl = __fmaf_rn((float)cc.z, coef, cbl);
     }
   }
-  out.sdf = dist * V::unit(v.t);
+  out.sdf = dist * v.t.trunc;
   out.w = V::w(raw0);
   out.r = cr;
   out.g = cg;
@@ -1650,7 +1645,7 @@ __device__ inline VoxelSample interp(const VolumeDev& v, F3 q, typename Vox<FP16
 // The interpolated colour at depth 'cur' of the ray q = o + cur * d (voxel
 // units); of an unobserved voxel its own.
 __device__ __noinline__ uchar4 mixed_colour(const VolumeDev& v, F3 o, F3 d, float cur) {
-  using V = Vox<true>;
+  using V = MixedVox;
   const F3 q = f3(__fmaf_rn(cur, d.x, o.x), __fmaf_rn(cur, d.y, o.y), __fmaf_rn(cur, d.z, o.z));
   const int gx = (int)floorf(q.x + 0.5f), gy = (int)floorf(q.y + 0.5f),
             gz = (int)floorf(q.z + 0.5f);
@@ -1659,9 +1654,9 @@ __device__ __noinline__ uchar4 mixed_colour(const VolumeDev& v, F3 o, F3 d, floa
   bc.ptr = -1;
   const int ptr = block_ptr(v, blk_of(gx), blk_of(gy), blk_of(gz), bc);
   const int lin = lin_of(gx, gy, gz);
-  const typename V::raw_t raw = V::load(v, ptr, lin);
-  if (V::w(raw) == 0) return V::color(v, raw, ptr, lin);
-  const VoxelSample vx = interp<true, true>(v, q, raw, ptr, lin, bc);
+  const unsigned raw = V::load(v, ptr, lin);
+  if (V::w(raw) == 0) return V::color(v, ptr, lin);
+  const VoxelSample vx = interp<true>(v, q, raw, ptr, lin, bc);
   return make_uchar4((uint8_t)vx.r, (uint8_t)vx.g, (uint8_t)vx.b, 0);
 }
 
@@ -1690,7 +1685,7 @@ __device__ inline bool mixed_hash_march(const VolumeDev& v, const DSensor& s, co
                                         int y, float skip_to, float skip_far,
                                         float* __restrict__ depth_out,
                                         uint8_t* __restrict__ rgb_out) {
-  using V = Vox<true>;
+  using V = MixedVox;
   const int i = y * s.cols + x;
   const DTsdf& t = v.t;
   const float inv_vs = 1.0f / t.vs;
@@ -1735,12 +1730,12 @@ __device__ inline bool mixed_hash_march(const VolumeDev& v, const DSensor& s, co
                         ? bc.ptr
                         : block_ptr(v, blk_of(gx), blk_of(gy), blk_of(gz), bc0);
     const int lin = lin_of(gx, gy, gz);
-    const typename V::raw_t raw = V::load(v, ptr, lin);
+    const unsigned raw = V::load(v, ptr, lin);
     if (V::w(raw) == 0) {
       cur += t.trunc;
       continue;
     }
-    const VoxelSample vx = interp<true, false>(v, q, raw, ptr, lin, bc);
+    const VoxelSample vx = interp<false>(v, q, raw, ptr, lin, bc);
     cur += vx.sdf;
     if (vx.sdf < t.vs) break;
   }
