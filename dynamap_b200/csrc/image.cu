@@ -50,10 +50,12 @@ __device__ inline float intensity_u8(const uint8_t* c) {
 //  * MASK false: where no staged pixel is invalid, no test per tap;
 //  * the taps of a window row unroll (DT the window size, 0: any), so that
 //    their weights overlap; only the two sums are serial.
-// A call at diameter 8, before -> now: 160x120 43.3 -> 12.4 us (the kernel 8),
-// 320x240 45 -> 14, 640x480 80 -> 33, 1280x720 146 -> 71.  Two pixels of a
-// column per thread, each staged depth read once for both, measured 16, 37 and
-// 72 us: the shared-memory reads are not what it waits for.  (They are in the
+// A call at diameter 8, before -> now: 160x120 43.1 -> 10.3 us, 320x240 45.1 ->
+// 15.3, 640x480 78.3 -> 32.9, 1280x720 145 -> 70.7.  Other diameters keep a loop of
+// unknown length with the test per tap: 640x480 at 4, 6, 7 and 16 24.8, 47.6, 61.4
+// and 278 us before, now 14.4, 25.7, 33.8 and 139.  Two pixels of a column per
+// thread, each staged depth read once for both, measured 16, 37 and 72 us from
+// 320x240 on: the shared-memory reads are not what it waits for.  (They are in the
 // mixed form, whose taps are six operations and an exponential: bilateral_pair.)
 constexpr int BTX = 32;
 

@@ -17,12 +17,12 @@ namespace {
 // (GridBox; z fastest): entry = first voxel of the block (512 x heap index),
 // or of the empty block after the heap.  A lookup is one multiply-add chain
 // and one load without branches, where the hash takes a bucket scan in a
-// divergent branch for every lane that changes block: with the exact march
-// below and hash lookups a 640x480 FP32 target took 257 M warp instructions at
-// 20 of 32 lanes (485 us, as before it); with the grid 138 M at 28 lanes
-// (260 us; 320x240 225 -> 98 us).  The mixed march, whose arithmetic did not
-// change: 640x480 136 -> 61 us, 1280x720 band 200 -> 100 us, and a 32-session
-// band batch 667 -> 351 us.
+// divergent branch for every lane that changes block.  A 640x480 FP32 target with
+// colours: 327 M warp instructions at 25 of 32 lanes and 485 us before, and no
+// faster with the exact march alone; with the grid 181 M at 28 lanes and 264 us
+// (320x240 225 -> 99).  The mixed march, whose arithmetic did not change: 640x480
+// 136 -> 62 us, 1280x720 band 200 -> 100 us, and a 32-session band batch 667 ->
+// 358 us.
 __device__ inline GridBox grid_box(const float* __restrict__ T, const DSensor& s, const DTsdf& t,
                                    int cap) {
   GridBox b;

@@ -687,9 +687,9 @@ __global__ void __launch_bounds__(kVisThreads) fused_surface_bound_kernel(const 
 //  * the merge's division by weight + 1: by the tabulated reciprocal with an
 //    exact correction (div_by), the colours' by a tabulated multiplier.
 // A 640x480 RGB frame (32,000 blocks): the CTA-per-block kernel before it took
-// 106 M warp instructions and waited on its barriers and on gathers of five
-// words per voxel (L1 at 76 %); this one takes 75 M and issues in 70 % of the
-// cycles (80 registers and 24 warps per SM: 57 %).  Live stage before -> now:
+// 123 M warp instructions and waited on its barriers and on gathers of five words
+// per voxel; this one takes 88 M and issues in 67 % of the cycles (with 80
+// registers and 24 warps per SM it was slower).  Live stage before -> now:
 // 640x480 RGB FP32 156 -> 112 us, mixed with its free-cell passes 195 -> 141,
 // 320x240 FP32 41 -> 36, 32-session band batch 357 -> 194; reading and writing
 // the blocks once would take 45 us of the first.
@@ -1894,7 +1894,7 @@ __global__ void __launch_bounds__(256)
 // hash (other sessions return), and per tile shape (every pixel's march is
 // independent of the tiling)
 // (at least 1024 threads resident per SM: the march waits on its own loads --
-// grid entry, voxel, corners -- and issues in 60 % of the cycles, and 4 CTAs of
+// grid entry, voxel, corners -- and issues in 67 % of the cycles, and 4 CTAs of
 // 256 hide more of it than the 3 that 76 registers allow.  A persistent launch
 // whose warps fetch 8x4 tiles from an even sample of the image balanced the
 // SMs but spilled in the loop: 272 against 253 us.  All nine loads of a sample
